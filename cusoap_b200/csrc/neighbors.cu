@@ -41,16 +41,16 @@ struct NLWork {
   int* bins_per_struct;      // (n_struct)
   int64_t* bin_off;          // (n_struct + 1)
   int* bin_count;            // (max_bins)
-  int64_t* bin_start;        // (max_bins + 1)
-  int* bin_cursor;           // (max_bins)
+  int* bin_start;            // (max_bins + 1)
+  int* arrival;              // (n_atoms) order in which the atoms reached their bins
   int* atom_bin;             // (n_atoms)
-  int* sorted_atom;          // (n_atoms)
+  int* sorted_atom;          // (n_atoms) atoms by bin, in arrival order inside a bin
   double4* sorted_pos;       // (n_atoms) {wrapped x, y, z, packed info} (see pack_info)
   double4* cpos;             // (n_centres) wrapped centre positions
   int4* cinfo;               // (n_centres) {bin xyz, struct, wrap, atom}
   int* counts;               // (n_centres)
   int64_t* partials;         // scan partials
-  int* status;               // error flags
+  int* status;               // {error flags, finished blocks of k_count, largest pair count of a centre, 0}
   int64_t max_bins;
 };
 
@@ -163,16 +163,18 @@ __device__ __forceinline__ int64_t block_incl_scan(int64_t v, int64_t* s_warp) {
   return v;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_blocks(const int* in, int64_t n, int64_t* out, int64_t* partials) {
+template <class Out>
+__global__ void __launch_bounds__(1024) k_scan_blocks(const int* in, int64_t n, Out* out, int64_t* partials) {
   __shared__ int64_t s_warp[32];
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t v = (i < n) ? in[i] : 0;
   const int64_t inc = block_incl_scan(v, s_warp);
-  if (i < n) out[i] = inc - v;
+  if (i < n) out[i] = (Out)(inc - v);
   if (threadIdx.x == blockDim.x - 1) partials[blockIdx.x] = inc;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_partials(int64_t* partials, int64_t nblk, int64_t* total_out) {
+template <class Out>
+__global__ void __launch_bounds__(1024) k_scan_partials(int64_t* partials, int64_t nblk, Out* total_out) {
   __shared__ int64_t s_warp[32];
   __shared__ int64_t s_carry;
   if (threadIdx.x == 0) s_carry = 0;
@@ -187,15 +189,17 @@ __global__ void __launch_bounds__(1024) k_scan_partials(int64_t* partials, int64
     if (threadIdx.x == blockDim.x - 1) s_carry = carry + inc;
     __syncthreads();
   }
-  if (threadIdx.x == 0) *total_out = s_carry;
+  if (threadIdx.x == 0) *total_out = (Out)s_carry;
 }
 
-__global__ void k_scan_add(int64_t* out, int64_t n, const int64_t* partials) {
+template <class Out>
+__global__ void k_scan_add(Out* out, int64_t n, const int64_t* partials) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += partials[i / 1024];
+  if (i < n) out[i] += (Out)partials[i / 1024];
 }
 
-static int exclusive_scan(const int* in, int64_t n, int64_t* out, int64_t* partials, cudaStream_t st) {
+template <class Out>
+static int exclusive_scan(const int* in, int64_t n, Out* out, int64_t* partials, cudaStream_t st) {
   const int64_t nblk = (n + 1023) / 1024;
   if (n > 0) {
     k_scan_blocks<<<(unsigned)nblk, 1024, 0, st>>>(in, n, out, partials);
@@ -205,13 +209,52 @@ static int exclusive_scan(const int* in, int64_t n, int64_t* out, int64_t* parti
   return check_launch("exclusive_scan", n > 0 ? 3 : 1);
 }
 
+// Exclusive scan of n ints by one block: every thread sums a contiguous chunk,
+// one block scan of the sums, then the chunk's offsets.  The inputs were
+// written by other blocks of the same launch: they are read from L2.  Returns
+// the total (every thread) and, in *largest, the largest input.
+template <class Out>
+__device__ __forceinline__ int64_t block_scan_chunks(const int* in, int64_t n, Out* out, int64_t* s_warp,
+                                                     int* s_max, int* largest) {
+  const int nth = blockDim.x;
+  const int64_t per = (n + nth - 1) / nth;
+  const int64_t i0 = min((int64_t)threadIdx.x * per, n), i1 = min(i0 + per, n);
+  int64_t sum = 0;
+  int mx = 0;
+#pragma unroll 8
+  for (int64_t i = i0; i < i1; ++i) {
+    const int v = __ldcg(in + i);
+    sum += v;
+    mx = max(mx, v);
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+  const int64_t inc = block_incl_scan(sum, s_warp);
+  int64_t run = inc - sum;
+#pragma unroll 8
+  for (int64_t i = i0; i < i1; ++i) {
+    const int v = __ldcg(in + i);
+    out[i] = (Out)run;
+    run += v;
+  }
+  __syncthreads();
+  if (largest) {
+    int m = 0;
+    for (int k = 0; k < (nth >> 5); ++k) m = max(m, s_max[k]);
+    *largest = m;
+  }
+  const int64_t total = s_warp[(nth >> 5) - 1];  // inclusive sum up to the last warp
+  if (threadIdx.x == 0) out[n] = (Out)total;
+  return total;
+}
+
 // ---------------------------------------------------------------------------
 // cell lists
 // ---------------------------------------------------------------------------
 
-__global__ void k_grid_init(soapb_structs s, NLWork w, double cutoff) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.n_struct) return;
+// Each stage below is a device function over (index, stride), so the separate
+// kernels of large inputs and the fused kernel of small ones (k_cells) share it.
+__device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& w, double cutoff, int i) {
   GridDesc g;
   int anyp = 0;
   for (int k = 0; k < 3; ++k) anyp |= s.d_pbc[i * 3 + k] ? 1 : 0;
@@ -260,13 +303,32 @@ __global__ void k_grid_init(soapb_structs s, NLWork w, double cutoff) {
   if (bad && anyp) atomicOr(w.status, 1);
 }
 
-// Fractional bounding box per structure.  Atoms of a structure are
-// contiguous, so a warp usually covers one structure: it reduces min / max
-// with shuffles and issues one atomic per bound instead of 32.
-__global__ void k_frac_bbox(soapb_structs s, NLWork w) {
+// Fractional bounding box of the open axes of every structure (warp-strided
+// over atoms base = first, first + stride, ...).  Atoms of a structure are
+// contiguous, so a warp keeps a running minimum and maximum while its atoms
+// belong to one structure and issues atomics only when the structure changes
+// or its atoms end.
+__device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& w, int64_t first, int64_t stride) {
   const int lane = threadIdx.x & 31;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < s.n_atoms; base += stride) {
+  int cur = -1;  // structure of the running bounds (warp-uniform)
+  double lo[3], hi[3];
+  auto flush = [&]() {
+    if (cur < 0) return;
+    for (int k = 0; k < 3; ++k) {
+      if (w.grids[cur].per[k]) continue;
+      double l = lo[k], h = hi[k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        l = fmin(l, __shfl_xor_sync(0xffffffffu, l, o));
+        h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
+      }
+      if (lane == 0) {
+        atomicMin(&w.fbox[cur * 6 + k], ord_encode(l));
+        atomicMax(&w.fbox[cur * 6 + 3 + k], ord_encode(h));
+      }
+    }
+  };
+  for (int64_t base = first; base < s.n_atoms; base += stride) {
     const int64_t a = base + lane;
     const bool valid = a < s.n_atoms;
     int si = 0;
@@ -277,20 +339,15 @@ __global__ void k_frac_bbox(soapb_structs s, NLWork w) {
     }
     const int si0 = __shfl_sync(0xffffffffu, si, 0);  // lane 0 is always valid here
     if (__all_sync(0xffffffffu, !valid || si == si0)) {
-      const GridDesc& g = w.grids[si0];
-      for (int k = 0; k < 3; ++k) {
-        if (g.per[k]) continue;
-        double lo = valid ? f[k] : INFINITY, hi = valid ? f[k] : -INFINITY;
+      if (si0 != cur) {
+        flush();
+        cur = si0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-          hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        }
-        if (lane == 0) {
-          atomicMin(&w.fbox[si0 * 6 + k], ord_encode(lo));
-          atomicMax(&w.fbox[si0 * 6 + 3 + k], ord_encode(hi));
-        }
+        for (int k = 0; k < 3; ++k) { lo[k] = INFINITY; hi[k] = -INFINITY; }
       }
+      if (valid)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { lo[k] = fmin(lo[k], f[k]); hi[k] = fmax(hi[k], f[k]); }
     } else if (valid) {
       const GridDesc& g = w.grids[si];
       for (int k = 0; k < 3; ++k) {
@@ -300,11 +357,10 @@ __global__ void k_frac_bbox(soapb_structs s, NLWork w) {
       }
     }
   }
+  flush();
 }
 
-__global__ void k_grid_setup(soapb_structs s, NLWork w, double cutoff) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.n_struct) return;
+__device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork& w, double cutoff, int i) {
   GridDesc g = w.grids[i];
   const double* H = g.H;
   const double det = fabs(H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
@@ -332,7 +388,7 @@ __global__ void k_grid_setup(soapb_structs s, NLWork w, double cutoff) {
       g.fmin[k] = 0.0;
       g.binw[k] = 1.0 / g.nb[k];
     } else {
-      double lo = ord_decode(w.fbox[i * 6 + k]), hi = ord_decode(w.fbox[i * 6 + 3 + k]);
+      double lo = ord_decode(__ldcg(&w.fbox[i * 6 + k])), hi = ord_decode(__ldcg(&w.fbox[i * 6 + 3 + k]));
       if (!(hi >= lo)) { lo = 0.0; hi = 0.0; }  // no atoms
       const double span = hi - lo;
       const int nb = (int)floor(span * perp[k] / bin_min);
@@ -363,100 +419,126 @@ __global__ void k_grid_setup(soapb_structs s, NLWork w, double cutoff) {
   w.bins_per_struct[i] = g.nb[0] * g.nb[1] * g.nb[2];
 }
 
-__global__ void k_bin_atoms(soapb_structs s, NLWork w) {
-  for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < s.n_atoms;
-       a += (int64_t)gridDim.x * blockDim.x) {
-    const int si = struct_of_atom(s.d_atom_off, s.n_struct, a);
-    const GridDesc& g = w.grids[si];
-    int b[3], wr[3];
-    double wp[3];
-    if (!locate(g, s.d_positions[3 * a], s.d_positions[3 * a + 1], s.d_positions[3 * a + 2], b, wr, wp))
-      atomicOr(w.status, 2);
-    const int64_t gb = w.bin_off[si] + ((int64_t)b[2] * g.nb[1] + b[1]) * g.nb[0] + b[0];
-    w.atom_bin[a] = (int)gb;
-    atomicAdd(&w.bin_count[gb], 1);
-  }
+__device__ __forceinline__ void bin_atom(const soapb_structs& s, const NLWork& w, int64_t a) {
+  const int si = struct_of_atom(s.d_atom_off, s.n_struct, a);
+  const GridDesc& g = w.grids[si];
+  int b[3], wr[3];
+  double wp[3];
+  if (!locate(g, s.d_positions[3 * a], s.d_positions[3 * a + 1], s.d_positions[3 * a + 2], b, wr, wp))
+    atomicOr(w.status, 2);
+  const int64_t gb = w.bin_off[si] + ((int64_t)b[2] * g.nb[1] + b[1]) * g.nb[0] + b[0];
+  w.atom_bin[a] = (int)gb;
+  w.arrival[a] = atomicAdd(&w.bin_count[gb], 1);
+}
+
+__device__ __forceinline__ void place_centre(const soapb_centres& c, const NLWork& w, int64_t i) {
+  const int si = c.d_struct[i];
+  const GridDesc& g = w.grids[si];
+  int b[3], wr[3];
+  double wp[3];
+  if (!locate(g, c.d_xyz[3 * i], c.d_xyz[3 * i + 1], c.d_xyz[3 * i + 2], b, wr, wp)) atomicOr(w.status, 2);
+  w.cpos[i] = make_double4(wp[0], wp[1], wp[2], 0.0);
+  w.cinfo[i] = make_int4(b[0] | (b[1] << 10) | (b[2] << 20), si, pack3(wr[0], wr[1], wr[2]), c.d_atom[i]);
+}
+
+// The atom of a slot goes to its final place in the bin, its rank by atom index
+// (the number of smaller indices in the bin), so the candidate order -- and the
+// FP32 accumulation order -- is deterministic.  Bins hold a few atoms: the
+// quadratic count is a few loads from L1, where sorting each bin by a warp took
+// a pass over all bins (1M atoms: 143 us for the sort kernel alone).
+__device__ __forceinline__ void gather_atom(const soapb_structs& s, const NLWork& w, int64_t slot) {
+  const int a = w.sorted_atom[slot];
+  const int gb = w.atom_bin[a];
+  const int s0 = w.bin_start[gb], s1 = w.bin_start[gb + 1];
+  int rank = 0;
+  for (int i = s0; i < s1; ++i) rank += w.sorted_atom[i] < a;
+  const int si = struct_of_atom(s.d_atom_off, s.n_struct, a);
+  const GridDesc& g = w.grids[si];
+  int b[3], wr[3];
+  double wp[3];
+  locate(g, s.d_positions[3 * (int64_t)a], s.d_positions[3 * (int64_t)a + 1], s.d_positions[3 * (int64_t)a + 2],
+         b, wr, wp);
+  w.sorted_pos[s0 + rank] =
+      make_double4(wp[0], wp[1], wp[2], pack_info(a, s.d_species[a], pack3(wr[0], wr[1], wr[2])));
+}
+
+// ---- large inputs: one kernel per stage ----
+
+__global__ void k_grid_init(soapb_structs s, NLWork w, double cutoff) {
+  const int64_t nth = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = t0; i < s.n_struct; i += nth) grid_init(s, w, cutoff, (int)i);
+  for (int64_t i = t0; i < w.max_bins; i += nth) w.bin_count[i] = 0;
+}
+
+__global__ void k_frac_bbox(soapb_structs s, NLWork w) {
+  frac_bbox(s, w, (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31), (int64_t)gridDim.x * blockDim.x);
+}
+
+__global__ void k_grid_setup(soapb_structs s, NLWork w, double cutoff) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < s.n_struct) grid_setup(s, w, cutoff, i);
+}
+
+__global__ void k_bin_atoms(soapb_structs s, soapb_centres c, NLWork w) {
+  const int64_t nth = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t a = t0; a < s.n_atoms; a += nth) bin_atom(s, w, a);
+  for (int64_t i = t0; i < c.n_centres; i += nth) place_centre(c, w, i);
 }
 
 __global__ void k_scatter_atoms(int64_t n_atoms, NLWork w) {
   for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n_atoms;
-       a += (int64_t)gridDim.x * blockDim.x) {
-    const int gb = w.atom_bin[a];
-    const int64_t slot = w.bin_start[gb] + atomicAdd(&w.bin_cursor[gb], 1);
-    w.sorted_atom[slot] = (int)a;
-  }
-}
-
-// Sort each bin's atoms by index (warp bitonic sort in shared memory), so
-// the candidate order -- and the FP32 accumulation order -- is deterministic.
-__global__ void __launch_bounds__(128) k_sort_bins(NLWork w) {
-  __shared__ int s_keys[4][1024];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int* keys = s_keys[wid];
-  const int64_t nwarps = (int64_t)gridDim.x * 4;
-  for (int64_t b = (int64_t)blockIdx.x * 4 + wid; b < w.max_bins; b += nwarps) {
-    const int64_t s0 = w.bin_start[b], s1 = w.bin_start[b + 1];
-    const int n = (int)(s1 - s0);
-    if (n <= 1) continue;
-    if (n > 1024) {  // rare fallback: insertion sort by one lane
-      if (lane == 0) {
-        int* p = w.sorted_atom + s0;
-        for (int i = 1; i < n; ++i) {
-          const int v = p[i];
-          int j = i - 1;
-          while (j >= 0 && p[j] > v) { p[j + 1] = p[j]; --j; }
-          p[j + 1] = v;
-        }
-      }
-      __syncwarp();
-      continue;
-    }
-    int n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    for (int i = lane; i < n2; i += 32) keys[i] = (i < n) ? w.sorted_atom[s0 + i] : 0x7fffffff;
-    __syncwarp();
-    for (int k = 2; k <= n2; k <<= 1)
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        for (int i = lane; i < n2; i += 32) {
-          const int ixj = i ^ j;
-          if (ixj > i) {
-            const int a = keys[i], c = keys[ixj];
-            const bool asc = (i & k) == 0;
-            if (asc ? (a > c) : (a < c)) { keys[i] = c; keys[ixj] = a; }
-          }
-        }
-        __syncwarp();
-      }
-    for (int i = lane; i < n; i += 32) w.sorted_atom[s0 + i] = keys[i];
-    __syncwarp();
-  }
+       a += (int64_t)gridDim.x * blockDim.x)
+    w.sorted_atom[w.bin_start[w.atom_bin[a]] + w.arrival[a]] = (int)a;
 }
 
 __global__ void k_gather_atoms(soapb_structs s, NLWork w) {
   for (int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; slot < s.n_atoms;
-       slot += (int64_t)gridDim.x * blockDim.x) {
-    const int a = w.sorted_atom[slot];
-    const int si = struct_of_atom(s.d_atom_off, s.n_struct, a);
-    const GridDesc& g = w.grids[si];
-    int b[3], wr[3];
-    double wp[3];
-    locate(g, s.d_positions[3 * (int64_t)a], s.d_positions[3 * (int64_t)a + 1], s.d_positions[3 * (int64_t)a + 2],
-           b, wr, wp);
-    w.sorted_pos[slot] = make_double4(wp[0], wp[1], wp[2], pack_info((int)a, s.d_species[a], pack3(wr[0], wr[1], wr[2])));
-  }
+       slot += (int64_t)gridDim.x * blockDim.x)
+    gather_atom(s, w, slot);
 }
 
-__global__ void k_centres(soapb_structs s, soapb_centres c, NLWork w) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < c.n_centres;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int si = c.d_struct[i];
-    const GridDesc& g = w.grids[si];
-    int b[3], wr[3];
-    double wp[3];
-    if (!locate(g, c.d_xyz[3 * i], c.d_xyz[3 * i + 1], c.d_xyz[3 * i + 2], b, wr, wp)) atomicOr(w.status, 2);
-    w.cpos[i] = make_double4(wp[0], wp[1], wp[2], 0.0);
-    w.cinfo[i] = make_int4(b[0] | (b[1] << 10) | (b[2] << 20), si, pack3(wr[0], wr[1], wr[2]), c.d_atom[i]);
-  }
+// ---- small inputs: every stage in one launch ----
+//
+// The stages are a chain of short dependent passes over few atoms, so separate
+// kernels cost their launches (16 launches and 3 memsets, 2-5 us each, for
+// 24 to 3000 atoms).  One cluster of up to 8 CTAs runs them all, with a cluster
+// barrier between stages (one CTA: a block barrier); intermediate arrays stay
+// in the workspace, in L2.
+constexpr int kCellsThreads = 512;
+constexpr int kCellsMaxCtas = 8;
+
+__global__ void __launch_bounds__(kCellsThreads) k_cells(soapb_structs s, soapb_centres c, NLWork w, double cutoff) {
+  __shared__ int64_t s_warp[32];
+  __shared__ int s_max[32];
+  // the grid is one cluster: blockIdx.x is the rank in it
+  const int nth = gridDim.x * kCellsThreads, t0 = blockIdx.x * kCellsThreads + threadIdx.x;
+  auto sync = [&]() {
+    if (gridDim.x == 1) {
+      __syncthreads();
+    } else {
+      asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    }
+  };
+  if (t0 < 4) w.status[t0] = 0;
+  for (int i = t0; i < s.n_struct; i += nth) grid_init(s, w, cutoff, i);
+  for (int64_t i = t0; i < w.max_bins; i += nth) w.bin_count[i] = 0;
+  sync();
+  frac_bbox(s, w, t0 & ~31, nth);
+  sync();
+  for (int i = t0; i < s.n_struct; i += nth) grid_setup(s, w, cutoff, i);
+  sync();
+  if (blockIdx.x == 0) block_scan_chunks(w.bins_per_struct, s.n_struct, w.bin_off, s_warp, s_max, nullptr);
+  sync();
+  for (int64_t a = t0; a < s.n_atoms; a += nth) bin_atom(s, w, a);
+  for (int64_t i = t0; i < c.n_centres; i += nth) place_centre(c, w, i);
+  sync();
+  if (blockIdx.x == 0)
+    block_scan_chunks(w.bin_count, __ldcg(w.bin_off + s.n_struct), w.bin_start, s_warp, s_max, nullptr);
+  sync();
+  for (int64_t a = t0; a < s.n_atoms; a += nth) w.sorted_atom[w.bin_start[w.atom_bin[a]] + w.arrival[a]] = (int)a;
+  sync();
+  for (int64_t slot = t0; slot < s.n_atoms; slot += nth) gather_atom(s, w, slot);
 }
 
 // ---------------------------------------------------------------------------
@@ -466,7 +548,7 @@ __global__ void k_centres(soapb_structs s, soapb_centres c, NLWork w) {
 struct VisitArgs {
   const GridDesc* grids;
   const int64_t* bin_off;
-  const int64_t* bin_start;
+  const int* bin_start;
   const double4* sorted_pos;
   const double4* cpos;
   const int4* cinfo;
@@ -747,18 +829,54 @@ __device__ __forceinline__ void visit_any(const VisitArgs& A, int64_t c, int* ru
   else visit(A, c, fn);
 }
 
-// 8 blocks of 4 warps per SM (64 registers): the count is latency-bound with
-// little work per candidate, so more resident warps pay more than pipelining.
-__global__ void __launch_bounds__(128, 8) k_count(VisitArgs A, int64_t n_centres, int* counts) {
+// Pairs of every centre, one warp per centre, 8 blocks of 4 warps per SM (64
+// registers): the count is latency-bound with little work per candidate, so
+// more resident warps pay more than pipelining.  The largest count goes to
+// status[2].  With pair_off, the last block to finish scans the counts into it
+// and, with stats, writes {total, largest, flags} -- the caller gets offsets and
+// summary from this launch (kLastBlockScan centres: the scan by 128 threads
+// costs less than the three launches of the general one).
+constexpr int64_t kLastBlockScan = 8192;
+
+__global__ void __launch_bounds__(128, 8) k_count(VisitArgs A, int64_t n_centres, int* counts, int64_t* pair_off,
+                                                  int64_t* stats) {
   __shared__ int s_runs[4][3 * kRunsPerPass];
-  const int lane = threadIdx.x & 31;
+  __shared__ int s_cnt[4];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t c = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < n_centres; c += nw) {
+  int most = 0;
+  for (int64_t c = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid; c < n_centres; c += nw) {
     int cnt = 0;
-    visit_any(A, c, s_runs[threadIdx.x >> 5], [&](bool ok, int, int, double, double, double, double) {
+    visit_any(A, c, s_runs[wid], [&](bool ok, int, int, double, double, double, double) {
       cnt += __popc(__ballot_sync(0xffffffffu, ok));
     });
     if (lane == 0) counts[c] = cnt;
+    most = max(most, cnt);
+  }
+  if (lane == 0) s_cnt[wid] = most;
+  __syncthreads();
+  if (!pair_off) {
+    if (threadIdx.x == 0) atomicMax(A.status + 2, max(max(s_cnt[0], s_cnt[1]), max(s_cnt[2], s_cnt[3])));
+    return;
+  }
+  __shared__ int s_last;
+  if (threadIdx.x == 0) {
+    __threadfence();  // this block's counts before its ticket (ordered after them by the barrier above)
+    s_last = atomicAdd(A.status + 1, 1) == (int)gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __shared__ int64_t s_warp[32];
+  int largest;
+  const int64_t total = block_scan_chunks(counts, n_centres, pair_off, s_warp, s_cnt, &largest);
+  if (threadIdx.x == 0) {
+    A.status[2] = largest;
+    if (stats) {
+      stats[0] = total;
+      stats[1] = largest;
+      stats[2] = __ldcg(A.status);
+    }
   }
 }
 
@@ -873,28 +991,12 @@ __global__ void __launch_bounds__(128) k_fill(VisitArgs A, int64_t n_centres, co
   }
 }
 
-// One block: total pairs, the largest per-centre count and the status flags,
-// so the host learns all three from one device-to-host copy.
-__global__ void __launch_bounds__(1024) k_stats(const int64_t* pair_off, int64_t n_centres, const int* status,
-                                                int64_t* out) {
-  __shared__ int64_t s_max[32];
-  int64_t m = 0;
-  for (int64_t c = threadIdx.x; c < n_centres; c += blockDim.x) {
-    const int64_t d = pair_off[c + 1] - pair_off[c];
-    m = d > m ? d : m;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const int64_t v = __shfl_xor_sync(0xffffffffu, m, o);
-    m = v > m ? v : m;
-  }
-  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) m = s_max[i] > m ? s_max[i] : m;
-    out[0] = pair_off[n_centres];
-    out[1] = m;
-    out[2] = status[0];
-  }
+// Total pairs, the largest per-centre count (from the count) and the status
+// flags, so the host learns all three from one read.
+__global__ void k_stats(const int64_t* pair_off, int64_t n_centres, const int* status, int64_t* out) {
+  out[0] = pair_off[n_centres];
+  out[1] = status[2];
+  out[2] = status[0];
 }
 
 // One block: out[0] = the list's total; when it exceeds capacity, every
@@ -916,7 +1018,7 @@ __global__ void __launch_bounds__(1024) k_clamp(int64_t* pair_off, int64_t n_cen
 // ---------------------------------------------------------------------------
 
 struct NLLayout {
-  int64_t grids, fbox, bps, bin_off, bin_count, bin_start, bin_cursor, atom_bin, sorted_atom, sorted_pos, cpos,
+  int64_t grids, fbox, bps, bin_off, bin_count, bin_start, arrival, atom_bin, sorted_atom, sorted_pos, cpos,
       cinfo, counts, partials, status, total;
   int64_t max_bins;
 };
@@ -933,8 +1035,8 @@ static NLLayout nl_layout(const soapb_structs* s, const soapb_centres* c) {
   L.bps = take(4 * ns);
   L.bin_off = take(8 * (ns + 1));
   L.bin_count = take(4 * L.max_bins);
-  L.bin_start = take(8 * (L.max_bins + 1));
-  L.bin_cursor = take(4 * L.max_bins);
+  L.bin_start = take(4 * (L.max_bins + 1));
+  L.arrival = take(4 * na);
   L.atom_bin = take(4 * na);
   L.sorted_atom = take(4 * na);
   L.sorted_pos = take(32 * na);
@@ -955,8 +1057,8 @@ static NLWork nl_work(const NLLayout& L, void* base_) {
   w.bins_per_struct = (int*)(base + L.bps);
   w.bin_off = (int64_t*)(base + L.bin_off);
   w.bin_count = (int*)(base + L.bin_count);
-  w.bin_start = (int64_t*)(base + L.bin_start);
-  w.bin_cursor = (int*)(base + L.bin_cursor);
+  w.bin_start = (int*)(base + L.bin_start);
+  w.arrival = (int*)(base + L.arrival);
   w.atom_bin = (int*)(base + L.atom_bin);
   w.sorted_atom = (int*)(base + L.sorted_atom);
   w.sorted_pos = (double4*)(base + L.sorted_pos);
@@ -1016,9 +1118,31 @@ extern "C" int soapb_neighbors_workspace(const soapb_basis* b, const soapb_struc
   return SOAPB_OK;
 }
 
-extern "C" int soapb_neighbors_count(const soapb_basis* b, const soapb_structs* s, const soapb_centres* c,
-                                     int32_t mode, void* d_work, int64_t work_bytes, int64_t* d_pair_off,
-                                     void* stream) {
+// Inputs up to this many atoms and centres build their cell lists in one
+// launch (k_cells).
+constexpr int64_t kCellsFused = 16384;
+
+static int launch_cells(const soapb_structs& s, const soapb_centres& c, const NLWork& w, double cutoff,
+                        cudaStream_t st) {
+  const int64_t most = s.n_atoms > c.n_centres ? s.n_atoms : c.n_centres;
+  int ctas = (int)((most + kCellsThreads - 1) / kCellsThreads);
+  ctas = ctas < 2 ? 1 : ctas < 4 ? 2 : ctas < 8 ? 4 : kCellsMaxCtas;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)ctas;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(kCellsThreads);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const int rc = check_cuda(cudaLaunchKernelEx(&cfg, k_cells, s, c, w, cutoff), "k_cells");
+  return rc ? rc : check_launch("k_cells");
+}
+
+static int neighbors_count(const soapb_basis* b, const soapb_structs* s, const soapb_centres* c, int32_t mode,
+                           void* d_work, int64_t work_bytes, int64_t* d_pair_off, int64_t* d_stats, void* stream) {
   int rc = check_inputs(b, s, c);
   if (rc) return rc;
   if (mode != SOAPB_NL_CREATE && mode != SOAPB_NL_ALL) return set_error(SOAPB_ERR_ARG, "bad neighbour mode");
@@ -1029,27 +1153,48 @@ extern "C" int soapb_neighbors_count(const soapb_basis* b, const soapb_structs* 
   cudaStream_t st = (cudaStream_t)stream;
   NLWork w = nl_work(L, d_work);
   const int ns = s->n_struct;
-  if ((rc = check_cuda(cudaMemsetAsync(w.status, 0, 16, st), "memset status"))) return rc;
-  if ((rc = check_cuda(cudaMemsetAsync(w.bin_count, 0, 4 * L.max_bins, st), "memset bins"))) return rc;
-  if ((rc = check_cuda(cudaMemsetAsync(w.bin_cursor, 0, 4 * L.max_bins, st), "memset cursor"))) return rc;
   const double cutoff = b->cutoff;
-  k_grid_init<<<(ns + 127) / 128, 128, 0, st>>>(*s, w, cutoff);
-  k_frac_bbox<<<grid_blocks(s->n_atoms, 256), 256, 0, st>>>(*s, w);
-  k_grid_setup<<<(ns + 127) / 128, 128, 0, st>>>(*s, w, cutoff);
-  if ((rc = check_launch("grid setup", 3))) return rc;
-  if ((rc = exclusive_scan(w.bins_per_struct, ns, w.bin_off, w.partials, st))) return rc;
-  k_bin_atoms<<<grid_blocks(s->n_atoms, 256), 256, 0, st>>>(*s, w);
-  if ((rc = check_launch("k_bin_atoms"))) return rc;
-  if ((rc = exclusive_scan(w.bin_count, L.max_bins, w.bin_start, w.partials, st))) return rc;
-  k_scatter_atoms<<<grid_blocks(s->n_atoms, 256), 256, 0, st>>>(s->n_atoms, w);
-  k_sort_bins<<<grid_blocks(L.max_bins, 4), 128, 0, st>>>(w);
-  k_gather_atoms<<<grid_blocks(s->n_atoms, 256), 256, 0, st>>>(*s, w);
-  k_centres<<<grid_blocks(c->n_centres, 256), 256, 0, st>>>(*s, *c, w);
-  if ((rc = check_launch("cell lists", 5))) return rc;
+  if (s->n_atoms <= kCellsFused && c->n_centres <= kCellsFused && ns <= kCellsFused) {
+    if ((rc = launch_cells(*s, *c, w, cutoff, st))) return rc;
+  } else {
+    if ((rc = check_cuda(cudaMemsetAsync(w.status, 0, 16, st), "memset status"))) return rc;
+    k_grid_init<<<grid_blocks(L.max_bins, 256), 256, 0, st>>>(*s, w, cutoff);
+    // at least 8 atoms a lane: a warp reduces its bounds once
+    k_frac_bbox<<<grid_blocks((s->n_atoms + 7) / 8, 256), 256, 0, st>>>(*s, w);
+    k_grid_setup<<<(ns + 127) / 128, 128, 0, st>>>(*s, w, cutoff);
+    if ((rc = check_launch("grid setup", 3))) return rc;
+    if ((rc = exclusive_scan(w.bins_per_struct, ns, w.bin_off, w.partials, st))) return rc;
+    k_bin_atoms<<<grid_blocks(s->n_atoms > c->n_centres ? s->n_atoms : c->n_centres, 256), 256, 0, st>>>(*s, *c, w);
+    if ((rc = check_launch("k_bin_atoms"))) return rc;
+    if ((rc = exclusive_scan(w.bin_count, L.max_bins, w.bin_start, w.partials, st))) return rc;
+    k_scatter_atoms<<<grid_blocks(s->n_atoms, 256), 256, 0, st>>>(s->n_atoms, w);
+    k_gather_atoms<<<grid_blocks(s->n_atoms, 256), 256, 0, st>>>(*s, w);
+    if ((rc = check_launch("cell lists", 2))) return rc;
+  }
   const VisitArgs A = visit_args(b, w, mode);
-  if (c->n_centres > 0) k_count<<<grid_blocks(c->n_centres, 4), 128, 0, st>>>(A, c->n_centres, w.counts);
+  const bool tail = c->n_centres > 0 && c->n_centres <= kLastBlockScan;
+  if (c->n_centres > 0)
+    k_count<<<grid_blocks(c->n_centres, 4), 128, 0, st>>>(A, c->n_centres, w.counts, tail ? d_pair_off : nullptr,
+                                                          tail ? d_stats : nullptr);
   if ((rc = check_launch("k_count", c->n_centres > 0 ? 1 : 0))) return rc;
-  return exclusive_scan(w.counts, c->n_centres, d_pair_off, w.partials, st);
+  if (tail) return SOAPB_OK;
+  if ((rc = exclusive_scan(w.counts, c->n_centres, d_pair_off, w.partials, st))) return rc;
+  if (!d_stats) return SOAPB_OK;
+  k_stats<<<1, 1, 0, st>>>(d_pair_off, c->n_centres, w.status, d_stats);
+  return check_launch("k_stats");
+}
+
+extern "C" int soapb_neighbors_count(const soapb_basis* b, const soapb_structs* s, const soapb_centres* c,
+                                     int32_t mode, void* d_work, int64_t work_bytes, int64_t* d_pair_off,
+                                     void* stream) {
+  return neighbors_count(b, s, c, mode, d_work, work_bytes, d_pair_off, nullptr, stream);
+}
+
+extern "C" int soapb_neighbors_count_stats(const soapb_basis* b, const soapb_structs* s, const soapb_centres* c,
+                                           int32_t mode, void* d_work, int64_t work_bytes, int64_t* d_pair_off,
+                                           int64_t* d_stats, void* stream) {
+  if (!d_stats) return set_error(SOAPB_ERR_ARG, "null stats");
+  return neighbors_count(b, s, c, mode, d_work, work_bytes, d_pair_off, d_stats, stream);
 }
 
 extern "C" int soapb_neighbors_fill(const soapb_basis* b, const soapb_structs* s, const soapb_centres* c,
@@ -1095,7 +1240,7 @@ extern "C" int soapb_neighbors_stats(const soapb_basis* b, const soapb_structs* 
   if (!d_work || !d_pair_off || !d_stats) return set_error(SOAPB_ERR_ARG, "null workspace, pair_off or stats");
   const NLLayout L = nl_layout(s, c);
   const NLWork w = nl_work(L, const_cast<void*>(d_work));
-  k_stats<<<1, 1024, 0, (cudaStream_t)stream>>>(d_pair_off, c->n_centres, w.status, d_stats);
+  k_stats<<<1, 1, 0, (cudaStream_t)stream>>>(d_pair_off, c->n_centres, w.status, d_stats);
   return check_launch("k_stats");
 }
 

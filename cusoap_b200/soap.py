@@ -293,13 +293,17 @@ class _Pairs:
         check(lib.soapb_neighbors_workspace(b, ctypes.byref(batch.cs), ctypes.byref(batch.cc), ctypes.byref(ws)))
         self.work = torch.empty(max(int(ws.value), 256), dtype=torch.uint8, device=dev)
         self.pair_off = torch.empty(batch.n_centres + 1, dtype=torch.int64, device=dev)
-        soap._call("neighbors_count", lib.soapb_neighbors_count, b, ctypes.byref(batch.cs), ctypes.byref(batch.cc),
-                   mode, _ptr(self.work), self.work.numel(), _ptr(self.pair_off), st)
-        # one device->host read: total pairs, largest per-centre count, status flags
-        stats = torch.empty(3, dtype=torch.int64, device=dev)
-        soap._call("neighbors_stats", lib.soapb_neighbors_stats, b, ctypes.byref(batch.cs), ctypes.byref(batch.cc),
-                   _ptr(self.work), _ptr(self.pair_off), _ptr(stats), st)
-        self.total, self.max_pairs, status = (int(v) for v in stats.cpu().tolist())
+        # total pairs, largest per-centre count and status flags, written by the count into
+        # page-locked host memory: read after one stream synchronisation
+        # (a buffer belongs to one call until it has been read, so threads may share the object)
+        pool = soap._stats_pool
+        stats = pool.pop() if pool else torch.empty(3, dtype=torch.int64, pin_memory=True)
+        soap._call("neighbors_count", lib.soapb_neighbors_count_stats, b, ctypes.byref(batch.cs),
+                   ctypes.byref(batch.cc), mode, _ptr(self.work), self.work.numel(), _ptr(self.pair_off), _ptr(stats),
+                   st)
+        torch.cuda.current_stream(dev).synchronize()
+        self.total, self.max_pairs, status = stats.tolist()
+        pool.append(stats)
         if status & 1:
             raise ValueError("singular cell in a periodic structure")
         if status & 2:
@@ -552,6 +556,7 @@ class SOAP:
         self._poly_grid = _poly_grid(self._r_cut, self._n_max, self.quad_n) if self._rbf == "polynomial" else None
         self._build_basis()
         self._counter = torch.zeros(1, dtype=torch.int32, device=self.device)
+        self._stats_pool: List[torch.Tensor] = []  # page-locked int64[3] buffers of the neighbour summaries
         self._topology = None  # device copies of the last batch's species, offsets, cells (see _Batch)
         self.n_features = int(self.get_number_of_features())
         # When a list, every library call appends (name, start_event, end_event)

@@ -181,6 +181,15 @@ int soapb_neighbors_status(const soapb_basis* b, const soapb_structs* s, const s
 int soapb_neighbors_stats(const soapb_basis* b, const soapb_structs* s, const soapb_centres* c, const void* d_work,
                           const int64_t* d_pair_off, int64_t* d_stats, void* stream);
 
+/* soapb_neighbors_count followed by soapb_neighbors_stats, in fewer launches:
+ * up to 8192 centres the count's last block scans the counts and writes the
+ * summary.  d_stats (int64[3]) is device memory, or page-locked host memory
+ * that the device can address: the caller then reads it after synchronising
+ * the stream, without a copy.  No single counterpart in the reference. */
+int soapb_neighbors_count_stats(const soapb_basis* b, const soapb_structs* s, const soapb_centres* c, int32_t mode,
+                                void* d_work, int64_t work_bytes, int64_t* d_pair_off, int64_t* d_stats,
+                                void* stream);
+
 /* For a pair buffer of fixed capacity (a captured CUDA graph replays with
  * the buffers it was captured with): after soapb_neighbors_fill, write the
  * list's total to *d_total (device int64) and, if it exceeds `capacity`,
