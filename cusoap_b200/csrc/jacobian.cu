@@ -26,14 +26,20 @@
 //
 // Two launches, sharing a workspace:
 //   k_jac_entries  per centre: the (row, edge) entries of its included atoms,
-//                  sorted by row, and a bitmap of its nonzero rows;
+//                  sorted by row, a bitmap of its nonzero rows, and its
+//                  compute tasks: runs of whole rows of about eb entries;
 //   k_jacobian     warp roles inside every block: warp 0 streams the block's
 //                  share of the zero rows (64-row chunks in global row order)
 //                  with TMA bulk copies of a zero tile in shared memory --
 //                  one issuing lane, no load/store-unit traffic -- while warps
-//                  1..7 compute the nonzero rows (entries staged in shared
-//                  memory, each thread four consecutive features of a row in
-//                  the three directions, stored as 16-byte vectors).
+//                  1..7 take compute tasks (entries staged in shared memory,
+//                  each thread four consecutive features of a row in the three
+//                  directions, stored as 16-byte vectors).
+// A task is one staged batch, not one centre: staging a batch is a chain of
+// barriers and shared-memory latencies, so with centres as tasks a centre's
+// batches ran one after the other in one block while most blocks had no centre
+// (50 centres of a 3000-atom cluster, F = 420: 452 us a launch, 179 us with
+// batches as tasks, 115 us to write the output; 1536 atoms, 12 GB: 2.35 and 2.08 ms).
 // Zero and nonzero rows are disjoint, so every element is written once and the
 // two roles never synchronise.
 #include "common.cuh"
@@ -52,13 +58,14 @@ struct JacArgs {
   const int* ftab;
   float* out;
   int* status;
-  int* counter;                  // work queue of the compute kernel
-  int* ent_cnt;                  // (n_centres) entries per centre
+  int* counter;                  // {next task, next zero chunk, tasks, 0}
+  int4* tasks;                   // {centre, entries (negative: the centre's own row), first entry in ent (low, high word)}
   unsigned long long* ent;       // sorted entries, centre c at ent_mult * pair_off[c]
   unsigned long long* ent_tmp;   // merge buffer of a centre with more than cap entries, same offsets
   unsigned int* bitmap;          // (n_centres * n_inc) nonzero-row bits
   int64_t n_centres, n_inc;
   int N, S, nseg, F, mode, attach, cap, eb, ent_mult;
+  int centre_eb;  // entries per batch of a moving centre's own row (centre_row), 0: as any other row
   float inv_h;
 };
 
@@ -187,7 +194,7 @@ __device__ int centre_entries(const JacArgs& a, int64_t p0, int P, int catom, in
 
 __global__ void __launch_bounds__(256) k_jac_entries(JacArgs a) {
   extern __shared__ __align__(16) unsigned long long skeys[];
-  __shared__ int s_nent;
+  __shared__ int s_nent, s_task0;
   for (int64_t c = blockIdx.x; c < a.n_centres; c += gridDim.x) {
     const int64_t p0 = a.pair_off[c];
     const int P = (int)(a.pair_off[c + 1] - p0);
@@ -200,7 +207,48 @@ __global__ void __launch_bounds__(256) k_jac_entries(JacArgs a) {
       const int64_t r = (int64_t)c * a.n_inc + (int64_t)(dst[i] >> 32);
       atomicOr(a.bitmap + (r >> 5), 1u << (r & 31));
     }
-    if (threadIdx.x == 0) a.ent_cnt[c] = nent;
+    // compute tasks: runs of about eb entries, both ends moved up to the next row boundary.  A
+    // moving centre's own row holds an entry of every edge: a task of its own (centre_row) splits
+    // the others into those before it, [0, g0), and after it, [g1, nent).
+    auto lower = [&](unsigned long long key) {  // first entry not below key
+      int lo = 0, hi = nent;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (dst[mid] < key) lo = mid + 1;
+        else hi = mid;
+      }
+      return lo;
+    };
+    auto row_boundary = [&](int i) {  // first entry >= i that starts a row
+      if (i == 0 || i >= nent) return min(i, nent);
+      const unsigned long long next = ((dst[i - 1] >> 32) + 1) << 32;  // first key of the following rows
+      return dst[i] >= next ? i : lower(next);
+    };
+    int g0 = nent, g1 = nent;
+    if (crow >= 0 && a.centre_eb > 0) {
+      g0 = lower((unsigned long long)crow << 32);
+      g1 = lower(((unsigned long long)crow + 1) << 32);
+      if (g1 - g0 <= a.eb) g0 = g1 = nent;
+    }
+    const int n0 = (g0 + a.eb - 1) / a.eb, n1 = (nent - g1 + a.eb - 1) / a.eb, own = g1 > g0 ? 1 : 0;
+    const int nt = n0 + n1 + own;
+    if (threadIdx.x == 0) s_task0 = nt > 0 ? atomicAdd(a.counter + 2, nt) : 0;
+    __syncthreads();
+    for (int k = threadIdx.x; k < nt; k += blockDim.x) {
+      int b, e;
+      if (k < own) {  // the long task first
+        b = g0;
+        e = g1;
+      } else if (k < own + n0) {
+        b = min(row_boundary((k - own) * a.eb), g0);
+        e = min(row_boundary((k - own + 1) * a.eb), g0);
+      } else {
+        b = row_boundary(g1 + (k - own - n0) * a.eb);
+        e = row_boundary(g1 + (k - own - n0 + 1) * a.eb);
+      }
+      const unsigned long long first = (unsigned long long)((size_t)a.ent_mult * p0 + b);
+      a.tasks[s_task0 + k] = make_int4((int)c, k < own ? b - e : e - b, (int)(unsigned)first, (int)(unsigned)(first >> 32));
+    }
     __syncthreads();
   }
 }
@@ -218,7 +266,7 @@ __device__ __forceinline__ void bulk_s2g(void* g, const void* s, uint32_t bytes)
 // (zq), by TMA bulk copies of the zero tile; lane 0 issues, the copies run
 // asynchronously and the lane waits for all of them before returning (the
 // tile must outlive them).  Every block's zero warp runs this from the start
-// and its compute warps join once the centre queue is empty, so the zero
+// and its compute warps join once the task queue is empty, so the zero
 // stream ends together with the compute work.  Rows are 12 F bytes, a
 // multiple of 16 (F % 4 == 0).
 __device__ void jac_zero_rows_tma(const JacArgs& a, const void* ztile, int* zq) {
@@ -273,58 +321,63 @@ __device__ __forceinline__ void compute_bar(int nthreads) {
   asm volatile("bar.sync 1, %0;\n" ::"r"(nthreads) : "memory");
 }
 
-// Stage entries [b0, b0 + nb) of the centre into ed (all threads; ends with a barrier).
+// Asynchronous copy of one T (4, 8 or 16 bytes) global -> shared.
+template <class T>
+__device__ __forceinline__ void copy_async(T* s, const T* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(s)), "l"(g),
+               "n"(sizeof(T))
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// Entry of thread tid (< nb): header, harmonics and their gradients.
 template <int L>
-__device__ void stage_entries(const JacArgs& a, int64_t p0, const unsigned long long* keys, int b0, int nb, int crow,
-                              const float* cs, float* ed, int EF, const float* sqrt_pref, int tid, int nth) {
+__device__ __forceinline__ void stage_harmonics(const JacArgs& a, const float4& pr, bool centre_row, float* h) {
+  constexpr int K = JacShape<L>::K;
+  const int NF = a.N * (L + 1);
+  const float r = sqrtf(pr.x * pr.x + pr.y * pr.y + pr.z * pr.z);
+  int seg;
+  float t;
+  seg_coord(r, a.inv_h, a.nseg, seg, t);
+  h[0] = pr.x; h[1] = pr.y; h[2] = pr.z;
+  h[3] = (float)((unsigned)__float_as_int(pr.w) >> kAtomBits);
+  h[4] = centre_row ? -1.0f : 1.0f;
+  h[5] = r; h[6] = t; h[7] = __int_as_float(seg);
+  float* R = h + 8 + 2 * NF;
+  float* dR = R + K;
+  SolidHarmonics<L>::with_gradients(pr.x, pr.y, pr.z, [&](int idx, float v, float dx, float dy, float dz) {
+    R[idx] = v; dR[idx] = dx; dR[K + idx] = dy; dR[2 * K + idx] = dz;
+  });
+}
+
+// Radial functions of the nb staged entries (all compute threads).
+__device__ __forceinline__ void stage_radial(const JacArgs& a, int nb, float* ed, int EF, int NF, int tid, int nth) {
+  auto one = [&](float* h, int fn) {
+    const float r = h[5], t = h[6];
+    const int seg = __float_as_int(h[7]);
+    float cb[kNCoef], cd[kNCoef];
+    load_coef(a.tab_b, seg, fn, NF, cb);
+    load_coef(a.tab_bh, seg, fn, NF, cd);
+    h[8 + fn] = (r > 0.0f) ? horner7(cb, t) : __ldg(a.selfv + fn);
+    h[8 + NF + fn] = (r > 0.0f) ? horner7(cd, t) / r : 0.0f;
+  };
+  if (NF <= nth) {  // thread owns radial function fn, entries stepped (division-free loop)
+    const int fn = tid % NF, istep = nth / NF;
+    if (tid < istep * NF)
+      for (int i = tid / NF; i < nb; i += istep) one(ed + (size_t)i * EF, fn);
+  } else {  // more radial functions than threads
+    for (int t = tid; t < nb * NF; t += nth) one(ed + (size_t)(t / NF) * EF, t % NF);
+  }
+}
+
+// ps: the pre-contracted vectors X0, X1 of the nb staged entries (all compute threads).
+template <int L>
+__device__ __forceinline__ void stage_vectors(const JacArgs& a, int nb, const float* cs, float* ed, int EF,
+                                              const float* sqrt_pref, int tid, int nth) {
   using Sh = JacShape<L>;
   constexpr int K = Sh::K, KC = Sh::KC, LP = Sh::LP;
   const int N = a.N, S = a.S, NF = N * LP, SNL = S * N * LP, XO = Sh::xoff(N);
-  for (int i = tid; i < nb; i += nth) {
-    const unsigned long long key = keys[b0 + i];
-    const float4 pr = a.pairs[p0 + (int)(key & 0xffffffffu)];
-    float* h = ed + (size_t)i * EF;
-    h[0] = pr.x; h[1] = pr.y; h[2] = pr.z;
-    h[3] = (float)((unsigned)__float_as_int(pr.w) >> kAtomBits);
-    h[4] = (a.attach && (int)(key >> 32) == crow) ? -1.0f : 1.0f;
-    float* R = h + 8 + 2 * NF;
-    float* dR = R + K;
-    SolidHarmonics<L>::with_gradients(pr.x, pr.y, pr.z, [&](int idx, float v, float dx, float dy, float dz) {
-      R[idx] = v; dR[idx] = dx; dR[K + idx] = dy; dR[2 * K + idx] = dz;
-    });
-  }
-  compute_bar(nth);
-  if (tid < (nth / NF) * NF) {  // thread owns radial function fn, entries stepped (division-free loop)
-    const int fn = tid % NF, istep = nth / NF;
-    for (int i = tid / NF; i < nb; i += istep) {
-      float* h = ed + (size_t)i * EF;
-      const float r = sqrtf(h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
-      int seg;
-      float tt;
-      seg_coord(r, a.inv_h, a.nseg, seg, tt);
-      float cf[kNCoef];
-      load_coef(a.tab_b, seg, fn, NF, cf);
-      h[8 + fn] = (r > 0.0f) ? horner7(cf, tt) : __ldg(a.selfv + fn);
-      load_coef(a.tab_bh, seg, fn, NF, cf);
-      h[8 + NF + fn] = (r > 0.0f) ? horner7(cf, tt) / r : 0.0f;
-    }
-  } else if (NF > nth) {  // more radial functions than threads: flat loop
-    for (int t = tid; t < nb * NF; t += nth) {
-      const int i = t / NF, fn = t % NF;
-      float* h = ed + (size_t)i * EF;
-      const float r = sqrtf(h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
-      int seg;
-      float tt;
-      seg_coord(r, a.inv_h, a.nseg, seg, tt);
-      float cf[kNCoef];
-      load_coef(a.tab_b, seg, fn, NF, cf);
-      h[8 + fn] = (r > 0.0f) ? horner7(cf, tt) : __ldg(a.selfv + fn);
-      load_coef(a.tab_bh, seg, fn, NF, cf);
-      h[8 + NF + fn] = (r > 0.0f) ? horner7(cf, tt) / r : 0.0f;
-    }
-  }
-  compute_bar(nth);
-  if (a.mode == SOAPB_OUT_PS) {
+  {
     // thread -> coefficient index ai = (l S + j) N + n (decoded once) and first entry;
     // entries stepped by istep (division-free loop)
     const bool small = SNL <= nth;
@@ -358,34 +411,63 @@ __device__ void stage_entries(const JacArgs& a, int64_t p0, const unsigned long 
         X[SNL + ai] = make_float4(h[1] * bh, v1, h[2] * bh, v2);
       }
     }
-    compute_bar(nth);
   }
 }
 
-// Values of the four features 4q .. 4q+3 in the three directions, summed over
+// The four features 4q .. 4q + 3 of a thread, decoded once per task.  ps: the
+// coefficient-pair code ia | ib << 12 | l << 24.  cc: species, radial function
+// index, source harmonic and output scale.
+struct QuadCode {
+  int code[4], sp[4], src[4];
+  float scale[4];
+};
+
+template <int L>
+__device__ __forceinline__ void quad_decode(const JacArgs& a, int q, QuadCode& qc) {
+  constexpr int K = JacShape<L>::K;
+  const int N = a.N, F = a.F;
+  if (a.mode == SOAPB_OUT_PS) {
+    if ((F & 3) == 0) {
+      const int4 c4 = __ldg(reinterpret_cast<const int4*>(a.ftab) + q);
+      qc.code[0] = c4.x; qc.code[1] = c4.y; qc.code[2] = c4.z; qc.code[3] = c4.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) qc.code[k] = (4 * q + k < F) ? __ldg(a.ftab + 4 * q + k) : 0;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int f = min(4 * q + k, F - 1);
+      const int sf = f / (N * K), rem = f - sf * N * K, n = rem / K, lo = rem - n * K;
+      int src = lo;
+      // DScribe cc layout: l = 1 stored (z, x, y) = source lm (2, 3, 1); lm >= 4 scaled by pi^-3/2
+      if (lo >= 1 && lo <= 3) src = (lo == 3) ? 1 : lo + 1;
+      int l = 0;
+      while ((l + 1) * (l + 1) <= src) ++l;
+      qc.code[k] = l * N + n;
+      qc.sp[k] = (4 * q + k < F) ? sf : -1;
+      qc.src[k] = src;
+      qc.scale[k] = lo >= 4 ? (float)(1.0 / (kPi * 1.7724538509055160273)) : 1.0f;
+    }
+  }
+}
+
+// Values of a thread's four features in the three directions, summed over
 // staged entries [g0, g1).  ps: X already carries sqrt(pref_l) on both sides.
 template <int L>
-__device__ __forceinline__ void quad_values(const JacArgs& a, const float* ed, int EF, int g0, int g1, int q,
-                                            float (&v)[3][4]) {
+__device__ __forceinline__ void quad_values(const JacArgs& a, const float* ed, int EF, int g0, int g1,
+                                            const QuadCode& qc, float (&v)[3][4]) {
   using Sh = JacShape<L>;
   constexpr int K = Sh::K, LP = Sh::LP;
-  const int N = a.N, S = a.S, NF = N * LP, SNL = S * N * LP, XO = Sh::xoff(N), F = a.F;
+  const int N = a.N, S = a.S, NF = N * LP, SNL = S * N * LP, XO = Sh::xoff(N);
 #pragma unroll
   for (int k = 0; k < 4; ++k) v[0][k] = v[1][k] = v[2][k] = 0.f;
   if (a.mode == SOAPB_OUT_PS) {
-    int code[4];
-    if ((F & 3) == 0) {
-      const int4 c4 = __ldg(reinterpret_cast<const int4*>(a.ftab) + q);  // pre-decoded: ia | ib << 12 | l << 24
-      code[0] = c4.x; code[1] = c4.y; code[2] = c4.z; code[3] = c4.w;
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) code[k] = (4 * q + k < F) ? __ldg(a.ftab + 4 * q + k) : 0;
-    }
     for (int i = g0; i < g1; ++i) {
       const float4* X = reinterpret_cast<const float4*>(ed + (size_t)i * EF + XO);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int ia = code[k] & 4095, ib = (code[k] >> 12) & 4095;
+        const int ia = qc.code[k] & 4095, ib = (qc.code[k] >> 12) & 4095;
         const float4 pa = X[ia], qa = X[SNL + ia], pb = X[ib], qb = X[SNL + ib];
         v[0][k] += pa.z * pb.x + pa.y * pb.w + pb.z * pa.x + pb.y * pa.w;
         v[1][k] += qa.x * pb.x + pa.y * qb.y + qb.x * pa.x + pb.y * qa.y;
@@ -393,35 +475,116 @@ __device__ __forceinline__ void quad_values(const JacArgs& a, const float* ed, i
       }
     }
   } else {
+    for (int i = g0; i < g1; ++i) {
+      const float* h = ed + (size_t)i * EF;
+      const float* R = h + 8 + 2 * NF;
+      const float* dR = R + K;
+      const int sp = (int)h[3];
+      const float sign = h[4], x = h[0], y = h[1], z = h[2];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int f = 4 * q + k;
-      if (f >= F) continue;
-      const int sf = f / (N * K), rem = f - sf * N * K, n = rem / K, lo = rem - n * K;
-      int src = lo;
-      float scale = 1.0f;
-      // DScribe cc layout: l = 1 stored (z, x, y) = source lm (2, 3, 1); lm >= 4 scaled by pi^-3/2
-      if (lo >= 1 && lo <= 3) src = (lo == 3) ? 1 : lo + 1;
-      if (lo >= 4) scale = (float)(1.0 / (kPi * 1.7724538509055160273));
-      const int l = (int)sqrtf((float)src + 0.5f);
-      for (int i = g0; i < g1; ++i) {
-        const float* h = ed + (size_t)i * EF;
-        if ((int)h[3] != sf) continue;
-        const float* R = h + 8 + 2 * NF;
-        const float* dR = R + K;
-        const float bh = h[4] * h[8 + NF + l * N + n] * R[src], b = h[4] * h[8 + l * N + n];
-        v[0][k] += scale * (h[0] * bh + b * dR[src]);
-        v[1][k] += scale * (h[1] * bh + b * dR[K + src]);
-        v[2][k] += scale * (h[2] * bh + b * dR[2 * K + src]);
+      for (int k = 0; k < 4; ++k) {
+        if (qc.sp[k] != sp) continue;
+        const int fn = qc.code[k], src = qc.src[k];
+        const float bh = sign * h[8 + NF + fn] * R[src], b = sign * h[8 + fn];
+        v[0][k] += qc.scale[k] * (x * bh + b * dR[src]);
+        v[1][k] += qc.scale[k] * (y * bh + b * dR[K + src]);
+        v[2][k] += qc.scale[k] * (z * bh + b * dR[2 * K + src]);
       }
     }
   }
 }
 
-// Nonzero rows: centres from a work queue, entries staged in batches, each
-// task = (row group, four consecutive features) stored as 16-byte vectors.
+// A moving centre's own row: minus the sum over all its n edges.  The sum of
+// dc / dx_d over the edges is formed first, D[d][s][n][lm] in shared memory
+// (3 N K FMAs an edge), and contracted with the coefficients once, instead of
+// 12 FMAs an edge for every feature in batches of eb that follow one another
+// (192 atoms, 130 edges a centre, cc: 195 us against 101 us, entries
+// included).  The edges are sorted by species, so a thread keeps its
+// (n, lm) in registers and adds it to D when the species changes.
 template <int L>
-__global__ void __launch_bounds__(256) k_jacobian(JacArgs a) {
+__device__ void centre_row(const JacArgs& a, int64_t p0, const unsigned long long* keys, int n, const float* cs,
+                           float* smem, float* orow, const float* sqrt_pref, int tid, int nth) {
+  using Sh = JacShape<L>;
+  constexpr int K = Sh::K, KC = Sh::KC;
+  const int N = a.N, SNK = a.S * N * K, NK = N * K, NF = N * (L + 1), EF = Sh::xoff(N), F = a.F;
+  float* D = smem;
+  float* ed = smem + ((3 * SNK + 3) & ~3);
+  for (int i = tid; i < 3 * SNK; i += nth) D[i] = 0.0f;
+  for (int b0 = 0; b0 < n; b0 += a.centre_eb) {
+    const int nb = min(a.centre_eb, n - b0);
+    if (tid < nb)
+      stage_harmonics<L>(a, a.pairs[p0 + (int)(keys[b0 + tid] & 0xffffffffu)], true, ed + (size_t)tid * EF);
+    compute_bar(nth);
+    stage_radial(a, nb, ed, EF, NF, tid, nth);
+    compute_bar(nth);
+    for (int it = tid; it < NK; it += nth) {
+      const int nn = it / K, lm = it - nn * K;
+      int l = 0;
+      while ((l + 1) * (l + 1) <= lm) ++l;
+      const int fn = 8 + l * N + nn, iR = 8 + 2 * NF + lm;
+      float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
+      int cur = (int)ed[3];
+      auto flush = [&]() {
+        float* d = D + cur * NK + it;
+        d[0] -= v0;
+        d[SNK] -= v1;
+        d[2 * SNK] -= v2;
+        v0 = v1 = v2 = 0.0f;
+      };
+      for (int i = 0; i < nb; ++i) {
+        const float* h = ed + (size_t)i * EF;
+        if ((int)h[3] != cur) {
+          flush();
+          cur = (int)h[3];
+        }
+        const float bR = h[fn + NF] * h[iR], b = h[fn];
+        v0 = fmaf(h[0], bR, fmaf(b, h[iR + K], v0));
+        v1 = fmaf(h[1], bR, fmaf(b, h[iR + 2 * K], v1));
+        v2 = fmaf(h[2], bR, fmaf(b, h[iR + 3 * K], v2));
+      }
+      flush();
+    }
+    compute_bar(nth);
+  }
+  if (a.mode == SOAPB_OUT_PS) {
+    for (int f = tid; f < F; f += nth) {
+      const int code = __ldg(a.ftab + f), l = code >> 24, base = l * a.S * N;
+      const int ja = (code & 4095) - base, jb = ((code >> 12) & 4095) - base;
+      const float *ca = cs + ja * KC + l * l, *cb = cs + jb * KC + l * l;
+      const float *da = D + ja * K + l * l, *db = D + jb * K + l * l;
+      float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
+      for (int m = 0; m < 2 * l + 1; ++m) {
+        const float x = ca[m], y = cb[m];
+        v0 += da[m] * y + x * db[m];
+        v1 += da[SNK + m] * y + x * db[SNK + m];
+        v2 += da[2 * SNK + m] * y + x * db[2 * SNK + m];
+      }
+      const float pref = sqrt_pref[l] * sqrt_pref[l];
+      __stcs(orow + f, pref * v0);
+      __stcs(orow + F + f, pref * v1);
+      __stcs(orow + 2 * F + f, pref * v2);
+    }
+  } else {
+    for (int f = tid; f < F; f += nth) {
+      const int sn = f / K, lo = f - sn * K;
+      const int src = (lo >= 1 && lo <= 3) ? ((lo == 3) ? 1 : lo + 1) : lo;  // as in quad_decode
+      const float scale = lo >= 4 ? (float)(1.0 / (kPi * 1.7724538509055160273)) : 1.0f;
+      for (int d = 0; d < 3; ++d) __stcs(orow + d * F + f, scale * D[d * SNK + sn * K + src]);
+    }
+  }
+  compute_bar(nth);  // D, the entries and cs are rewritten by the next task
+}
+
+// Nonzero rows: tasks from a work queue, a task's entries staged in batches of
+// eb (one batch, unless a row has many entries), each thread (row group, four
+// consecutive features), stored as 16-byte vectors.  A task is a chain of short
+// stages, so its global loads run ahead: the next task is claimed while the
+// harmonics are computed, its keys are loaded during the radial stage and its
+// pairs during the contraction, and the centre's coefficient row comes in by
+// asynchronous copies.  1536 atoms: 2.08 ms without this, 1.83 ms with it,
+// entries included (1.81 ms to write the output).
+template <int L>
+__global__ void __launch_bounds__(256, 2) k_jacobian(JacArgs a) {
   using Sh = JacShape<L>;
   constexpr int K = Sh::K, KC = Sh::KC;
   constexpr int kCT = 224;  // compute threads (warps 1..7)
@@ -434,9 +597,13 @@ __global__ void __launch_bounds__(256) k_jacobian(JacArgs a) {
   float* ed = cs + Sh::cs_floats(N, S);
   const int EF = Sh::entry_floats(N, S, a.mode);
   __shared__ float s_sqrt_pref[kMaxL + 1];
-  __shared__ int s_gstart[33];
+  __shared__ int s_gstart[33], s_grow[32];  // first entry and output row of each row group of the batch
   __shared__ int s_ng;
-  __shared__ int s_c;
+  __shared__ int4 s_task[2];
+  // the next task's offset, keys and pairs (an entry's key and pair are written and read by its own thread)
+  __shared__ int64_t s_p0;
+  __shared__ unsigned long long s_key[32];
+  __shared__ __align__(16) float4 s_pair[32];
   if (threadIdx.x <= L) s_sqrt_pref[threadIdx.x] = sqrtf(sqrtf(8.0f * (float)(kPi * kPi) / (2.0f * threadIdx.x + 1.0f)));
   for (int i = threadIdx.x; i < kZeroTile / 4; i += blockDim.x) ztile[i] = 0.0f;
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // tile visible to the bulk-copy engine
@@ -452,43 +619,101 @@ __global__ void __launch_bounds__(256) k_jacobian(JacArgs a) {
   const int qstep = Q >= kCT ? kCT : Q, gstep = Q >= kCT ? 1 : kCT / Q;
   const int q0 = Q >= kCT ? tid : tid % Q;
   const int g0t = Q >= kCT ? 0 : (tid < gstep * Q ? tid / Q : 1 << 30);
-  for (;;) {
-    if (tid == 0) s_c = atomicAdd(a.counter, 1);
-    compute_bar(kCT);
-    const int64_t c = s_c;
-    if (c >= a.n_centres) break;
-    const int64_t p0 = a.pair_off[c];
-    const int nent = a.ent_cnt[c];
-    const unsigned long long* keys = a.ent + (size_t)a.ent_mult * p0;
+  const int ntasks = a.counter[2];
+  const int NF = N * (L + 1), SNK = S * N * K;
+  auto claim = [&]() {
+    const int t = atomicAdd(a.counter, 1);
+    return t < ntasks ? a.tasks[t] : make_int4(-1, 0, 0, 0);
+  };
+  auto keys_of = [&](const int4& t) {
+    return a.ent + (((unsigned long long)(unsigned)t.w << 32) | (unsigned)t.z);
+  };
+  if (tid == 0) s_task[0] = claim();
+  compute_bar(kCT);
+  int4 task = s_task[0];
+  if (task.x >= 0 && tid < min(task.y, a.eb)) {
+    s_key[tid] = keys_of(task)[tid];
+    s_pair[tid] = a.pairs[a.pair_off[task.x] + (int)(s_key[tid] & 0xffffffffu)];
+  }
+  for (int it = 1; task.x >= 0; it ^= 1) {
+    const int64_t c = task.x;
+    const int nent = task.y;
+    const unsigned long long* keys = keys_of(task);
+    int4 next = make_int4(-1, 0, 0, 0);
+    if (tid == 0) next = claim();
+    for (int i = tid; i < SNK; i += kCT) copy_async(cs + (i / K) * KC + (i % K), a.coeff + (size_t)c * SNK + i);
     const int catom = a.attach ? a.centre_atom[c] : -1;
     const int crow = (catom >= 0) ? a.inc_row[catom] : -1;
-    const int SNK = S * N * K;
-    for (int i = tid; i < SNK; i += kCT) cs[(i / K) * KC + (i % K)] = a.coeff[(size_t)c * SNK + i];
-    compute_bar(kCT);
     float* obase = a.out + (size_t)c * a.n_inc * 3 * F;
-    int last_row = -1;
-    for (int b0 = 0; b0 < nent; b0 += a.eb) {
-      const int nb = min(a.eb, nent - b0);
-      stage_entries<L>(a, p0, keys, b0, nb, crow, cs, ed, EF, s_sqrt_pref, tid, kCT);
-      if (tid == 0) {  // row groups of this batch
-        int ng = 0, prev = -1;
-        for (int i = 0; i < nb; ++i) {
-          const int row = (int)(keys[b0 + i] >> 32);
-          if (row != prev) { s_gstart[ng++] = i; prev = row; }
-        }
-        s_gstart[ng] = nb;
-        s_ng = ng;
-      }
+    if (nent < 0) {
+      copy_async_wait();  // cs: visible to all after centre_row's first barrier
+      centre_row<L>(a, a.pair_off[c], keys, -nent, cs, ed, obase + (size_t)crow * 3 * F, s_sqrt_pref, tid, kCT);
+      if (tid == 0) s_task[it] = next;
       compute_bar(kCT);
+      task = s_task[it];
+      if (task.x >= 0 && tid < min(task.y, a.eb)) {
+        s_key[tid] = keys_of(task)[tid];
+        s_pair[tid] = a.pairs[a.pair_off[task.x] + (int)(s_key[tid] & 0xffffffffu)];
+      }
+      continue;
+    }
+    int last_row = -1;
+    for (int b0 = 0; b0 == 0 || b0 < nent; b0 += a.eb) {
+      const int nb = min(a.eb, nent - b0);
+      const bool in = tid < nb;
+      int row = -1;
+      float4 pr = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (in) {
+        unsigned long long key;
+        if (b0 == 0) {
+          key = s_key[tid];
+          pr = s_pair[tid];
+        } else {  // a row with more entries than one batch holds
+          key = keys[b0 + tid];
+          pr = a.pairs[a.pair_off[c] + (int)(key & 0xffffffffu)];
+        }
+        row = (int)(key >> 32);
+      }
+      if (tid < 32) {  // row groups of this batch (eb <= 32: one lane per entry)
+        const int prev = __shfl_up_sync(0xffffffffu, row, 1);
+        const unsigned starts = __ballot_sync(0xffffffffu, in && (tid == 0 || row != prev));
+        if ((starts >> tid) & 1u) {
+          const int g = __popc(starts & ((1u << tid) - 1u));
+          s_gstart[g] = tid;
+          s_grow[g] = row;
+        }
+        if (tid == 0) {
+          s_ng = __popc(starts);
+          s_gstart[__popc(starts)] = nb;
+        }
+      }
+      if (in) stage_harmonics<L>(a, pr, a.attach && row == crow, ed + (size_t)tid * EF);
+      if (b0 == 0 && tid == 0) s_task[it] = next;
+      compute_bar(kCT);
+      if (b0 == 0 && tid < 32 && s_task[it].x >= 0) {
+        const int4 tn = s_task[it];
+        if (tid < min(tn.y, a.eb)) copy_async(&s_key[tid], keys_of(tn) + tid);
+        if (tid == 0) copy_async(&s_p0, a.pair_off + tn.x);
+      }
+      stage_radial(a, nb, ed, EF, NF, tid, kCT);
+      copy_async_wait();
+      compute_bar(kCT);
+      if (b0 == 0 && s_task[it].x >= 0 && tid < min(s_task[it].y, a.eb))
+        copy_async(&s_pair[tid], a.pairs + s_p0 + (int)(s_key[tid] & 0xffffffffu));
+      if (a.mode == SOAPB_OUT_PS) {
+        stage_vectors<L>(a, nb, cs, ed, EF, s_sqrt_pref, tid, kCT);
+        compute_bar(kCT);
+      }
       const int ng = s_ng;
       for (int q = q0; q < Q; q += qstep) {
+        QuadCode qc;
+        quad_decode<L>(a, q, qc);
         for (int g = g0t; g < ng; g += gstep) {
-          const int g0 = s_gstart[g], g1 = s_gstart[g + 1];
-          const int row = (int)(keys[b0 + g0] >> 32);
-          const bool cont = (g == 0 && row == last_row);  // continues from the previous batch
+          const int grow = s_grow[g];
+          const bool cont = (g == 0 && grow == last_row);  // continues from the previous batch
           float v[3][4];
-          quad_values<L>(a, ed, EF, g0, g1, q, v);
-          float* orow = obase + (size_t)row * 3 * F;
+          quad_values<L>(a, ed, EF, s_gstart[g], s_gstart[g + 1], qc, v);
+          float* orow = obase + (size_t)grow * 3 * F;
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
             float* p = orow + d * F + 4 * q;
@@ -505,11 +730,13 @@ __global__ void __launch_bounds__(256) k_jacobian(JacArgs a) {
           }
         }
       }
-      last_row = (int)(keys[b0 + nb - 1] >> 32);
-      compute_bar(kCT);  // staged entries are rewritten by the next batch
+      last_row = ng > 0 ? s_grow[ng - 1] : -1;
+      copy_async_wait();
+      compute_bar(kCT);  // staged entries, groups and cs are rewritten by the next batch
     }
+    task = s_task[it];
   }
-  // centre queue empty: this warp joins the zero-row stream
+  // task queue empty: this warp joins the zero-row stream
   if (vec) jac_zero_rows_tma(a, ztile, a.counter + 1);
 }
 
@@ -518,15 +745,17 @@ __global__ void __launch_bounds__(256) k_jacobian(JacArgs a) {
 // ---------------------------------------------------------------------------
 
 struct JacLayout {
-  int64_t counter, ent_cnt, ent, ent_tmp, bitmap, total;
+  int64_t counter, tasks, ent, ent_tmp, bitmap, total;
 };
+
+constexpr int kMinBatch = 4;  // smallest eb (staged entries per task)
 
 static JacLayout jac_layout(int64_t n_centres, int64_t n_pairs, int64_t n_inc, int attach) {
   JacLayout L{};
   int64_t off = 0;
   auto take = [&](int64_t bytes) { const int64_t o = off; off = align_up(off + bytes, 256); return o; };
   L.counter = take(16);
-  L.ent_cnt = take(4 * n_centres);
+  L.tasks = take(16 * ((attach ? 2 : 1) * n_pairs / kMinBatch + n_centres));
   L.ent = take(8 * (attach ? 2 : 1) * (n_pairs > 0 ? n_pairs : 1));
   L.ent_tmp = take(8 * (attach ? 2 : 1) * (n_pairs > 0 ? n_pairs : 1));
   L.bitmap = take(4 * ((n_centres * n_inc + 31) / 32));
@@ -546,12 +775,25 @@ struct JacDispatch {
   static int run(JacArgs a, cudaStream_t st) {
     using Sh = JacShape<L>;
     const int nsm = sm_count();
-    // 1. entries + bitmap
+    int rc;
+    const int EF = Sh::entry_floats(a.N, a.S, a.mode);
+    const size_t base = kZeroTile + 4 * (size_t)Sh::cs_floats(a.N, a.S);
+    const size_t budget = 56 * 1024;  // four CTAs per SM
+    int eb = base < budget ? (int)((budget - base) / (4 * (size_t)EF)) : 0;
+    eb = eb > 32 ? 32 : eb;
+    if (eb < kMinBatch) eb = kMinBatch;
+    a.eb = eb;
+    a.centre_eb = 0;
+    if (a.attach) {  // what the batch buffer leaves beside D, if it is worth having
+      const int left = eb * EF - ((3 * a.S * a.N * Sh::K + 3) & ~3), ceb = left > 0 ? left / Sh::xoff(a.N) : 0;
+      if (ceb >= kMinBatch) a.centre_eb = ceb > 224 ? 224 : ceb;
+    }
+    // 1. entries, bitmap and tasks
     {
       const size_t smem = 8 * (size_t)a.cap;
       auto kern = k_jac_entries;
-      int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                          "entries smem attribute");
+      rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                      "entries smem attribute");
       if (rc) return rc;
       int occ = 1;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, smem);
@@ -561,14 +803,6 @@ struct JacDispatch {
       if ((rc = check_launch("k_jac_entries"))) return rc;
     }
     // 2. one launch: in every block warp 0 streams zero rows, warps 1..7 compute
-    int rc;
-    const int EF = Sh::entry_floats(a.N, a.S, a.mode);
-    const size_t base = kZeroTile + 4 * (size_t)Sh::cs_floats(a.N, a.S);
-    const size_t budget = 56 * 1024;  // four CTAs per SM
-    int eb = base < budget ? (int)((budget - base) / (4 * (size_t)EF)) : 0;
-    eb = eb > 32 ? 32 : eb;
-    if (eb < 4) eb = 4;
-    a.eb = eb;
     const size_t smem = base + 4 * (size_t)eb * EF;
     if (smem > 220 * 1024) return set_error(SOAPB_ERR_UNSUPPORTED, "jacobian shared memory %zu B too large", smem);
     auto kern = k_jacobian<L>;
@@ -630,7 +864,7 @@ extern "C" int soapb_jacobian(const soapb_basis* b, int64_t n_centres, const int
   a.out = d_out;
   a.status = d_status;
   a.counter = (int*)(w + Lw.counter);
-  a.ent_cnt = (int*)(w + Lw.ent_cnt);
+  a.tasks = (int4*)(w + Lw.tasks);
   a.ent = (unsigned long long*)(w + Lw.ent);
   a.ent_tmp = (unsigned long long*)(w + Lw.ent_tmp);
   a.bitmap = (unsigned int*)(w + Lw.bitmap);

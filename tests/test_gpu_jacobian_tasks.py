@@ -1,0 +1,70 @@
+"""The Jacobian's compute tasks: whole rows in batches of staged entries, rows
+with more entries than a batch (images of a tiny cell), and the row of a centre
+that moves with its atom."""
+import numpy as np
+import pytest
+import torch
+
+from cusoap_b200 import workloads as W
+from oracle.soap_oracle import OracleSOAP, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# FP32 values (2^-24 relative each) summed over at most some hundred edges, relative to the block
+TOL = 1e-5
+
+BASES = [dict(r_cut=5.0, n_max=4, l_max=3, sigma=0.5), dict(r_cut=4.0, n_max=3, l_max=2, sigma=0.5),
+         dict(r_cut=4.0, n_max=8, l_max=6, sigma=0.5), dict(r_cut=3.0, n_max=10, l_max=9, sigma=0.5)]
+
+
+def _soap(**kw):
+    from cusoap_b200 import SOAP
+    return SOAP(species=[1, 8], **kw)
+
+
+@pytest.mark.parametrize("average", ["off", "cc"])
+@pytest.mark.parametrize("basis", BASES)
+def test_fixed_centres_vs_oracle(basis, average):
+    s = W.water_cluster(3, 3, 3, seed=4)
+    centres, include = [0, 40, 80], [0, 3, 4, 40, 41, 77, 80]
+    J = _soap(average=average, **basis).derivatives(s, centers=centres, include=include, return_descriptor=False)
+    Jo, _ = OracleSOAP(species=[1, 8], average=average, **basis).derivatives(
+        s["positions"], s["atomic_numbers"], centers=centres, include=include)
+    for k in range(3):
+        assert rel_l2(J[k].cpu().numpy(), Jo[k]) < TOL
+
+
+def _structure(kind):
+    if kind == "cluster":
+        return W.water_cluster(4, 4, 4, seed=2)
+    if kind == "tiny":  # every atom of the cell many times within the cutoff
+        return {"positions": np.array([[0.0, 0.0, 0.0], [1.1, 0.9, 1.3], [0.2, 1.9, 0.4]]),
+                "atomic_numbers": np.array([8, 1, 1]), "pbc": [True] * 3,
+                "cell": np.array([[2.9, 0.0, 0.0], [0.3, 3.0, 0.0], [0.1, -0.2, 3.1]])}
+    return W.water_box(20, 8.5, seed=3)
+
+
+@pytest.mark.parametrize("average", ["off", "cc"])
+@pytest.mark.parametrize("kind", ["cluster", "tiny", "box"])
+@pytest.mark.parametrize("basis", BASES)
+def test_moving_centres(basis, kind, average):
+    """With attached centres the rows of a centre sum to zero, the other rows
+    are those of fixed centres, and an excluded centre atom leaves them so."""
+    s = _structure(kind)
+    soap = _soap(average=average, periodic=kind != "cluster", **basis)
+    n = len(s["atomic_numbers"])
+    centres = [0, 1, n - 1]
+    Ja = soap.derivatives(s, centers=centres, attach=True, return_descriptor=False).double()
+    Jf = soap.derivatives(s, centers=centres, return_descriptor=False).double()
+    inc = [i for i in range(n) if i != 1]
+    Jx = soap.derivatives(s, centers=centres, include=inc, attach=True, return_descriptor=False).double()
+    for k, c in enumerate(centres):
+        scale = Ja[k].abs().sum(0).norm()
+        assert Ja[k].sum(0).norm() <= TOL * scale
+        rest = [i for i in range(n) if i != c]
+        assert (Ja[k, rest] - Jf[k, rest]).norm() <= TOL * Jf[k, rest].norm()
+        keep = [i for i in inc if i != c]
+        assert (Jx[k, [inc.index(i) for i in keep]] - Ja[k, keep]).norm() <= TOL * Ja[k, keep].norm()
+    # the centre whose atom is left out has no centre row; the others keep theirs
+    assert (Jx[0, 0] - Ja[0, 0]).norm() <= TOL * Ja[0, 0].norm()
+    assert torch.isfinite(Jx).all()
