@@ -45,6 +45,7 @@ struct BasisDev {
   double* beta;
   const double* poly;  // rx[Q] | wr[Q] | g[N][Q]
   float* tab_b;
+  float* tab_p;   // pair-interleaved copy of tab_b (pair_coef)
   float* tab_bh;
   float* tabf;     // function-major [fn][2 nseg][8]: w B on half-width segments
   float* selfv;    // w0 B_nl(0) per function fn = l N + n
@@ -298,6 +299,14 @@ __global__ void __launch_bounds__(512) k_basis_build(BasisDev a) {
     }
     cheb_to_mono(f, a.tabf + ((size_t)fn * force_tab_stride(a.nseg) + seg) * kNCoef);
   }
+  __syncthreads();
+  for (int i = tid; N <= 8 && i < a.nseg * NF; i += blockDim.x) {  // i = seg NF + l N + n
+    const int seg = i / NF, fn = i % NF, l = fn / N, n = fn % N, NP = stream_lanes(N);
+    for (int k = 0; k < kNCoef; ++k) {
+      const int c = pair_coef(l, L, k);
+      a.tab_p[(size_t)seg * NP * (L + 1) * kNCoef + (c / 4 * NP + n) * 4 + c % 4] = a.tab_b[(size_t)i * kNCoef + k];
+    }
+  }
   // self values: the centre's own Gaussian, w0 B_nl(0) (SG:765-819)
   for (int fn = tid; fn < NF; fn += blockDim.x) {
     double b, bh;
@@ -462,7 +471,7 @@ extern "C" int soapb_basis_plan(soapb_basis* b) {
   int64_t off = 0;
   b->off_alpha = off; off = align_up(off + 8 * (int64_t)NF, 256);
   b->off_beta = off; off = align_up(off + 8 * (int64_t)NF * N, 256);
-  b->off_tab_b = off; off = align_up(off + 4 * (int64_t)b->n_seg * NF * kNCoef, 256);
+  b->off_tab_b = off; off = off_tab_pairs(b) + tab_pairs_bytes(b);
   b->off_tab_bh = off; off = align_up(off + 4 * (int64_t)b->n_seg * NF * kNCoef, 256);
   b->off_ftab = off; off = align_up(off + 4 * (int64_t)b->n_feat_ps, 256);
   b->off_widx = off; off = align_up(off + 4 * (int64_t)(L + 1) * (S * N) * (S * N), 256);
@@ -496,6 +505,7 @@ extern "C" int soapb_basis_build(soapb_basis* b, void* dev_buf, void* stream) {
   a.beta = (double*)(base + b->off_beta);
   a.poly = (const double*)(base + b->off_poly);
   a.tab_b = (float*)(base + b->off_tab_b);
+  a.tab_p = (float*)(base + off_tab_pairs(b));
   a.tab_bh = (float*)(base + b->off_tab_bh);
   a.tabf = (float*)(base + b->off_tabf);
   a.selfv = (float*)(base + b->off_self);

@@ -73,6 +73,50 @@ __device__ __forceinline__ void load_coef(const float* __restrict__ tab, int seg
   a[4] = v.x; a[5] = v.y; a[6] = v.z; a[7] = v.w;
 }
 
+// Pair-interleaved radial table of the radial-index-lane descriptor, behind
+// tab_b.  The (l_max + 1) kNCoef coefficients of a radial index n in a segment
+// are ordered as operands of packed FMAs: the l pairs (l_max, l_max - 1),
+// (l_max - 2, l_max - 3), ... interleaved coefficient by coefficient {a_0(hi),
+// a_0(lo), a_1(hi), ...}, then l = 0 alone when l_max is even.  Segments hold
+// them as [16-byte chunk][n][4 floats], n padded to the lanes of a stream: the
+// lanes load a chunk from consecutive addresses, at immediate offsets.
+__host__ __device__ inline int stream_lanes(int N) { return N <= 4 ? 4 : 8; }
+inline int64_t off_tab_pairs(const soapb_basis* b) {
+  return b->off_tab_b + align_up(4 * (int64_t)b->n_seg * b->n_max * (b->l_max + 1) * kNCoef, 256);
+}
+inline int64_t tab_pairs_bytes(const soapb_basis* b) {  // built for n_max <= 8
+  return b->n_max > 8 ? 0 : align_up(4 * (int64_t)b->n_seg * stream_lanes(b->n_max) * (b->l_max + 1) * kNCoef, 256);
+}
+// Position of coefficient k of l among a radial index's coefficients.
+__host__ __device__ inline int pair_coef(int l, int L, int k) {
+  const int p = (L - l) >> 1;  // pair index, l = L - 2p (first) or L - 2p - 1 (second)
+  return (L % 2 == 0 && l == 0) ? L * kNCoef + k : 2 * p * kNCoef + 2 * k + ((L - l) & 1);
+}
+
+// ---- packed FP32 ----
+// Two FP32 values in a register pair.  fma2 is two IEEE FMAs in one issue slot
+// (the FMA pipe's rate is that of scalar FMAs, measured 68 against 62-65
+// TFLOP/s, so it pays where instruction issue is the bound).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // Segment index and local coordinate t in [-1, 1] of radius r.
 __device__ __forceinline__ void seg_coord(float r, float inv_h, int nseg, int& seg, float& t) {
   float u = r * inv_h;
@@ -207,6 +251,69 @@ struct SolidHarmonics {
     }
   }
 };
+
+// Real solid harmonics without their normalisation: R_lm = norm(l, m) R'_lm
+// with R'_l^{+-m} = q_l^m {Re, Im}(x + i y)^m and q_l^m monic in z,
+//   q_m^m = 1, q_{m+1}^m = z, q_l^m = z q_{l-1}^m - b r^2 q_{l-2}^m,
+//   b = (l+m-1)(l-m-1) / ((2l-1)(2l-3)).
+// A kernel that sums over neighbours applies norm once per sum: 42 instead of
+// 98 operations per vector at l_max 4.
+template <int L>
+struct MonicHarmonics {
+  template <class Store>
+  __device__ __forceinline__ static void values(float x, float y, float z, float r2, Store&& store) {
+    float C = 1.0f, S = 0.0f;
+#pragma unroll
+    for (int m = 0; m <= L; ++m) {
+      if (m == 1) {
+        C = x;
+        S = y;
+      } else if (m > 1) {
+        const float Cn = x * C - y * S;
+        S = x * S + y * C;
+        C = Cn;
+      }
+      float q2 = 0.0f, q1 = 0.0f, q = 1.0f;
+#pragma unroll
+      for (int l = m; l <= L; ++l) {
+        if (l == m + 1) {
+          q = z;
+        } else if (l > m + 1) {
+          const float b = (float)((l + m - 1) * (l - m - 1)) / (float)((2 * l - 1) * (2 * l - 3));
+          q = (l == m + 2) ? fmaf(-b, r2, z * z) : fmaf(-b, r2 * q2, z * q1);
+        }
+        if (m == 0) {
+          store(l * l + l, q);
+        } else {
+          store(l * l + l + m, l == m ? C : q * C);
+          store(l * l + l - m, l == m ? S : q * S);
+        }
+        q2 = q1;
+        q1 = q;
+      }
+    }
+  }
+};
+namespace detail {
+// norm(l, m) = N_lm x leading coefficient of Q_l^m in z, index l^2 + l + m
+struct MonicNorm {
+  float v[(kMaxL + 1) * (kMaxL + 1)];
+};
+constexpr MonicNorm make_monic_norm() {
+  MonicNorm t{};
+  for (int m = 0; m <= kMaxL; ++m) {
+    double lead = 1.0;
+    for (int k = 2 * m - 1; k > 0; k -= 2) lead *= (double)k;
+    for (int l = m; l <= kMaxL; ++l) {
+      if (l > m) lead *= (2.0 * l - 1.0) / (l - m);
+      const double base = (2.0 * l + 1.0) / (4.0 * kPi) * (m == 0 ? 1.0 : 2.0) * cfact(l - m) / cfact(l + m);
+      t.v[l * l + l + m] = t.v[l * l + l - m] = (float)(csqrt(base) * lead);
+    }
+  }
+  return t;
+}
+}  // namespace detail
+__device__ constexpr detail::MonicNorm kMonicNorm = detail::make_monic_norm();
 
 // Dispatch a functor templated on l_max (0..kMaxL).
 template <template <int> class F, class... Args>

@@ -31,10 +31,11 @@ struct DescArgs {
   const float4* pairs;
   int64_t n_centres;
   const float* tab_b;
+  const float* tab_p;  // pair-interleaved table (radial-index lanes)
   const float* selfv;  // w0 B_nl(0): value of r = 0 edges (the centre's own Gaussian)
   float* out;
   float* coeff_out;  // optional raw c[s][n][lm] rows (S N K floats per centre)
-  int* counter;
+  int* counter;        // work queue; nullptr: at least as many warps as centres, one each
   int N, S, nseg, F, mode, crossover;
   float inv_h;
   float self_ratio;  // w0 / w(0): an r = 0 edge's table value times this is its self value
@@ -245,10 +246,17 @@ __device__ __forceinline__ void descriptor_body(const DescArgs& a) {
     selfb[g] = (active && n < N) ? __ldg(a.selfv + fn_index(n, lme, N)) : 0.0f;
   }
 
+  bool first = true;
   for (;;) {
-    int c32 = 0;
-    if (lane == 0) c32 = atomicAdd(a.counter, 1);
-    const int64_t c = __shfl_sync(0xffffffffu, c32, 0);
+    int64_t c;
+    if (a.counter) {
+      int c32 = 0;
+      if (lane == 0) c32 = atomicAdd(a.counter, 1);
+      c = __shfl_sync(0xffffffffu, c32, 0);
+    } else {
+      c = first ? (int64_t)blockIdx.x * (blockDim.x >> 5) + wid : a.n_centres;
+      first = false;
+    }
     if (c >= a.n_centres) break;
     for (int i = lane; i < cbn; i += 32) cbuf[i] = 0.0f;
     float acc[GN][M];
@@ -370,21 +378,69 @@ __global__ void __launch_bounds__(128, 4) k_descriptor_2s(DescArgs a) {
   descriptor_body<L, GN, 2>(a);
 }
 
+// Order of the (l, m) slots in the rows of the radial-index-lane kernel:
+// slots are the operands of packed FMAs, so the row is made of pairs (lm, lm')
+// whose radial functions sit in one register pair.  The l pairs (L, L - 1),
+// (L - 2, L - 3), ... of the interleaved table give 2 lo + 1 slot pairs each
+// and leave two slots of their larger l; the leftovers of two l pairs are
+// paired with each other, those of a last one among themselves, and l = 0 is
+// the single last slot when L is even.  With plain order, half of the pairs
+// would mix neighbouring l and need two moves each to assemble an operand.
+template <int L>
+struct YOrder {
+  static constexpr int K = (L + 1) * (L + 1), NS = K / 2;  // NS packed slots, K odd: one scalar (lm = 0)
+  static constexpr int NLP = (L + 1) / 2;                  // l pairs
+  int lm[K];   // lm at each position
+  int pos[K];  // position of each lm
+  constexpr YOrder() : lm(), pos() {
+    int i = 0;
+    for (int p = 0; p < NLP; ++p) {
+      const int hi = L - 2 * p, lo = hi - 1;
+      for (int m = 0; m < 2 * lo + 1; ++m) {
+        lm[i++] = hi * hi + m;
+        lm[i++] = lo * lo + m;
+      }
+    }
+    for (int p = 0; p + 1 < NLP; p += 2)
+      for (int k = 0; k < 2; ++k) {
+        const int h0 = L - 2 * p, h1 = L - 2 * p - 2;
+        lm[i++] = h0 * h0 + 2 * h0 - 1 + k;
+        lm[i++] = h1 * h1 + 2 * h1 - 1 + k;
+      }
+    if (NLP % 2 == 1) {
+      const int h = L - 2 * (NLP - 1);
+      lm[i++] = h * h + 2 * h - 1;
+      lm[i++] = h * h + 2 * h;
+    }
+    if (K % 2 == 1) lm[i++] = 0;
+    for (int k = 0; k < K; ++k) pos[lm[k]] = k;
+  }
+  static constexpr int l_of(int lm_) {
+    int l = 0;
+    while ((l + 1) * (l + 1) <= lm_) ++l;
+    return l;
+  }
+};
+template <int L>
+__device__ constexpr YOrder<L> kYOrder{};
+
 // Epilogue of the radial-index-lane kernel: coefficient rows KR = K4 floats
-// apart (16-byte aligned).  For the power spectrum each lane takes one (n, n')
-// pair of a species block and walks every l with compile-time m loops,
-// reading the two rows as float4; for each l the lanes write consecutive
+// apart (16-byte aligned), slots in YOrder.  For the power spectrum each lane
+// takes one (n, n') pair of a species block and contracts the two rows with
+// packed FMAs, reading them as float4; for each l the lanes write consecutive
 // features (coalesced).  Same outputs and DScribe order as desc_epilogue.
 template <int L, int KR>
 __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, const float* cbuf, int lane,
-                                                const float* s_pref, const int* s_blk, const unsigned char* s_tri) {
+                                                const float* s_pref, const int* s_blk, const unsigned char* s_tri,
+                                                const unsigned char* s_pos) {
   constexpr int K = (L + 1) * (L + 1);
+  using YO = YOrder<L>;
   const int N = a.N, S = a.S;
   if (a.coeff_out) {
     float* crow = a.coeff_out + (size_t)c * S * N * K;
     for (int f = lane; f < S * N * K; f += 32) {
       const int sn = f / K;
-      crow[f] = cbuf[sn * KR + (f - sn * K)];
+      crow[f] = cbuf[sn * KR + s_pos[f - sn * K]];
     }
   }
   float* orow = a.out + (size_t)c * a.F;
@@ -400,7 +456,7 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
         if (lm >= 1 && lm <= 3) src = (lm == 3) ? 1 : lm + 1;
         if (lm >= 4) scale = pi_m15;
       }
-      orow[f] = cbuf[sn * KR + src] * scale;
+      orow[f] = cbuf[sn * KR + s_pos[src]] * scale;
     }
     return;
   }
@@ -419,27 +475,47 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
         n = p / N;
         nd = p - n * N;
       }
-      const float4* x4 = reinterpret_cast<const float4*>(cbuf + (j * N + n) * KR);
-      const float4* y4 = reinterpret_cast<const float4*>(cbuf + (jd * N + nd) * KR);
+      const ulonglong2* x2 = reinterpret_cast<const ulonglong2*>(cbuf + (j * N + n) * KR);
+      const ulonglong2* y2 = reinterpret_cast<const ulonglong2*>(cbuf + (jd * N + nd) * KR);
+      // sums of slot pairs with the same two l: one per l pair of the table, then the leftovers
+      constexpr int NLP = YO::NLP, NSUM = NLP + (NLP + 1) / 2;
+      f32x2 sum[NSUM > 0 ? NSUM : 1];
+#pragma unroll
+      for (int k = 0; k < NSUM; ++k) sum[k] = 0ull;
+      float s0 = 0.0f;
+#pragma unroll
+      for (int q = 0; q < (K + 3) / 4; ++q) {
+        const ulonglong2 u = x2[q], v = y2[q];
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const int i = 2 * q + hh;  // slot pair
+          if (i < YO::NS) {
+            const int la = YO::l_of(kYOrder<L>.lm[2 * i]), lb = YO::l_of(kYOrder<L>.lm[2 * i + 1]);
+            const int k = (lb == la - 1) ? (L - la) / 2 : NLP + (L - la) / 4;
+            sum[k] = fma2(hh ? u.y : u.x, hh ? v.y : v.x, sum[k]);
+          } else if (K % 2 == 1 && i == YO::NS) {
+            float xa, xb, ya, yb;
+            unpack2(hh ? u.y : u.x, xa, xb);
+            unpack2(hh ? v.y : v.x, ya, yb);
+            s0 = xa * ya;
+          }
+        }
+      }
+      float sl[L + 1];
+      sl[0] = s0;
+#pragma unroll
+      for (int k = 0; k < NLP; ++k) unpack2(sum[k], sl[L - 2 * k], sl[L - 2 * k - 1]);
+#pragma unroll
+      for (int k = NLP; k < NSUM; ++k) {
+        const int ha = L - 4 * (k - NLP), hb = (2 * (k - NLP) + 1 < NLP) ? ha - 2 : ha;
+        float xa, xb;
+        unpack2(sum[k], xa, xb);
+        sl[ha] += xa;
+        sl[hb] += xb;
+      }
       float* o = orow + fb0 + p;
 #pragma unroll
-      for (int l = 0; l <= L; ++l) {
-        const int q0 = (l * l) / 4, q1 = ((l + 1) * (l + 1) - 1) / 4;  // float4 chunks holding slots l^2..(l+1)^2-1
-        float xv[16], yv[16];
-#pragma unroll
-        for (int q = q0; q <= q1; ++q) {
-          const float4 u = x4[q], v = y4[q];
-          xv[4 * (q - q0)] = u.x; xv[4 * (q - q0) + 1] = u.y; xv[4 * (q - q0) + 2] = u.z; xv[4 * (q - q0) + 3] = u.w;
-          yv[4 * (q - q0)] = v.x; yv[4 * (q - q0) + 1] = v.y; yv[4 * (q - q0) + 2] = v.z; yv[4 * (q - q0) + 3] = v.w;
-        }
-        float acc = 0.0f;
-#pragma unroll
-        for (int m = 0; m < 2 * l + 1; ++m) {
-          const int i = l * l + m - 4 * q0;
-          acc = fmaf(xv[i], yv[i], acc);
-        }
-        o[l * np] = acc * s_pref[l];
-      }
+      for (int l = 0; l <= L; ++l) o[l * np] = sl[l] * s_pref[l];
     }
   }
 }
@@ -456,6 +532,22 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
 // per lane, as rows of solid harmonics in shared memory; rows have an odd
 // stride, so the streams' reads of the same slot k from their rows hit
 // different banks and the staging writes are conflict-free.
+//
+// Instruction issue is the bound (1M atoms: 35 warp instructions per pair, of
+// which 15 are the algorithmic FMAs), so two values go into each FMA: the
+// table interleaves pairs of l, whose Horner passes run packed, and the row's
+// slots are ordered so that most slot pairs take such a register pair as it
+// is (YOrder).  The harmonics are staged without their normalisation
+// (MonicHarmonics), which the flush applies.  The pair loop is unrolled over
+// the batch and branches around the coefficient reloads: 27 warp instructions
+// per pair.  1M atoms (l_max 4): 14.65 -> 14.15 ms; 48 cells (l_max 6): 268 ->
+// 256 us; 3000 atoms (l_max 3): 73 -> 68 us.  The gain is less than the
+// instructions saved because packed and scalar FMAs with three distinct
+// operands share the register ports (2.3 - 2.7 and 1.6 - 1.9 cycles each,
+// measured) and 4 warps per scheduler leave 47 % of the issue slots to the
+// latency of the reloads and row reads.  Measured slower: the polynomials as
+// trees over t^2, t^4 (14.36 ms), two pairs per step (16.0 ms), 3 blocks per SM
+// (14.8 ms), the loop unrolled by 2 (14.7 ms).
 //
 // The r = 0 edge of the centre's own atom needs no test in the pair loop:
 // its solid harmonics are (Y00, 0, ..., 0) and its table value is
@@ -480,46 +572,119 @@ struct NShape {
   __host__ __device__ static int warp_floats(int S, int N) { return (YF + 4 * 32 + S * N * KC + 3) & ~3; }
 };
 
+// A radial-index lane's coefficients of one segment: interleaved l pairs and,
+// for even L, l = 0.
+template <int L, int NP>
+struct LaneCoefs {
+  static constexpr int NLP = (L + 1) / 2;
+  f32x2 p[NLP > 0 ? NLP : 1][kNCoef];
+  float s[kNCoef];
+  // blk: the segment's first chunk of the lane's n; chunks NP float4 apart
+  __device__ __forceinline__ void load(const float* __restrict__ blk) {
+    const ulonglong2* q = reinterpret_cast<const ulonglong2*>(blk);
+#pragma unroll
+    for (int i = 0; i < NLP; ++i)
+#pragma unroll
+      for (int k = 0; k < kNCoef; k += 2) {
+        const ulonglong2 v = __ldg(q + (i * (kNCoef / 2) + k / 2) * NP);
+        p[i][k] = v.x;
+        p[i][k + 1] = v.y;
+      }
+    if (L % 2 == 0) {
+      const float4* f = reinterpret_cast<const float4*>(blk) + NLP * (kNCoef / 2) * NP;
+      const float4 u = __ldg(f), v = __ldg(f + NP);
+      s[0] = u.x; s[1] = u.y; s[2] = u.z; s[3] = u.w;
+      s[4] = v.x; s[5] = v.y; s[6] = v.z; s[7] = v.w;
+    }
+  }
+};
+
+// A lane's accumulators, packed as its row's slots.
+template <int L>
+struct LaneSums {
+  static constexpr int K = (L + 1) * (L + 1), NS = K / 2;
+  f32x2 p[NS > 0 ? NS : 1];
+  float s;
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < NS; ++i) p[i] = 0ull;
+    s = 0.0f;
+  }
+};
+
 // One pair's contribution to a radial-index lane: the lane's l_max + 1 radial
-// functions at t (Horner), then acc[lm] += B_l R_lm over the pair's harmonic
-// row, read as float4.
-template <int L, int K4>
-__device__ __forceinline__ void accumulate_pair(float (&acc)[(L + 1) * (L + 1)], const float (&cf)[L + 1][kNCoef],
-                                                float t, const float* yrow) {
-  constexpr int K = (L + 1) * (L + 1);
-  float B[L + 1];
+// functions at t (Horner, two l per FMA), then acc[lm] += B_l R'_lm over the
+// pair's harmonic row, two slots per FMA.
+template <int L, int NP, int K4>
+__device__ __forceinline__ void accumulate_pair(LaneSums<L>& acc, const LaneCoefs<L, NP>& cf, f32x2 t2,
+                                                const float* yrow) {
+  using YO = YOrder<L>;
+  constexpr int K = YO::K, NLP = YO::NLP;
+  f32x2 B[NLP > 0 ? NLP : 1];
+  float hi[NLP > 0 ? NLP : 1], lo[NLP > 0 ? NLP : 1], b0 = 0.0f;
 #pragma unroll
-  for (int l = 0; l <= L; ++l) B[l] = horner7(cf[l], t);
-  const float4* yr = reinterpret_cast<const float4*>(yrow);
+  for (int i = 0; i < NLP; ++i) {
+    f32x2 b = cf.p[i][kDeg];
 #pragma unroll
-  for (int k4 = 0; k4 < K4 / 4; ++k4) {
-    const float4 v = yr[k4];
-    const float vv[4] = {v.x, v.y, v.z, v.w};
+    for (int k = kDeg - 1; k >= 0; --k) b = fma2(b, t2, cf.p[i][k]);
+    B[i] = b;
+    unpack2(b, hi[i], lo[i]);
+  }
+  if (L % 2 == 0) {
+    float t, t_;
+    unpack2(t2, t, t_);
+    b0 = horner7(cf.s, t);
+  }
+  const ulonglong2* yr = reinterpret_cast<const ulonglong2*>(yrow);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = 4 * k4 + i;
-      if (k < K) {
-        int l = 0;
-        while ((l + 1) * (l + 1) <= k) ++l;  // compile time: k is unrolled
-        acc[k] = fmaf(B[l], vv[i], acc[k]);
+  for (int q = 0; q < K4 / 4; ++q) {
+    const ulonglong2 v = yr[q];
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int i = 2 * q + hh;  // slot pair: compile time
+      const f32x2 y = hh ? v.y : v.x;
+      if (i < YO::NS) {
+        const int la = YO::l_of(kYOrder<L>.lm[2 * i]), lb = YO::l_of(kYOrder<L>.lm[2 * i + 1]);
+        if (lb == la - 1) {
+          acc.p[i] = fma2(B[(L - la) / 2], y, acc.p[i]);
+        } else {  // two slots of larger l left over: scalar FMAs on the halves (a packed operand would take two moves)
+          float ya, yb, sa, sb;
+          unpack2(y, ya, yb);
+          unpack2(acc.p[i], sa, sb);
+          sa = fmaf(hi[(L - la) / 2], ya, sa);
+          sb = fmaf(hi[(L - lb) / 2], yb, sb);
+          acc.p[i] = pack2(sa, sb);
+        }
+      } else if (K % 2 == 1 && i == YO::NS) {
+        float ya, yb;
+        unpack2(y, ya, yb);
+        acc.s = fmaf(b0, ya, acc.s);
       }
     }
   }
 }
 
-// Adds a lane's K accumulators to its 16-byte-aligned coefficient row (float4
-// read-modify-write; the row's K4 - K padding slots stay zero).
-template <int K, int K4>
-__device__ __forceinline__ void flush_row(float* row, const float (&acc)[K]) {
+// Adds a lane's K accumulators, times the harmonics' norms, to its
+// 16-byte-aligned coefficient row (float4 read-modify-write; the row's K4 - K
+// padding slots stay zero).
+template <int L, int K4>
+__device__ __forceinline__ void flush_row(float* row, const LaneSums<L>& acc) {
+  constexpr int K = (L + 1) * (L + 1);
   float4* r4 = reinterpret_cast<float4*>(row);
 #pragma unroll
   for (int q = 0; q < K4 / 4; ++q) {
-    float4 v = r4[q];
-    v.x += acc[4 * q];
-    if (4 * q + 1 < K) v.y += acc[4 * q + 1];
-    if (4 * q + 2 < K) v.z += acc[4 * q + 2];
-    if (4 * q + 3 < K) v.w += acc[4 * q + 3];
-    r4[q] = v;
+    const float4 v = r4[q];
+    float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int i = 2 * q + hh;
+      float x = 0.0f, y = 0.0f;
+      if (i < K / 2) unpack2(acc.p[i], x, y);
+      else if (K % 2 == 1 && i == K / 2) x = acc.s;
+      if (2 * i < K) w[2 * hh] = fmaf(x, kMonicNorm.v[kYOrder<L>.lm[2 * i]], w[2 * hh]);
+      if (2 * i + 1 < K) w[2 * hh + 1] = fmaf(y, kMonicNorm.v[kYOrder<L>.lm[2 * i + 1]], w[2 * hh + 1]);
+    }
+    r4[q] = make_float4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -531,24 +696,37 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
   __shared__ float s_pref[kMaxL + 1];
   __shared__ int s_blk[2 * kMaxBlocks];
   __shared__ unsigned char s_tri[2 * kMaxTri];
+  __shared__ unsigned char s_pos[K];  // row position of each lm
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int N = a.N, S = a.S, NF = N * (L + 1);
+  const int N = a.N, S = a.S;
   float* Y = sm + (size_t)wid * Sh::warp_floats(S, N);
-  float* tt = Y + Sh::YF;  // per staged pair: segment coordinate t, segment, species
+  // per staged pair: segment coordinate (t, t), segment, species
+  f32x2* tt = reinterpret_cast<f32x2*>(Y + Sh::YF);
   int* sg = reinterpret_cast<int*>(tt + 32);
   int* spp = sg + 32;
   float* cbuf = Y + Sh::YF + 4 * 32;
   desc_tables<L>(a, s_pref, s_blk, s_tri);
+  for (int k = threadIdx.x; k < K; k += blockDim.x) s_pos[kYOrder<L>.lm[k]] = (unsigned char)k;
   __syncthreads();
   const int h = lane / NP, n = lane - h * NP;
+  const float* tab = a.tab_p + 4 * n;  // this lane's first chunk of segment 0
+  constexpr int seg_floats = NP * (L + 1) * kNCoef;
+  bool first = true;
+  const unsigned row_mask = NP == 8 ? 0x01010101u : 0x11111111u;  // row j of every stream's block, shifted by j
   const bool active = n < N;
   const int cbn = S * N * KC;
   float4* myrow = reinterpret_cast<float4*>(Y + lane * K4 + 4 * h);  // the row this lane stages
 
   for (;;) {
-    int c32 = 0;
-    if (lane == 0) c32 = atomicAdd(a.counter, 1);
-    const int64_t c = __shfl_sync(0xffffffffu, c32, 0);
+    int64_t c;
+    if (a.counter) {
+      int c32 = 0;
+      if (lane == 0) c32 = atomicAdd(a.counter, 1);
+      c = __shfl_sync(0xffffffffu, c32, 0);
+    } else {
+      c = first ? (int64_t)blockIdx.x * (blockDim.x >> 5) + wid : a.n_centres;
+      first = false;
+    }
     if (c >= a.n_centres) break;
     for (int i = lane; i < cbn / 4; i += 32) reinterpret_cast<float4*>(cbuf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // offsets inside the centre's list are 32-bit: 2^31 pairs of one centre would be 34 GB of list
@@ -557,14 +735,9 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
     const float4* pc = a.pairs + p0;
     const int s0 = (int)(((int64_t)P * h) / H), s1 = (int)(((int64_t)P * (h + 1)) / H);  // this stream's pairs
     const int rounds = (P + H - 1) / H;                                                  // longest stream
-    float acc[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = 0.0f;
-    float cf[L + 1][kNCoef];
-#pragma unroll
-    for (int l = 0; l <= L; ++l)
-#pragma unroll
-      for (int k = 0; k < kNCoef; ++k) cf[l][k] = 0.0f;
+    LaneSums<L> acc;
+    acc.clear();
+    LaneCoefs<L, NP> cf = {};
     // each stream starts on the species of its first pair, so the centre's first batch takes the
     // fast path unless a species changes inside it
     int cur_sp = (s0 < s1) ? (int)((unsigned)__float_as_int(__ldg(&pc[s0].w)) >> kAtomBits) : -1;
@@ -587,12 +760,13 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
         const float4 pr = valid ? __ldg(pc + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         // the stream's pair of the next batch: into L1 while this batch runs
         if (e + NP < s1) asm volatile("prefetch.global.L1 [%0];" ::"l"(pc + e + NP));
-        const float r = sqrtf(pr.x * pr.x + pr.y * pr.y + pr.z * pr.z);
+        const float r2 = pr.x * pr.x + pr.y * pr.y + pr.z * pr.z;
+        const float r = sqrtf(r2);
         seg_coord(r, a.inv_h, a.nseg, seg, t);
         sp = (int)((unsigned)__float_as_int(pr.w) >> kAtomBits);
-        SolidHarmonics<L>::values(pr.x, pr.y, pr.z, [&](int idx, float v) { yv[idx] = v; });
+        MonicHarmonics<L>::values(pr.x, pr.y, pr.z, r2, [&](int idx, float v) { yv[kYOrder<L>.pos[idx]] = v; });
         // the centre's own Gaussian (r = 0): w0 B_n0(0) Y00
-        yv[0] *= valid ? ((r > 0.0f) ? 1.0f : a.self_ratio) : 0.0f;
+        yv[kYOrder<L>.pos[0]] = valid ? ((r > 0.0f) ? 1.0f : a.self_ratio) : 0.0f;
         if (!valid) {
           seg = -1;
           sp = -1;
@@ -618,24 +792,23 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
       }
       const unsigned seg_chg = __ballot_sync(0xffffffffu, seg != seg_prev);
       const unsigned sp_chg = __ballot_sync(0xffffffffu, sp != sp_prev);
-      tt[lane] = t;
+      tt[lane] = pack2(t, t);
       sg[lane] = seg;
       spp[lane] = sp;
       __syncwarp();
       if (sp_chg == 0) {
         // no species change in any stream: t, a coefficient reload where the segment changes,
         // Horner and the K FMAs per pair
-#pragma unroll 2
+#pragma unroll
         for (int j = 0; j < NP; ++j) {
           const int q = h * NP + j;
-          if ((seg_chg >> q) & 1u) {
-            const int sq = sg[q];
-            if (active) {
-#pragma unroll
-              for (int l = 0; l <= L; ++l) load_coef(a.tab_b, sq, fn_index(n, l, N), NF, cf[l]);
-            }
+          // one warp-uniform branch for the streams' reloads, kept a branch by the barrier: the ten
+          // loads of a reload are otherwise issued, predicated off, for every pair
+          if (seg_chg & (row_mask << j)) {
+            __syncwarp();
+            if (((seg_chg >> q) & 1u) && active) cf.load(tab + (size_t)sg[q] * seg_floats);
           }
-          accumulate_pair<L, K4>(acc, cf, tt[q], Y + q * K4 + 4 * h);
+          accumulate_pair<L, NP, K4>(acc, cf, tt[q], Y + q * K4 + 4 * h);
         }
       } else {
 #pragma unroll 1
@@ -647,23 +820,19 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
             for (int hh = 0; hh < H; ++hh) {  // streams flush one after the other
               if (h == hh && spq != cur_sp) {
                 if (cur_sp >= 0 && active) {
-                  flush_row<K, K4>(cbuf + (cur_sp * N + n) * KC, acc);
+                  flush_row<L, K4>(cbuf + (cur_sp * N + n) * KC, acc);
                 }
-#pragma unroll
-                for (int k = 0; k < K; ++k) acc[k] = 0.0f;
+                acc.clear();
                 cur_sp = spq;
               }
               __syncwarp();
             }
           }
-          if ((seg_chg >> q) & 1u) {
-            const int sq = sg[q];
-            if (active) {
-#pragma unroll
-              for (int l = 0; l <= L; ++l) load_coef(a.tab_b, sq, fn_index(n, l, N), NF, cf[l]);
-            }
+          if (seg_chg & (row_mask << j)) {
+            __syncwarp();
+            if (((seg_chg >> q) & 1u) && active) cf.load(tab + (size_t)sg[q] * seg_floats);
           }
-          accumulate_pair<L, K4>(acc, cf, tt[q], Y + q * K4 + 4 * h);
+          accumulate_pair<L, NP, K4>(acc, cf, tt[q], Y + q * K4 + 4 * h);
         }
       }
       cur_seg = sg[h * NP + NP - 1];
@@ -673,11 +842,11 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
 #pragma unroll
     for (int hh = 0; hh < H; ++hh) {
       if (h == hh && cur_sp >= 0 && active) {
-        flush_row<K, K4>(cbuf + (cur_sp * N + n) * KC, acc);
+        flush_row<L, K4>(cbuf + (cur_sp * N + n) * KC, acc);
       }
       __syncwarp();
     }
-    desc_epilogue_n<L, KC>(a, c, cbuf, lane, s_pref, s_blk, s_tri);
+    desc_epilogue_n<L, KC>(a, c, cbuf, lane, s_pref, s_blk, s_tri, s_pos);
     __syncwarp();
   }
 }
@@ -709,9 +878,14 @@ static int launch_descriptor_n(const DescArgs& a, int wpb_tuned, cudaStream_t st
   if (occ < 1) occ = 1;
   int64_t blocks = (int64_t)nsm * occ;
   const int64_t need = (a.n_centres + wpb - 1) / wpb;
-  if (blocks > need) blocks = need;
-  if (blocks < 1) blocks = 1;
-  kern<<<(unsigned)blocks, 32 * wpb, smem, st>>>(a);
+  DescArgs b = a;
+  if (blocks >= need) {  // one centre per warp: no work queue to reset
+    blocks = need;
+    b.counter = nullptr;
+  } else if ((rc = check_cuda(cudaMemsetAsync(a.counter, 0, sizeof(int32_t), st), "reset work counter"))) {
+    return rc;
+  }
+  kern<<<(unsigned)blocks, 32 * wpb, smem, st>>>(b);
   return check_launch("k_descriptor_n");
 }
 
@@ -724,7 +898,10 @@ static int launch_descriptor(const DescArgs& a, int wpb_tuned, cudaStream_t st) 
   if ((wpb_tuned == 1 || wpb_tuned == 2 || wpb_tuned == 4) && wpb_tuned <= wpb) wpb = wpb_tuned;
   if (wpb < 1) return set_error(SOAPB_ERR_UNSUPPORTED, "descriptor shared memory %d B per warp too large", per_warp);
   const int smem = wpb * per_warp;
-  auto kern = (H == 2) ? k_descriptor_2s<L, GN> : k_descriptor<L, GN>;
+  auto kern = [] {
+    if constexpr (H == 2) return k_descriptor_2s<L, GN>;
+    else return k_descriptor<L, GN>;
+  }();
   int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                       "descriptor smem attribute");
   if (rc) return rc;
@@ -735,9 +912,14 @@ static int launch_descriptor(const DescArgs& a, int wpb_tuned, cudaStream_t st) 
   if (occ < 1) occ = 1;
   int64_t blocks = (int64_t)nsm * occ;
   const int64_t need = (a.n_centres + wpb - 1) / wpb;
-  if (blocks > need) blocks = need;
-  if (blocks < 1) blocks = 1;
-  kern<<<(unsigned)blocks, 32 * wpb, smem, st>>>(a);
+  DescArgs b = a;
+  if (blocks >= need) {  // one centre per warp: no work queue to reset
+    blocks = need;
+    b.counter = nullptr;
+  } else if ((rc = check_cuda(cudaMemsetAsync(a.counter, 0, sizeof(int32_t), st), "reset work counter"))) {
+    return rc;
+  }
+  kern<<<(unsigned)blocks, 32 * wpb, smem, st>>>(b);
   return check_launch("k_descriptor");
 }
 
@@ -794,6 +976,7 @@ extern "C" int soapb_descriptor(const soapb_basis* b, int64_t n_centres, const i
   a.pairs = (const float4*)d_pairs;
   a.n_centres = n_centres;
   a.tab_b = (const float*)((const char*)b->dev + b->off_tab_b);
+  a.tab_p = (const float*)((const char*)b->dev + off_tab_pairs(b));
   a.selfv = (const float*)((const char*)b->dev + b->off_self);
   a.out = d_out;
   a.coeff_out = d_coeff;
@@ -815,8 +998,6 @@ extern "C" int soapb_descriptor(const soapb_basis* b, int64_t n_centres, const i
     else if (b->weighting == SOAPB_W_EXP) w_at0 = b->w_c / (b->w_d + 1.0);
     a.self_ratio = (float)(w0 / w_at0);
   }
-  int rc = check_cuda(cudaMemsetAsync(d_counter, 0, sizeof(int32_t), st), "reset work counter");
-  if (rc) return rc;
   int gn = desc_group(N, L);
   const int tg = b->tune[1];
   if (tg > gn && (tg == 2 || tg == 3 || tg == 4 || tg == 6)) gn = tg;
