@@ -5,18 +5,19 @@
 // (:382-396) and _perpendicular_lengths (:369-379).  The reference
 // replicates every atom over all (2 n_rep + 1)^3 image offsets and runs an
 // all-pairs GEMM distance test; here atoms are binned once per structure
-// (counting sort into bins in the cell's fractional frame, periodic axes
-// wrapped) and each centre scans only the bins of its window, generating
-// images on the fly.  Diagonal frames use bins a quarter of the cutoff wide
-// and a window trimmed to the cutoff sphere (visit_fine); other frames use
-// bins of perpendicular width >= half the cutoff and a +-2 window (visit).  The image set is
-// the reference's: image offset n = T - w_atom + w_centre (T the cell-window
-// shift, w the wrap shifts) must satisfy |n_i| <= n_rep_i on periodic axes.
+// (counting sort into bins in the cell's fractional frame, a quarter of the
+// cutoff wide, periodic axes wrapped) and each centre scans only the runs of
+// bins that its cutoff sphere reaches, generating images on the fly.  The image
+// set is the reference's: image offset n = T - w_atom + w_centre (T the
+// cell-window shift, w the wrap shifts) must satisfy |n_i| <= n_rep_i on
+// periodic axes.
 //
 // Pairs of a centre are written sorted by (neighbour species, radial table
 // segment) -- the order the descriptor kernels consume them in -- and, inside
 // a key, in a deterministic candidate order (bins are sorted by atom index).
-// Distances are tested and differences taken in FP64; rvec is stored FP32.
+// Whether a candidate is within the cutoff is decided in FP64: FP32 copies of
+// the positions decide all candidates but those within their rounding of the
+// cutoff.  Differences are taken in FP64; rvec is stored FP32.
 #include <math.h>
 
 #include <mutex>
@@ -30,9 +31,18 @@ struct GridDesc {
   double Hinv[9];  // f_j = sum_i x_i Hinv[i*3+j]
   double fmin[3];  // bin origin in fractional coordinates (non-periodic axes)
   double binw[3];  // fractional bin width
-  int nb[3], win[3], nrep[3], per[3];
+  int nb[3], nrep[3];
+  signed char per[4];
   int any_per;
-  int orth;  // diagonal frame (every non-periodic structure, rectangular cells): sphere-trimmed enumeration
+  int orth;     // diagonal frame (every non-periodic structure, rectangular cells)
+  int wrapped;  // an atom has a wrap shift: pairs need the image test
+  // FP32 geometry of the window (Angstrom): perpendicular bin widths and their reciprocals; for
+  // other than diagonal frames the direction of lattice row a, the reciprocal of a bin's length
+  // along it, the edges of a bin along b and c, and the largest distance of a bin's point from
+  // the bin row's axis
+  float wp[3], iw[3], dir[3], ialong, eb[3], ec[3], rho;
+  // squared FP32 distances up to c2lo are within the cutoff, above c2hi beyond it
+  float c2lo, c2hi;
 };
 
 struct NLWork {
@@ -42,10 +52,11 @@ struct NLWork {
   int64_t* bin_off;          // (n_struct + 1)
   int* bin_count;            // (max_bins)
   int* bin_start;            // (max_bins + 1)
-  int* arrival;              // (n_atoms) order in which the atoms reached their bins
+  int* arrival;              // (n_atoms) order in which the atoms reached their bins (in sorted_f's memory)
   int* atom_bin;             // (n_atoms)
   int* sorted_atom;          // (n_atoms) atoms by bin, in arrival order inside a bin
   double4* sorted_pos;       // (n_atoms) {wrapped x, y, z, packed info} (see pack_info)
+  float4* sorted_f;          // (n_atoms) {x, y, z} of sorted_pos from the origin of coord_origin
   double4* cpos;             // (n_centres) wrapped centre positions
   int4* cinfo;               // (n_centres) {bin xyz, struct, wrap, atom}
   int* counts;               // (n_centres)
@@ -279,9 +290,9 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
     g.fmin[k] = 0.0;
     g.binw[k] = 1.0;
     g.nb[k] = 1;
-    g.win[k] = 1;
     g.nrep[k] = 0;
   }
+  g.wrapped = 0;
   g.any_per = anyp;
   g.orth = 1;
   for (int k = 0; k < 9; ++k)
@@ -373,24 +384,22 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
     perp[k] = det / (sqrt(cx * cx + cy * cy + cz * cz) + 1e-300);
   }
   const int64_t A = s.d_atom_off[i + 1] - s.d_atom_off[i];
-  // Diagonal frames: bins of width >= cutoff / 4, each window row trimmed to
-  // the cutoff sphere (visit_fine), unless a periodic x axis would get fewer
-  // than 3 bins (a row of the window would wrap into more than 4 runs).
-  // Other frames: bins of perpendicular width >= cutoff / 2 and the full
-  // +-2 window: 5^3 half-width bins hold 15.6 cutoff^3 of candidates against
-  // 27 cutoff^3 for full-width bins.
-  if (g.orth && g.per[0] && perp[0] < 0.75 * cutoff) g.orth = 0;
-  const double bin_min = (g.orth ? 0.25 : 0.5) * cutoff;
+  // Bins of perpendicular width >= cutoff / 4; every bin row of the window is
+  // trimmed to the cutoff sphere (visit).
+  const double bin_min = 0.25 * cutoff;
+  double far[3];  // largest |fractional coordinate| of a wrapped atom, from the origin of the FP32 copies
   for (int k = 0; k < 3; ++k) {
     if (g.per[k]) {
       const int nb = (int)floor(perp[k] / bin_min);
       g.nb[k] = min(max(nb, 1), 1023);
       g.fmin[k] = 0.0;
       g.binw[k] = 1.0 / g.nb[k];
+      far[k] = 1.0;
     } else {
       double lo = ord_decode(__ldcg(&w.fbox[i * 6 + k])), hi = ord_decode(__ldcg(&w.fbox[i * 6 + 3 + k]));
       if (!(hi >= lo)) { lo = 0.0; hi = 0.0; }  // no atoms
       const double span = hi - lo;
+      far[k] = g.any_per ? fmax(fabs(lo), fabs(hi)) : span;
       const int nb = (int)floor(span * perp[k] / bin_min);
       g.nb[k] = min(max(nb, 1), 1023);
       g.fmin[k] = lo;
@@ -407,16 +416,43 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
     g.nb[k] = max(1, g.nb[k] / 2);
     g.binw[k] = span / g.nb[k];
   }
-  if (g.orth && g.per[0] && g.nb[0] < 3) g.orth = 0;
   for (int k = 0; k < 3; ++k) {
-    const double bw_perp = g.binw[k] * perp[k];  // perpendicular width of one bin
-    int win = (int)ceil(cutoff / bw_perp);
-    if (!(bw_perp > 0.0)) win = 1;
-    if (!g.per[k]) win = min(win, g.nb[k]);
-    g.win[k] = max(win, 1);
+    g.wp[k] = (float)(g.binw[k] * perp[k]);
+    g.iw[k] = 1.0f / g.wp[k];
   }
+  if (!g.orth) {
+    const double la = sqrt(H[0] * H[0] + H[1] * H[1] + H[2] * H[2]);
+    double p2 = 0.0, m2 = 0.0;
+    for (int k = 0; k < 3; ++k) {
+      const double eb = g.binw[1] * H[3 + k], ec = g.binw[2] * H[6 + k];
+      g.dir[k] = (float)(la > 0.0 ? H[k] / la : 0.0);
+      g.eb[k] = (float)eb;
+      g.ec[k] = (float)ec;
+      p2 += (eb + ec) * (eb + ec);
+      m2 += (eb - ec) * (eb - ec);
+    }
+    g.ialong = (float)(1.0 / (g.binw[0] * la));
+    g.rho = (float)(0.5 * sqrt(fmax(p2, m2)) + 1e-4);
+  }
+  // FP32 test: copies of coordinates up to m, shifts up to m + cutoff and differences up to the
+  // cutoff are each rounded by 2^-24 of their size, so a component is off by at most 1.2e-7 (m +
+  // cutoff); twice that is allowed for, and the rounding of the squares
+  double m = 0.0;
+  for (int k = 0; k < 3; ++k)
+    m = fmax(m, far[0] * fabs(H[k]) + far[1] * fabs(H[3 + k]) + far[2] * fabs(H[6 + k]));
+  const double band = 3.5 * cutoff * 2.4e-7 * (m + 2.0 * cutoff) + 1e-6 * cutoff * cutoff;
+  const bool fits = band < 0.5 * cutoff * cutoff;  // false for NaN as well
+  g.c2lo = fits ? (float)(cutoff * cutoff - band) : -1.0f;
+  g.c2hi = fits ? (float)(cutoff * cutoff + band) : INFINITY;
   w.grids[i] = g;
   w.bins_per_struct[i] = g.nb[0] * g.nb[1] * g.nb[2];
+}
+
+// Origin of the FP32 coordinates: the corner of an open structure's box, else
+// the cell's (positions are wrapped into it).
+__device__ __forceinline__ void coord_origin(const GridDesc& g, double (&o)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) o[k] = g.any_per ? 0.0 : g.fmin[k];
 }
 
 __device__ __forceinline__ void bin_atom(const soapb_structs& s, const NLWork& w, int64_t a) {
@@ -426,6 +462,7 @@ __device__ __forceinline__ void bin_atom(const soapb_structs& s, const NLWork& w
   double wp[3];
   if (!locate(g, s.d_positions[3 * a], s.d_positions[3 * a + 1], s.d_positions[3 * a + 2], b, wr, wp))
     atomicOr(w.status, 2);
+  if ((wr[0] | wr[1] | wr[2]) != 0 && !g.wrapped) atomicOr(&w.grids[si].wrapped, 1);
   const int64_t gb = w.bin_off[si] + ((int64_t)b[2] * g.nb[1] + b[1]) * g.nb[0] + b[0];
   w.atom_bin[a] = (int)gb;
   w.arrival[a] = atomicAdd(&w.bin_count[gb], 1);
@@ -460,6 +497,9 @@ __device__ __forceinline__ void gather_atom(const soapb_structs& s, const NLWork
          b, wr, wp);
   w.sorted_pos[s0 + rank] =
       make_double4(wp[0], wp[1], wp[2], pack_info(a, s.d_species[a], pack3(wr[0], wr[1], wr[2])));
+  double o[3];
+  coord_origin(g, o);
+  w.sorted_f[s0 + rank] = make_float4((float)(wp[0] - o[0]), (float)(wp[1] - o[1]), (float)(wp[2] - o[2]), 0.0f);
 }
 
 // ---- large inputs: one kernel per stage ----
@@ -550,6 +590,7 @@ struct VisitArgs {
   const int64_t* bin_off;
   const int* bin_start;
   const double4* sorted_pos;
+  const float4* sorted_f;
   const double4* cpos;
   const int4* cinfo;
   int* status;
@@ -557,281 +598,323 @@ struct VisitArgs {
   int mode;
 };
 
-template <class Fn>
-__device__ __forceinline__ void visit(const VisitArgs& A, int64_t c, Fn&& fn) {
-  const int lane = threadIdx.x & 31;
-  const double4 cp = A.cpos[c];
-  const int4 ci = A.cinfo[c];
-  const GridDesc& g = A.grids[ci.y];
-  const int cb[3] = {ci.x & 1023, (ci.x >> 10) & 1023, (ci.x >> 20) & 1023};
+// Shared memory of a warp's enumeration: per nonempty run, the slot of its
+// first atom minus its place in the candidate stream, and for periodic
+// structures that place and the image shift minus the centre (FP32), packed T in w.
+struct VisitMem {
+  float4 shift[64];
+  int start[64], adj[64];
+};
+
+// The centre of a warp.
+struct VisitCentre {
+  double4 cp;
+  int atom;  // centre atom or -1
   int cw[3];
-  unpack3(ci.z, cw);
-  const int64_t boff = A.bin_off[ci.y];
-  for (int dz = -g.win[2]; dz <= g.win[2]; ++dz) {
-    int bz = cb[2] + dz, Tz = 0;
-    if (g.per[2]) { Tz = floordiv(bz, g.nb[2]); bz -= Tz * g.nb[2]; }
-    else if (bz < 0 || bz >= g.nb[2]) continue;
-    for (int dy = -g.win[1]; dy <= g.win[1]; ++dy) {
-      int by = cb[1] + dy, Ty = 0;
-      if (g.per[1]) { Ty = floordiv(by, g.nb[1]); by -= Ty * g.nb[1]; }
-      else if (by < 0 || by >= g.nb[1]) continue;
-      // the row's x bins as runs of consecutive bins with one image shift Tx:
-      // a run is one contiguous range of bin-sorted atoms
-      int dx = -g.win[0];
-      while (dx <= g.win[0]) {
-        int bx = cb[0] + dx, Tx = 0, run_end;
-        if (g.per[0]) {
-          Tx = floordiv(bx, g.nb[0]);
-          bx -= Tx * g.nb[0];
-          run_end = min(g.win[0], dx + (g.nb[0] - 1 - bx));
-        } else {
-          if (bx < 0) { dx = -cb[0]; continue; }
-          if (bx >= g.nb[0]) break;
-          run_end = min(g.win[0], g.nb[0] - 1 - cb[0]);
-        }
-        const int bx1 = bx + (run_end - dx);
-        dx = run_end + 1;
-        const double sx = Tx * g.H[0] + Ty * g.H[3] + Tz * g.H[6] - cp.x;
-        const double sy = Tx * g.H[1] + Ty * g.H[4] + Tz * g.H[7] - cp.y;
-        const double sz = Tx * g.H[2] + Ty * g.H[5] + Tz * g.H[8] - cp.z;
-        const int T[3] = {Tx, Ty, Tz};
-        const int64_t gb = boff + ((int64_t)bz * g.nb[1] + by) * g.nb[0];
-        const int64_t s0 = A.bin_start[gb + bx], s1 = A.bin_start[gb + bx1 + 1];
-        for (int64_t base = s0; base < s1; base += 32) {
-          const int64_t i = base + lane;
-          bool ok = false;
-          int atom = 0, sp = 0;
-          double rx = 0.0, ry = 0.0, rz = 0.0, r2 = 0.0;
-          if (i < s1) {
-            const double4 p = A.sorted_pos[i];
-            int wrap;
-            unpack_info(p.w, atom, sp, wrap);
-            rx = p.x + sx;
-            ry = p.y + sy;
-            rz = p.z + sz;
-            r2 = rx * rx + ry * ry + rz * rz;
-            ok = r2 <= A.cutoff2;
-            if (ok && g.any_per) {
-              int aw[3];
-              unpack3(wrap, aw);
-#pragma unroll
-              for (int k = 0; k < 3; ++k)
-                if (g.per[k]) ok &= abs(T[k] - aw[k] + cw[k]) <= g.nrep[k];
-            }
-            // create(): drop r <= 1e-12 edges except the centre's own atom (SG:1171-1179)
-            if (ok && A.mode == SOAPB_NL_CREATE && r2 <= 1e-24 && atom != ci.w) ok = false;
-          }
-          fn(ok, atom, sp, rx, ry, rz, r2);
-        }
-      }
-    }
+  const GridDesc* g;
+  bool per;
+};
+
+// One sorted-atom record through the read-only path (the lists are built by earlier kernels).
+__device__ __forceinline__ double4 load_record(const double4* p) {
+  const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+  return make_double4(a.x, a.y, b.x, b.y);
+}
+
+// rvec of the candidate in a slot with cell-window shift T, in FP64.
+__device__ __forceinline__ void exact_rvec(const VisitCentre& C, const double4& p, int Tpacked, double& rx, double& ry,
+                                           double& rz) {
+  if (!C.per) {
+    rx = p.x - C.cp.x;
+    ry = p.y - C.cp.y;
+    rz = p.z - C.cp.z;
+  } else {
+    const double* H = C.g->H;
+    int T[3];
+    unpack3(Tpacked, T);
+    rx = p.x + (T[0] * H[0] + T[1] * H[3] + T[2] * H[6] - C.cp.x);
+    ry = p.y + (T[0] * H[1] + T[1] * H[4] + T[2] * H[7] - C.cp.y);
+    rz = p.z + (T[0] * H[2] + T[1] * H[5] + T[2] * H[8] - C.cp.z);
   }
 }
 
-// Sphere-trimmed enumeration for diagonal frames (x = f diag(L)): the rows
-// (bz, by) of unwrapped bins whose slab comes within the cutoff of the
-// centre, each trimmed to the bins x that the sphere's cross-section reaches
-// (conservatively: the cutoff plus 1e-8 A).  Up to 32 rows are laid out at a
-// time, one per lane; a row's x bins are at most 4 runs of contiguous
-// bin-sorted atoms (periodic x axes have >= 3 bins).  The runs of the 32 rows
-// form one candidate stream that all lanes walk 32 at a time: a lane finds
-// its run from the run starts inside its tile (one OR-reduction and a
-// popcount).  Candidate order: z rows, then y, then x, then atom index --
-// deterministic, like the full window's.  PIPE: the candidate records of the
-// next tile are looked up and loaded while this tile is tested (the fill,
-// whose per-candidate work covers the load; the count, which has little work
-// per candidate, runs more warps instead).
-constexpr int kRunsPerPass = 128;  // 32 rows x at most 4 runs
+// Whether a candidate is a pair, in FP64: the cutoff, the image set, and for
+// create() the r <= 1e-12 edges other than the centre's own (SG:1171-1179).
+__device__ __forceinline__ bool exact_test(const VisitArgs& A, const VisitCentre& C, int slot, int Tpacked) {
+  const double4 p = load_record(A.sorted_pos + slot);
+  double rx, ry, rz;
+  exact_rvec(C, p, Tpacked, rx, ry, rz);
+  const double r2 = rx * rx + ry * ry + rz * rz;
+  if (!(r2 <= A.cutoff2)) return false;
+  int atom, sp, wrap;
+  unpack_info(p.w, atom, sp, wrap);
+  if (C.per) {
+    int T[3], aw[3];
+    unpack3(Tpacked, T);
+    unpack3(wrap, aw);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (C.g->per[k] && abs(T[k] - aw[k] + C.cw[k]) > C.g->nrep[k]) return false;
+  }
+  return !(A.mode == SOAPB_NL_CREATE && r2 <= 1e-24 && atom != C.atom);
+}
 
-template <bool PIPE, class Fn>
-__device__ __forceinline__ void visit_fine(const VisitArgs& A, int64_t c, int* runs, Fn&& fn) {
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Candidate enumeration of one centre by a warp.  The rows (by, bz) of unwrapped
+// bins within the cutoff are taken 32 at a time, one per lane, each trimmed to
+// the bins x that the cutoff sphere reaches (in FP32, against the cutoff plus
+// 1e-3 A, which covers its rounding).  A row is one run of bin-sorted atoms, or
+// in a cell periodic along x one per image Tx, two images at a time.  The runs
+// form one candidate stream that all lanes walk 32 at a time: the runs that
+// start inside a tile give one bit each (an OR-reduction), and a lane's run is
+// the number of bits up to its own.  An FP32 copy of the position settles almost every
+// candidate; those within rounding of the cutoff (or near r = 0 in create(), or
+// all of them when wrap shifts make the image set matter) take the FP64 test.
+// Order: pairs of images, z rows, y, x, then atom index -- deterministic.
+// fn(ok, slot, T) is called with all lanes.
+//
+// The enumeration is bound by instruction issue and the latency of the loads: 5
+// warp instructions per pair in the count, against 8 with FP64 row geometry
+// (six divisions and a square root a centre, one a row) and tests (1M atoms:
+// count 3.31 -> 2.2 ms; 48 periodic cells 85 -> 41 us).  Other than diagonal
+// frames scanned the full window of half-cutoff bins before, 4 candidates a
+// pair against 2 (501 atoms, triclinic: count 38 -> 19 us, fill 45 -> 23 us).
+// Writing the candidate slots of all runs into a list first, instead of finding
+// each lane's run, took as many instructions as it saved.
+template <bool PER, int UNROLL, class Fn>
+__device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, const VisitCentre& C, const int4& ci,
+                                           Fn&& fn) {
   const int lane = threadIdx.x & 31;
-  const double4 cp = A.cpos[c];
-  const int4 ci = A.cinfo[c];
-  const GridDesc& g = A.grids[ci.y];
-  int cw[3];
-  unpack3(ci.z, cw);
-  const int64_t boff = A.bin_off[ci.y];
-  const double cm = A.cutoff + 1e-8;
-  const double Lv[3] = {g.H[0], g.H[4], g.H[8]};
-  const double cv[3] = {cp.x, cp.y, cp.z};
-  // bin coordinate u = x / (L binw) - fmin / binw (reciprocals: the 1e-8 A margin covers the rounding)
-  const double ib[3] = {1.0 / (Lv[0] * g.binw[0]), 1.0 / (Lv[1] * g.binw[1]), 1.0 / (Lv[2] * g.binw[2])};
-  const double ub[3] = {g.fmin[0] / g.binw[0], g.fmin[1] / g.binw[1], g.fmin[2] / g.binw[2]};
-  // unwrapped bins of axis k that meet [x0, x1] (clamped to the grid on open axes)
-  auto brange = [&](int k, double x0, double x1, int& lo, int& hi) {
-    double u0 = fma(x0, ib[k], -ub[k]), u1 = fma(x1, ib[k], -ub[k]);
-    if (!g.per[k]) {
-      u0 = fmin(fmax(u0, -1.0), (double)g.nb[k]);
-      u1 = fmin(fmax(u1, -1.0), (double)g.nb[k]);
+  const GridDesc& g = *C.g;
+  const int cb[3] = {ci.x & 1023, (ci.x >> 10) & 1023, (ci.x >> 20) & 1023};
+  const float R = (float)A.cutoff + 1e-3f;
+  // the centre inside its bin (beyond [0, 1] for centres outside an open structure's box), and
+  // the bins, from its own, that the cutoff reaches on each axis
+  float f[3];
+  int lo[3], hi[3];
+  {
+    double fr[3];
+    if (PER) {
+      to_frac(g, C.cp.x, C.cp.y, C.cp.z, fr);
+    } else {  // the identity frame
+      fr[0] = C.cp.x;
+      fr[1] = C.cp.y;
+      fr[2] = C.cp.z;
     }
-    lo = (int)floor(u0);
-    hi = (int)floor(u1);
-    if (!g.per[k]) {
-      lo = max(lo, 0);
-      hi = min(hi, g.nb[k] - 1);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      // bins of an open axis are binw wide in the frame's coordinate: binw = wp for the identity
+      // frame; a mixed frame divides (few structures have one)
+      const double d = fr[k] - fma((double)cb[k], g.binw[k], g.fmin[k]);
+      f[k] = PER ? (float)(d / g.binw[k]) : (float)d * g.iw[k];
+      f[k] = fminf(fmaxf(f[k], -1e6f), 1e6f);
+      const float reach = fmaf(R, g.iw[k], 1e-3f);
+      lo[k] = (int)floorf(fmaxf(f[k] - reach, -1e6f));
+      hi[k] = (int)floorf(fminf(f[k] + reach, 1e6f));
+      if (!PER || !g.per[k]) {
+        lo[k] = max(lo[k], -cb[k]);
+        hi[k] = min(hi[k], g.nb[k] - 1 - cb[k]);
+      }
     }
-  };
-  // distance from the centre to the slab of unwrapped bin b on axis k
-  auto dmin = [&](int k, int b) {
-    const double lo = (g.fmin[k] + b * g.binw[k]) * Lv[k], hi = (g.fmin[k] + (b + 1) * g.binw[k]) * Lv[k];
-    return fmax(0.0, fmax(lo - cv[k], cv[k] - hi));
-  };
-  int bz0, bz1, by0, by1;
-  brange(2, cp.z - cm, cp.z + cm, bz0, bz1);
-  brange(1, cp.y - cm, cp.y + cm, by0, by1);
-  const int ny = by1 - by0 + 1, nz = bz1 - bz0 + 1;
-  const int nrows = (ny > 0 && nz > 0) ? ny * nz : 0;
-  int* r_start = runs;
-  int* r_s0 = runs + kRunsPerPass;
-  int* r_T = runs + 2 * kRunsPerPass;
-  for (int p0 = 0; p0 < nrows; p0 += 32) {
-    // this lane's row and its x runs (slots with len 0 are unused)
+  }
+  const int ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
+  int T0 = 0, nT = 1;
+  if (PER && g.per[0]) {
+    T0 = floordiv(cb[0] + lo[0], g.nb[0]);
+    nT = floordiv(cb[0] + hi[0], g.nb[0]) - T0 + 1;
+  }
+  const int nrows = (ny > 0 && nz > 0 && lo[0] <= hi[0]) ? ny * nz : 0;
+  const float inv_ny = 1.0f / (float)ny;  // quotients below 2^20: exact with the half added
+  const int boff = (int)A.bin_off[ci.y];
+  double o[3];
+  coord_origin(g, o);
+  const float sx0 = (float)(o[0] - C.cp.x), sy0 = (float)(o[1] - C.cp.y), sz0 = (float)(o[2] - C.cp.z);
+  const bool image_test = PER && (g.wrapped || (C.cw[0] | C.cw[1] | C.cw[2]) != 0);
+  const float c2lo = image_test ? -1.0f : g.c2lo, c2hi = g.c2hi;
+  const float near2 = A.mode == SOAPB_NL_CREATE ? 1e-4f : -1.0f;
+  const unsigned upto = 0xffffffffu >> (31 - lane);
+  const bool orth = !PER || g.orth;
+  const int groups = PER ? (nT + 1) >> 1 : 1;
+  for (int p0 = 0, tg = 0; tg < groups; p0 += 32) {
+    if (p0 >= nrows) {  // the next two images
+      if (nrows == 0) break;
+      p0 = -32;
+      ++tg;
+      continue;
+    }
     const int row = p0 + lane;
-    int rs0[4], rlen[4], rT[4];
+    constexpr int Q = PER ? 2 : 1;  // runs of a row
+    int len[Q], s0[Q];
+    float4 sh[Q];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) { rs0[q] = 0; rlen[q] = 0; rT[q] = 0; }
+    for (int q = 0; q < Q; ++q) {
+      len[q] = s0[q] = 0;
+      sh[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
     if (row < nrows) {
-      const int bz = bz0 + row / ny, by = by0 + row % ny;
-      const double dy = dmin(1, by), dz = dmin(2, bz), d2 = dy * dy + dz * dz;
-      if (d2 <= cm * cm) {
-        const double ext = sqrt(cm * cm - d2);
-        int bx0, bx1;
-        brange(0, cp.x - ext, cp.x + ext, bx0, bx1);
-        int Ty = 0, byw = by, Tz = 0, bzw = bz;
-        if (g.per[1]) { Ty = floordiv(by, g.nb[1]); byw = by - Ty * g.nb[1]; }
-        if (g.per[2]) { Tz = floordiv(bz, g.nb[2]); bzw = bz - Tz * g.nb[2]; }
-        const int64_t gb = boff + ((int64_t)bzw * g.nb[1] + byw) * g.nb[0];
-        int bx = bx0;
+      const int iz = (int)(((float)row + 0.5f) * inv_ny), dz = lo[2] + iz, dy = lo[1] + row - iz * ny;
+      float mid, ext2, slack = 1e-3f, iwx;  // x range in bins from the centre's: mid +- (sqrt(ext2) iwx + slack)
+      if (orth) {
+        const float ay = fmaxf(0.0f, fmaxf((float)dy - f[1], f[1] - (float)(dy + 1)) * g.wp[1]);
+        const float az = fmaxf(0.0f, fmaxf((float)dz - f[2], f[2] - (float)(dz + 1)) * g.wp[2]);
+        ext2 = R * R - ay * ay - az * az;
+        mid = f[0];
+        iwx = g.iw[0];
+      } else {
+        const float qy = (float)dy + 0.5f - f[1], qz = (float)dz + 0.5f - f[2];
+        const float vx = qy * g.eb[0] + qz * g.ec[0], vy = qy * g.eb[1] + qz * g.ec[1],
+                    vz = qy * g.eb[2] + qz * g.ec[2];
+        const float par = vx * g.dir[0] + vy * g.dir[1] + vz * g.dir[2];
+        const float px = vx - par * g.dir[0], py = vy - par * g.dir[1], pz = vz - par * g.dir[2];
+        const float perp = fmaxf(0.0f, sqrt_approx(px * px + py * py + pz * pz) - g.rho - 1e-4f);
+        ext2 = R * R - perp * perp;
+        iwx = g.ialong;
+        mid = f[0] - par * iwx;
+        slack += g.rho * iwx;
+      }
+      if (ext2 >= 0.0f) {
+        const float e = fmaf(sqrt_approx(ext2), iwx, slack);
+        const int x0 = max((int)floorf(fmaxf(mid - e, -1e6f)), lo[0]),
+                  x1 = min((int)floorf(fminf(mid + e, 1e6f)), hi[0]);
+        int byw = cb[1] + dy, bzw = cb[2] + dz, Ty = 0, Tz = 0;
+        if (PER) {
+          if (g.per[1]) { Ty = floordiv(byw, g.nb[1]); byw -= Ty * g.nb[1]; }
+          if (g.per[2]) { Tz = floordiv(bzw, g.nb[2]); bzw -= Tz * g.nb[2]; }
+        }
+        const int gb = boff + (bzw * g.nb[1] + byw) * g.nb[0];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (bx <= bx1) {
-            int Tx = 0, lx = bx, rend = bx1;
-            if (g.per[0]) {
-              Tx = floordiv(bx, g.nb[0]);
-              lx = bx - Tx * g.nb[0];
-              rend = min(bx1, bx + (g.nb[0] - 1 - lx));
+        for (int q = 0; q < Q; ++q) {
+          const int Tx = T0 + 2 * tg + q;
+          int bx = cb[0], xa = x0, xb = x1;
+          if (PER && g.per[0]) {  // the part of the row in this image
+            bx -= Tx * g.nb[0];
+            xa = max(xa, -bx);
+            xb = min(xb, g.nb[0] - 1 - bx);
+          }
+          if (xa <= xb && (q == 0 || 2 * tg + q < nT)) {
+            s0[q] = __ldg(A.bin_start + gb + bx + xa);
+            len[q] = __ldg(A.bin_start + gb + bx + xb + 1) - s0[q];
+            if (PER) {
+              const double* H = g.H;
+              sh[q] = make_float4((float)(Tx * H[0] + Ty * H[3] + Tz * H[6] - C.cp.x),
+                                  (float)(Tx * H[1] + Ty * H[4] + Tz * H[7] - C.cp.y),
+                                  (float)(Tx * H[2] + Ty * H[5] + Tz * H[8] - C.cp.z),
+                                  __int_as_float(pack3(Tx, Ty, Tz)));
             }
-            const int64_t s0 = A.bin_start[gb + lx], s1 = A.bin_start[gb + lx + (rend - bx) + 1];
-            rs0[q] = (int)s0;
-            rlen[q] = (int)(s1 - s0);
-            rT[q] = pack3(Tx, Ty, Tz);
-            bx = rend + 1;
           }
         }
-        if (bx <= bx1) atomicOr(A.status, 8);  // more than 4 runs: cannot happen with >= 3 bins on x
       }
     }
-    int nr = 0, cnt = 0;
+    const int mine = PER ? len[0] + len[Q - 1] : len[0];
+    int end = mine;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      nr += rlen[q] > 0;
-      cnt += rlen[q];
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, d);
+      if (lane >= d) end += v;
     }
-    int nr_inc = nr, cnt_inc = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int a = __shfl_up_sync(0xffffffffu, nr_inc, o), b = __shfl_up_sync(0xffffffffu, cnt_inc, o);
-      if (lane >= o) {
-        nr_inc += a;
-        cnt_inc += b;
-      }
-    }
-    const int nruns = __shfl_sync(0xffffffffu, nr_inc, 31), total = __shfl_sync(0xffffffffu, cnt_inc, 31);
+    const int total = __shfl_sync(0xffffffffu, end, 31);
+    int nruns = 0;
     {
-      int slot = nr_inc - nr, start = cnt_inc - cnt;
+      const unsigned b0 = __ballot_sync(0xffffffffu, len[0] > 0), before = upto >> 1;
+      int ord = __popc(b0 & before), start = end - mine;
+      nruns = __popc(b0);
+      if (PER) {
+        const unsigned b1 = __ballot_sync(0xffffffffu, len[Q - 1] > 0);
+        ord += __popc(b1 & before);
+        nruns += __popc(b1);
+      }
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (rlen[q] > 0) {
-          r_start[slot] = start;
-          r_s0[slot] = rs0[q];
-          r_T[slot] = rT[q];
-          start += rlen[q];
-          ++slot;
+      for (int q = 0; q < Q; ++q)
+        if (len[q] > 0) {
+          M.adj[ord] = s0[q] - start;
+          if (PER) {
+            M.start[ord] = start;
+            M.shift[ord] = sh[q];
+          }
+          start += len[q];
+          ++ord;
         }
     }
     __syncwarp();
-    // the run of each lane's position in the tile at k0, given the run rb of the position
-    // before the tile; returns the run of the tile's last position
-    auto lookup = [&](int k0, int rb, int& run) {
-      const int idx = rb + 1 + lane;
-      const int pos = (idx < nruns) ? r_start[idx] - k0 : 32;
-      const unsigned mask = __reduce_or_sync(0xffffffffu, (pos >= 0 && pos < 32) ? (1u << pos) : 0u);
-      run = rb + __popc(mask & ((2u << lane) - 1u));
-      return __shfl_sync(0xffffffffu, run, 31);
+    int before = -1;  // runs started before the tile, minus one
+    // the run of this lane's candidate in the tile at k0
+    auto run_of = [&](int k0) {
+      unsigned d = 32u;
+      if (PER) {
+        const int idx = before + 1 + lane;
+        if (idx < nruns) d = (unsigned)(M.start[idx] - k0);
+      } else if (len[0] > 0) {  // this lane's own run
+        d = (unsigned)(end - len[0] - k0);
+      }
+      const unsigned mask = __reduce_or_sync(0xffffffffu, d < 32u ? 1u << d : 0u);
+      const int run = before + __popc(mask & upto);
+      before += __popc(mask);
+      return run;
     };
-    auto load = [&](int k, int run) { return A.sorted_pos[(int64_t)r_s0[run] + (k - r_start[run])]; };
-    const double4 zero4 = make_double4(0.0, 0.0, 0.0, 0.0);
-    int rb = -1;  // run of the position before the tile
-    int run_n = 0;
-    double4 rec_n = zero4;
-    if constexpr (PIPE) {
-      rb = lookup(0, -1, run_n);
-      if (lane < total) rec_n = load(lane, run_n);
-    }
+    // the next tile's position is loaded while this one is tested
+    int run_n = run_of(0), slot_n = lane < total ? M.adj[run_n] + lane : 0;
+    float4 pos_n = __ldg(A.sorted_f + slot_n);
+#pragma unroll (UNROLL)
     for (int k0 = 0; k0 < total; k0 += 32) {
-      const int k = k0 + lane;
-      int run;
-      double4 p = zero4;
-      if constexpr (PIPE) {
-        run = run_n;
-        p = rec_n;
-        rec_n = zero4;
-        if (k0 + 32 < total) {
-          rb = lookup(k0 + 32, rb, run_n);
-          if (k + 32 < total) rec_n = load(k + 32, run_n);
-        }
-      } else {
-        rb = lookup(k0, rb, run);
-        if (k < total) p = load(k, run);
+      const bool valid = k0 + lane < total;
+      const int slot = slot_n, run = run_n;
+      const float4 p = pos_n;
+      if (k0 + 32 < total) {
+        run_n = run_of(k0 + 32);
+        slot_n = k0 + 32 + lane < total ? M.adj[run_n] + k0 + 32 + lane : 0;
+        pos_n = __ldg(A.sorted_f + slot_n);
       }
-      bool ok = false;
-      int atom = 0, sp = 0;
-      double rx = 0.0, ry = 0.0, rz = 0.0, r2 = 0.0;
-      if (k < total) {
-        int wrap;
-        unpack_info(p.w, atom, sp, wrap);
-        if (!g.any_per) {  // open structure: no image shifts (warp-uniform)
-          rx = p.x - cp.x;
-          ry = p.y - cp.y;
-          rz = p.z - cp.z;
-          r2 = rx * rx + ry * ry + rz * rz;
-          ok = r2 <= A.cutoff2;
-        } else {
-          int T[3];
-          unpack3(r_T[run], T);
-          rx = p.x + (T[0] * Lv[0] - cp.x);
-          ry = p.y + (T[1] * Lv[1] - cp.y);
-          rz = p.z + (T[2] * Lv[2] - cp.z);
-          r2 = rx * rx + ry * ry + rz * rz;
-          ok = r2 <= A.cutoff2;
-          if (ok) {
-            int aw[3];
-            unpack3(wrap, aw);
-#pragma unroll
-            for (int kk = 0; kk < 3; ++kk)
-              if (g.per[kk]) ok &= abs(T[kk] - aw[kk] + cw[kk]) <= g.nrep[kk];
-          }
-        }
-        if (ok && A.mode == SOAPB_NL_CREATE && r2 <= 1e-24 && atom != ci.w) ok = false;
+      float sx = sx0, sy = sy0, sz = sz0;
+      int T = 0;
+      if (PER) {
+        const float4 v = M.shift[valid ? run : 0];
+        sx = v.x;
+        sy = v.y;
+        sz = v.z;
+        T = __float_as_int(v.w);
       }
-      fn(ok, atom, sp, rx, ry, rz, r2);
+      const float rx = p.x + sx, ry = p.y + sy, rz = p.z + sz;
+      const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+      bool ok = valid && r2 <= c2lo && r2 > near2;
+      const bool unsure = valid && !ok && !(r2 > c2hi);
+      if (__any_sync(0xffffffffu, unsure)) {
+        if (unsure) ok = exact_test(A, C, slot, T);
+        __syncwarp();
+      }
+      fn(ok, slot, T);
     }
-    __syncwarp();  // the next pass rewrites the run table
+    __syncwarp();  // the run table is rewritten
   }
 }
 
-// The enumeration for the centre's structure: sphere-trimmed for diagonal
-// frames, the full window otherwise (runs: kRunsPerPass * 3 ints of the warp's shared memory).
-template <bool PIPE = false, class Fn>
-__device__ __forceinline__ void visit_any(const VisitArgs& A, int64_t c, int* runs, Fn&& fn) {
-  if (A.grids[A.cinfo[c].y].orth) visit_fine<PIPE>(A, c, runs, fn);
-  else visit(A, c, fn);
+template <int UNROLL, class Fn>
+__device__ __forceinline__ void visit(const VisitArgs& A, int64_t c, VisitMem& M, VisitCentre& C, Fn&& fn) {
+  const int4 ci = A.cinfo[c];
+  C.g = A.grids + ci.y;
+  C.cp = A.cpos[c];
+  C.atom = ci.w;
+  C.per = C.g->any_per != 0;
+  unpack3(ci.z, C.cw);
+  if (C.per) visit_runs<true, UNROLL>(A, M, C, ci, fn);
+  else visit_runs<false, UNROLL>(A, M, C, ci, fn);
+}
+
+// The i-th centre of a warp, or n_centres.  A block takes consecutive centres,
+// its warps in turn: neighbouring centres share most of their candidates, so
+// the warps find each other's records in L1.
+__device__ __forceinline__ int64_t nth_centre(int i, int64_t n_centres) {
+  const int64_t W = blockDim.x >> 5, per = (n_centres + gridDim.x * W - 1) / (gridDim.x * W);
+  return i < per ? min((blockIdx.x * per + i) * W + (threadIdx.x >> 5), n_centres) : n_centres;
 }
 
 // Pairs of every centre, one warp per centre, 8 blocks of 4 warps per SM (64
 // registers): the count is latency-bound with little work per candidate, so
-// more resident warps pay more than pipelining.  The largest count goes to
+// more resident warps pay.  The largest count goes to
 // status[2].  With pair_off, the last block to finish scans the counts into it
 // and, with stats, writes {total, largest, flags} -- the caller gets offsets and
 // summary from this launch (kLastBlockScan centres: the scan by 128 threads
@@ -840,16 +923,17 @@ constexpr int64_t kLastBlockScan = 8192;
 
 __global__ void __launch_bounds__(128, 8) k_count(VisitArgs A, int64_t n_centres, int* counts, int64_t* pair_off,
                                                   int64_t* stats) {
-  __shared__ int s_runs[4][3 * kRunsPerPass];
+  __shared__ VisitMem s_mem[4];
   __shared__ int s_cnt[4];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
   int most = 0;
-  for (int64_t c = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid; c < n_centres; c += nw) {
+  for (int i = 0;; ++i) {
+    const int64_t c = nth_centre(i, n_centres);
+    if (c >= n_centres) break;
     int cnt = 0;
-    visit_any(A, c, s_runs[wid], [&](bool ok, int, int, double, double, double, double) {
-      cnt += __popc(__ballot_sync(0xffffffffu, ok));
-    });
+    VisitCentre C;
+    visit<2>(A, c, s_mem[wid], C, [&](bool ok, int, int) { cnt += ok; });
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
     if (lane == 0) counts[c] = cnt;
     most = max(most, cnt);
   }
@@ -880,33 +964,40 @@ __global__ void __launch_bounds__(128, 8) k_count(VisitArgs A, int64_t n_centres
   }
 }
 
-constexpr int kFillStage = 512;  // pairs per centre collected in shared memory
+// Fill: one warp per centre.  The slots and image shifts of the centre's pairs are
+// collected in shared memory in candidate order (one enumeration, 8 bytes a
+// pair), then ranked within their key (species, radial segment) by a stable
+// counting sort and written to the centre's CSR slice from the FP64 records.  A
+// centre with more than `stage` pairs, or in a cell so small that shifts need
+// more than 4 bits an axis, enumerates twice instead (histogram, then scatter).
+// Either way the order is: by key, and by candidate order within a key.  The key
+// is computed from the FP32 pair record (the radius and segment the descriptor
+// kernels compute).
+//
+// The latency of the record loads and of the ranking bounds this kernel, so it
+// keeps little per pair: 20 bytes (the FP32 record, key and rank, a tile's
+// records loaded while the next is tested) leave fewer warps and less L1 and
+// measured slower (1M atoms: 7.0 ms).  1M atoms: 7.25 -> 5.9 ms; 3000 atoms at
+// 700 pairs a centre: 63 -> 42 us (768 staged pairs, no second enumeration); 48
+// cells: 126 -> 76 us.  7 blocks per SM: 6 take 6.1 ms, 8 spill.
+__host__ __device__ inline int fill_warp_bytes(int nkeys, int stage) {
+  return (int)sizeof(VisitMem) + 8 * stage + ((4 * nkeys + 15) & ~15);
+}
 
-// Fill: one warp per centre.  The centre's accepted candidates are collected
-// in shared memory in candidate order (one enumeration), then placed by a
-// stable counting sort on the key (species, radial segment) and written to the
-// centre's CSR slice.  A centre with more than kFillStage pairs enumerates
-// twice instead (histogram, then scatter).  Either way the order is: by key,
-// and by candidate order within a key.  The key is recomputed from the FP32
-// pair record whenever it is needed (the radius and segment the descriptor
-// kernels compute), so no key array takes shared memory.
-__global__ void __launch_bounds__(128) k_fill(VisitArgs A, int64_t n_centres, const int64_t* pair_off, float4* pairs,
-                                              int64_t capacity, int nseg, float inv_h, int nkeys, int* status) {
+__global__ void __launch_bounds__(128, 7) k_fill(VisitArgs A, int64_t n_centres, const int64_t* pair_off, float4* pairs,
+                                              int64_t capacity, int nseg, float inv_h, int nkeys, int stage,
+                                              int* status) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  float4* stage = reinterpret_cast<float4*>(s_raw) + (size_t)wid * kFillStage;
-  int* hist = reinterpret_cast<int*>(reinterpret_cast<float4*>(s_raw) + (size_t)(blockDim.x >> 5) * kFillStage) +
-              (size_t)wid * nkeys;
-  int* runs = reinterpret_cast<int*>(reinterpret_cast<float4*>(s_raw) + (size_t)(blockDim.x >> 5) * kFillStage) +
-              (size_t)(blockDim.x >> 5) * nkeys + (size_t)wid * 3 * kRunsPerPass;
-  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  unsigned char* mine = s_raw + (size_t)wid * fill_warp_bytes(nkeys, stage);
+  VisitMem& M = *reinterpret_cast<VisitMem*>(mine);
+  int* st_slot = reinterpret_cast<int*>(mine + sizeof(VisitMem));
+  unsigned* st_meta = reinterpret_cast<unsigned*>(st_slot + stage);  // T + 8 per axis (4 bits) | key << 12 | rank << 22
+  int* hist = reinterpret_cast<int*>(st_meta + stage);
   if (pair_off[n_centres] > capacity) {
     if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(status, 4);
     return;
   }
-  auto record = [](int atom, int sp, double rx, double ry, double rz) {
-    return make_float4((float)rx, (float)ry, (float)rz, __int_as_float(atom | (sp << kAtomBits)));
-  };
   auto keyof = [&](const float4& p) {  // species * nseg + segment of the FP32 record
     const float r = sqrtf(p.x * p.x + p.y * p.y + p.z * p.z);
     return (int)((unsigned)__float_as_int(p.w) >> kAtomBits) * nseg + min((int)(r * inv_h), nseg - 1);
@@ -930,61 +1021,80 @@ __global__ void __launch_bounds__(128) k_fill(VisitArgs A, int64_t n_centres, co
     }
     __syncwarp();
   };
-  for (int64_t c = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid; c < n_centres; c += nw) {
+  for (int ic = 0;; ++ic) {
+    const int64_t c = nth_centre(ic, n_centres);
+    if (c >= n_centres) break;
     for (int k = lane; k < nkeys; k += 32) hist[k] = 0;
     const int64_t base = pair_off[c];
     const int64_t P = pair_off[c + 1] - base;
     __syncwarp();
-    if (P <= kFillStage) {
+    VisitCentre C;
+    auto record = [&](int slot, int T) {
+      const double4 p = load_record(A.sorted_pos + slot);
+      double rx, ry, rz;
+      exact_rvec(C, p, T, rx, ry, rz);
+      // the record's low word is atom | species << kAtomBits already
+      return make_float4((float)rx, (float)ry, (float)rz, __int_as_float((int)__double_as_longlong(p.w)));
+    };
+    auto staged = [&](int i) {
+      const unsigned t = st_meta[i];
+      return record(st_slot[i], C.per ? pack3((int)(t & 15u) - 8, (int)((t >> 4) & 15u) - 8, (int)((t >> 8) & 15u) - 8)
+                                      : 0);
+    };
+    // slots of one key in a warp's 32 pairs, ranked in lane order behind those counted before
+    auto rank_in_key = [&](bool ok, int key) {
+      const unsigned peers = __match_any_sync(0xffffffffu, ok ? key : -1 - lane);
+      const int before = ok ? hist[key] : 0;
+      __syncwarp();
+      if (ok && lane == __ffs(peers) - 1) hist[key] = before + __popc(peers);
+      __syncwarp();
+      return before + __popc(peers & ((1u << lane) - 1u));
+    };
+    const GridDesc& g = A.grids[A.cinfo[c].y];
+    // positions are wrapped: a pair's |T| is at most ceil(cutoff / width) = n_rep on each axis
+    if (P <= stage && max(g.nrep[0], max(g.nrep[1], g.nrep[2])) <= 7) {
       int n = 0;
-      visit_any<true>(A, c, runs, [&](bool ok, int atom, int sp, double rx, double ry, double rz, double) {
+      visit<1>(A, c, M, C, [&](bool ok, int slot, int T) {
         const unsigned bal = __ballot_sync(0xffffffffu, ok);
-        if (ok) {
-          const int pos = n + __popc(bal & ((1u << lane) - 1u));
-          if (pos < kFillStage) {
-            const float4 rec = record(atom, sp, rx, ry, rz);
-            stage[pos] = rec;
-            atomicAdd(&hist[keyof(rec)], 1);
-          }
+        const int pos = n + __popc(bal & ((1u << lane) - 1u));
+        if (ok && pos < stage) {
+          st_slot[pos] = slot;
+          int v[3];
+          unpack3(T, v);
+          st_meta[pos] = C.per ? (unsigned)(v[0] + 8) | (unsigned)(v[1] + 8) << 4 | (unsigned)(v[2] + 8) << 8 : 0u;
         }
         n += __popc(bal);
       });
       __syncwarp();
-      scan_hist();
-      const int m = min(n, kFillStage);
-      for (int i0 = 0; i0 < m; i0 += 32) {
-        const int i = i0 + lane;
-        const bool ok = i < m;
-        const float4 rec = ok ? stage[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const int key = ok ? keyof(rec) : -1 - lane;
-        const unsigned peers = __match_any_sync(0xffffffffu, key);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        const int start = ok ? hist[key] : 0;
-        __syncwarp();
-        if (ok) {
-          pairs[base + start + rank] = rec;
-          if (rank == 0) hist[key] = start + __popc(peers);
+      const int m = min(n, stage);
+      for (int i0 = 0; i0 < m; i0 += 64) {  // two tiles' records in flight
+        int key[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) key[u] = keyof(staged(min(i0 + 32 * u + lane, m - 1)));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int i = i0 + 32 * u + lane;
+          const int rank = rank_in_key(i < m, key[u]);
+          if (i < m) st_meta[i] |= (unsigned)key[u] << 12 | (unsigned)rank << 22;
         }
-        __syncwarp();
+      }
+      scan_hist();
+#pragma unroll 4
+      for (int i = lane; i < m; i += 32) {
+        const unsigned t = st_meta[i];
+        pairs[base + hist[(t >> 12) & 1023u] + (t >> 22)] = staged(i);
       }
     } else {
-      visit_any<true>(A, c, runs, [&](bool ok, int atom, int sp, double rx, double ry, double rz, double) {
-        if (ok) atomicAdd(&hist[keyof(record(atom, sp, rx, ry, rz))], 1);
+      visit<1>(A, c, M, C, [&](bool ok, int slot, int T) {
+        if (ok) atomicAdd(&hist[keyof(record(slot, T))], 1);
       });
       __syncwarp();
       scan_hist();
-      visit_any<true>(A, c, runs, [&](bool ok, int atom, int sp, double rx, double ry, double rz, double) {
-        const float4 rec = record(atom, sp, rx, ry, rz);
-        const int key = ok ? keyof(rec) : -1 - lane;
-        const unsigned peers = __match_any_sync(0xffffffffu, key);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        const int start = ok ? hist[key] : 0;
-        __syncwarp();
-        if (ok) {
-          pairs[base + start + rank] = rec;
-          if (rank == 0) hist[key] = start + __popc(peers);
-        }
-        __syncwarp();
+      visit<1>(A, c, M, C, [&](bool ok, int slot, int T) {
+        float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ok) rec = record(slot, T);
+        const int pos = rank_in_key(ok, ok ? keyof(rec) : 0);
+        if (ok) pairs[base + pos] = rec;
       });
     }
     __syncwarp();
@@ -1018,7 +1128,7 @@ __global__ void __launch_bounds__(1024) k_clamp(int64_t* pair_off, int64_t n_cen
 // ---------------------------------------------------------------------------
 
 struct NLLayout {
-  int64_t grids, fbox, bps, bin_off, bin_count, bin_start, arrival, atom_bin, sorted_atom, sorted_pos, cpos,
+  int64_t grids, fbox, bps, bin_off, bin_count, bin_start, atom_bin, sorted_atom, sorted_pos, sorted_f, cpos,
       cinfo, counts, partials, status, total;
   int64_t max_bins;
 };
@@ -1027,7 +1137,8 @@ static NLLayout nl_layout(const soapb_structs* s, const soapb_centres* c) {
   NLLayout L{};
   const int64_t ns = s->n_struct, na = s->n_atoms, nc = c->n_centres;
   L.max_bins = 2 * na + 8 * ns + 64;
-  const int64_t maxn = (na > nc ? na : nc) + L.max_bins + 2;
+  int64_t maxn = L.max_bins > nc ? L.max_bins : nc;  // longest scan
+  if (maxn < ns) maxn = ns;
   int64_t off = 0;
   auto take = [&](int64_t bytes) { const int64_t o = off; off = align_up(off + bytes, 256); return o; };
   L.grids = take(sizeof(GridDesc) * ns);
@@ -1036,10 +1147,10 @@ static NLLayout nl_layout(const soapb_structs* s, const soapb_centres* c) {
   L.bin_off = take(8 * (ns + 1));
   L.bin_count = take(4 * L.max_bins);
   L.bin_start = take(4 * (L.max_bins + 1));
-  L.arrival = take(4 * na);
   L.atom_bin = take(4 * na);
   L.sorted_atom = take(4 * na);
   L.sorted_pos = take(32 * na);
+  L.sorted_f = take(16 * na);
   L.cpos = take(32 * nc);
   L.cinfo = take(16 * nc);
   L.counts = take(4 * nc);
@@ -1058,7 +1169,8 @@ static NLWork nl_work(const NLLayout& L, void* base_) {
   w.bin_off = (int64_t*)(base + L.bin_off);
   w.bin_count = (int*)(base + L.bin_count);
   w.bin_start = (int*)(base + L.bin_start);
-  w.arrival = (int*)(base + L.arrival);
+  w.sorted_f = (float4*)(base + L.sorted_f);
+  w.arrival = (int*)(base + L.sorted_f);  // read by the scatter, before the gather writes sorted_f
   w.atom_bin = (int*)(base + L.atom_bin);
   w.sorted_atom = (int*)(base + L.sorted_atom);
   w.sorted_pos = (double4*)(base + L.sorted_pos);
@@ -1089,6 +1201,7 @@ static VisitArgs visit_args(const soapb_basis* b, const NLWork& w, int mode) {
   A.bin_off = w.bin_off;
   A.bin_start = w.bin_start;
   A.sorted_pos = w.sorted_pos;
+  A.sorted_f = w.sorted_f;
   A.cpos = w.cpos;
   A.cinfo = w.cinfo;
   A.status = w.status;
@@ -1210,13 +1323,16 @@ extern "C" int soapb_neighbors_fill(const soapb_basis* b, const soapb_structs* s
   NLWork w = nl_work(L, d_work);
   const VisitArgs A = visit_args(b, w, mode);
   if (c->n_centres > 0) {
-    const int smem = 4 * (16 * kFillStage + 4 * b->n_keys + 4 * 3 * kRunsPerPass);
+    // staged pairs per centre: 512, or 768 when the cutoff sphere holds more at condensed-matter
+    // density (0.12 atoms / A^3); more would cost resident warps
+    const int stage = 4.19 * b->cutoff * b->cutoff * b->cutoff * 0.12 > 512.0 ? 768 : 512;
+    const int smem = 4 * fill_warp_bytes(b->n_keys, stage);
     int rc2 = check_cuda(cudaFuncSetAttribute(k_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                          "fill smem attribute");
     if (rc2) return rc2;
     k_fill<<<grid_blocks(c->n_centres, 4), 128, smem, st>>>(A, c->n_centres, d_pair_off, (float4*)d_pairs,
                                                             capacity, b->n_seg, (float)(1.0 / b->seg_width),
-                                                            b->n_keys, w.status);
+                                                            b->n_keys, stage, w.status);
   }
   return check_launch("k_fill", c->n_centres > 0 ? 1 : 0);
 }

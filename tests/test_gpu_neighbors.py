@@ -14,6 +14,13 @@ def _soap(periodic, r_cut=4.0):
     return SOAP(species=[1, 8], r_cut=r_cut, n_max=2, l_max=1, sigma=0.3, periodic=periodic)
 
 
+def _lattice(kind):
+    """Cells of every enumeration: diagonal, sheared both ways, and with an open axis."""
+    return {"cubic": np.eye(3), "flat": np.diag([1.9, 1.1, 0.5]),
+            "sheared": np.array([[1.0, 0.0, 0.0], [0.7, 0.8, 0.0], [-0.5, 0.4, 0.9]]),
+            "rotated": np.array([[0.6, 0.8, 0.0], [-0.8, 0.6, 0.1], [0.0, 0.1, 1.0]])}[kind]
+
+
 def _system(n, periodic, rng, density=0.05):
     side = (n / density) ** (1.0 / 3.0)
     s = {"positions": rng.uniform(0.0, side, (n, 3)) + (0.0 if periodic else -3.0 * side),
@@ -27,10 +34,11 @@ def _brute(soap, s):
     """(centre, atom, x, y, z) of every pair of one structure, r = 0 own edges included."""
     pos = torch.as_tensor(s["positions"], device="cuda")
     shifts = torch.zeros((1, 3), dtype=torch.float64, device="cuda")
-    if "cell" in s:
-        n = int(np.ceil(soap._cutoff / s["cell"][0, 0]))
-        g = torch.arange(-n, n + 1, dtype=torch.float64, device="cuda")
-        shifts = torch.cartesian_prod(g, g, g) * s["cell"][0, 0]
+    if "cell" in s:  # the image offsets of the atoms as given: |n_i| <= ceil(cutoff / width_i) on periodic axes
+        width = 1.0 / np.linalg.norm(np.linalg.inv(s["cell"]), axis=0)
+        g = [torch.arange(-k, k + 1, dtype=torch.float64, device="cuda")
+             for k in (int(np.ceil(soap._cutoff / w)) if p else 0 for w, p in zip(width, s["pbc"]))]
+        shifts = torch.cartesian_prod(*g) @ torch.as_tensor(s["cell"], device="cuda")
     img = (pos[None] + shifts[:, None]).reshape(-1, 3)
     rows = []
     step = max(1, (1 << 25) // img.shape[0])
@@ -102,3 +110,31 @@ def test_coincident_and_clustered_atoms():
     pos = np.concatenate([rng.uniform(0, 0.5, (600, 3)), [[0.1, 0.1, 0.1], [0.1, 0.1, 0.1]],
                           [[5e4, 0, 0], [0, -3e4, 2e4]]])
     _check(_soap(False), [{"positions": pos, "atomic_numbers": np.ones(len(pos), np.int64)}])
+
+
+@pytest.mark.parametrize("wrapped", [True, False])
+@pytest.mark.parametrize("pbc", [[True, True, True], [True, False, True], [False, True, False]])
+@pytest.mark.parametrize("kind", ["cubic", "flat", "sheared", "rotated"])
+@pytest.mark.parametrize("n", [2, 9, 150, 1200])
+def test_frames_and_images(n, kind, pbc, wrapped):
+    """Cells much smaller than the cutoff to several times it; positions in the
+    cell and up to two cells outside (the image set is that of the atoms as given)."""
+    rng = np.random.default_rng(n + len(kind))
+    cell = _lattice(kind)
+    cell = cell * (n / 0.06 / abs(np.linalg.det(cell))) ** (1.0 / 3.0)
+    frac = rng.uniform(0.0, 1.0, (n, 3))
+    if not wrapped:
+        frac += rng.integers(-2, 3, (n, 3))
+    _check(_soap(True), [{"positions": frac @ cell, "atomic_numbers": rng.choice(np.array([1, 8]), n),
+                          "cell": cell, "pbc": pbc}])
+
+
+@pytest.mark.parametrize("n,side", [(700, 9.0), (1000, 9.5), (2000, 10.0), (60, 1.2)])
+def test_dense_centres(n, side):
+    """More pairs per centre than the fill stages, and a cell whose shifts do not fit its packed form."""
+    rng = np.random.default_rng(n)
+    s = {"positions": rng.uniform(0.0, side, (n, 3)), "atomic_numbers": rng.choice(np.array([1, 8]), n)}
+    if n == 60:
+        s = {"positions": rng.uniform(0.0, 0.5, (2, 3)), "atomic_numbers": np.array([1, 8]),
+             "cell": np.diag([0.5, 2.0, 5.0]), "pbc": [True] * 3}
+    _check(_soap(n == 60, r_cut=5.0), [s])
