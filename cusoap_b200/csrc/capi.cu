@@ -33,3 +33,7 @@ extern "C" const char* soapb_last_error(void) { return soapb::g_err; }
 extern "C" const char* soapb_version(void) { return "soapb200 0.1.0 (sm_100a)"; }
 
 extern "C" int64_t soapb_kernel_launches(void) { return soapb::g_launches.load(std::memory_order_relaxed); }
+
+extern "C" int soapb_stream_synchronize(void* stream) {
+  return soapb::check_cuda(cudaStreamSynchronize((cudaStream_t)stream), "stream synchronize");
+}

@@ -26,6 +26,7 @@ Differences from the reference, by design:
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 from typing import Any, Dict, List, Optional, Sequence, Tuple, Union
@@ -70,7 +71,40 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def _on_device(device: torch.device):
+    """``torch.cuda.device(device)``, or nothing when it is the current one."""
+    return _NO_GUARD if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+def _index_centres(centres) -> bool:
+    """Whether a centre list holds atom indices only."""
+    return all(isinstance(c, (int, np.integer)) for c in centres)
+
+
+_TORCH_TYPES = {np.dtype(np.int32): torch.int32, np.dtype(np.int64): torch.int64,
+                np.dtype(np.float64): torch.float64, np.dtype(np.uint8): torch.uint8}
+
+
+class _DevArrays:
+    """Named host arrays copied to the device in one buffer: addresses for the
+    library, tensor views made when asked for."""
+
+    def __init__(self, buf: torch.Tensor, where: Dict[str, Tuple[int, np.ndarray]], stage: torch.Tensor):
+        self.buf, self.base, self.stage = buf, buf.data_ptr(), stage
+        self.where = {name: (off, a.dtype, a.shape, a.nbytes) for name, (off, a) in where.items()}
+
+    def ptr(self, name: str) -> int:
+        return self.base + self.where[name][0]
+
+    def tensor(self, name: str) -> torch.Tensor:
+        off, dtype, shape, nbytes = self.where[name]
+        return self.buf[off:off + nbytes].view(_TORCH_TYPES[dtype]).reshape(shape)
 
 
 def _resolve_z(s) -> int:
@@ -156,28 +190,33 @@ def _poly_grid(r_cut: float, n_max: int, quad_n: int) -> np.ndarray:
 
 class _Batch:
     """Device buffers describing a batch of structures and their centres.
-    Host arrays are concatenated first and copied with one transfer each."""
+    Host arrays go to the device in one transfer.  ``own_positions``: the
+    positions are a copy even where the caller's tensor could be used as it is."""
 
-    def __init__(self, soap: "SOAP", systems: List[Any], centers_list: List[Optional[Sequence[Any]]]):
+    def __init__(self, soap: "SOAP", systems: List[Any], centers_list: List[Optional[Sequence[Any]]],
+                 own_positions: bool = False):
         dev = soap.device
         raw = [soap._system_arrays(s) for s in systems]
+        centers_list = [None if c is None else list(c) for c in centers_list]
+        n_struct = len(raw)
         counts_a = [int(r[0].shape[0]) for r in raw]
-        atom_off = np.concatenate([[0], np.cumsum(counts_a)]).astype(np.int64)
+        atom_off = np.zeros(n_struct + 1, np.int64)
+        np.cumsum(counts_a, out=atom_off[1:])
         self.atom_off_list = atom_off.tolist()
-        self.n_atoms = int(atom_off[-1])
+        self.n_atoms = self.atom_off_list[-1]
         self.pos_tensors = [r[0] for r in raw if isinstance(r[0], torch.Tensor)]
-        host_pos = all(isinstance(r[0], np.ndarray) for r in raw)
-        Zall = np.concatenate([r[1] for r in raw]) if raw else np.zeros(0, np.int64)
-        cells = np.zeros((len(raw), 9))
-        pbcs = np.zeros((len(raw), 3), np.uint8)
+        host_pos = not self.pos_tensors
+        Zall = raw[0][1] if n_struct == 1 else np.concatenate([r[1] for r in raw]) if raw else np.zeros(0, np.int64)
+        cells = np.zeros((n_struct, 9))
+        pbcs = np.zeros((n_struct, 3), np.uint8)
         if soap.periodic:
             if any(r[2] is None or r[3] is None for r in raw):
                 raise ValueError("periodic=True requires cell and pbc.")
             try:  # one conversion for the whole list (numpy / nested-list cells and flags)
                 if any(isinstance(r[2], torch.Tensor) or isinstance(r[3], torch.Tensor) for r in raw):
                     raise TypeError
-                cells[:] = np.asarray([r[2] for r in raw], dtype=np.float64).reshape(len(raw), 9)
-                pbcs[:] = np.asarray([r[3] for r in raw], dtype=bool).reshape(len(raw), 3)
+                cells[:] = np.asarray([r[2] for r in raw], dtype=np.float64).reshape(n_struct, 9)
+                pbcs[:] = np.asarray([r[3] for r in raw], dtype=bool).reshape(n_struct, 3)
             except (TypeError, ValueError):
                 for i, r in enumerate(raw):
                     cells[i] = np.asarray(r[2].detach().cpu() if isinstance(r[2], torch.Tensor) else r[2],
@@ -193,43 +232,60 @@ class _Batch:
                                        and np.array_equal(cached["cells"], cells)
                                        and np.array_equal(cached["pbcs"], pbcs)):
             cached = None
+        # centres that are all atom indices (or every atom) are described by host arrays
+        by_index = not all_atoms and all(c is None or _index_centres(c) for c in centers_list)
         if cached is not None:
-            dev_arrays = cached["dev"]
+            self._dev = cached["dev"]
         else:
             # the small host arrays (and host positions) go to the device in ONE
             # asynchronous copy from a pinned staging buffer
             arrays = [("species", soap._species_lookup(Zall)), ("atom_off", atom_off), ("cells", cells),
                       ("pbc", pbcs)]
-            if all_atoms:
-                arrays.append(("centre_struct", np.repeat(np.arange(len(raw), dtype=np.int32), counts_a)))
-                arrays.append(("centre_atom", np.arange(int(atom_off[-1]), dtype=np.int32)))
+            host = None
             if host_pos:
-                host = np.concatenate([r[0] for r in raw]) if raw else np.zeros((0, 3))
-                arrays.append(("positions", np.ascontiguousarray(host, dtype=np.float64)))
-            dev_arrays = soap._upload(arrays)
+                host = raw[0][0] if n_struct == 1 else np.concatenate([r[0] for r in raw]) if raw else np.zeros((0, 3))
+                arrays.append(("positions", host))
+            if all_atoms:
+                struct = np.zeros(self.n_atoms, np.int32) if n_struct == 1 else \
+                    np.repeat(np.arange(n_struct, dtype=np.int32), counts_a)
+                arrays.append(("centre_struct", struct))
+                arrays.append(("centre_atom", np.arange(self.n_atoms, dtype=np.int32)))
+            elif by_index:
+                arrays += self._index_arrays(centers_list, counts_a, host)
+            self._dev = soap._upload(arrays)
             if all_atoms and not host_pos:
                 soap._topology = {"counts": list(counts_a), "Z": Zall.copy(), "cells": cells.copy(),
-                                  "pbcs": pbcs.copy(), "dev": dev_arrays}
-        self.species, self.atom_off = dev_arrays["species"], dev_arrays["atom_off"]
-        self.cells, self.pbc = dev_arrays["cells"], dev_arrays["pbc"]
+                                  "pbcs": pbcs.copy(), "dev": self._dev}
+        self._alias = {"centre_attach": "centre_atom"}
+        self.grad_positions = None
         if host_pos:
-            self.positions = dev_arrays["positions"]
-            self.pos_tensors = []
-        elif all(isinstance(r[0], torch.Tensor) and r[0].device == dev for r in raw):
-            # device tensors: one concatenation, one conversion
-            self.positions = torch.cat([r[0].detach() for r in raw]).to(torch.float64).contiguous()
+            pos_ptr = self._dev.ptr("positions")
         else:
-            parts = [r[0].detach().to(dev, torch.float64) if isinstance(r[0], torch.Tensor)
-                     else torch.as_tensor(r[0], dtype=torch.float64, device=dev) for r in raw]
-            self.positions = torch.cat(parts).contiguous()
+            if len(self.pos_tensors) == n_struct and all(p.device == dev for p in self.pos_tensors):
+                # device tensors: one concatenation (differentiable), one conversion
+                cat = self.pos_tensors[0] if n_struct == 1 else torch.cat(self.pos_tensors)
+                self.grad_positions = cat
+                self.positions = cat.detach().to(torch.float64).contiguous().resolve_neg()
+                if own_positions and self.positions.data_ptr() == cat.data_ptr():
+                    self.positions = self.positions.clone()
+            else:
+                parts = [r[0].detach().to(dev, torch.float64) if isinstance(r[0], torch.Tensor)
+                         else torch.as_tensor(r[0], dtype=torch.float64, device=dev) for r in raw]
+                self.positions = torch.cat(parts).contiguous()
+            pos_ptr = self.positions.data_ptr()
         if all_atoms:
             # every atom is a centre, attached to itself (SG:977-979)
             self.counts = counts_a
-            self.n_centres = self.n_atoms
-            self.centre_xyz = self.positions
-            self.centre_atom = dev_arrays["centre_atom"]
-            self.centre_attach = self.centre_atom
-            self.centre_struct = dev_arrays["centre_struct"]
+            self._alias["centre_xyz"] = "positions"
+            xyz_ptr, struct_ptr, atom_ptr = pos_ptr, self._dev.ptr("centre_struct"), self._dev.ptr("centre_atom")
+        elif by_index:
+            self.counts = [n if c is None else len(c) for n, c in zip(counts_a, centers_list)]
+            if host_pos:
+                xyz_ptr = self._dev.ptr("centre_xyz")
+            else:
+                self.centre_xyz = self.positions.index_select(0, self._dev.tensor("centre_index"))
+                xyz_ptr = self.centre_xyz.data_ptr()
+            struct_ptr, atom_ptr = self._dev.ptr("centre_struct"), self._dev.ptr("centre_atom")
         else:
             cxyz, cstruct, catom, cattach, self.counts = [], [], [], [], []
             for i, cen in enumerate(centers_list):
@@ -241,12 +297,57 @@ class _Batch:
                 cattach.append(torch.where(attach >= 0, attach + off, attach))
                 cstruct.append(torch.full((xyz.shape[0],), i, dtype=torch.int32, device=dev))
                 self.counts.append(int(xyz.shape[0]))
-            self.n_centres = sum(self.counts)
             self.centre_xyz = torch.cat([c.detach() for c in cxyz]).contiguous()
             self.centre_struct = torch.cat(cstruct).contiguous()
             self.centre_atom = torch.cat(catom).to(torch.int32).contiguous()
             self.centre_attach = torch.cat(cattach).to(torch.int32).contiguous()
-        self._describe(len(raw))
+            xyz_ptr, struct_ptr, atom_ptr = (self.centre_xyz.data_ptr(), self.centre_struct.data_ptr(),
+                                             self.centre_atom.data_ptr())
+        self.n_centres = sum(self.counts)
+        d = self._dev
+        self.cs = Structs(n_struct, self.n_atoms, d.ptr("atom_off"), pos_ptr, d.ptr("species"), d.ptr("cells"),
+                          d.ptr("pbc"))
+        self.cc = Centres(self.n_centres, xyz_ptr, struct_ptr, atom_ptr)
+
+    @staticmethod
+    def _index_arrays(centers_list, counts_a, host):
+        """Host arrays of centres given by atom index: structure, self atom
+        (a negative index counts from the end and has none, SG:966-1003) and
+        the coordinates of host positions, or the index to gather device ones."""
+        structs, atoms, index, off = [], [], [], 0
+        for i, (n, cen) in enumerate(zip(counts_a, centers_list)):
+            c = np.arange(n, dtype=np.int64) if cen is None else np.array([int(v) for v in cen], dtype=np.int64)
+            if c.size and (c.min() < -n or c.max() >= n):
+                raise IndexError(f"centre index out of range for a structure of {n} atoms")
+            structs.append(np.full(c.size, i, np.int32))
+            atoms.append(np.where(c >= 0, c + off, c).astype(np.int32))
+            index.append(np.where(c >= 0, c, c + n) + off)
+            off += n
+        idx = np.concatenate(index)
+        where = ("centre_index", idx) if host is None else ("centre_xyz", host[idx])
+        return [("centre_struct", np.concatenate(structs)), ("centre_atom", np.concatenate(atoms)), where]
+
+    def __getattr__(self, name):
+        # tensor views of the uploaded arrays, made on first use
+        dev = self.__dict__.get("_dev")
+        if dev is not None:
+            alias = self.__dict__["_alias"].get(name)
+            if alias is not None:
+                value = getattr(self, alias)
+            elif name in dev.where:
+                value = dev.tensor(name)
+            else:
+                raise AttributeError(name)
+            setattr(self, name, value)
+            return value
+        raise AttributeError(name)
+
+    def staged(self, soap: "SOAP") -> None:
+        """The stream of the upload has been synchronised: its staging buffer is free."""
+        dev = self.__dict__.get("_dev")
+        if dev is not None and dev.stage is not None:
+            soap._stage_pool.append(dev.stage)
+            dev.stage = None
 
     def _describe(self, n_struct: int):
         self.cs = Structs(n_struct, self.n_atoms, _ptr(self.atom_off), _ptr(self.positions),
@@ -301,7 +402,8 @@ class _Pairs:
         soap._call("neighbors_count", lib.soapb_neighbors_count_stats, b, ctypes.byref(batch.cs),
                    ctypes.byref(batch.cc), mode, _ptr(self.work), self.work.numel(), _ptr(self.pair_off), _ptr(stats),
                    st)
-        torch.cuda.current_stream(dev).synchronize()
+        check(lib.soapb_stream_synchronize(st))
+        batch.staged(soap)
         self.total, self.max_pairs, status = stats.tolist()
         pool.append(stats)
         if status & 1:
@@ -314,6 +416,11 @@ class _Pairs:
         self.pairs = torch.empty((max(self.total, 1), 4), dtype=torch.float32, device=dev)
         soap._call("neighbors_fill", lib.soapb_neighbors_fill, b, ctypes.byref(batch.cs), ctypes.byref(batch.cc),
                    mode, _ptr(self.work), self.work.numel(), _ptr(self.pair_off), _ptr(self.pairs), self.total, st)
+
+
+def _negated(forces: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """-forces in another type, in one pass."""
+    return torch.mul(forces, -1.0, out=torch.empty(forces.shape, dtype=dtype, device=forces.device))
 
 
 class _SOAPFunction(torch.autograd.Function):
@@ -332,22 +439,23 @@ class _SOAPFunction(torch.autograd.Function):
         soap, batch, pairs = ctx.soap, ctx.batch, ctx.pairs
         forces = soap._run_forces(batch, pairs, ctx.coeff, grad_out.contiguous().to(torch.float32), attach=True,
                                   mode=ctx.mode)
-        return (-forces).to(torch.float64), None, None, None
+        return _negated(forces, torch.float64), None, None, None
 
 
 class SOAPBatch:
     """A fixed batch of structures (every atom a centre) whose descriptor and
-    adjoint run as two captured CUDA graphs, for loops that re-evaluate the
+    adjoint run as captured CUDA graphs, for loops that re-evaluate the
     same structures at new positions (molecular dynamics, relaxations).
 
     Built by ``SOAP.batch(systems)``.  All buffers are allocated once: the
     pair buffer with ``headroom`` over the first neighbour count.  Per call,
     ``create(positions)`` copies the positions into the batch's position
-    buffer and replays the forward graph (neighbour count and fill, a clamp
-    that empties the lists if they overflowed the pair buffer, descriptor);
-    the one device-to-host read checks the pair total, and an overflow
-    rebuilds the plan with a larger buffer and replays.  The backward graph is
-    the adjoint: ``create`` is differentiable w.r.t. ``positions``.
+    buffer and replays the neighbour graph (count and fill, a clamp that
+    empties the lists if they overflowed the pair buffer and writes the pair
+    total to page-locked host memory) and the descriptor graph; the host reads
+    the total when the neighbour graph is done, while the descriptor runs, and
+    an overflow rebuilds the plan with a larger buffer and replays.  The third
+    graph is the adjoint: ``create`` is differentiable w.r.t. ``positions``.
 
     The descriptor returned is the plan's output buffer, overwritten by the
     next replay (clone it to keep it).  Cells, pbc, species and atom counts
@@ -359,7 +467,7 @@ class SOAPBatch:
         self.mode = soap._out_mode()
         self.headroom = float(headroom)
         with torch.cuda.device(soap.device):
-            self.b = _Batch(soap, systems, [None] * len(systems))
+            self.b = _Batch(soap, systems, [None] * len(systems), own_positions=True)
             self.counts = list(self.b.counts)
             self.n_atoms = self.b.n_atoms
             self._build(capacity=None)
@@ -373,7 +481,7 @@ class SOAPBatch:
                                             ctypes.byref(ws)))
         self.work = torch.empty(max(int(ws.value), 256), dtype=torch.uint8, device=dev)
         self.pair_off = torch.empty(C + 1, dtype=torch.int64, device=dev)
-        self.total = torch.zeros(1, dtype=torch.int64, device=dev)
+        self.total = torch.zeros(1, dtype=torch.int64, pin_memory=True)  # written by the neighbour graph
         if capacity is None:
             check(lib.soapb_neighbors_count(ctypes.byref(soap._basis), ctypes.byref(b.cs), ctypes.byref(b.cc),
                                             _lib.NL_ALL, _ptr(self.work), self.work.numel(), _ptr(self.pair_off), st))
@@ -390,18 +498,24 @@ class SOAPBatch:
         check(lib.soapb_forces_workspace(ctypes.byref(soap._basis), C, ctypes.byref(wsb)))
         self.fwork = torch.empty(max(int(wsb.value), 256), dtype=torch.uint8, device=dev)
         self.counter = torch.zeros(1, dtype=torch.int32, device=dev)
-        # run once eagerly (sets kernel attributes), then capture both graphs
-        self._forward_calls()
+        # run once eagerly (sets kernel attributes), then capture the graphs
+        self._list_calls()
+        self._descriptor_calls()
         self._backward_calls()
         torch.cuda.synchronize(dev)
-        self.g_fwd, self.g_bwd = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.g_fwd):
-            self._forward_calls()
+        self.listed = torch.cuda.Event()
+        self.g_list, self.g_desc, self.g_bwd = (torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph(),
+                                                torch.cuda.CUDAGraph())
+        with torch.cuda.graph(self.g_list):
+            self._list_calls()
+        with torch.cuda.graph(self.g_desc):
+            self._descriptor_calls()
         with torch.cuda.graph(self.g_bwd):
             self._backward_calls()
         torch.cuda.synchronize(dev)
+        b.staged(soap)
 
-    def _forward_calls(self):
+    def _list_calls(self):
         soap, b, lib = self.soap, self.b, _lib.load()
         st = _stream(soap.device)
         bb, cs, cc = ctypes.byref(soap._basis), ctypes.byref(b.cs), ctypes.byref(b.cc)
@@ -410,8 +524,12 @@ class SOAPBatch:
         check(lib.soapb_neighbors_fill(bb, cs, cc, _lib.NL_ALL, _ptr(self.work), self.work.numel(),
                                        _ptr(self.pair_off), _ptr(self.pairs), self.capacity, st))
         check(lib.soapb_neighbors_clamp(_ptr(self.pair_off), b.n_centres, self.capacity, _ptr(self.total), st))
-        check(lib.soapb_descriptor(bb, b.n_centres, _ptr(self.pair_off), _ptr(self.pairs), self.mode,
-                                   _ptr(self.desc), _ptr(self.coeff), _ptr(self.counter), st))
+
+    def _descriptor_calls(self):
+        soap, b, lib = self.soap, self.b, _lib.load()
+        check(lib.soapb_descriptor(ctypes.byref(soap._basis), b.n_centres, _ptr(self.pair_off), _ptr(self.pairs),
+                                   self.mode, _ptr(self.desc), _ptr(self.coeff), _ptr(self.counter),
+                                   _stream(soap.device)))
 
     def _backward_calls(self):
         soap, b, lib = self.soap, self.b, _lib.load()
@@ -424,18 +542,22 @@ class SOAPBatch:
     def _replay_forward(self, positions: Optional[torch.Tensor]):
         if positions is not None:
             self.b.positions.copy_(positions.detach().reshape(-1, 3))
-        self.g_fwd.replay()
+        self.g_list.replay()
+        self.listed.record()
+        self.g_desc.replay()
+        self.listed.synchronize()
         need = int(self.total.item())
         if need > self.capacity:  # the lists outgrew the pair buffer: re-plan and run again
             self._build(capacity=int(need * self.headroom) + 1024)
-            self.g_fwd.replay()
+            self.g_list.replay()
+            self.g_desc.replay()
         return self.desc
 
     def create(self, positions: Optional[torch.Tensor] = None) -> torch.Tensor:
         """(n_atoms, F) descriptors of the whole batch at ``positions``
         ((n_atoms, 3), the structures' atoms concatenated; None: unchanged).
         Differentiable w.r.t. ``positions`` through the adjoint graph."""
-        with torch.cuda.device(self.soap.device):
+        with _on_device(self.soap.device):
             if positions is not None and torch.is_grad_enabled() and positions.requires_grad:
                 return _BatchFunction.apply(positions, self)
             return self._replay_forward(positions)
@@ -443,7 +565,7 @@ class SOAPBatch:
     def forces_from(self, dEdp: torch.Tensor) -> torch.Tensor:
         """-dE/dx (n_atoms, 3) for a given dE/dp (n_atoms, F), at the
         positions of the last ``create``."""
-        with torch.cuda.device(self.soap.device):
+        with _on_device(self.soap.device):
             self.dEdp.copy_(dEdp)
             self.g_bwd.replay()
             return self.forces
@@ -463,7 +585,7 @@ class _BatchFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         forces = ctx.plan.forces_from(grad_out.contiguous().to(torch.float32))
-        return (-forces).to(ctx.dtype), None
+        return _negated(forces, ctx.dtype), None
 
 
 class SOAP:
@@ -503,6 +625,11 @@ class SOAP:
         self._atomic_number_set = set(self._atomic_numbers_list)
         self._Z_to_species_index = {z: i for i, z in enumerate(self._atomic_numbers_list)}
         self.n_species = len(self._atomic_numbers_list)
+        top = min(max(self._atomic_numbers_list[-1], 0), 1023)
+        self._species_table = np.full(top + 1, -1, dtype=np.int32)  # atomic number -> species index
+        for z, i in self._Z_to_species_index.items():
+            if 0 <= z <= top:
+                self._species_table[z] = i
         self._n_max = int(n_max)
         self._l_max = int(l_max)
         # limits of the compiled kernels (the reference has none): refused here, before any device work
@@ -554,6 +681,7 @@ class SOAP:
         self._poly_grid = _poly_grid(self._r_cut, self._n_max, self.quad_n) if self._rbf == "polynomial" else None
         self._build_basis()
         self._counter = torch.zeros(1, dtype=torch.int32, device=self.device)
+        self._stage_pool: List[torch.Tensor] = []  # page-locked staging buffers of uploads
         self._stats_pool: List[torch.Tensor] = []  # page-locked int64[3] buffers of the neighbour summaries
         self._topology = None  # device copies of the last batch's species, offsets, cells (see _Batch)
         self.n_features = int(self.get_number_of_features())
@@ -677,47 +805,42 @@ class SOAP:
         """Host int32 species index of every atom; ValueError for atomic
         numbers outside the species list (SG:1782-1784)."""
         Zc = Z.detach().cpu().numpy() if isinstance(Z, torch.Tensor) else np.asarray(Z, dtype=np.int64)
+        if Zc.size == 0:
+            return np.zeros(0, np.int32)
+        if Zc.min() >= 0 and Zc.max() < self._species_table.size:
+            idx = self._species_table[Zc]
+            if idx.min() >= 0:
+                return idx
         bad = set(np.unique(Zc).tolist()) - self._atomic_number_set
         if bad:
             raise ValueError(f"System contains atomic numbers not in species list: {sorted(bad)}")
-        lut = np.full(int(Zc.max()) + 1 if Zc.size else 1, -1, dtype=np.int32)
-        for z, i in self._Z_to_species_index.items():
-            if z < lut.size:
-                lut[z] = i
-        return lut[Zc] if Zc.size else np.zeros(0, np.int32)
+        # species numbers outside the table
+        return np.searchsorted(np.asarray(self._atomic_numbers_list), Zc).astype(np.int32)
 
     def _species_index(self, Z) -> torch.Tensor:
         return torch.as_tensor(self._species_lookup(Z)).to(self.device)
 
-    def _upload(self, arrays) -> Dict[str, torch.Tensor]:
-        """Copy named host arrays to the device in one asynchronous copy
-        through a pinned staging buffer kept by this object; returns typed
-        device views.  The staging buffer is reused once its last copy has
-        completed."""
-        offs, off = [], 0
+    def _upload(self, arrays) -> _DevArrays:
+        """Copy named host arrays to the device in one asynchronous copy from a
+        page-locked staging buffer.  The buffer goes back to this object's pool
+        once the stream has been synchronised (``_Batch.staged``), so calls of
+        other threads take their own."""
+        where, off = {}, 0
         for name, a in arrays:
             a = np.ascontiguousarray(a)
-            offs.append((name, a, off))
-            off = (off + a.nbytes + 255) // 256 * 256
+            where[name] = (off, a)
+            off = (off + a.nbytes + 255) & ~255
         total = max(off, 256)
-        if getattr(self, "_stage", None) is None or self._stage.numel() < total:
-            self._stage = torch.empty(max(total, 1 << 16), dtype=torch.uint8, pin_memory=True)
-            self._stage_done = None
-        if self._stage_done is not None:
-            self._stage_done.synchronize()
-        host = self._stage.numpy()
-        for name, a, o in offs:
-            host[o:o + a.nbytes] = a.view(np.uint8).reshape(-1)
+        pool = self._stage_pool
+        stage = pool.pop() if pool else None
+        if stage is None or stage.numel() < total:
+            stage = torch.empty(max(total, 1 << 16), dtype=torch.uint8, pin_memory=True)
+        base = stage.data_ptr()
+        for o, a in where.values():
+            ctypes.memmove(base + o, a.__array_interface__["data"][0], a.nbytes)
         dbuf = torch.empty(total, dtype=torch.uint8, device=self.device)
-        dbuf.copy_(self._stage[:total], non_blocking=True)
-        self._stage_done = torch.cuda.Event()
-        self._stage_done.record(torch.cuda.current_stream(self.device))
-        tmap = {np.dtype(np.int32): torch.int32, np.dtype(np.int64): torch.int64,
-                np.dtype(np.float64): torch.float64, np.dtype(np.uint8): torch.uint8}
-        out = {}
-        for name, a, o in offs:
-            out[name] = dbuf[o:o + a.nbytes].view(tmap[a.dtype]).reshape(a.shape)
-        return out
+        dbuf.copy_(stage[:total], non_blocking=True)
+        return _DevArrays(dbuf, where, stage)
 
     def _prepare_centres(self, pos: torch.Tensor, centers):
         """(xyz, self atom, attached atom) per centre.  Index centres are
@@ -806,7 +929,7 @@ class SOAP:
 
     def generate(self, system, centers=None, n_jobs: int = 1, only_physical_cores: bool = False,
                  verbose: bool = False):
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             if isinstance(system, list):
                 systems = system
                 if centers is None:
@@ -821,6 +944,8 @@ class SOAP:
                     return []
                 out = self._evaluate_batch(systems, centers_list)
                 parts = list(torch.split(out, [int(c) for c in self._last_counts]))
+                if len(set(self._last_counts)) > 1 and not self.sparse:
+                    return parts  # uneven shapes do not stack
                 if self.sparse:  # each system's rows in COO, then stacked if possible (SG:1716-1737)
                     parts = [p.to_sparse_coo() for p in parts]
                 try:
@@ -843,7 +968,7 @@ class SOAP:
         centers_list = [None] * len(systems) if centers is None else list(centers)
         if len(centers_list) != len(systems):
             raise ValueError("centers list must match number of systems.")
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             if not systems:
                 return (torch.zeros((0, self.get_number_of_features()), dtype=self.dtype, device=self.device),
                         torch.zeros(1, dtype=torch.int64))
@@ -860,7 +985,9 @@ class SOAP:
         if grad:
             if len(batch.pos_tensors) != len(systems):
                 raise ValueError("differentiable create() needs every structure's positions as a tensor")
-            pos = batch.pos_tensors[0] if len(batch.pos_tensors) == 1 else torch.cat(batch.pos_tensors)
+            pos = batch.grad_positions  # None: tensors of other devices, concatenated by their own rules
+            if pos is None:
+                pos = batch.pos_tensors[0] if len(batch.pos_tensors) == 1 else torch.cat(batch.pos_tensors)
             out = _SOAPFunction.apply(pos, self, batch, mode)
         else:
             pairs = _Pairs(self, batch, _lib.NL_CREATE)
@@ -893,27 +1020,32 @@ class SOAP:
                                               only_physical_cores=only_physical_cores, verbose=verbose)
         if method not in ("auto", "analytical"):
             raise ValueError("method must be one of: 'auto', 'analytical', 'numerical'.")
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             batch = _Batch(self, [system], [centers])
             n_atoms = batch.n_atoms
-            idx = list(range(n_atoms)) if include is None else [int(i) for i in include]
-            if exclude is not None:
-                ex = set(int(i) for i in exclude)
-                idx = [i for i in idx if i not in ex]
-            n_inc = len(idx)
+            every = include is None and exclude is None  # every atom, in order: row = atom
+            if every:
+                n_inc = n_atoms
+            else:
+                idx = list(range(n_atoms)) if include is None else [int(i) for i in include]
+                if exclude is not None:
+                    ex = set(int(i) for i in exclude)
+                    idx = [i for i in idx if i not in ex]
+                n_inc = len(idx)
             mode = self._out_mode()
             F = self.get_number_of_features()
             pairs = _Pairs(self, batch, _lib.NL_ALL)
             desc, coeff = self._run_descriptor(batch, pairs, mode, want_coeff=True)
             deriv = torch.empty((batch.n_centres, n_inc, 3, F), dtype=torch.float32, device=self.device)
             if n_inc > 0 and batch.n_centres > 0:
-                if include is None and exclude is None:  # every atom, in order: row = atom
-                    inc_row = torch.arange(max(n_atoms, 1), dtype=torch.int32, device=self.device)
+                if every:
+                    inc_row = (batch.centre_atom if centers is None else
+                               torch.arange(max(n_atoms, 1), dtype=torch.int32, device=self.device))
                 else:
                     h = np.full(max(n_atoms, 1), -1, dtype=np.int32)
                     h[np.asarray(idx, dtype=np.int64)] = np.arange(n_inc, dtype=np.int32)
                     inc_row = torch.from_numpy(h).to(self.device)
-                status = torch.zeros(1, dtype=torch.int32, device=self.device)
+                status = torch.empty(1, dtype=torch.int32, device=self.device)  # never set, see below
                 lib = _lib.load()
                 wsb = ctypes.c_int64(0)
                 check(lib.soapb_jacobian_workspace(ctypes.byref(self._basis), batch.n_centres, pairs.total, n_inc,
@@ -971,7 +1103,7 @@ class SOAP:
         d = float(self.FD_STEP if d is None else d)
         if not d > 0.0:
             raise ValueError("d must be positive")
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             desc0 = self.create(system, centers) if return_descriptor else None
             pos, Z, cell, pbc = self._system_arrays(system)
             pos = (pos.detach() if isinstance(pos, torch.Tensor) else torch.as_tensor(pos)).to(self.device,
@@ -1041,7 +1173,7 @@ class SOAP:
         """E = sum(dEdp * p) over all atoms as centres, and F = -dE/dx from the
         adjoint kernel (centres attached to their atoms).  dEdp: (F,) weights
         shared by every centre, or (n_atoms, F)."""
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             batch = _Batch(self, [system], [None])
             pairs = _Pairs(self, batch, _lib.NL_ALL)
             desc, coeff = self._run_descriptor(batch, pairs, _lib.OUT_PS, want_coeff=True)

@@ -194,7 +194,8 @@ int soapb_neighbors_count_stats(const soapb_basis* b, const soapb_structs* s, co
  * set every offset of d_pair_off to 0 so that the descriptor / Jacobian /
  * adjoint kernels launched after it see empty lists instead of reading past
  * the buffer.  The caller compares *d_total with its capacity and rebuilds
- * with a larger buffer.  Stream-ordered, no sync.  No counterpart in the
+ * with a larger buffer.  d_total may also be page-locked host memory that the
+ * device can address.  Stream-ordered, no sync.  No counterpart in the
  * reference (it allocates per call, SG:1128-1181). */
 int soapb_neighbors_clamp(int64_t* d_pair_off, int64_t n_centres, int64_t capacity, int64_t* d_total, void* stream);
 
@@ -286,6 +287,10 @@ int soapb_forces_status(const soapb_basis* b, int64_t n_centres, const void* d_w
  * normally).  Stream-ordered; no copy is in flight, so the context stays
  * usable.  No counterpart in the reference. */
 int soapb_check_bounded_wait(int32_t* d_status, void* stream);
+
+/* Waits for the stream.  For callers that read a summary written to
+ * page-locked host memory (soapb_neighbors_count_stats). */
+int soapb_stream_synchronize(void* stream);
 
 /* Message describing the last error on the calling thread ("" if none). */
 const char* soapb_last_error(void);
