@@ -30,7 +30,7 @@ struct GridDesc {
   double H[9];     // rows: lattice a, b, c (identity for non-periodic structures)
   double Hinv[9];  // f_j = sum_i x_i Hinv[i*3+j]
   double fmin[3];  // bin origin in fractional coordinates (non-periodic axes)
-  double binw[3];  // fractional bin width
+  double ibinw[3]; // bins per fractional unit
   int nb[3], nrep[3];
   signed char per[4];
   int any_per;
@@ -137,7 +137,7 @@ __device__ __forceinline__ bool locate(const GridDesc& g, double x, double y, do
       ok &= (w[i] > -512 && w[i] < 511);
     } else {
       w[i] = 0;
-      const int bi = (int)floor((f[i] - g.fmin[i]) / g.binw[i]);
+      const int bi = (int)floor((f[i] - g.fmin[i]) * g.ibinw[i]);
       b[i] = min(max(bi, 0), g.nb[i] - 1);
     }
   }
@@ -228,25 +228,41 @@ template <class Out>
 __device__ __forceinline__ int64_t block_scan_chunks(const int* in, int64_t n, Out* out, int64_t* s_warp,
                                                      int* s_max, int* largest) {
   const int nth = blockDim.x;
-  const int64_t per = (n + nth - 1) / nth;
+  // chunks of a multiple of 4, loaded as int4 (in is 16-byte aligned)
+  const int64_t per = ((n + nth - 1) / nth + 3) & ~(int64_t)3;
   const int64_t i0 = min((int64_t)threadIdx.x * per, n), i1 = min(i0 + per, n);
+  auto load4 = [&](int64_t i, int (&v)[4]) {
+    if (i + 4 <= i1) {
+      const int4 q = __ldcg(reinterpret_cast<const int4*>(in + i));
+      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = i + k < i1 ? __ldcg(in + i + k) : 0;
+    }
+  };
   int64_t sum = 0;
   int mx = 0;
-#pragma unroll 8
-  for (int64_t i = i0; i < i1; ++i) {
-    const int v = __ldcg(in + i);
-    sum += v;
-    mx = max(mx, v);
+#pragma unroll 4
+  for (int64_t i = i0; i < i1; i += 4) {
+    int v[4];
+    load4(i, v);
+    sum += (int64_t)v[0] + v[1] + v[2] + v[3];
+    mx = max(max(mx, max(v[0], v[1])), max(v[2], v[3]));
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
   const int64_t inc = block_incl_scan(sum, s_warp);
   int64_t run = inc - sum;
-#pragma unroll 8
-  for (int64_t i = i0; i < i1; ++i) {
-    const int v = __ldcg(in + i);
-    out[i] = (Out)run;
-    run += v;
+  int next[4];
+  load4(i0, next);
+  for (int64_t i = i0; i < i1; i += 4) {  // the next four are loaded before these are stored
+    const int v[4] = {next[0], next[1], next[2], next[3]};
+    load4(i + 4, next);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k < i1) out[i + k] = (Out)run;
+      run += v[k];
+    }
   }
   __syncthreads();
   if (largest) {
@@ -274,7 +290,7 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   const double det = H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
                      H[2] * (H[3] * H[7] - H[4] * H[6]);
   int bad = fabs(det) < 1e-300;
-  const double id = bad ? 0.0 : 1.0 / det;
+  const double id = !anyp ? 1.0 : bad ? 0.0 : 1.0 / det;
   // inverse of the row-vector matrix: x = f H  =>  f = x H^-1
   g.Hinv[0] = (H[4] * H[8] - H[5] * H[7]) * id;
   g.Hinv[1] = (H[2] * H[7] - H[1] * H[8]) * id;
@@ -288,7 +304,7 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   for (int k = 0; k < 3; ++k) {
     g.per[k] = anyp ? (s.d_pbc[i * 3 + k] ? 1 : 0) : 0;
     g.fmin[k] = 0.0;
-    g.binw[k] = 1.0;
+    g.ibinw[k] = 1.0;
     g.nb[k] = 1;
     g.nrep[k] = 0;
   }
@@ -298,14 +314,14 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   for (int k = 0; k < 9; ++k)
     if (k % 4 == 0 ? !(H[k] > 0.0) : H[k] != 0.0) g.orth = 0;
   // perpendicular widths |det| / |cross of the other two rows| (SG:369-379)
-  double perp[3];
-  for (int k = 0; k < 3; ++k) {
-    const double* u = H + 3 * ((k + 1) % 3);
-    const double* v = H + 3 * ((k + 2) % 3);
-    const double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2], cz = u[0] * v[1] - u[1] * v[0];
-    perp[k] = fabs(det) / (sqrt(cx * cx + cy * cy + cz * cz) + 1e-12);
-    if (g.per[k]) g.nrep[k] = (int)ceil(cutoff / (perp[k] + 1e-12));  // SG:389
-  }
+  if (anyp)
+    for (int k = 0; k < 3; ++k) {
+      const double* u = H + 3 * ((k + 1) % 3);
+      const double* v = H + 3 * ((k + 2) % 3);
+      const double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2], cz = u[0] * v[1] - u[1] * v[0];
+      const double perp = fabs(det) / (sqrt(cx * cx + cy * cy + cz * cz) + 1e-12);
+      if (g.per[k]) g.nrep[k] = (int)ceil(cutoff / (perp + 1e-12));  // SG:389
+    }
   w.grids[i] = g;
   for (int k = 0; k < 3; ++k) {
     w.fbox[i * 6 + k] = ord_encode(INFINITY);
@@ -314,28 +330,32 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   if (bad && anyp) atomicOr(w.status, 1);
 }
 
+// FP32 keys in the order of the values they encode (NaN above infinity).
+__device__ __forceinline__ unsigned ord_key(float v) {
+  const unsigned b = __float_as_uint(v);
+  return (b >> 31) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ double key_value(unsigned e) {
+  return (double)__uint_as_float((e >> 31) ? (e & 0x7fffffffu) : ~e);
+}
+
 // Fractional bounding box of the open axes of every structure (warp-strided
-// over atoms base = first, first + stride, ...).  Atoms of a structure are
-// contiguous, so a warp keeps a running minimum and maximum while its atoms
-// belong to one structure and issues atomics only when the structure changes
-// or its atoms end.
+// over atoms base = first, first + stride, ...), in FP32 rounded outwards.
+// Atoms of a structure are contiguous, so a warp keeps a running minimum and
+// maximum while its atoms belong to one structure and issues atomics only when
+// the structure changes or its atoms end.
 __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& w, int64_t first, int64_t stride) {
   const int lane = threadIdx.x & 31;
   int cur = -1;  // structure of the running bounds (warp-uniform)
-  double lo[3], hi[3];
+  unsigned lo[3], hi[3];
   auto flush = [&]() {
     if (cur < 0) return;
-    for (int k = 0; k < 3; ++k) {
-      if (w.grids[cur].per[k]) continue;
-      double l = lo[k], h = hi[k];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        l = fmin(l, __shfl_xor_sync(0xffffffffu, l, o));
-        h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
-      }
-      if (lane == 0) {
-        atomicMin(&w.fbox[cur * 6 + k], ord_encode(l));
-        atomicMax(&w.fbox[cur * 6 + 3 + k], ord_encode(h));
+    for (int k = 0; k < 3; ++k) {
+      const unsigned l = __reduce_min_sync(0xffffffffu, lo[k]), h = __reduce_max_sync(0xffffffffu, hi[k]);
+      if (lane == 0 && !w.grids[cur].per[k]) {
+        atomicMin(&w.fbox[cur * 6 + k], ord_encode(key_value(l)));
+        atomicMax(&w.fbox[cur * 6 + 3 + k], ord_encode(key_value(h)));
       }
     }
   };
@@ -343,10 +363,16 @@ __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& 
     const int64_t a = base + lane;
     const bool valid = a < s.n_atoms;
     int si = 0;
-    double f[3] = {0.0, 0.0, 0.0};
+    unsigned kl[3], kh[3];
     if (valid) {
       si = struct_of_atom(s.d_atom_off, s.n_struct, a);
+      double f[3];
       to_frac(w.grids[si], s.d_positions[3 * a], s.d_positions[3 * a + 1], s.d_positions[3 * a + 2], f);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        kl[k] = ord_key(__double2float_rd(f[k]));
+        kh[k] = ord_key(__double2float_ru(f[k]));
+      }
     }
     const int si0 = __shfl_sync(0xffffffffu, si, 0);  // lane 0 is always valid here
     if (__all_sync(0xffffffffu, !valid || si == si0)) {
@@ -354,17 +380,16 @@ __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& 
         flush();
         cur = si0;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { lo[k] = INFINITY; hi[k] = -INFINITY; }
+        for (int k = 0; k < 3; ++k) { lo[k] = 0xffffffffu; hi[k] = 0u; }
       }
       if (valid)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { lo[k] = fmin(lo[k], f[k]); hi[k] = fmax(hi[k], f[k]); }
+        for (int k = 0; k < 3; ++k) { lo[k] = min(lo[k], kl[k]); hi[k] = max(hi[k], kh[k]); }
     } else if (valid) {
-      const GridDesc& g = w.grids[si];
       for (int k = 0; k < 3; ++k) {
-        if (g.per[k]) continue;
-        atomicMin(&w.fbox[si * 6 + k], ord_encode(f[k]));
-        atomicMax(&w.fbox[si * 6 + 3 + k], ord_encode(f[k]));
+        if (w.grids[si].per[k]) continue;
+        atomicMin(&w.fbox[si * 6 + k], ord_encode(key_value(kl[k])));
+        atomicMax(&w.fbox[si * 6 + 3 + k], ord_encode(key_value(kh[k])));
       }
     }
   }
@@ -376,34 +401,35 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
   const double* H = g.H;
   const double det = fabs(H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
                           H[2] * (H[3] * H[7] - H[4] * H[6]));
-  double perp[3];
-  for (int k = 0; k < 3; ++k) {
-    const double* u = H + 3 * ((k + 1) % 3);
-    const double* v = H + 3 * ((k + 2) % 3);
-    const double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2], cz = u[0] * v[1] - u[1] * v[0];
-    perp[k] = det / (sqrt(cx * cx + cy * cy + cz * cz) + 1e-300);
-  }
+  double perp[3] = {1.0, 1.0, 1.0}, binw[3];
+  if (g.any_per)
+    for (int k = 0; k < 3; ++k) {
+      const double* u = H + 3 * ((k + 1) % 3);
+      const double* v = H + 3 * ((k + 2) % 3);
+      const double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2], cz = u[0] * v[1] - u[1] * v[0];
+      perp[k] = det / (sqrt(cx * cx + cy * cy + cz * cz) + 1e-300);
+    }
   const int64_t A = s.d_atom_off[i + 1] - s.d_atom_off[i];
   // Bins of perpendicular width >= cutoff / 4; every bin row of the window is
   // trimmed to the cutoff sphere (visit).
-  const double bin_min = 0.25 * cutoff;
+  const double ibin_min = 4.0 / cutoff;
   double far[3];  // largest |fractional coordinate| of a wrapped atom, from the origin of the FP32 copies
   for (int k = 0; k < 3; ++k) {
     if (g.per[k]) {
-      const int nb = (int)floor(perp[k] / bin_min);
+      const int nb = (int)floor(perp[k] * ibin_min);
       g.nb[k] = min(max(nb, 1), 1023);
       g.fmin[k] = 0.0;
-      g.binw[k] = 1.0 / g.nb[k];
+      binw[k] = 1.0 / g.nb[k];
       far[k] = 1.0;
     } else {
       double lo = ord_decode(__ldcg(&w.fbox[i * 6 + k])), hi = ord_decode(__ldcg(&w.fbox[i * 6 + 3 + k]));
       if (!(hi >= lo)) { lo = 0.0; hi = 0.0; }  // no atoms
       const double span = hi - lo;
       far[k] = g.any_per ? fmax(fabs(lo), fabs(hi)) : span;
-      const int nb = (int)floor(span * perp[k] / bin_min);
+      const int nb = (int)floor(span * perp[k] * ibin_min);
       g.nb[k] = min(max(nb, 1), 1023);
       g.fmin[k] = lo;
-      g.binw[k] = span > 0.0 ? span / g.nb[k] : 1.0;
+      binw[k] = span > 1e-3 ? span / g.nb[k] : 1.0;  // (one bin below that)
     }
   }
   // cap the bin count of the structure at 2 A + 8
@@ -412,26 +438,27 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
     int k = 0;
     if (g.nb[1] > g.nb[k]) k = 1;
     if (g.nb[2] > g.nb[k]) k = 2;
-    const double span = g.binw[k] * g.nb[k];
+    const double span = binw[k] * g.nb[k];
     g.nb[k] = max(1, g.nb[k] / 2);
-    g.binw[k] = span / g.nb[k];
+    binw[k] = span / g.nb[k];
   }
   for (int k = 0; k < 3; ++k) {
-    g.wp[k] = (float)(g.binw[k] * perp[k]);
+    g.ibinw[k] = 1.0 / binw[k];
+    g.wp[k] = (float)(binw[k] * perp[k]);
     g.iw[k] = 1.0f / g.wp[k];
   }
   if (!g.orth) {
     const double la = sqrt(H[0] * H[0] + H[1] * H[1] + H[2] * H[2]);
     double p2 = 0.0, m2 = 0.0;
     for (int k = 0; k < 3; ++k) {
-      const double eb = g.binw[1] * H[3 + k], ec = g.binw[2] * H[6 + k];
+      const double eb = binw[1] * H[3 + k], ec = binw[2] * H[6 + k];
       g.dir[k] = (float)(la > 0.0 ? H[k] / la : 0.0);
       g.eb[k] = (float)eb;
       g.ec[k] = (float)ec;
       p2 += (eb + ec) * (eb + ec);
       m2 += (eb - ec) * (eb - ec);
     }
-    g.ialong = (float)(1.0 / (g.binw[0] * la));
+    g.ialong = (float)(1.0 / (binw[0] * la));
     g.rho = (float)(0.5 * sqrt(fmax(p2, m2)) + 1e-4);
   }
   // FP32 test: copies of coordinates up to m, shifts up to m + cutoff and differences up to the
@@ -445,7 +472,12 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
   g.c2lo = fits ? (float)(cutoff * cutoff - band) : -1.0f;
   g.c2hi = fits ? (float)(cutoff * cutoff + band) : INFINITY;
   w.grids[i] = g;
-  w.bins_per_struct[i] = g.nb[0] * g.nb[1] * g.nb[2];
+  const int bins = g.nb[0] * g.nb[1] * g.nb[2];
+  w.bins_per_struct[i] = bins;
+  if (s.n_struct == 1) {  // no scan needed
+    w.bin_off[0] = 0;
+    w.bin_off[1] = bins;
+  }
 }
 
 // Origin of the FP32 coordinates: the corner of an open structure's box, else
@@ -455,17 +487,33 @@ __device__ __forceinline__ void coord_origin(const GridDesc& g, double (&o)[3]) 
   for (int k = 0; k < 3; ++k) o[k] = g.any_per ? 0.0 : g.fmin[k];
 }
 
-__device__ __forceinline__ void bin_atom(const soapb_structs& s, const NLWork& w, int64_t a) {
-  const int si = struct_of_atom(s.d_atom_off, s.n_struct, a);
-  const GridDesc& g = w.grids[si];
-  int b[3], wr[3];
+// An atom's place: bin, order of arrival in it, wrapped position and wrap shift.
+struct AtomPlace {
+  int bin, arrival, wrap, si;
   double wp[3];
-  if (!locate(g, s.d_positions[3 * a], s.d_positions[3 * a + 1], s.d_positions[3 * a + 2], b, wr, wp))
+};
+
+__device__ __forceinline__ AtomPlace bin_atom(const soapb_structs& s, const NLWork& w, int64_t a) {
+  AtomPlace p;
+  p.si = struct_of_atom(s.d_atom_off, s.n_struct, a);
+  const GridDesc& g = w.grids[p.si];
+  int b[3], wr[3];
+  if (!locate(g, s.d_positions[3 * a], s.d_positions[3 * a + 1], s.d_positions[3 * a + 2], b, wr, p.wp))
     atomicOr(w.status, 2);
-  if ((wr[0] | wr[1] | wr[2]) != 0 && !g.wrapped) atomicOr(&w.grids[si].wrapped, 1);
-  const int64_t gb = w.bin_off[si] + ((int64_t)b[2] * g.nb[1] + b[1]) * g.nb[0] + b[0];
-  w.atom_bin[a] = (int)gb;
-  w.arrival[a] = atomicAdd(&w.bin_count[gb], 1);
+  if ((wr[0] | wr[1] | wr[2]) != 0 && !g.wrapped) atomicOr(&w.grids[p.si].wrapped, 1);
+  p.bin = (int)(w.bin_off[p.si] + ((int64_t)b[2] * g.nb[1] + b[1]) * g.nb[0] + b[0]);
+  p.arrival = atomicAdd(&w.bin_count[p.bin], 1);
+  p.wrap = pack3(wr[0], wr[1], wr[2]);
+  return p;
+}
+
+// The records of atom a in its final slot.
+__device__ __forceinline__ void write_records(const NLWork& w, const GridDesc& g, int a, int species, const double* wp,
+                                              int wrap, int slot) {
+  w.sorted_pos[slot] = make_double4(wp[0], wp[1], wp[2], pack_info(a, species, wrap));
+  double o[3];
+  coord_origin(g, o);
+  w.sorted_f[slot] = make_float4((float)(wp[0] - o[0]), (float)(wp[1] - o[1]), (float)(wp[2] - o[2]), 0.0f);
 }
 
 __device__ __forceinline__ void place_centre(const soapb_centres& c, const NLWork& w, int64_t i) {
@@ -495,11 +543,7 @@ __device__ __forceinline__ void gather_atom(const soapb_structs& s, const NLWork
   double wp[3];
   locate(g, s.d_positions[3 * (int64_t)a], s.d_positions[3 * (int64_t)a + 1], s.d_positions[3 * (int64_t)a + 2],
          b, wr, wp);
-  w.sorted_pos[s0 + rank] =
-      make_double4(wp[0], wp[1], wp[2], pack_info(a, s.d_species[a], pack3(wr[0], wr[1], wr[2])));
-  double o[3];
-  coord_origin(g, o);
-  w.sorted_f[s0 + rank] = make_float4((float)(wp[0] - o[0]), (float)(wp[1] - o[1]), (float)(wp[2] - o[2]), 0.0f);
+  write_records(w, g, a, s.d_species[a], wp, pack3(wr[0], wr[1], wr[2]), s0 + rank);
 }
 
 // ---- large inputs: one kernel per stage ----
@@ -521,7 +565,11 @@ __global__ void k_grid_setup(soapb_structs s, NLWork w, double cutoff) {
 
 __global__ void k_bin_atoms(soapb_structs s, soapb_centres c, NLWork w) {
   const int64_t nth = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (int64_t a = t0; a < s.n_atoms; a += nth) bin_atom(s, w, a);
+  for (int64_t a = t0; a < s.n_atoms; a += nth) {
+    const AtomPlace p = bin_atom(s, w, a);
+    w.atom_bin[a] = p.bin;
+    w.arrival[a] = p.arrival;
+  }
   for (int64_t i = t0; i < c.n_centres; i += nth) place_centre(c, w, i);
 }
 
@@ -568,17 +616,46 @@ __global__ void __launch_bounds__(kCellsThreads) k_cells(soapb_structs s, soapb_
   sync();
   for (int i = t0; i < s.n_struct; i += nth) grid_setup(s, w, cutoff, i);
   sync();
-  if (blockIdx.x == 0) block_scan_chunks(w.bins_per_struct, s.n_struct, w.bin_off, s_warp, s_max, nullptr);
-  sync();
-  for (int64_t a = t0; a < s.n_atoms; a += nth) bin_atom(s, w, a);
-  for (int64_t i = t0; i < c.n_centres; i += nth) place_centre(c, w, i);
+  if (s.n_struct > 1) {
+    if (blockIdx.x == 0) block_scan_chunks(w.bins_per_struct, s.n_struct, w.bin_off, s_warp, s_max, nullptr);
+    sync();
+  }
+  // an atom per thread stays in registers through the sort; centres are taken from the last
+  // thread on, so with threads for both neither waits for the other
+  const bool one = s.n_atoms <= nth;
+  AtomPlace p = {};
+  for (int64_t a = t0; a < s.n_atoms; a += nth) {
+    p = bin_atom(s, w, a);
+    if (!one) {
+      w.atom_bin[a] = p.bin;
+      w.arrival[a] = p.arrival;
+    }
+  }
+  for (int64_t i = nth - 1 - t0; i < c.n_centres; i += nth) place_centre(c, w, i);
   sync();
   if (blockIdx.x == 0)
     block_scan_chunks(w.bin_count, __ldcg(w.bin_off + s.n_struct), w.bin_start, s_warp, s_max, nullptr);
   sync();
-  for (int64_t a = t0; a < s.n_atoms; a += nth) w.sorted_atom[w.bin_start[w.atom_bin[a]] + w.arrival[a]] = (int)a;
-  sync();
-  for (int64_t slot = t0; slot < s.n_atoms; slot += nth) gather_atom(s, w, slot);
+  if (one) {
+    const bool mine = t0 < s.n_atoms;
+    int s0 = 0, n = 0;
+    if (mine) {
+      s0 = __ldcg(w.bin_start + p.bin);
+      n = __ldcg(w.bin_start + p.bin + 1) - s0;
+      w.sorted_atom[s0 + p.arrival] = t0;
+    }
+    sync();
+    if (mine) {
+      int rank = 0;
+#pragma unroll 4
+      for (int i = 0; i < n; ++i) rank += __ldcg(w.sorted_atom + s0 + i) < t0;
+      write_records(w, w.grids[p.si], t0, s.d_species[t0], p.wp, p.wrap, s0 + rank);
+    }
+  } else {
+    for (int64_t a = t0; a < s.n_atoms; a += nth) w.sorted_atom[w.bin_start[w.atom_bin[a]] + w.arrival[a]] = (int)a;
+    sync();
+    for (int64_t slot = t0; slot < s.n_atoms; slot += nth) gather_atom(s, w, slot);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -708,10 +785,7 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      // bins of an open axis are binw wide in the frame's coordinate: binw = wp for the identity
-      // frame; a mixed frame divides (few structures have one)
-      const double d = fr[k] - fma((double)cb[k], g.binw[k], g.fmin[k]);
-      f[k] = PER ? (float)(d / g.binw[k]) : (float)d * g.iw[k];
+      f[k] = (float)fma(fr[k] - g.fmin[k], g.ibinw[k], -(double)cb[k]);
       f[k] = fminf(fmaxf(f[k], -1e6f), 1e6f);
       const float reach = fmaf(R, g.iw[k], 1e-3f);
       lo[k] = (int)floorf(fmaxf(f[k] - reach, -1e6f));
@@ -1237,9 +1311,9 @@ constexpr int64_t kCellsFused = 16384;
 
 static int launch_cells(const soapb_structs& s, const soapb_centres& c, const NLWork& w, double cutoff,
                         cudaStream_t st) {
-  const int64_t most = s.n_atoms > c.n_centres ? s.n_atoms : c.n_centres;
-  int ctas = (int)((most + kCellsThreads - 1) / kCellsThreads);
-  ctas = ctas < 2 ? 1 : ctas < 4 ? 2 : ctas < 8 ? 4 : kCellsMaxCtas;
+  // a thread for every atom and centre, as far as one cluster goes
+  int ctas = 1;
+  while (ctas < kCellsMaxCtas && ctas * kCellsThreads < s.n_atoms + c.n_centres) ctas *= 2;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeClusterDimension;
   at.val.clusterDim.x = (unsigned)ctas;
