@@ -815,7 +815,8 @@ static JacLayout jac_layout(int64_t n_centres, int64_t n_pairs, int64_t n_inc, i
   auto take = [&](int64_t bytes) { const int64_t o = off; off = align_up(off + bytes, 256); return o; };
   L.counter = take(16);  // and the bitmap behind it: cleared together
   L.bitmap = take(4 * ((n_centres * n_inc + 31) / 32));
-  L.tasks = take(16 * ((attach ? 2 : 1) * n_pairs / kMinBatch + n_centres));
+  // a centre has at most entries / eb + 2 tasks (the parts before and after its own row)
+  L.tasks = take(16 * ((attach ? 2 : 1) * n_pairs / kMinBatch + 2 * n_centres + 1));
   L.ent = take(8 * (attach ? 2 : 1) * (n_pairs > 0 ? n_pairs : 1));
   L.ent_tmp = take(8 * (attach ? 2 : 1) * (n_pairs > 0 ? n_pairs : 1));
   L.total = off;
