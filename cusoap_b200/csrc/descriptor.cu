@@ -529,9 +529,9 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
 // a warp walk contiguous, equal parts of the centre's pair list, so each
 // stream sees only its part's species and segment runs and reloads its
 // coefficients rarely.  32 pairs (NP per stream) are staged per batch, one
-// per lane, as rows of solid harmonics in shared memory; rows have an odd
-// stride, so the streams' reads of the same slot k from their rows hit
-// different banks and the staging writes are conflict-free.
+// per lane, as rows of solid harmonics in shared memory; the rows of different
+// streams are 4 floats off each other, so the streams' reads of the same slots
+// hit different groups of four banks.
 //
 // Instruction issue is the bound (1M atoms: 35 warp instructions per pair, of
 // which 15 are the algorithmic FMAs), so two values go into each FMA: the
@@ -540,14 +540,16 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
 // is (YOrder).  The harmonics are staged without their normalisation
 // (MonicHarmonics), which the flush applies.  The pair loop is unrolled over
 // the batch and branches around the coefficient reloads: 27 warp instructions
-// per pair.  1M atoms (l_max 4): 14.65 -> 14.15 ms; 48 cells (l_max 6): 268 ->
+// per pair.  1M atoms (l_max 4): 14.65 -> 13.95 ms; 48 cells (l_max 6): 268 ->
 // 256 us; 3000 atoms (l_max 3): 73 -> 68 us.  The gain is less than the
 // instructions saved because packed and scalar FMAs with three distinct
 // operands share the register ports (2.3 - 2.7 and 1.6 - 1.9 cycles each,
 // measured) and 4 warps per scheduler leave 47 % of the issue slots to the
 // latency of the reloads and row reads.  Measured slower: the polynomials as
 // trees over t^2, t^4 (14.36 ms), two pairs per step (16.0 ms), 3 blocks per SM
-// (14.8 ms), the loop unrolled by 2 (14.7 ms).
+// (14.8 ms; l_max 6, where they spill: 288 against 268 us for the 48 cells), the
+// loop unrolled by 2 (14.7 ms); a block per centre (its sums would depend on
+// the number of centres, or cost 24 % where there are many).
 //
 // The r = 0 edge of the centre's own atom needs no test in the pair loop:
 // its solid harmonics are (Y00, 0, ..., 0) and its table value is

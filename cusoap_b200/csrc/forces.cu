@@ -395,7 +395,7 @@ struct PairCoefs {
 // against 2.3 - 2.7 for a packed one (measured), so the sums over n run packed: even and odd n
 // in the halves, added once per (l, m).  The table lies in 16-byte chunks by segment, so a
 // warp's load of a chunk touches the few lines of its lanes' segments (64-byte rows per segment
-// took 3.6 ms).  512 cells (l_max 6): 2.56 -> 2.2 ms a launch; 2001 atoms: 122 -> 98 us.  3
+// took 3.6 ms).  512 cells (l_max 6): 2.56 -> 2.27 ms a launch; 2001 atoms: 122 -> 115 us.  3
 // blocks per SM at 168 registers; 4 with small spills take 14 % longer at 2001 atoms.
 template <int L, bool FAST>
 __global__ void __launch_bounds__(128, 3) k_forces(ForceArgs a) {

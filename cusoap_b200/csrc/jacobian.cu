@@ -38,8 +38,8 @@
 // A task is one staged batch, not one centre: staging a batch is a chain of
 // barriers and shared-memory latencies, so with centres as tasks a centre's
 // batches ran one after the other in one block while most blocks had no centre
-// (50 centres of a 3000-atom cluster, F = 420: 452 us a launch, 179 us with
-// batches as tasks, 115 us to write the output; 1536 atoms, 12 GB: 2.35 and 2.08 ms).
+// (50 centres of a 3000-atom cluster, F = 420: 452 us a launch, 152 us as it is
+// now, 115 us of it to write the output; 1536 atoms, 12 GB: 2.35 and 1.76 ms).
 // Zero and nonzero rows are disjoint, so every element is written once and the
 // two roles never synchronise.
 #include "common.cuh"
@@ -557,7 +557,7 @@ __device__ __forceinline__ void quad_values(const JacArgs& a, const float* ed, i
 // dc / dx_d over the edges is formed first, D[d][s][n][lm] in shared memory
 // (3 N K FMAs an edge), and contracted with the coefficients once, instead of
 // 12 FMAs an edge for every feature in batches of eb that follow one another
-// (192 atoms, 130 edges a centre, cc: 195 us against 101 us, entries
+// (192 atoms, 130 edges a centre, cc: 193 us against 89 us, entries
 // included).  The edges are sorted by species, so a thread keeps its
 // (n, lm) in registers and adds it to D when the species changes.
 template <int L>
@@ -640,8 +640,8 @@ __device__ void centre_row(const JacArgs& a, int64_t p0, const unsigned long lon
 // stages, so its global loads run ahead: the next task is claimed while the
 // harmonics are computed, its keys are loaded during the radial stage and its
 // pairs during the contraction, and the centre's coefficient row comes in by
-// asynchronous copies.  1536 atoms: 2.08 ms without this, 1.83 ms with it,
-// entries included (1.81 ms to write the output).
+// asynchronous copies.  1536 atoms, entries (then 67 us) included: 2.08 ms
+// without this, 1.83 ms with it (12 GB take 1.81 ms at the measured copy rate).
 template <int L>
 __global__ void __launch_bounds__(256, 2) k_jacobian(JacArgs a) {
   using Sh = JacShape<L>;
