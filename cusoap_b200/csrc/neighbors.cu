@@ -5,8 +5,8 @@
 // (:382-396) and _perpendicular_lengths (:369-379).  The reference
 // replicates every atom over all (2 n_rep + 1)^3 image offsets and runs an
 // all-pairs GEMM distance test; here atoms are binned once per structure
-// (counting sort into bins in the cell's fractional frame, a quarter of the
-// cutoff wide, periodic axes wrapped) and each centre scans only the runs of
+// (counting sort into bins in the cell's fractional frame, a quarter or half of
+// the cutoff wide, periodic axes wrapped) and each centre scans only the runs of
 // bins that its cutoff sphere reaches, generating images on the fly.  The image
 // set is the reference's: image offset n = T - w_atom + w_centre (T the
 // cell-window shift, w the wrap shifts) must satisfy |n_i| <= n_rep_i on
@@ -14,7 +14,10 @@
 //
 // Pairs of a centre are written sorted by (neighbour species, radial table
 // segment) -- the order the descriptor kernels consume them in -- and, inside
-// a key, in a deterministic candidate order (bins are sorted by atom index).
+// a key, by bin (z, y, x, counted on through the images) and atom index.  That
+// order fixes the FP32 sums over a centre's neighbours, so the bins (grid_setup,
+// locate) are part of the results: they are computed in FP64, and another width
+// or another order of the images moves every gradient in its last digits.
 // Whether a candidate is within the cutoff is decided in FP64: FP32 copies of
 // the positions decide all candidates but those within their rounding of the
 // cutoff.  Differences are taken in FP64; rvec is stored FP32.
@@ -30,20 +33,23 @@ struct GridDesc {
   double H[9];     // rows: lattice a, b, c (identity for non-periodic structures)
   double Hinv[9];  // f_j = sum_i x_i Hinv[i*3+j]
   double fmin[3];  // bin origin in fractional coordinates (non-periodic axes)
-  double ibinw[3]; // bins per fractional unit
-  int nb[3], nrep[3];
-  signed char per[4];
-  int any_per;
-  int orth;     // diagonal frame (every non-periodic structure, rectangular cells)
-  int wrapped;  // an atom has a wrap shift: pairs need the image test
-  // FP32 geometry of the window (Angstrom): perpendicular bin widths and their reciprocals; for
-  // other than diagonal frames the direction of lattice row a, the reciprocal of a bin's length
-  // along it, the edges of a bin along b and c, and the largest distance of a bin's point from
-  // the bin row's axis
-  float wp[3], iw[3], dir[3], ialong, eb[3], ec[3], rho;
+  double binw[3];  // fractional bin width (locate)
+  double ibinw[3]; // bins per fractional unit (the window)
+  int nrep[3];
+  int wrapped;     // an atom has a wrap shift: pairs need the image test
+  short nb[3];
+  signed char per[3];
+  signed char orth;  // diagonal frame (every non-periodic structure, rectangular cells)
+  // FP32 geometry of the window (Angstrom): perpendicular bin widths; for other than diagonal
+  // frames the direction of lattice row a, the reciprocal of a bin's length along it, the edges
+  // of a bin along b and c, and the largest distance of a bin's point from the bin row's axis
+  float wp[3], dir[3], ialong, eb[3], ec[3], rho;
   // squared FP32 distances up to c2lo are within the cutoff, above c2hi beyond it
   float c2lo, c2hi;
+  __device__ __forceinline__ bool any_per() const { return (per[0] | per[1] | per[2]) != 0; }
 };
+// the workspace per structure must not grow: soapb_neighbors_noalloc has a fixed one
+static_assert(sizeof(GridDesc) <= 312, "GridDesc");
 
 struct NLWork {
   GridDesc* grids;
@@ -137,7 +143,7 @@ __device__ __forceinline__ bool locate(const GridDesc& g, double x, double y, do
       ok &= (w[i] > -512 && w[i] < 511);
     } else {
       w[i] = 0;
-      const int bi = (int)floor((f[i] - g.fmin[i]) * g.ibinw[i]);
+      const int bi = (int)floor((f[i] - g.fmin[i]) / g.binw[i]);
       b[i] = min(max(bi, 0), g.nb[i] - 1);
     }
   }
@@ -304,12 +310,11 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   for (int k = 0; k < 3; ++k) {
     g.per[k] = anyp ? (s.d_pbc[i * 3 + k] ? 1 : 0) : 0;
     g.fmin[k] = 0.0;
-    g.ibinw[k] = 1.0;
+    g.binw[k] = g.ibinw[k] = 1.0;
     g.nb[k] = 1;
     g.nrep[k] = 0;
   }
   g.wrapped = 0;
-  g.any_per = anyp;
   g.orth = 1;
   for (int k = 0; k < 9; ++k)
     if (k % 4 == 0 ? !(H[k] > 0.0) : H[k] != 0.0) g.orth = 0;
@@ -330,32 +335,31 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   if (bad && anyp) atomicOr(w.status, 1);
 }
 
-// FP32 keys in the order of the values they encode (NaN above infinity).
-__device__ __forceinline__ unsigned ord_key(float v) {
-  const unsigned b = __float_as_uint(v);
-  return (b >> 31) ? ~b : (b | 0x80000000u);
+// Smallest (largest) key of a warp: the high words, then the low words of those that have it.
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
+  const unsigned hi = (unsigned)(v >> 32), h = __reduce_min_sync(0xffffffffu, hi);
+  const unsigned l = __reduce_min_sync(0xffffffffu, hi == h ? (unsigned)v : 0xffffffffu);
+  return (unsigned long long)h << 32 | l;
 }
-__device__ __forceinline__ double key_value(unsigned e) {
-  return (double)__uint_as_float((e >> 31) ? (e & 0x7fffffffu) : ~e);
-}
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) { return ~warp_min(~v); }
 
 // Fractional bounding box of the open axes of every structure (warp-strided
-// over atoms base = first, first + stride, ...), in FP32 rounded outwards.
-// Atoms of a structure are contiguous, so a warp keeps a running minimum and
-// maximum while its atoms belong to one structure and issues atomics only when
-// the structure changes or its atoms end.
+// over atoms base = first, first + stride, ...), without atoms whose
+// coordinate is NaN.  Atoms of a structure are contiguous, so a warp keeps a
+// running minimum and maximum while its atoms belong to one structure and
+// issues atomics only when the structure changes or its atoms end.
 __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& w, int64_t first, int64_t stride) {
   const int lane = threadIdx.x & 31;
   int cur = -1;  // structure of the running bounds (warp-uniform)
-  unsigned lo[3], hi[3];
+  unsigned long long lo[3], hi[3];
   auto flush = [&]() {
     if (cur < 0) return;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const unsigned l = __reduce_min_sync(0xffffffffu, lo[k]), h = __reduce_max_sync(0xffffffffu, hi[k]);
+      const unsigned long long l = warp_min(lo[k]), h = warp_max(hi[k]);
       if (lane == 0 && !w.grids[cur].per[k]) {
-        atomicMin(&w.fbox[cur * 6 + k], ord_encode(key_value(l)));
-        atomicMax(&w.fbox[cur * 6 + 3 + k], ord_encode(key_value(h)));
+        atomicMin(&w.fbox[cur * 6 + k], l);
+        atomicMax(&w.fbox[cur * 6 + 3 + k], h);
       }
     }
   };
@@ -363,15 +367,16 @@ __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& 
     const int64_t a = base + lane;
     const bool valid = a < s.n_atoms;
     int si = 0;
-    unsigned kl[3], kh[3];
+    unsigned long long key[3];
+    bool num[3] = {false, false, false};
     if (valid) {
       si = struct_of_atom(s.d_atom_off, s.n_struct, a);
       double f[3];
       to_frac(w.grids[si], s.d_positions[3 * a], s.d_positions[3 * a + 1], s.d_positions[3 * a + 2], f);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        kl[k] = ord_key(__double2float_rd(f[k]));
-        kh[k] = ord_key(__double2float_ru(f[k]));
+        key[k] = ord_encode(f[k]);
+        num[k] = f[k] == f[k];
       }
     }
     const int si0 = __shfl_sync(0xffffffffu, si, 0);  // lane 0 is always valid here
@@ -380,16 +385,16 @@ __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& 
         flush();
         cur = si0;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { lo[k] = 0xffffffffu; hi[k] = 0u; }
+        for (int k = 0; k < 3; ++k) { lo[k] = ~0ull; hi[k] = 0ull; }
       }
-      if (valid)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { lo[k] = min(lo[k], kl[k]); hi[k] = max(hi[k], kh[k]); }
-    } else if (valid) {
+      for (int k = 0; k < 3; ++k)
+        if (num[k]) { lo[k] = min(lo[k], key[k]); hi[k] = max(hi[k], key[k]); }
+    } else {
       for (int k = 0; k < 3; ++k) {
-        if (w.grids[si].per[k]) continue;
-        atomicMin(&w.fbox[si * 6 + k], ord_encode(key_value(kl[k])));
-        atomicMax(&w.fbox[si * 6 + 3 + k], ord_encode(key_value(kh[k])));
+        if (!num[k] || w.grids[si].per[k]) continue;
+        atomicMin(&w.fbox[si * 6 + k], key[k]);
+        atomicMax(&w.fbox[si * 6 + 3 + k], key[k]);
       }
     }
   }
@@ -402,7 +407,7 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
   const double det = fabs(H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
                           H[2] * (H[3] * H[7] - H[4] * H[6]));
   double perp[3] = {1.0, 1.0, 1.0}, binw[3];
-  if (g.any_per)
+  if (g.any_per())
     for (int k = 0; k < 3; ++k) {
       const double* u = H + 3 * ((k + 1) % 3);
       const double* v = H + 3 * ((k + 2) % 3);
@@ -410,13 +415,17 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
       perp[k] = det / (sqrt(cx * cx + cy * cy + cz * cz) + 1e-300);
     }
   const int64_t A = s.d_atom_off[i + 1] - s.d_atom_off[i];
-  // Bins of perpendicular width >= cutoff / 4; every bin row of the window is
-  // trimmed to the cutoff sphere (visit).
-  const double ibin_min = 4.0 / cutoff;
+  // Bins of perpendicular width >= cutoff / 4 in diagonal frames, unless a
+  // periodic x axis would get fewer than 3 of them, and >= cutoff / 2 in the
+  // others; every bin row of the window is trimmed to the cutoff sphere (visit).
+  // The line is where it always was: the bins set the order of the pairs.
+  // Quarter bins everywhere would gain little (501 atoms, triclinic: count 18
+  // instead of 19 us, fill 22 instead of 23).
+  const double bin_min = (g.orth && !(g.per[0] && perp[0] < 0.75 * cutoff) ? 0.25 : 0.5) * cutoff;
   double far[3];  // largest |fractional coordinate| of a wrapped atom, from the origin of the FP32 copies
   for (int k = 0; k < 3; ++k) {
     if (g.per[k]) {
-      const int nb = (int)floor(perp[k] * ibin_min);
+      const int nb = (int)floor(perp[k] / bin_min);
       g.nb[k] = min(max(nb, 1), 1023);
       g.fmin[k] = 0.0;
       binw[k] = 1.0 / g.nb[k];
@@ -425,11 +434,11 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
       double lo = ord_decode(__ldcg(&w.fbox[i * 6 + k])), hi = ord_decode(__ldcg(&w.fbox[i * 6 + 3 + k]));
       if (!(hi >= lo)) { lo = 0.0; hi = 0.0; }  // no atoms
       const double span = hi - lo;
-      far[k] = g.any_per ? fmax(fabs(lo), fabs(hi)) : span;
-      const int nb = (int)floor(span * perp[k] * ibin_min);
+      far[k] = g.any_per() ? fmax(fabs(lo), fabs(hi)) : span;
+      const int nb = (int)floor(span * perp[k] / bin_min);
       g.nb[k] = min(max(nb, 1), 1023);
       g.fmin[k] = lo;
-      binw[k] = span > 1e-3 ? span / g.nb[k] : 1.0;  // (one bin below that)
+      binw[k] = span > 0.0 ? span / g.nb[k] : 1.0;
     }
   }
   // cap the bin count of the structure at 2 A + 8
@@ -443,9 +452,11 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
     binw[k] = span / g.nb[k];
   }
   for (int k = 0; k < 3; ++k) {
+    g.binw[k] = binw[k];
+    // a single bin of an open axis may be as thin as its atoms; the window takes it at least 1e-3 A wide
+    if (!g.per[k] && g.nb[k] == 1) binw[k] = fmax(binw[k], 1e-3 / perp[k]);
     g.ibinw[k] = 1.0 / binw[k];
     g.wp[k] = (float)(binw[k] * perp[k]);
-    g.iw[k] = 1.0f / g.wp[k];
   }
   if (!g.orth) {
     const double la = sqrt(H[0] * H[0] + H[1] * H[1] + H[2] * H[2]);
@@ -484,7 +495,7 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
 // the cell's (positions are wrapped into it).
 __device__ __forceinline__ void coord_origin(const GridDesc& g, double (&o)[3]) {
 #pragma unroll
-  for (int k = 0; k < 3; ++k) o[k] = g.any_per ? 0.0 : g.fmin[k];
+  for (int k = 0; k < 3; ++k) o[k] = g.any_per() ? 0.0 : g.fmin[k];
 }
 
 // An atom's place: bin, order of arrival in it, wrapped position and wrap shift.
@@ -746,21 +757,21 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 // bins within the cutoff are taken 32 at a time, one per lane, each trimmed to
 // the bins x that the cutoff sphere reaches (in FP32, against the cutoff plus
 // 1e-3 A, which covers its rounding).  A row is one run of bin-sorted atoms, or
-// in a cell periodic along x one per image Tx, two images at a time.  The runs
+// in a cell periodic along x one per image Tx, two of them to a lane.  The runs
 // form one candidate stream that all lanes walk 32 at a time: the runs that
 // start inside a tile give one bit each (an OR-reduction), and a lane's run is
 // the number of bits up to its own.  An FP32 copy of the position settles almost every
 // candidate; those within rounding of the cutoff (or near r = 0 in create(), or
 // all of them when wrap shifts make the image set matter) take the FP64 test.
-// Order: pairs of images, z rows, y, x, then atom index -- deterministic.
+// Order: z, y and x bins (through the images), then atom index.
 // fn(ok, slot, T) is called with all lanes.
 //
 // The enumeration is bound by instruction issue and the latency of the loads: 5
 // warp instructions per pair in the count, against 8 with FP64 row geometry
 // (six divisions and a square root a centre, one a row) and tests (1M atoms:
-// count 3.31 -> 2.2 ms; 48 periodic cells 85 -> 41 us).  Other than diagonal
-// frames scanned the full window of half-cutoff bins before, 4 candidates a
-// pair against 2 (501 atoms, triclinic: count 38 -> 19 us, fill 45 -> 23 us).
+// count 3.31 -> 2.2 ms; 48 periodic cells 85 -> 40 us).  Other than diagonal
+// frames scanned the full window of half-cutoff bins before
+// (501 atoms, triclinic: count 38 -> 19 us, fill 45 -> 23 us).
 // Writing the candidate slots of all runs into a list first, instead of finding
 // each lane's run, took as many instructions as it saved.
 template <bool PER, int UNROLL, class Fn>
@@ -772,7 +783,7 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
   const float R = (float)A.cutoff + 1e-3f;
   // the centre inside its bin (beyond [0, 1] for centres outside an open structure's box), and
   // the bins, from its own, that the cutoff reaches on each axis
-  float f[3];
+  float f[3], iw[3];
   int lo[3], hi[3];
   {
     double fr[3];
@@ -787,7 +798,8 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
     for (int k = 0; k < 3; ++k) {
       f[k] = (float)fma(fr[k] - g.fmin[k], g.ibinw[k], -(double)cb[k]);
       f[k] = fminf(fmaxf(f[k], -1e6f), 1e6f);
-      const float reach = fmaf(R, g.iw[k], 1e-3f);
+      iw[k] = 1.0f / g.wp[k];
+      const float reach = fmaf(R, iw[k], 1e-3f);
       lo[k] = (int)floorf(fmaxf(f[k] - reach, -1e6f));
       hi[k] = (int)floorf(fminf(f[k] + reach, 1e6f));
       if (!PER || !g.per[k]) {
@@ -813,15 +825,15 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
   const float near2 = A.mode == SOAPB_NL_CREATE ? 1e-4f : -1.0f;
   const unsigned upto = 0xffffffffu >> (31 - lane);
   const bool orth = !PER || g.orth;
-  const int groups = PER ? (nT + 1) >> 1 : 1;
-  for (int p0 = 0, tg = 0; tg < groups; p0 += 32) {
-    if (p0 >= nrows) {  // the next two images
-      if (nrows == 0) break;
-      p0 = -32;
-      ++tg;
-      continue;
+  const int groups = PER ? (nT + 1) >> 1 : 1;  // pairs of images of a row
+  const int nlanes = nrows * groups;
+  for (int p0 = 0; p0 < nlanes; p0 += 32) {
+    int row = p0 + lane, tg = 0;
+    if (PER && groups > 1) {
+      const int i = row;
+      row = i / groups;
+      tg = i - row * groups;
     }
-    const int row = p0 + lane;
     constexpr int Q = PER ? 2 : 1;  // runs of a row
     int len[Q], s0[Q];
     float4 sh[Q];
@@ -838,7 +850,7 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
         const float az = fmaxf(0.0f, fmaxf((float)dz - f[2], f[2] - (float)(dz + 1)) * g.wp[2]);
         ext2 = R * R - ay * ay - az * az;
         mid = f[0];
-        iwx = g.iw[0];
+        iwx = iw[0];
       } else {
         const float qy = (float)dy + 0.5f - f[1], qz = (float)dz + 0.5f - f[2];
         const float vx = qy * g.eb[0] + qz * g.ec[0], vy = qy * g.eb[1] + qz * g.ec[1],
@@ -972,7 +984,7 @@ __device__ __forceinline__ void visit(const VisitArgs& A, int64_t c, VisitMem& M
   C.g = A.grids + ci.y;
   C.cp = A.cpos[c];
   C.atom = ci.w;
-  C.per = C.g->any_per != 0;
+  C.per = C.g->any_per();
   unpack3(ci.z, C.cw);
   if (C.per) visit_runs<true, UNROLL>(A, M, C, ci, fn);
   else visit_runs<false, UNROLL>(A, M, C, ci, fn);
