@@ -308,8 +308,10 @@ __global__ void __launch_bounds__(512) k_basis_build(BasisDev a) {
   __syncthreads();
   for (int i = tid; N <= 8 && i < a.nseg * NF; i += blockDim.x) {  // i = seg NF + l N + n
     const int seg = i / NF, fn = i % NF, l = fn / N, n = fn % N, NP = stream_lanes(N);
-    for (int k = 0; k < kNCoef; ++k)
-      a.tab_p[(size_t)seg * pair_seg_floats(L, NP) + pair_coef(l, n, L, NP, k)] = a.tab_b[(size_t)i * kNCoef + k];
+    for (int k = 0; k < kNCoef; ++k) {
+      const int c = pair_coef(l, L, k);
+      a.tab_p[(size_t)seg * NP * (L + 1) * kNCoef + (c / 4 * NP + n) * 4 + c % 4] = a.tab_b[(size_t)i * kNCoef + k];
+    }
   }
   // self values: the centre's own Gaussian, w0 B_nl(0) (SG:765-819)
   for (int fn = tid; fn < NF; fn += blockDim.x) {

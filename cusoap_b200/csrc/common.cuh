@@ -87,30 +87,19 @@ __device__ __forceinline__ void load_coef(const float* __restrict__ tab, int seg
 // are ordered as operands of packed FMAs: the l pairs (l_max, l_max - 1),
 // (l_max - 2, l_max - 3), ... interleaved coefficient by coefficient {a_0(hi),
 // a_0(lo), a_1(hi), ...}, then l = 0 alone when l_max is even.  Segments hold
-// them as [16-byte chunk][lane][4 floats], n padded to the lanes of a stream: the
-// lanes load a chunk from consecutive addresses, at immediate offsets.  l_max 6
-// has two lanes per n: (6, 4), (1, -) in lane n and (5, 3), (2, 0) in lane NP + n.
+// them as [16-byte chunk][n][4 floats], n padded to the lanes of a stream: the
+// lanes load a chunk from consecutive addresses, at immediate offsets.
 __host__ __device__ inline int stream_lanes(int N) { return N <= 4 ? 4 : 8; }
-__host__ __device__ constexpr int pair_seg_floats(int L, int NP) { return NP * (L == 6 ? 8 : L + 1) * kNCoef; }
 inline int64_t off_tab_pairs(const soapb_basis* b) {
   return b->off_tab_b + align_up(4 * (int64_t)b->n_seg * b->n_max * (b->l_max + 1) * kNCoef, 256);
 }
 inline int64_t tab_pairs_bytes(const soapb_basis* b) {  // built for n_max <= 8
-  return b->n_max > 8 ? 0 : align_up(4 * (int64_t)b->n_seg * pair_seg_floats(b->l_max, stream_lanes(b->n_max)), 256);
+  return b->n_max > 8 ? 0 : align_up(4 * (int64_t)b->n_seg * stream_lanes(b->n_max) * (b->l_max + 1) * kNCoef, 256);
 }
-// Position of coefficient k of (l, n) in a segment.
-__host__ __device__ inline int pair_coef(int l, int n, int L, int NP, int k) {
-  int c, lane = n, lanes = NP;
-  if (L == 6) {
-    const int half = l == 5 || l == 3 || l == 2 || l == 0;
-    lane += half * NP;
-    lanes *= 2;
-    c = (l <= 2 ? 2 * kNCoef : 0) + 2 * k + (l == 4 || l == 3 || l == 0);
-  } else {
-    const int p = (L - l) >> 1;  // pair index, l = L - 2p (first) or L - 2p - 1 (second)
-    c = (L % 2 == 0 && l == 0) ? L * kNCoef + k : 2 * p * kNCoef + 2 * k + ((L - l) & 1);
-  }
-  return (c / 4 * lanes + lane) * 4 + c % 4;
+// Position of coefficient k of l among a radial index's coefficients.
+__host__ __device__ inline int pair_coef(int l, int L, int k) {
+  const int p = (L - l) >> 1;  // pair index, l = L - 2p (first) or L - 2p - 1 (second)
+  return (L % 2 == 0 && l == 0) ? L * kNCoef + k : 2 * p * kNCoef + 2 * k + ((L - l) & 1);
 }
 
 // ---- packed FP32 ----

@@ -415,58 +415,26 @@ struct YOrder {
     if (K % 2 == 1) lm[i++] = 0;
     for (int k = 0; k < K; ++k) pos[lm[k]] = k;
   }
+  static constexpr int l_of(int lm_) {
+    int l = 0;
+    while ((l + 1) * (l + 1) <= lm_) ++l;
+    return l;
+  }
 };
 template <int L>
 __device__ constexpr YOrder<L> kYOrder{};
-constexpr int l_of(int lm) {
-  int l = 0;
-  while ((l + 1) * (l + 1) <= lm) ++l;
-  return l;
-}
 
 // Epilogue of the radial-index-lane kernel: coefficient rows KR = K4 floats
 // apart (16-byte aligned), slots in YOrder.  For the power spectrum each lane
 // takes one (n, n') pair of a species block and contracts the two rows with
 // packed FMAs, reading them as float4; for each l the lanes write consecutive
-// features (coalesced).  With TILE 2 a lane takes columns n', n' + 1 of the
-// N x N block (a diagonal block skips those below the diagonal) and reads the
-// row of n once for both.  Same outputs and DScribe order as desc_epilogue.
-// Slot order of a coefficient row of KR floats (pads -1) and the grouping of its slot pairs by
-// their two l: pairs with the same l add into one packed sum.
-template <class Layout>
-struct RowSums {
-  static constexpr int KR = Layout::K4;
-  int key[KR / 2];            // sum of each slot pair, -1: both slots are pads
-  int la[KR / 2], lb[KR / 2]; // l of each sum's halves, -1: pads
-  int n;
-  constexpr RowSums() : key(), la(), lb(), n(0) {
-    const typename Layout::Order o;
-    for (int i = 0; i < KR / 2; ++i) {
-      const int ma = 2 * i < Layout::NLM ? o.lm[2 * i] : -1, mb = 2 * i + 1 < Layout::NLM ? o.lm[2 * i + 1] : -1;
-      const int a = ma < 0 ? -1 : l_of(ma), b = mb < 0 ? -1 : l_of(mb);
-      key[i] = -1;
-      if (a < 0 && b < 0) continue;
-      int k = 0;
-      while (k < n && !((a < 0 || la[k] < 0 || la[k] == a) && (b < 0 || lb[k] < 0 || lb[k] == b))) ++k;
-      if (k == n) {
-        la[k] = a;
-        lb[k] = b;
-        ++n;
-      }
-      if (la[k] < 0) la[k] = a;
-      if (lb[k] < 0) lb[k] = b;
-      key[i] = k;
-    }
-  }
-};
-template <class Layout>
-__device__ constexpr RowSums<Layout> kRowSums{};
-
-template <class Layout>
+// features (coalesced).  Same outputs and DScribe order as desc_epilogue.
+template <int L, int KR>
 __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, const float* cbuf, int lane,
                                                 const float* s_pref, const int* s_blk, const unsigned char* s_tri,
                                                 const unsigned char* s_pos) {
-  constexpr int L = Layout::L, K = (L + 1) * (L + 1), KR = Layout::K4;
+  constexpr int K = (L + 1) * (L + 1);
+  using YO = YOrder<L>;
   const int N = a.N, S = a.S;
   if (a.coeff_out) {
     float* crow = a.coeff_out + (size_t)c * S * N * K;
@@ -498,67 +466,62 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
     const int j = jj & 255, jd = jj >> 8;
     const bool diag = j == jd;
     const int np = diag ? N * (N + 1) / 2 : N * N;
-    constexpr int T = Layout::TILE;
-    const int nt = (N + T - 1) / T;
-    for (int p = lane; p < (T == 1 ? np : N * nt); p += 32) {
+    for (int p = lane; p < np; p += 32) {
       int n, nd;
-      if (T == 1 && diag) {
+      if (diag) {
         n = s_tri[2 * p];
         nd = s_tri[2 * p + 1];
       } else {
-        n = p / nt;
-        nd = T * (p - n * nt);
+        n = p / N;
+        nd = p - n * N;
       }
-      const int cols = min(T, N - nd);
-      if (T > 1 && diag && nd + cols <= n) continue;  // below the diagonal
       const ulonglong2* x2 = reinterpret_cast<const ulonglong2*>(cbuf + (j * N + n) * KR);
       const ulonglong2* y2 = reinterpret_cast<const ulonglong2*>(cbuf + (jd * N + nd) * KR);
-      constexpr int NSUM = RowSums<Layout>().n;
-      f32x2 sum[T][NSUM];
-      int y_off[T];  // a column past the end repeats the last one
+      // sums of slot pairs with the same two l: one per l pair of the table, then the leftovers
+      constexpr int NLP = YO::NLP, NSUM = NLP + (NLP + 1) / 2;
+      f32x2 sum[NSUM > 0 ? NSUM : 1];
 #pragma unroll
-      for (int c = 0; c < T; ++c) {
-        y_off[c] = min(c, cols - 1) * (KR / 4);
+      for (int k = 0; k < NSUM; ++k) sum[k] = 0ull;
+      float s0 = 0.0f;
 #pragma unroll
-        for (int k = 0; k < NSUM; ++k) sum[c][k] = 0ull;
-      }
+      for (int q = 0; q < (K + 3) / 4; ++q) {
+        const ulonglong2 u = x2[q], v = y2[q];
 #pragma unroll
-      for (int q = 0; q < KR / 4; ++q) {
-        const ulonglong2 u = x2[q];
-        const int k0 = kRowSums<Layout>.key[2 * q], k1 = kRowSums<Layout>.key[2 * q + 1];
-#pragma unroll
-        for (int c = 0; c < T; ++c) {
-          const ulonglong2 v = y2[y_off[c] + q];
-          if (k0 >= 0) sum[c][k0] = fma2(u.x, v.x, sum[c][k0]);
-          if (k1 >= 0) sum[c][k1] = fma2(u.y, v.y, sum[c][k1]);
+        for (int hh = 0; hh < 2; ++hh) {
+          const int i = 2 * q + hh;  // slot pair
+          if (i < YO::NS) {
+            const int la = YO::l_of(kYOrder<L>.lm[2 * i]), lb = YO::l_of(kYOrder<L>.lm[2 * i + 1]);
+            const int k = (lb == la - 1) ? (L - la) / 2 : NLP + (L - la) / 4;
+            sum[k] = fma2(hh ? u.y : u.x, hh ? v.y : v.x, sum[k]);
+          } else if (K % 2 == 1 && i == YO::NS) {
+            float xa, xb, ya, yb;
+            unpack2(hh ? u.y : u.x, xa, xb);
+            unpack2(hh ? v.y : v.x, ya, yb);
+            s0 = xa * ya;
+          }
         }
       }
+      float sl[L + 1];
+      sl[0] = s0;
 #pragma unroll
-      for (int c = 0; c < T; ++c) {
-        float sl[L + 1];
+      for (int k = 0; k < NLP; ++k) unpack2(sum[k], sl[L - 2 * k], sl[L - 2 * k - 1]);
 #pragma unroll
-        for (int l = 0; l <= L; ++l) sl[l] = 0.0f;
-#pragma unroll
-        for (int k = 0; k < NSUM; ++k) {
-          float xa, xb;
-          unpack2(sum[c][k], xa, xb);
-          if (kRowSums<Layout>.la[k] >= 0) sl[kRowSums<Layout>.la[k]] += xa;
-          if (kRowSums<Layout>.lb[k] >= 0) sl[kRowSums<Layout>.lb[k]] += xb;
-        }
-        if (c < cols && (T == 1 || !diag || nd + c >= n)) {
-          const int f = T == 1 ? p : (diag ? n * N - n * (n - 1) / 2 + nd + c - n : n * N + nd + c);
-          float* o = orow + fb0 + f;
-#pragma unroll
-          for (int l = 0; l <= L; ++l) o[l * np] = sl[l] * s_pref[l];
-        }
+      for (int k = NLP; k < NSUM; ++k) {
+        const int ha = L - 4 * (k - NLP), hb = (2 * (k - NLP) + 1 < NLP) ? ha - 2 : ha;
+        float xa, xb;
+        unpack2(sum[k], xa, xb);
+        sl[ha] += xa;
+        sl[hb] += xb;
       }
+      float* o = orow + fb0 + p;
+#pragma unroll
+      for (int l = 0; l <= L; ++l) o[l * np] = sl[l] * s_pref[l];
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Radial-index lanes (n_max <= 8, l_max <= 6; at l_max 6 two lanes share an n,
-// see HalfLanes): lane n of a stream owns the
+// Radial-index lanes (n_max <= 8, l_max <= 6): lane n of a stream owns the
 // radial index n and ALL K = (l_max+1)^2 accumulators c[n][lm] of it, so
 // every lane does the same work per pair -- l_max+1 Horner evaluations
 // (its functions (n, 0..l_max)) and K FMAs -- with no idle m slots.  NP
@@ -577,14 +540,15 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
 // is (YOrder).  The harmonics are staged without their normalisation
 // (MonicHarmonics), which the flush applies.  The pair loop is unrolled over
 // the batch and branches around the coefficient reloads: 27 warp instructions
-// per pair.  1M atoms (l_max 4): 14.65 -> 13.8 ms; 48 cells (l_max 6): 268 ->
-// 256 us before HalfLanes; 3000 atoms (l_max 3): 73 -> 68 us.  The gain is less than the
+// per pair.  1M atoms (l_max 4): 14.65 -> 13.95 ms; 48 cells (l_max 6): 268 ->
+// 256 us; 3000 atoms (l_max 3): 73 -> 68 us.  The gain is less than the
 // instructions saved because packed and scalar FMAs with three distinct
 // operands share the register ports (2.3 - 2.7 and 1.6 - 1.9 cycles each,
 // measured) and 4 warps per scheduler leave 47 % of the issue slots to the
 // latency of the reloads and row reads.  Measured slower: the polynomials as
 // trees over t^2, t^4 (14.36 ms), two pairs per step (16.0 ms), 3 blocks per SM
-// (14.8 ms), the loop unrolled by 2 (14.7 ms); a block per centre (its sums would depend on
+// (14.8 ms; l_max 6, where they spill: 288 against 268 us for the 48 cells), the
+// loop unrolled by 2 (14.7 ms); a block per centre (its sums would depend on
 // the number of centres, or cost 24 % where there are many).
 //
 // The r = 0 edge of the centre's own atom needs no test in the pair loop:
@@ -682,7 +646,7 @@ __device__ __forceinline__ void accumulate_pair(LaneSums<L>& acc, const LaneCoef
       const int i = 2 * q + hh;  // slot pair: compile time
       const f32x2 y = hh ? v.y : v.x;
       if (i < YO::NS) {
-        const int la = l_of(kYOrder<L>.lm[2 * i]), lb = l_of(kYOrder<L>.lm[2 * i + 1]);
+        const int la = YO::l_of(kYOrder<L>.lm[2 * i]), lb = YO::l_of(kYOrder<L>.lm[2 * i + 1]);
         if (lb == la - 1) {
           acc.p[i] = fma2(B[(L - la) / 2], y, acc.p[i]);
         } else {  // two slots of larger l left over: scalar FMAs on the halves (a packed operand would take two moves)
@@ -726,169 +690,10 @@ __device__ __forceinline__ void flush_row(float* row, const LaneSums<L>& acc) {
   }
 }
 
-// One lane per radial index: all K accumulators of n in a lane, NP lanes a stream.
-template <int L_, int NP>
-struct FullLanes : NShape<L_, NP> {
-  static constexpr int L = L_, NPL = NP, STREAM = NP, SEG = pair_seg_floats(L_, NP);
-  using Coefs = LaneCoefs<L, NP>;
-  using Sums = LaneSums<L>;
-  using Order = YOrder<L>;
-  static constexpr int NLM = NShape<L_, NP>::K;
-  static constexpr int TILE = 1;
-  static constexpr int UNROLL_FLUSH = 32 / NP, UNROLL_PAIRS = NP;
-  static constexpr int NORMS = 1;  // unused: the norms are immediates
-  __device__ __forceinline__ static void norm_table(float*) {}
-  static constexpr int kSumBatches = 0;  // sums run on until the species changes
-  __device__ static constexpr int pos_of(int lm) { return kYOrder<L>.pos[lm]; }
-  __device__ static constexpr int lm_at(int slot) { return slot < NLM ? kYOrder<L>.lm[slot] : -1; }
-  __host__ __device__ static constexpr int stream_off(int h) { return 4 * h; }
-  __device__ __forceinline__ static void accumulate(Sums& acc, const Coefs& cf, f32x2 t2, const float* yrow, int) {
-    accumulate_pair<L, NP, NShape<L_, NP>::K4>(acc, cf, t2, yrow);
-  }
-  __device__ __forceinline__ static void flush(float* row, const Sums& acc, int, const float*) {
-    flush_row<L, NShape<L_, NP>::K4>(row, acc);
-  }
-};
-
-// Two lanes per radial index, for l_max 6, whose 49 accumulators and 7 x 8 coefficients in one
-// lane leave room for 8 warps per SM, too few to cover the latency of the coefficient reloads
-// (a stream meets a new segment every few pairs) and of the row reads.  Lane A of n owns l =
-// 6, 4, 1 (25 accumulators), lane B l = 5, 3, 2, 0 (24): P0 = (6, 4) or (5, 3) and P1 = (1, -) or
-// (2, 0) are its Horner pairs, and its 12 slot pairs and one single slot take
-//   7 x P0; 2 x (6, 4) or (5, 2); 3 x (6, 1) or (5, 2); 6 or 0
-// so the two lanes run the same instructions on operands that differ in two selects a pair.
-// Row: A's 24 packed slots, B's 24 (one a pad), the two single ones, 2 pads.
-// 16 warps per SM instead of 8: 512 cells 2624 -> 2255 us, 48 cells 257 -> 236 us, 2001 atoms
-// 75 -> 72 us.  Shared-memory wavefronts bound it then (70 % of their rate), so the epilogue
-// takes two columns a lane (2470 -> 2270 us).  Half as many streams as with one lane walk twice
-// the pairs: sums are written out every 64 pairs, which keeps their rounding below that of one
-// lane per n (512-cell atoms 2.4e-7 against 2.6e-7; 2.7e-7 without) for 4 % of the time.
-struct HalfOrder {
-  static constexpr int K = 49, K4 = 52;
-  int lm[K4];   // lm at each position, -1: pad
-  int pos[K];
-  constexpr HalfOrder() : lm(), pos() {
-    int next[7] = {0, 1, 4, 9, 16, 25, 36};  // next lm of each l
-    for (int i = 0; i < 12; ++i) {
-      lm[2 * i] = next[6]++;
-      lm[2 * i + 1] = i < 9 ? next[4]++ : next[1]++;
-      lm[24 + 2 * i] = i < 11 ? next[5]++ : -1;
-      lm[24 + 2 * i + 1] = i < 7 ? next[3]++ : next[2]++;
-    }
-    lm[48] = next[6]++;
-    lm[49] = next[0]++;
-    lm[50] = lm[51] = -1;
-    for (int k = 0; k < K4; ++k)
-      if (lm[k] >= 0) pos[lm[k]] = k;
-  }
-};
-__device__ constexpr HalfOrder kHalfOrder{};
-struct HalfNorm {
-  float v[2][28];  // norms of a half's 24 packed slots and its single one (0: pad)
-  constexpr HalfNorm() : v() {
-    const HalfOrder o;
-    const detail::MonicNorm t = detail::make_monic_norm();
-    for (int g = 0; g < 2; ++g) {
-      for (int k = 0; k < 24; ++k) v[g][k] = o.lm[24 * g + k] < 0 ? 0.0f : t.v[o.lm[24 * g + k]];
-      v[g][24] = t.v[o.lm[48 + g]];
-    }
-  }
-};
-__device__ constexpr HalfNorm kHalfNorm{};
-
-template <int NP>
-struct HalfLanes {
-  static constexpr int L = 6, NPL = NP, STREAM = 2 * NP, SEG = pair_seg_floats(6, NP);
-  static constexpr int K = 49, K4 = 52, KC = 52, H = 32 / STREAM;
-  // the streams' rows STREAM apart start on the same group of four banks, A's and B's slots 6
-  // groups apart: offsets of 0, 1 (H = 2) and 0, 1, 4, 5 (H = 4) groups keep all apart
-  __host__ __device__ static constexpr int stream_off(int h) { return 4 * ((h & 1) + 4 * (h >> 1)); }
-  static constexpr int YF = 32 * K4 + 24;
-  __host__ __device__ static int warp_floats(int S, int N) { return (YF + 4 * 32 + S * N * KC + 3) & ~3; }
-  using Order = HalfOrder;
-  static constexpr int NLM = 52;
-  static constexpr int TILE = NP == 8 ? 2 : 1;  // epilogue columns a lane (n_max <= 4: too few pairs for two)
-  static constexpr int kSumBatches = 64 / STREAM;
-  // the code of 16 unrolled pairs and its flushes exceeds the instruction cache: 2340 us
-  static constexpr int UNROLL_FLUSH = 2, UNROLL_PAIRS = 8;
-  static constexpr int NORMS = 56;
-  __device__ __forceinline__ static void norm_table(float* s_norm) {
-    for (int k = threadIdx.x; k < NORMS; k += blockDim.x) s_norm[k] = kHalfNorm.v[k / 28][k % 28];
-  }
-  __device__ static constexpr int pos_of(int lm) { return kHalfOrder.pos[lm]; }
-  __device__ static constexpr int lm_at(int slot) { return kHalfOrder.lm[slot]; }
-  struct Coefs {
-    f32x2 p[2][kNCoef];
-    __device__ __forceinline__ void load(const float* __restrict__ blk) {
-      const ulonglong2* q = reinterpret_cast<const ulonglong2*>(blk);
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int k = 0; k < kNCoef; k += 2) {
-          const ulonglong2 v = __ldg(q + (i * (kNCoef / 2) + k / 2) * STREAM);
-          p[i][k] = v.x;
-          p[i][k + 1] = v.y;
-        }
-    }
-  };
-  struct Sums {
-    f32x2 p[12];
-    float s;
-    __device__ __forceinline__ void clear() {
-#pragma unroll
-      for (int i = 0; i < 12; ++i) p[i] = 0ull;
-      s = 0.0f;
-    }
-  };
-  __device__ __forceinline__ static void accumulate(Sums& acc, const Coefs& cf, f32x2 t2, const float* yrow, int g) {
-    f32x2 B[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      f32x2 b = cf.p[i][kDeg];
-#pragma unroll
-      for (int k = kDeg - 1; k >= 0; --k) b = fma2(b, t2, cf.p[i][k]);
-      B[i] = b;
-    }
-    float a0, a1, b0, b1;
-    unpack2(B[0], a0, a1);
-    unpack2(B[1], b0, b1);
-    const f32x2 q1 = pack2(a0, g ? b0 : a1), q2 = pack2(a0, b0);
-    const ulonglong2* yr = reinterpret_cast<const ulonglong2*>(yrow + 24 * g);
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      const ulonglong2 v = yr[q];
-      const int i = 2 * q;
-      acc.p[i] = fma2(i < 7 ? B[0] : (i < 9 ? q1 : q2), v.x, acc.p[i]);
-      acc.p[i + 1] = fma2(i + 1 < 7 ? B[0] : (i + 1 < 9 ? q1 : q2), v.y, acc.p[i + 1]);
-    }
-    acc.s = fmaf(g ? b1 : a0, yrow[48 + g], acc.s);
-  }
-  __device__ __forceinline__ static void flush(float* row, const Sums& acc, int g, const float* s_norm) {
-    float4* r4 = reinterpret_cast<float4*>(row + 24 * g);
-    const float4* n4 = reinterpret_cast<const float4*>(s_norm + 28 * g);
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      float4 v = r4[q];
-      float x0, x1, x2, x3;
-      unpack2(acc.p[2 * q], x0, x1);
-      unpack2(acc.p[2 * q + 1], x2, x3);
-      const float4 nrm = n4[q];
-      v.x = fmaf(x0, nrm.x, v.x);
-      v.y = fmaf(x1, nrm.y, v.y);
-      v.z = fmaf(x2, nrm.z, v.z);
-      v.w = fmaf(x3, nrm.w, v.w);
-      r4[q] = v;
-    }
-    row[48 + g] = fmaf(acc.s, s_norm[28 * g + 24], row[48 + g]);
-  }
-};
-
-template <class Sh>
+template <int L, int NP>
 __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
-  constexpr int L = Sh::L, K = Sh::K, K4 = Sh::K4, KC = Sh::KC, H = Sh::H;
-  __shared__ __align__(16) float s_norm[Sh::NORMS];
-  constexpr int UF = Sh::UNROLL_FLUSH, UJ = Sh::UNROLL_PAIRS;
-  constexpr int NP = Sh::STREAM;  // lanes of a stream, and its pairs per batch
+  using Sh = NShape<L, NP>;
+  constexpr int K = Sh::K, K4 = Sh::K4, KC = Sh::KC, H = Sh::H;
   extern __shared__ __align__(16) float sm[];
   __shared__ float s_pref[kMaxL + 1];
   __shared__ int s_blk[2 * kMaxBlocks];
@@ -903,18 +708,16 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
   int* spp = sg + 32;
   float* cbuf = Y + Sh::YF + 4 * 32;
   desc_tables<L>(a, s_pref, s_blk, s_tri);
-  for (int k = threadIdx.x; k < K4; k += blockDim.x)
-    if (Sh::lm_at(k) >= 0) s_pos[Sh::lm_at(k)] = (unsigned char)k;
-  Sh::norm_table(s_norm);
+  for (int k = threadIdx.x; k < K; k += blockDim.x) s_pos[kYOrder<L>.lm[k]] = (unsigned char)k;
   __syncthreads();
   const int h = lane / NP, n = lane - h * NP;
-  const int rn = n % Sh::NPL, g = n / Sh::NPL;  // radial index, and which of its lanes
-  const float* tab = a.tab_p + 4 * n;           // this lane's first chunk of segment 0
+  const float* tab = a.tab_p + 4 * n;  // this lane's first chunk of segment 0
+  constexpr int seg_floats = NP * (L + 1) * kNCoef;
   bool first = true;
-  const unsigned row_mask = NP == 16 ? 0x00010001u : (NP == 8 ? 0x01010101u : 0x11111111u);  // row j of every stream's block, shifted by j
-  const bool active = rn < N;
+  const unsigned row_mask = NP == 8 ? 0x01010101u : 0x11111111u;  // row j of every stream's block, shifted by j
+  const bool active = n < N;
   const int cbn = S * N * KC;
-  float4* myrow = reinterpret_cast<float4*>(Y + lane * K4 + Sh::stream_off(h));  // the row this lane stages
+  float4* myrow = reinterpret_cast<float4*>(Y + lane * K4 + 4 * h);  // the row this lane stages
 
   for (;;) {
     int64_t c;
@@ -934,16 +737,15 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
     const float4* pc = a.pairs + p0;
     const int s0 = (int)(((int64_t)P * h) / H), s1 = (int)(((int64_t)P * (h + 1)) / H);  // this stream's pairs
     const int rounds = (P + H - 1) / H;                                                  // longest stream
-    typename Sh::Sums acc;
+    LaneSums<L> acc;
     acc.clear();
-    typename Sh::Coefs cf = {};
+    LaneCoefs<L, NP> cf = {};
     // each stream starts on the species of its first pair, so the centre's first batch takes the
     // fast path unless a species changes inside it
     int cur_sp = (s0 < s1) ? (int)((unsigned)__float_as_int(__ldg(&pc[s0].w)) >> kAtomBits) : -1;
     int cur_seg = -1;
     __syncwarp();
 
-    int batches = 0;  // since the sums were last flushed for their length
     for (int base = 0; base < rounds; base += NP) {
       // stage: lane (h, n) takes pair s0 + base + n of its stream into row `lane`
       const int e = s0 + base + n;
@@ -956,8 +758,7 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
         // with R_00 scaled to 0: a zero row that adds nothing
         float yv[K4];
 #pragma unroll
-        for (int k = 0; k < K4; ++k)
-          if (Sh::lm_at(k) < 0) yv[k] = 0.0f;
+        for (int k = K; k < K4; ++k) yv[k] = 0.0f;
         const float4 pr = valid ? __ldg(pc + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         // the stream's pair of the next batch: into L1 while this batch runs
         if (e + NP < s1) asm volatile("prefetch.global.L1 [%0];" ::"l"(pc + e + NP));
@@ -965,9 +766,9 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
         const float r = sqrtf(r2);
         seg_coord(r, a.inv_h, a.nseg, seg, t);
         sp = (int)((unsigned)__float_as_int(pr.w) >> kAtomBits);
-        MonicHarmonics<L>::values(pr.x, pr.y, pr.z, r2, [&](int idx, float v) { yv[Sh::pos_of(idx)] = v; });
+        MonicHarmonics<L>::values(pr.x, pr.y, pr.z, r2, [&](int idx, float v) { yv[kYOrder<L>.pos[idx]] = v; });
         // the centre's own Gaussian (r = 0): w0 B_n0(0) Y00
-        yv[Sh::pos_of(0)] = valid ? ((r > 0.0f) ? 1.0f : a.self_ratio) : 0.0f;
+        yv[kYOrder<L>.pos[0]] = valid ? ((r > 0.0f) ? 1.0f : a.self_ratio) : 0.0f;
         if (!valid) {
           seg = -1;
           sp = -1;
@@ -1000,16 +801,16 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
       if (sp_chg == 0) {
         // no species change in any stream: t, a coefficient reload where the segment changes,
         // Horner and the K FMAs per pair
-#pragma unroll UJ
+#pragma unroll
         for (int j = 0; j < NP; ++j) {
           const int q = h * NP + j;
           // one warp-uniform branch for the streams' reloads, kept a branch by the barrier: the ten
           // loads of a reload are otherwise issued, predicated off, for every pair
           if (seg_chg & (row_mask << j)) {
             __syncwarp();
-            if (((seg_chg >> q) & 1u) && active) cf.load(tab + (size_t)sg[q] * Sh::SEG);
+            if (((seg_chg >> q) & 1u) && active) cf.load(tab + (size_t)sg[q] * seg_floats);
           }
-          Sh::accumulate(acc, cf, tt[q], Y + q * K4 + Sh::stream_off(h), g);
+          accumulate_pair<L, NP, K4>(acc, cf, tt[q], Y + q * K4 + 4 * h);
         }
       } else {
 #pragma unroll 1
@@ -1017,11 +818,11 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
           const int q = h * NP + j;
           const int spq = spp[q];
           if (__any_sync(0xffffffffu, spq != cur_sp)) {
-#pragma unroll UF
+#pragma unroll
             for (int hh = 0; hh < H; ++hh) {  // streams flush one after the other
               if (h == hh && spq != cur_sp) {
                 if (cur_sp >= 0 && active) {
-                  Sh::flush(cbuf + (cur_sp * N + rn) * KC, acc, g, s_norm);
+                  flush_row<L, K4>(cbuf + (cur_sp * N + n) * KC, acc);
                 }
                 acc.clear();
                 cur_sp = spq;
@@ -1031,48 +832,37 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
           }
           if (seg_chg & (row_mask << j)) {
             __syncwarp();
-            if (((seg_chg >> q) & 1u) && active) cf.load(tab + (size_t)sg[q] * Sh::SEG);
+            if (((seg_chg >> q) & 1u) && active) cf.load(tab + (size_t)sg[q] * seg_floats);
           }
-          Sh::accumulate(acc, cf, tt[q], Y + q * K4 + Sh::stream_off(h), g);
+          accumulate_pair<L, NP, K4>(acc, cf, tt[q], Y + q * K4 + 4 * h);
         }
       }
       cur_seg = sg[h * NP + NP - 1];
       cur_sp = spp[h * NP + NP - 1];
       __syncwarp();
-      // the centre's last batch, or sums of kSumBatches batches: into the coefficient buffer
-      if (base + NP >= rounds || (Sh::kSumBatches > 0 && ++batches == Sh::kSumBatches)) {
-        batches = 0;
-#pragma unroll UF
-        for (int hh = 0; hh < H; ++hh) {  // streams flush one after the other
-          if (h == hh && cur_sp >= 0 && active) Sh::flush(cbuf + (cur_sp * N + rn) * KC, acc, g, s_norm);
-          __syncwarp();
-        }
-        acc.clear();
-      }
     }
-    desc_epilogue_n<Sh>(a, c, cbuf, lane, s_pref, s_blk, s_tri, s_pos);
+#pragma unroll
+    for (int hh = 0; hh < H; ++hh) {
+      if (h == hh && cur_sp >= 0 && active) {
+        flush_row<L, K4>(cbuf + (cur_sp * N + n) * KC, acc);
+      }
+      __syncwarp();
+    }
+    desc_epilogue_n<L, KC>(a, c, cbuf, lane, s_pref, s_blk, s_tri, s_pos);
     __syncwarp();
   }
 }
 
+// l_max <= 4: 4 blocks of 4 warps per SM at 128 registers; l_max 5: 3 blocks; l_max 6: 2 blocks,
+// so its 49 accumulators and 7 x 8 coefficients per lane stay in registers (at 3 blocks they spill)
 template <int L, int NP>
-struct LanesFor {
-  using T = FullLanes<L, NP>;
-};
-template <int NP>
-struct LanesFor<6, NP> {
-  using T = HalfLanes<NP>;
-};
-
-// l_max <= 4 and 6: 4 blocks of 4 warps per SM at 128 registers; l_max 5: 3 blocks
-template <int L, int NP>
-__global__ void __launch_bounds__(128, L == 5 ? 3 : 4) k_descriptor_n(DescArgs a) {
-  descriptor_n_body<typename LanesFor<L, NP>::T>(a);
+__global__ void __launch_bounds__(128, (L <= 4) ? 4 : (L == 5 ? 3 : 2)) k_descriptor_n(DescArgs a) {
+  descriptor_n_body<L, NP>(a);
 }
 
 template <int L, int NP>
 static int launch_descriptor_n(const DescArgs& a, int wpb_tuned, cudaStream_t st) {
-  const int per_warp = 4 * LanesFor<L, NP>::T::warp_floats(a.S, a.N);
+  const int per_warp = 4 * NShape<L, NP>::warp_floats(a.S, a.N);
   if (per_warp % 16 != 0) return set_error(SOAPB_ERR_ARG, "descriptor: warp slice of %d B not 16-byte aligned", per_warp);
   int wpb = (200 * 1024) / per_warp;
   wpb = wpb > 4 ? 4 : wpb;
