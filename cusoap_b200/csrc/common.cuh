@@ -261,69 +261,6 @@ struct SolidHarmonics {
   }
 };
 
-// Real solid harmonics without their normalisation: R_lm = norm(l, m) R'_lm
-// with R'_l^{+-m} = q_l^m {Re, Im}(x + i y)^m and q_l^m monic in z,
-//   q_m^m = 1, q_{m+1}^m = z, q_l^m = z q_{l-1}^m - b r^2 q_{l-2}^m,
-//   b = (l+m-1)(l-m-1) / ((2l-1)(2l-3)).
-// A kernel that sums over neighbours applies norm once per sum: 42 instead of
-// 98 operations per vector at l_max 4.
-template <int L>
-struct MonicHarmonics {
-  template <class Store>
-  __device__ __forceinline__ static void values(float x, float y, float z, float r2, Store&& store) {
-    float C = 1.0f, S = 0.0f;
-#pragma unroll
-    for (int m = 0; m <= L; ++m) {
-      if (m == 1) {
-        C = x;
-        S = y;
-      } else if (m > 1) {
-        const float Cn = x * C - y * S;
-        S = x * S + y * C;
-        C = Cn;
-      }
-      float q2 = 0.0f, q1 = 0.0f, q = 1.0f;
-#pragma unroll
-      for (int l = m; l <= L; ++l) {
-        if (l == m + 1) {
-          q = z;
-        } else if (l > m + 1) {
-          const float b = (float)((l + m - 1) * (l - m - 1)) / (float)((2 * l - 1) * (2 * l - 3));
-          q = (l == m + 2) ? fmaf(-b, r2, z * z) : fmaf(-b, r2 * q2, z * q1);
-        }
-        if (m == 0) {
-          store(l * l + l, q);
-        } else {
-          store(l * l + l + m, l == m ? C : q * C);
-          store(l * l + l - m, l == m ? S : q * S);
-        }
-        q2 = q1;
-        q1 = q;
-      }
-    }
-  }
-};
-namespace detail {
-// norm(l, m) = N_lm x leading coefficient of Q_l^m in z, index l^2 + l + m
-struct MonicNorm {
-  float v[(kMaxL + 1) * (kMaxL + 1)];
-};
-constexpr MonicNorm make_monic_norm() {
-  MonicNorm t{};
-  for (int m = 0; m <= kMaxL; ++m) {
-    double lead = 1.0;
-    for (int k = 2 * m - 1; k > 0; k -= 2) lead *= (double)k;
-    for (int l = m; l <= kMaxL; ++l) {
-      if (l > m) lead *= (2.0 * l - 1.0) / (l - m);
-      const double base = (2.0 * l + 1.0) / (4.0 * kPi) * (m == 0 ? 1.0 : 2.0) * cfact(l - m) / cfact(l + m);
-      t.v[l * l + l + m] = t.v[l * l + l - m] = (float)(csqrt(base) * lead);
-    }
-  }
-  return t;
-}
-}  // namespace detail
-__device__ constexpr detail::MonicNorm kMonicNorm = detail::make_monic_norm();
-
 // Dispatch a functor templated on l_max (0..kMaxL).
 template <template <int> class F, class... Args>
 inline int dispatch_l(int l, Args&&... args) {

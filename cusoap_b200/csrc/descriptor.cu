@@ -537,11 +537,13 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
 // which 15 are the algorithmic FMAs), so two values go into each FMA: the
 // table interleaves pairs of l, whose Horner passes run packed, and the row's
 // slots are ordered so that most slot pairs take such a register pair as it
-// is (YOrder).  The harmonics are staged without their normalisation
-// (MonicHarmonics), which the flush applies.  The pair loop is unrolled over
-// the batch and branches around the coefficient reloads: 27 warp instructions
-// per pair.  1M atoms (l_max 4): 14.65 -> 13.95 ms; 48 cells (l_max 6): 268 ->
-// 256 us; 3000 atoms (l_max 3): 73 -> 68 us.  The gain is less than the
+// is (YOrder).  Each half of a packed FMA is the scalar one, every sum keeps its
+// order over the neighbours, and the harmonics are staged with their norms: the
+// coefficients are those of scalar FMAs bit by bit, as float64 position gradients
+// need (norms applied to the sums instead: 13.95 against 14.05 ms for 1M atoms, and
+// a larger error).  The pair loop is unrolled over the batch and branches around
+// the coefficient reloads.  1M atoms (l_max 4): 14.65 -> 14.05 ms; 48 cells
+// (l_max 6): 268 -> 262 us; 3000 atoms (l_max 3): 73 -> 70 us.  The gain is less than the
 // instructions saved because packed and scalar FMAs with three distinct
 // operands share the register ports (2.3 - 2.7 and 1.6 - 1.9 cycles each,
 // measured) and 4 warps per scheduler leave 47 % of the issue slots to the
@@ -615,7 +617,7 @@ struct LaneSums {
 };
 
 // One pair's contribution to a radial-index lane: the lane's l_max + 1 radial
-// functions at t (Horner, two l per FMA), then acc[lm] += B_l R'_lm over the
+// functions at t (Horner, two l per FMA), then acc[lm] += B_l R_lm over the
 // pair's harmonic row, two slots per FMA.
 template <int L, int NP, int K4>
 __device__ __forceinline__ void accumulate_pair(LaneSums<L>& acc, const LaneCoefs<L, NP>& cf, f32x2 t2,
@@ -666,9 +668,8 @@ __device__ __forceinline__ void accumulate_pair(LaneSums<L>& acc, const LaneCoef
   }
 }
 
-// Adds a lane's K accumulators, times the harmonics' norms, to its
-// 16-byte-aligned coefficient row (float4 read-modify-write; the row's K4 - K
-// padding slots stay zero).
+// Adds a lane's K accumulators to its 16-byte-aligned coefficient row (float4
+// read-modify-write; the row's K4 - K padding slots stay zero).
 template <int L, int K4>
 __device__ __forceinline__ void flush_row(float* row, const LaneSums<L>& acc) {
   constexpr int K = (L + 1) * (L + 1);
@@ -683,8 +684,8 @@ __device__ __forceinline__ void flush_row(float* row, const LaneSums<L>& acc) {
       float x = 0.0f, y = 0.0f;
       if (i < K / 2) unpack2(acc.p[i], x, y);
       else if (K % 2 == 1 && i == K / 2) x = acc.s;
-      if (2 * i < K) w[2 * hh] = fmaf(x, kMonicNorm.v[kYOrder<L>.lm[2 * i]], w[2 * hh]);
-      if (2 * i + 1 < K) w[2 * hh + 1] = fmaf(y, kMonicNorm.v[kYOrder<L>.lm[2 * i + 1]], w[2 * hh + 1]);
+      if (2 * i < K) w[2 * hh] += x;
+      if (2 * i + 1 < K) w[2 * hh + 1] += y;
     }
     r4[q] = make_float4(w[0], w[1], w[2], w[3]);
   }
@@ -762,13 +763,12 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
         const float4 pr = valid ? __ldg(pc + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         // the stream's pair of the next batch: into L1 while this batch runs
         if (e + NP < s1) asm volatile("prefetch.global.L1 [%0];" ::"l"(pc + e + NP));
-        const float r2 = pr.x * pr.x + pr.y * pr.y + pr.z * pr.z;
-        const float r = sqrtf(r2);
+        const float r = sqrtf(pr.x * pr.x + pr.y * pr.y + pr.z * pr.z);
         seg_coord(r, a.inv_h, a.nseg, seg, t);
         sp = (int)((unsigned)__float_as_int(pr.w) >> kAtomBits);
-        MonicHarmonics<L>::values(pr.x, pr.y, pr.z, r2, [&](int idx, float v) { yv[kYOrder<L>.pos[idx]] = v; });
+        SolidHarmonics<L>::values(pr.x, pr.y, pr.z, [&](int idx, float v) { yv[kYOrder<L>.pos[idx]] = v; });
         // the centre's own Gaussian (r = 0): w0 B_n0(0) Y00
-        yv[kYOrder<L>.pos[0]] = valid ? ((r > 0.0f) ? 1.0f : a.self_ratio) : 0.0f;
+        yv[kYOrder<L>.pos[0]] *= valid ? ((r > 0.0f) ? 1.0f : a.self_ratio) : 0.0f;
         if (!valid) {
           seg = -1;
           sp = -1;

@@ -36,6 +36,48 @@ PAIRS = {
     ("slab", 12.0, 150, 3, 3.0): "8b1417e9a2456a36e8aa58ac604bf0d0",
     ("slab", 12.0, 150, 3, 6.0): "0a40912671618706edacae3b1509cf77",
 }
+COEFFICIENTS = {
+    ("open", 14.0, 260, 2, 4, 0): "ae9d6416e85553d3", ("open", 14.0, 260, 2, 8, 1): "fab634dc0752b73c",
+    ("open", 14.0, 260, 2, 3, 2): "e6a0840a7efca690", ("open", 14.0, 260, 2, 4, 3): "a24cb3a7ec66c1a4",
+    ("open", 14.0, 260, 2, 8, 4): "e69bf4e45fbaee18", ("open", 14.0, 260, 2, 7, 5): "00a004a01588bea3",
+    ("open", 14.0, 260, 2, 8, 6): "576874da62956518", ("open", 14.0, 260, 2, 2, 6): "d90adcbd9fbd6e24",
+    ("open", 14.0, 260, 2, 10, 4): "02ddea5f327a89bd", ("open", 14.0, 260, 2, 8, 8): "ab830cc19375b6c7",
+    ("open", 5.0, 9, 4, 4, 0): "a3f24c8de86ff91c", ("open", 5.0, 9, 4, 8, 1): "9d83066bb015c6b4",
+    ("open", 5.0, 9, 4, 3, 2): "dc827ffa84584bfb", ("open", 5.0, 9, 4, 4, 3): "84e1a1ecce37a342",
+    ("open", 5.0, 9, 4, 8, 4): "a6f387f6c3c39596", ("open", 5.0, 9, 4, 7, 5): "6d37cff72f4f9d07",
+    ("open", 5.0, 9, 4, 8, 6): "6a3c9a8963cb51ab", ("open", 5.0, 9, 4, 2, 6): "a038cec30acb5ea7",
+    ("open", 5.0, 9, 4, 10, 4): "045a6f90b10ec5f4", ("open", 5.0, 9, 4, 8, 8): "b1aabe7de014665a",
+    ("cubic", 4.5, 11, 4, 4, 0): "67733d6b497a9e83", ("cubic", 4.5, 11, 4, 8, 1): "0e2888a0a4aa341f",
+    ("cubic", 4.5, 11, 4, 3, 2): "9dd299974689dbe9", ("cubic", 4.5, 11, 4, 4, 3): "ca009219b359311f",
+    ("cubic", 4.5, 11, 4, 8, 4): "4460289e32826ca0", ("cubic", 4.5, 11, 4, 7, 5): "9e739ff933e72414",
+    ("cubic", 4.5, 11, 4, 8, 6): "68dcd04bafd2df79", ("cubic", 4.5, 11, 4, 2, 6): "0c1f22a132aa489a",
+    ("cubic", 4.5, 11, 4, 10, 4): "e90d76c787a941e0", ("cubic", 4.5, 11, 4, 8, 8): "82c5ec77d2f5fa32",
+    ("cubic", 15.0, 300, 2, 4, 0): "f9f0ff141617e1ce", ("cubic", 15.0, 300, 2, 8, 1): "10e129186acfe562",
+    ("cubic", 15.0, 300, 2, 3, 2): "99606ce9bc6575ca", ("cubic", 15.0, 300, 2, 4, 3): "0cb7b88397c21d6b",
+    ("cubic", 15.0, 300, 2, 8, 4): "0eba5a046266e2f3", ("cubic", 15.0, 300, 2, 7, 5): "d77bb4bba924c9a9",
+    ("cubic", 15.0, 300, 2, 8, 6): "e994b7061c75097a", ("cubic", 15.0, 300, 2, 2, 6): "cd2c65b7873b2cda",
+    ("cubic", 15.0, 300, 2, 10, 4): "fdd678fe5463ae2e", ("cubic", 15.0, 300, 2, 8, 8): "28d543763998c535",
+    ("thin", 7.0, 40, 2, 4, 0): "2f2dfc574a1d614f", ("thin", 7.0, 40, 2, 8, 1): "eee7548ec658cacf",
+    ("thin", 7.0, 40, 2, 3, 2): "e2eddd5abade0789", ("thin", 7.0, 40, 2, 4, 3): "71e769e3b5c685bf",
+    ("thin", 7.0, 40, 2, 8, 4): "130d4be81714ce09", ("thin", 7.0, 40, 2, 7, 5): "e1fa9ec942794a42",
+    ("thin", 7.0, 40, 2, 8, 6): "d4846c47a354f85d", ("thin", 7.0, 40, 2, 2, 6): "91f925a2d4e227ae",
+    ("thin", 7.0, 40, 2, 10, 4): "e7e166542f6e0de3", ("thin", 7.0, 40, 2, 8, 8): "d4df1e2b45ed9e60",
+    ("triclinic", 6.0, 21, 2, 4, 0): "1737714268557601", ("triclinic", 6.0, 21, 2, 8, 1): "774244156029f3c8",
+    ("triclinic", 6.0, 21, 2, 3, 2): "02194f37cb1d7627", ("triclinic", 6.0, 21, 2, 4, 3): "264613f3eb224b61",
+    ("triclinic", 6.0, 21, 2, 8, 4): "5cc9b80bdd9cc9a5", ("triclinic", 6.0, 21, 2, 7, 5): "e06e9b75f3e890aa",
+    ("triclinic", 6.0, 21, 2, 8, 6): "ea8472c426c5e7db", ("triclinic", 6.0, 21, 2, 2, 6): "7cb25e7230ae1b33",
+    ("triclinic", 6.0, 21, 2, 10, 4): "7e62261c0ff65a17", ("triclinic", 6.0, 21, 2, 8, 8): "7b6fde5b6ebb26a8",
+    ("triclinic", 16.0, 330, 4, 4, 0): "112c9f688b09f2d6", ("triclinic", 16.0, 330, 4, 8, 1): "c53dbcc326d7ba3d",
+    ("triclinic", 16.0, 330, 4, 3, 2): "aa4d9b199cf62227", ("triclinic", 16.0, 330, 4, 4, 3): "427cb64aa4aeba6b",
+    ("triclinic", 16.0, 330, 4, 8, 4): "4002ef0b987aba05", ("triclinic", 16.0, 330, 4, 7, 5): "c71fefa41122083e",
+    ("triclinic", 16.0, 330, 4, 8, 6): "426dddfd5bff9ba0", ("triclinic", 16.0, 330, 4, 2, 6): "e1d3d3185ba031df",
+    ("triclinic", 16.0, 330, 4, 10, 4): "505e71980aec1ae9", ("triclinic", 16.0, 330, 4, 8, 8): "dec873998e04cad4",
+    ("slab", 12.0, 150, 3, 4, 0): "f5de31adc52f1cce", ("slab", 12.0, 150, 3, 8, 1): "0836b7d570e65b4f",
+    ("slab", 12.0, 150, 3, 3, 2): "4ddd82ec6229f191", ("slab", 12.0, 150, 3, 4, 3): "99c6563be0587636",
+    ("slab", 12.0, 150, 3, 8, 4): "f4f068b62a70d534", ("slab", 12.0, 150, 3, 7, 5): "d9b3e2a01711e082",
+    ("slab", 12.0, 150, 3, 8, 6): "54b9699fa995686d", ("slab", 12.0, 150, 3, 2, 6): "ce1afbeb42808416",
+    ("slab", 12.0, 150, 3, 10, 4): "18362965da9ddd29", ("slab", 12.0, 150, 3, 8, 8): "19e3079dbdce3d21",
+}
 
 
 def _digest(t):
@@ -65,6 +107,7 @@ def _soap(kind, n_species, **basis):
 # ones, an open axis; every l_max of the radial-index lanes with both stream widths, and beyond
 C_STRUCTURES = [("open", 14.0, 260, 2), ("open", 5.0, 9, 4), ("cubic", 4.5, 11, 4), ("cubic", 15.0, 300, 2),
                 ("thin", 7.0, 40, 2), ("triclinic", 6.0, 21, 2), ("triclinic", 16.0, 330, 4), ("slab", 12.0, 150, 3)]
+C_BASES = [(4, 0), (8, 1), (3, 2), (4, 3), (8, 4), (7, 5), (8, 6), (2, 6), (10, 4), (8, 8)]
 
 
 def pairs(structure, r_cut):
@@ -76,7 +119,19 @@ def pairs(structure, r_cut):
     return _digest(p.pair_off) + _digest(p.pairs.view(torch.int32))
 
 
+def coefficients(structure, basis):
+    kind, _, _, ns = structure
+    soap = _soap(kind, ns, r_cut=6.0, n_max=basis[0], l_max=basis[1], sigma=0.4, average="cc")
+    return _digest(soap.create(_structure(*structure)))
+
+
 @pytest.mark.parametrize("r_cut", [3.0, 6.0])
 @pytest.mark.parametrize("structure", C_STRUCTURES)
 def test_pair_lists(structure, r_cut):
     assert pairs(structure, r_cut) == PAIRS[structure + (r_cut,)]
+
+
+@pytest.mark.parametrize("basis", C_BASES)
+@pytest.mark.parametrize("structure", C_STRUCTURES)
+def test_coefficients(structure, basis):
+    assert coefficients(structure, basis) == COEFFICIENTS[structure + basis]
