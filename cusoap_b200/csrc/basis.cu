@@ -47,7 +47,7 @@ struct BasisDev {
   float* tab_b;
   float* tab_p;   // pair-interleaved copy of tab_b (pair_coef)
   float* tab_bh;
-  float* tabf;     // w B on half-width segments (force_coef)
+  float* tabf;     // function-major [fn][2 nseg][8]: w B on half-width segments
   float* selfv;    // w0 B_nl(0) per function fn = l N + n
   int* ftab;
   int* widx;
@@ -285,8 +285,8 @@ __global__ void __launch_bounds__(512) k_basis_build(BasisDev a) {
     cheb_to_mono(fb, a.tab_b + ((size_t)seg * NF + fn) * kNCoef);
     cheb_to_mono(fh, a.tab_bh + ((size_t)seg * NF + fn) * kNCoef);
   }
-  // Force table: w B alone on segments of half the width, by radial function;
-  // its polynomial's derivative is D (the derivative of a degree-7 interpolant
+  // Force table: w B alone on segments of half the width, function-major; its
+  // polynomial's derivative is D (the derivative of a degree-7 interpolant
   // loses about h per order, halving h wins back 2^7).
   for (int task = tid; task < 2 * a.nseg * NF; task += blockDim.x) {
     const int seg = task % (2 * a.nseg), fn = task / (2 * a.nseg);
@@ -297,13 +297,7 @@ __global__ void __launch_bounds__(512) k_basis_build(BasisDev a) {
       double d;
       exact_BD(a, s_gamma, s_pref, fn, r, f[j], d);
     }
-    float c[kNCoef];
-    cheb_to_mono(f, c);
-    const int l = fn / N, n = fn % N, fs = force_tab_stride(a.nseg);
-    for (int k = 0; k < kNCoef; ++k) {
-      a.tabf[force_coef(l, n, N, fs, seg, k)] = c[k];
-      if (N % 2 == 1 && n == N - 1) a.tabf[force_coef(l, n + 1, N + 1, fs, seg, k)] = 0.0f;
-    }
+    cheb_to_mono(f, a.tabf + ((size_t)fn * force_tab_stride(a.nseg) + seg) * kNCoef);
   }
   __syncthreads();
   for (int i = tid; N <= 8 && i < a.nseg * NF; i += blockDim.x) {  // i = seg NF + l N + n
@@ -354,8 +348,7 @@ __global__ void __launch_bounds__(512) k_basis_build(BasisDev a) {
       }
     } else {  // the force table: value, and derivative d/dr = (4 / h) d/dt
       const int sf = seg - a.nseg;
-      float cf[kNCoef];
-      for (int k = 0; k < kNCoef; ++k) cf[k] = a.tabf[force_coef(fn / N, fn % N, N, force_tab_stride(a.nseg), sf, k)];
+      const float* cf = a.tabf + ((size_t)fn * force_tab_stride(a.nseg) + sf) * kNCoef;
       for (int j = 0; j <= 16; ++j) {
         const double t = -1.0 + j / 8.0;
         const double r = (sf + 0.5 * (t + 1.0)) * (0.5 * a.h);
@@ -483,8 +476,7 @@ extern "C" int soapb_basis_plan(soapb_basis* b) {
   b->off_ftab = off; off = align_up(off + 4 * (int64_t)b->n_feat_ps, 256);
   b->off_widx = off; off = align_up(off + 4 * (int64_t)(L + 1) * (S * N) * (S * N), 256);
   b->off_err = off; off = align_up(off + 16, 256);
-  b->off_tabf = off; 
-  off = align_up(off + 4 * (int64_t)force_tab_stride(b->n_seg) * radial_pairs(N) * (L + 1) * 2 * kNCoef, 256);
+  b->off_tabf = off; off = align_up(off + 4 * (int64_t)force_tab_stride(b->n_seg) * NF * kNCoef, 256);
   b->off_self = off; off = align_up(off + 4 * (int64_t)NF, 256);
   b->off_poly = off;
   if (b->rbf == SOAPB_RBF_POLY) off = align_up(off + 8 * (int64_t)(2 + N) * b->quad_n, 256);

@@ -16,15 +16,6 @@ constexpr int kForceSegStride = 64;
 __host__ __device__ inline int force_tab_stride(int nseg) {
   return 2 * nseg <= kForceSegStride ? kForceSegStride : 2 * nseg;
 }
-// Force table: the coefficients of a pair of radial functions on a half segment,
-// interleaved one by one (operands of packed FMAs; the partner of an odd last n
-// is zero), in four 16-byte chunks: [l][pair][chunk][half segment][4 floats].
-// Lanes on neighbouring segments load a chunk from neighbouring addresses.
-__host__ __device__ inline int radial_pairs(int N) { return (N + 1) >> 1; }
-__host__ __device__ inline size_t force_coef(int l, int n, int N, int fstride, int seg, int k) {
-  const int i = 2 * k + (n & 1);
-  return (((size_t)(l * radial_pairs(N) + (n >> 1)) * 4 + i / 4) * fstride + seg) * 4 + i % 4;
-}
 constexpr int kMaxL = 12;
 constexpr int kMaxN = 16;
 constexpr int kMaxS = 16;

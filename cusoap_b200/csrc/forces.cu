@@ -27,7 +27,7 @@
 //               w B on half-width segments (value and derivative of the
 //               segment polynomial in one Horner pass; lanes on nearby
 //               segments share cache lines), its solid harmonics in registers,
-//               and contracts l by l, two radial indices per packed FMA:
+//               and contracts l by l:
 //                 xi_lm = sum_n G[s, n, lm] B_nl, zeta_lm = sum_n G[s, n, lm] Bhat_nl,
 //                 dE/drvec = sum_lm (rvec zeta_lm R_lm + xi_lm grad R_lm),
 //               the last sum accumulated as five per-edge scalars, with G
@@ -44,7 +44,7 @@ struct ForceArgs {
   const float* coeff;
   const float* dEdp;
   const int* centre_atom;
-  const float* tabf;     // w B on half-width segments (force_coef); its derivative is D = d(w B)/dr
+  const float* tabf;     // [fn][nsegf][8]: w B on half-width segments; its derivative is D = d(w B)/dr
   const int* widx;
   const int* ftab;       // l-major pair indices of every feature
   float* G;              // (n_centres, S N K) workspace
@@ -363,58 +363,45 @@ __global__ void k_adjoint_g_cc(ForceArgs a, int K) {
   }
 }
 
-// Shared memory of a warp of k_forces: G of the centre with radial indices in
-// pairs, {G[n], G[n + 1]} for each (species, pair, lm), every l block padded to
-// an even number of slots (16-byte aligned): slot of lm = lm + l.
+// Q_l^m table and the powers (x + i y)^m of one vector, for per-(l, m) solid
+// harmonics and gradients (same recurrences and normalisation as SolidHarmonics).
 template <int L>
-struct ForceShape {
-  static constexpr int K = (L + 1) * (L + 1);
-  static constexpr int KP = (L + 1) * (L + 2);
-  __host__ __device__ static int warp_floats(int S, int N) { return S * radial_pairs(N) * 2 * KP; }
-};
-
-// Coefficients of a pair of radial functions on one half segment.
-struct PairCoefs {
-  f32x2 c[kNCoef];
-  __device__ __forceinline__ void load(const float* __restrict__ p, int fstride) {
-    const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p);
+struct EdgeHarmonics {
+  static constexpr int NQ = (L + 1) * (L + 2) / 2;
+  float Q[NQ], C[L + 1], Sn[L + 1];
+  __device__ __forceinline__ EdgeHarmonics(float x, float y, float z) {
+    SolidHarmonics<L>::legendre(z, x * x + y * y + z * z, Q);
+    C[0] = 1.0f;
+    Sn[0] = 0.0f;
 #pragma unroll
-    for (int k = 0; k < kNCoef; k += 2) {
-      const ulonglong2 v = __ldg(q + k / 2 * fstride);
-      c[k] = v.x;
-      c[k + 1] = v.y;
+    for (int m = 1; m <= L; ++m) {
+      C[m] = x * C[m - 1] - y * Sn[m - 1];
+      Sn[m] = x * Sn[m - 1] + y * C[m - 1];
     }
   }
 };
 
+template <int L>
+struct ForceShape {
+  static constexpr int K = (L + 1) * (L + 1);
+  static constexpr int KC = K | 1;
+  __host__ __device__ static int warp_floats(int S, int N) { return (S * N * KC + 3) & ~3; }
+};
+
 // FAST: n_max 8 and the table stride kForceSegStride at compile time, so the radial loop
 // unrolls fully and every G and table offset is an immediate; else both come from the arguments.
-//
-// FMAs bound this kernel (per edge 28 N (L+1) in the radial functions and their derivatives, 4
-// N K in the contractions), and an FMA with three distinct registers takes 1.6 - 1.9 cycles
-// against 2.3 - 2.7 for a packed one (measured), so the sums over n run packed: even and odd n
-// in the halves, added once per (l, m).  The table lies in 16-byte chunks by segment, so a
-// warp's load of a chunk touches the few lines of its lanes' segments (64-byte rows per segment
-// took 3.6 ms).  512 cells (l_max 6): 2.56 -> 2.27 ms a launch; 2001 atoms: 122 -> 115 us.  3
-// blocks per SM at 168 registers; 4 with small spills take 14 % longer at 2001 atoms.
+// The radial indices are added one after the other: float64 position gradients depend on that
+// order.  Even and odd ones in the halves of packed FMAs took 2.27 instead of 2.56 ms for 512
+// cells and moved every gradient by 4e-7.
 template <int L, bool FAST>
-__global__ void __launch_bounds__(128, 3) k_forces(ForceArgs a) {
+__global__ void __launch_bounds__(128) k_forces(ForceArgs a) {
   using Sh = ForceShape<L>;
-  constexpr int K = Sh::K, KP = Sh::KP;
+  constexpr int K = Sh::K, KC = Sh::KC;
   extern __shared__ __align__(16) float sm[];
-  __shared__ unsigned char s_slot[K];  // slot of each lm
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int N = FAST ? 8 : a.N, NP = radial_pairs(N), SN = a.S * N, nsegf = a.nsegf;
+  const int N = FAST ? 8 : a.N, SN = a.S * N, nsegf = a.nsegf;
   const int fstride = FAST ? kForceSegStride : a.fstride;
   float* G = sm + (size_t)wid * Sh::warp_floats(a.S, N);
-  for (int lm = threadIdx.x; lm < K; lm += blockDim.x) {
-    int l = 0;
-    while ((l + 1) * (l + 1) <= lm) ++l;
-    s_slot[lm] = (unsigned char)(lm + l);
-  }
-  // padding slots and the partner of an odd last n stay zero
-  for (int i = lane; i < Sh::warp_floats(a.S, N); i += 32) G[i] = 0.0f;
-  __syncthreads();
 
   for (;;) {
     int c32 = 0;
@@ -423,11 +410,7 @@ __global__ void __launch_bounds__(128, 3) k_forces(ForceArgs a) {
     if (c >= a.n_centres) break;
     const int catom = a.attach ? a.centre_atom[c] : -1;
     const float* grow = a.G + (size_t)c * SN * K;
-#pragma unroll 4
-    for (int i = lane; i < SN * K; i += 32) {
-      const int sn = i / K, sp = sn / N, n = sn - sp * N;
-      G[((sp * NP + (n >> 1)) * KP + s_slot[i - sn * K]) * 2 + (n & 1)] = __ldg(grow + i);
-    }
+    for (int i = lane; i < SN * K; i += 32) G[(i / K) * KC + (i % K)] = grow[i];
     __syncwarp();
 
     float fcx = 0.f, fcy = 0.f, fcz = 0.f;
@@ -439,104 +422,65 @@ __global__ void __launch_bounds__(128, 3) k_forces(ForceArgs a) {
       const float x = pr.x, y = pr.y, z = pr.z;
       int seg;
       float t;
-      const float r2 = x * x + y * y + z * z, r = sqrtf(r2);
+      const float r = sqrtf(x * x + y * y + z * z);
       seg_coord(r, a.inv_hf, nsegf, seg, t);
       const bool self_edge = !(r > 0.0f);
       const float dt_r = self_edge ? 0.0f : 2.0f * a.inv_hf / r;  // (dt/dr) / r: Bhat = D / r = dP/dt dt_r
-      const f32x2 t2 = pack2(t, t);
-      const float* gs = G + (size_t)sp * NP * 2 * KP;
-      const float* tab = a.tabf + 4 * seg;
+      const EdgeHarmonics<L> eh(x, y, z);
+      const float* gs = G + sp * N * KC;
       // sum_lm (rvec zeta_lm R_lm + xi_lm grad R_lm), grouped: with u = nrm xi, Phi_m = C_m or S_m,
       //   P1 = sum u Q_{l-1}^{m+1} Phi_m, Pz = sum u (l+m) Q_{l-1}^m Phi_m, Rz = sum zeta R_lm,
       //   Tx, Ty = sum m Q_l^m (d Phi_m / dx, dy) u:  dE/drvec = (x (Rz - P1) + Tx, y (Rz - P1) + Ty, z Rz + Pz)
       float P1 = 0.f, Pz = 0.f, Rz = 0.f, Tx = 0.f, Ty = 0.f;
-      // (x + i y)^m and Q_l^m (as SolidHarmonics) of this l and the one below
-      float C[L + 1], Sn[L + 1], Q[L + 1], Qm[L + 1], Qmm[L + 1];
-      C[0] = 1.0f;
-      Sn[0] = 0.0f;
 #pragma unroll
       for (int l = 0; l <= L; ++l) {
+        float xi[2 * L + 1], ze[2 * L + 1];
 #pragma unroll
-        for (int m = 0; m <= l; ++m) {
-          Qmm[m] = (m <= l - 2) ? Qm[m] : 0.0f;
-          Qm[m] = (m <= l - 1) ? Q[m] : 0.0f;
-        }
-        if (l > 0) {
-          C[l] = x * C[l - 1] - y * Sn[l - 1];
-          Sn[l] = x * Sn[l - 1] + y * C[l - 1];
-        }
+        for (int m = 0; m < 2 * l + 1; ++m) { xi[m] = 0.0f; ze[m] = 0.0f; }
+        // function-major table: row fn = l N + n, column seg.  The next function's two
+        // float4 loads are issued before this one is evaluated, so their latency overlaps
+        // the Horner pass and the G contraction.
+        float cf[kNCoef];
+        load_coef(a.tabf, l * N, seg, fstride, cf);
+#pragma unroll (FAST ? 8 : 2)
+        for (int n = 0; n < N; ++n) {
+          float nx[kNCoef];
+          load_coef(a.tabf, l * N + min(n + 1, N - 1), seg, fstride, nx);
+          float p, dp;
+          horner7_d(cf, t, p, dp);
 #pragma unroll
-        for (int m = 0; m <= l; ++m) {
-          if (m == l) {
-            float dfact = 1.0f;
-#pragma unroll
-            for (int k = 2 * m - 1; k > 0; k -= 2) dfact *= (float)k;
-            Q[m] = dfact;
-          } else if (m == l - 1) {
-            Q[m] = (float)(2 * m + 1) * z * Qm[m];
-          } else {
-            Q[m] = (float)(2 * l - 1) / (float)(l - m) * z * Qm[m] - (float)(l + m - 1) / (float)(l - m) * r2 * Qmm[m];
-          }
-        }
-        f32x2 xi[2 * L + 1], ze[2 * L + 1];
-#pragma unroll
-        for (int m = 0; m < 2 * l + 1; ++m) xi[m] = ze[m] = 0ull;
-        // The next pair's loads are issued before this one is evaluated, so their latency
-        // overlaps the polynomials and the G contraction.
-        const float* tl = tab + (size_t)l * NP * fstride * 16;
-        PairCoefs cf;
-        cf.load(tl, fstride);
-#pragma unroll (FAST ? 4 : 1)
-        for (int p = 0; p < NP; ++p) {
-          PairCoefs nx;
-          nx.load(tl + (size_t)min(p + 1, NP - 1) * fstride * 16, fstride);
-          f32x2 v = fma2(cf.c[7], t2, cf.c[6]), d = cf.c[7];
-#pragma unroll
-          for (int k = kDeg - 2; k >= 0; --k) {
-            d = fma2(d, t2, v);
-            v = fma2(v, t2, cf.c[k]);
-          }
-          cf = nx;
+          for (int k = 0; k < kNCoef; ++k) cf[k] = nx[k];
           // xi sums G B, ze sums G dB/dt: the factor (dt/dr) / r of zeta is applied once, to Rz
-          const ulonglong2* gr = reinterpret_cast<const ulonglong2*>(gs + (p * KP + l * l + l) * 2);
+          const float* gr = gs + n * KC + l * l;
 #pragma unroll
-          for (int m = 0; m < 2 * l + 2; m += 2) {
-            const ulonglong2 g = gr[m / 2];
-            xi[m] = fma2(g.x, v, xi[m]);
-            ze[m] = fma2(g.x, d, ze[m]);
-            if (m + 1 < 2 * l + 1) {
-              xi[m + 1] = fma2(g.y, v, xi[m + 1]);
-              ze[m + 1] = fma2(g.y, d, ze[m + 1]);
-            }
+          for (int m = 0; m < 2 * l + 1; ++m) {
+            const float gv = gr[m];
+            xi[m] = fmaf(gv, p, xi[m]);
+            ze[m] = fmaf(gv, dp, ze[m]);
           }
         }
         // this l's terms of the grouped sums (xi / ze index l + m within the l block)
-        auto both = [](f32x2 w) {
-          float even, odd;
-          unpack2(w, even, odd);
-          return even + odd;
-        };
 #pragma unroll
         for (int m = 0; m <= l; ++m) {
           const float nrm = c_shnorm[l * (kMaxL + 1) + m];
-          const float q = Q[m];
-          const float qp = (l >= 1 && m + 1 <= l - 1) ? Qm[m + 1] : 0.0f;
-          const float qz = (l >= 1 && m <= l - 1) ? (float)(l + m) * Qm[m] : 0.0f;
+          const float q = eh.Q[tri(l, m)];
+          const float qp = (l >= 1 && m + 1 <= l - 1) ? eh.Q[tri(l - 1, m + 1)] : 0.0f;
+          const float qz = (l >= 1 && m <= l - 1) ? (float)(l + m) * eh.Q[tri(l - 1, m)] : 0.0f;
           if (m == 0) {
-            const float u = nrm * both(xi[l]);
+            const float u = nrm * xi[l];
             P1 = fmaf(u, qp, P1);
             Pz = fmaf(u, qz, Pz);
-            Rz = fmaf(nrm * q, both(ze[l]), Rz);
+            Rz = fmaf(nrm * q, ze[l], Rz);
           } else {
-            const float Cm = C[m], Sm = Sn[m], Cp = C[m - 1], Sp = Sn[m - 1];
-            const float u = nrm * both(xi[l + m]), v = nrm * both(xi[l - m]);
+            const float Cm = eh.C[m], Sm = eh.Sn[m], Cp = eh.C[m - 1], Sp = eh.Sn[m - 1];
+            const float u = nrm * xi[l + m], v = nrm * xi[l - m];
             const float U = fmaf(u, Cm, v * Sm);
             P1 = fmaf(U, qp, P1);
             Pz = fmaf(U, qz, Pz);
             const float mq = (float)m * q;
             Tx = fmaf(mq, fmaf(u, Cp, v * Sp), Tx);
             Ty = fmaf(mq, fmaf(v, Cp, -u * Sp), Ty);
-            Rz = fmaf(nrm * q, fmaf(both(ze[l + m]), Cm, both(ze[l - m]) * Sm), Rz);
+            Rz = fmaf(nrm * q, fmaf(ze[l + m], Cm, ze[l - m] * Sm), Rz);
           }
         }
       }

@@ -78,6 +78,32 @@ COEFFICIENTS = {
     ("slab", 12.0, 150, 3, 8, 6): "54b9699fa995686d", ("slab", 12.0, 150, 3, 2, 6): "ce1afbeb42808416",
     ("slab", 12.0, 150, 3, 10, 4): "18362965da9ddd29", ("slab", 12.0, 150, 3, 8, 8): "19e3079dbdce3d21",
 }
+GRADIENTS = {
+    ("open", 7.0, 45, 2, 8, 6): "0e4c131121a1829b", ("open", 7.0, 45, 2, 8, 3): "6fecf0c5a716f983",
+    ("open", 7.0, 45, 2, 8, 1): "6c7e3c4069012cac", ("open", 7.0, 45, 2, 4, 3): "b554970a29a1fc8c",
+    ("open", 7.0, 45, 2, 7, 4): "6aa82edc58c8b95d", ("open", 7.0, 45, 2, 1, 2): "059dbd5a5c45c8c4",
+    ("open", 7.0, 45, 2, 6, 6): "3feb0586d616894f", ("open", 7.0, 45, 2, 8, 9): "aab829f2d81072e0",
+    ("open", 7.0, 45, 2, 5, 8): "6eea00807697286a", ("open", 7.0, 45, 2, 10, 9): "b45c2ec9678715c1",
+    ("open", 7.0, 45, 2, 8, 12): "36e4467c4017f36b",
+    ("cubic", 8.4, 60, 3, 8, 6): "00069470f4ac900a", ("cubic", 8.4, 60, 3, 8, 3): "5df8b18a0e890450",
+    ("cubic", 8.4, 60, 3, 8, 1): "d41d9fbce057bafd", ("cubic", 8.4, 60, 3, 4, 3): "dde284545268f745",
+    ("cubic", 8.4, 60, 3, 7, 4): "b6fe14a5e932f517", ("cubic", 8.4, 60, 3, 1, 2): "088b698ba9018f3e",
+    ("cubic", 8.4, 60, 3, 6, 6): "0920ace064257b20", ("cubic", 8.4, 60, 3, 8, 9): "3c677abdc6240923",
+    ("cubic", 8.4, 60, 3, 5, 8): "f83a647a24d35920", ("cubic", 8.4, 60, 3, 10, 9): "1fbe41256e57b421",
+    ("cubic", 8.4, 60, 3, 8, 12): "0aa5298a40b7a876",
+    ("triclinic", 9.0, 75, 2, 8, 6): "9738954def761f57", ("triclinic", 9.0, 75, 2, 8, 3): "870d8a42bf2a0c98",
+    ("triclinic", 9.0, 75, 2, 8, 1): "d4afcd04f4d325bd", ("triclinic", 9.0, 75, 2, 4, 3): "84b58eb2e22c5736",
+    ("triclinic", 9.0, 75, 2, 7, 4): "a181dc909a36420e", ("triclinic", 9.0, 75, 2, 1, 2): "5aa3d09443a8a481",
+    ("triclinic", 9.0, 75, 2, 6, 6): "88bd991a25990ea6", ("triclinic", 9.0, 75, 2, 8, 9): "4c4c76c07d0acd43",
+    ("triclinic", 9.0, 75, 2, 5, 8): "b53cd7eff6912d30", ("triclinic", 9.0, 75, 2, 10, 9): "4e44535bea287642",
+    ("triclinic", 9.0, 75, 2, 8, 12): "bb1507c5e4d59103",
+    ("slab", 9.6, 60, 2, 8, 6): "3c1e4d5e756b17b1", ("slab", 9.6, 60, 2, 8, 3): "cd19ad4867cb0973",
+    ("slab", 9.6, 60, 2, 8, 1): "3df4eebeb5f7bba3", ("slab", 9.6, 60, 2, 4, 3): "259a63cd04e5a67a",
+    ("slab", 9.6, 60, 2, 7, 4): "ee2ab37b8929cfcd", ("slab", 9.6, 60, 2, 1, 2): "cea884d9f5cea66c",
+    ("slab", 9.6, 60, 2, 6, 6): "cc35ba3141689072", ("slab", 9.6, 60, 2, 8, 9): "a1b2648f4f94acbe",
+    ("slab", 9.6, 60, 2, 5, 8): "72232f60c063be68", ("slab", 9.6, 60, 2, 10, 9): "7506b0d9b5c8265a",
+    ("slab", 9.6, 60, 2, 8, 12): "5449e267224e6d63",
+}
 
 
 def _digest(t):
@@ -108,6 +134,9 @@ def _soap(kind, n_species, **basis):
 C_STRUCTURES = [("open", 14.0, 260, 2), ("open", 5.0, 9, 4), ("cubic", 4.5, 11, 4), ("cubic", 15.0, 300, 2),
                 ("thin", 7.0, 40, 2), ("triclinic", 6.0, 21, 2), ("triclinic", 16.0, 330, 4), ("slab", 12.0, 150, 3)]
 C_BASES = [(4, 0), (8, 1), (3, 2), (4, 3), (8, 4), (7, 5), (8, 6), (2, 6), (10, 4), (8, 8)]
+# (cells at least twice the 4.1 A cutoff wide)
+G_STRUCTURES = [("open", 7.0, 45, 2), ("cubic", 8.4, 60, 3), ("triclinic", 9.0, 75, 2), ("slab", 9.6, 60, 2)]
+G_BASES = [(8, 6), (8, 3), (8, 1), (4, 3), (7, 4), (1, 2), (6, 6), (8, 9), (5, 8), (10, 9), (8, 12)]
 
 
 def pairs(structure, r_cut):
@@ -125,6 +154,20 @@ def coefficients(structure, basis):
     return _digest(soap.create(_structure(*structure)))
 
 
+def gradients(structure, basis):
+    kind, _, n, ns = structure
+    soap = _soap(kind, ns, r_cut=3.0, n_max=basis[0], l_max=basis[1], sigma=0.3)
+    s = _structure(*structure)
+    w = torch.as_tensor(np.random.default_rng(3).standard_normal(soap.get_number_of_features()), dtype=torch.float32,
+                        device="cuda")
+    out = []
+    for c in (0, n // 2, n - 1):
+        pos = torch.as_tensor(s["positions"], device="cuda").requires_grad_(True)
+        (soap.create(dict(s, positions=pos))[c] @ w).backward()
+        out.append(pos.grad)
+    return _digest(torch.stack(out))
+
+
 @pytest.mark.parametrize("r_cut", [3.0, 6.0])
 @pytest.mark.parametrize("structure", C_STRUCTURES)
 def test_pair_lists(structure, r_cut):
@@ -135,3 +178,9 @@ def test_pair_lists(structure, r_cut):
 @pytest.mark.parametrize("structure", C_STRUCTURES)
 def test_coefficients(structure, basis):
     assert coefficients(structure, basis) == COEFFICIENTS[structure + basis]
+
+
+@pytest.mark.parametrize("basis", G_BASES)
+@pytest.mark.parametrize("structure", G_STRUCTURES)
+def test_gradient_of_one_centre(structure, basis):
+    assert gradients(structure, basis) == GRADIENTS[structure + basis]
