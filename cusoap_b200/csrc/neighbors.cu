@@ -39,7 +39,8 @@ struct GridDesc {
   int wrapped;     // an atom has a wrap shift: pairs need the image test
   short nb[3];
   signed char per[3];
-  signed char orth;  // diagonal frame (every non-periodic structure, rectangular cells)
+  signed char orth;  // 1: diagonal frame (every non-periodic structure, rectangular cells), 0: another,
+                     // -1: no frame (a periodic cell without a volume, or not of numbers): no pairs
   // FP32 geometry of the window (Angstrom): perpendicular bin widths; for other than diagonal
   // frames the direction of lattice row a, the reciprocal of a bin's length along it, the edges
   // of a bin along b and c, and the largest distance of a bin's point from the bin row's axis
@@ -318,6 +319,7 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   g.orth = 1;
   for (int k = 0; k < 9; ++k)
     if (k % 4 == 0 ? !(H[k] > 0.0) : H[k] != 0.0) g.orth = 0;
+  if (anyp && !(fabs(det) >= 1e-300 && fabs(det) < INFINITY)) g.orth = -1;
   // perpendicular widths |det| / |cross of the other two rows| (SG:369-379)
   if (anyp)
     for (int k = 0; k < 3; ++k) {
@@ -403,6 +405,14 @@ __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& 
 
 __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork& w, double cutoff, int i) {
   GridDesc g = w.grids[i];
+  if (g.orth < 0) {  // one bin of which nothing is visited (its window would have no end)
+    w.bins_per_struct[i] = 1;
+    if (s.n_struct == 1) {
+      w.bin_off[0] = 0;
+      w.bin_off[1] = 1;
+    }
+    return;
+  }
   const double* H = g.H;
   const double det = fabs(H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
                           H[2] * (H[3] * H[7] - H[4] * H[6]));
@@ -814,8 +824,9 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
     T0 = floordiv(cb[0] + lo[0], g.nb[0]);
     nT = floordiv(cb[0] + hi[0], g.nb[0]) - T0 + 1;
   }
-  const int nrows = (ny > 0 && nz > 0 && lo[0] <= hi[0]) ? ny * nz : 0;
-  const float inv_ny = 1.0f / (float)ny;  // quotients below 2^20: exact with the half added
+  // (a cell far thinner than 1e-2 A can have more rows than an int holds)
+  const int64_t nrows64 = (ny > 0 && nz > 0 && lo[0] <= hi[0]) ? (int64_t)ny * nz : 0;
+  const float inv_ny = 1.0f / (float)ny;  // row / ny for rows below 2^20: exact with the half added
   const int boff = (int)A.bin_off[ci.y];
   double o[3];
   coord_origin(g, o);
@@ -826,7 +837,7 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
   const unsigned upto = 0xffffffffu >> (31 - lane);
   const bool orth = !PER || g.orth;
   const int groups = PER ? (nT + 1) >> 1 : 1;  // pairs of images of a row
-  const int nlanes = nrows * groups;
+  const int nrows = (int)min(nrows64, (int64_t)0x7fffff00 / groups), nlanes = nrows * groups;
   for (int p0 = 0; p0 < nlanes; p0 += 32) {
     int row = p0 + lane, tg = 0;
     if (PER && groups > 1) {
@@ -843,7 +854,7 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
       sh[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     if (row < nrows) {
-      const int iz = (int)(((float)row + 0.5f) * inv_ny), dz = lo[2] + iz, dy = lo[1] + row - iz * ny;
+      const int iz = nrows <= 1 << 20 ? (int)(((float)row + 0.5f) * inv_ny) : row / ny, dz = lo[2] + iz, dy = lo[1] + row - iz * ny;
       float mid, ext2, slack = 1e-3f, iwx;  // x range in bins from the centre's: mid +- (sqrt(ext2) iwx + slack)
       if (orth) {
         const float ay = fmaxf(0.0f, fmaxf((float)dy - f[1], f[1] - (float)(dy + 1)) * g.wp[1]);
@@ -985,6 +996,7 @@ __device__ __forceinline__ void visit(const VisitArgs& A, int64_t c, VisitMem& M
   C.cp = A.cpos[c];
   C.atom = ci.w;
   C.per = C.g->any_per();
+  if (C.g->orth < 0) return;
   unpack3(ci.z, C.cw);
   if (C.per) visit_runs<true, UNROLL>(A, M, C, ci, fn);
   else visit_runs<false, UNROLL>(A, M, C, ci, fn);

@@ -25,3 +25,39 @@ def test_atom_without_a_position(at):
     want = soap.create({"positions": pos, "atomic_numbers": Z})
     got = soap.create({"positions": np.insert(pos, at, [np.nan, 1.0, 2.0], 0), "atomic_numbers": np.insert(Z, at, 1)})
     assert torch.equal(got[torch.arange(201, device="cuda") != at], want)
+
+
+FLAT = {"no third vector": np.diag([9.0, 8.0, 0.0]), "no cell": np.zeros((3, 3)),
+        "in a plane": np.array([[9.0, 0.0, 0.0], [0.0, 8.0, 0.0], [9.0, 8.0, 0.0]])}
+
+
+@pytest.mark.parametrize("n", [1, 60, 17000])  # (the last one builds its lists in separate launches)
+@pytest.mark.parametrize("pbc", [[True, True, True], [True, True, False], [False, False, True]])
+@pytest.mark.parametrize("cell", FLAT)
+def test_cell_without_a_volume(cell, pbc, n):
+    soap = _soap(True)
+    pos, Z = _atoms(n, 3)
+    flat = {"positions": pos, "atomic_numbers": Z, "cell": FLAT[cell], "pbc": pbc}
+    with pytest.raises(ValueError, match="singular cell"):
+        soap.create(flat)
+    if n == 60:
+        good = dict(flat, cell=np.eye(3) * 11.0)
+        want = soap.create(good)
+        with pytest.raises(ValueError, match="singular cell"):
+            soap.create([good, flat, good])
+        with pytest.raises(ValueError, match="singular cell"):
+            soap.derivatives(flat, centers=[0])
+        assert torch.equal(soap.create(good), want)
+        # not periodic: the cell is not read
+        assert soap.create(dict(flat, pbc=[False] * 3)).shape == want.shape
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("n", [1, 60, 17000])
+def test_cell_not_of_numbers(n, value):
+    """No atom has a place in such a cell."""
+    pos, Z = _atoms(n, 3)
+    cell = np.eye(3) * 11.0
+    cell[1, 1] = value
+    with pytest.raises(ValueError, match="outside its periodic cell"):
+        _soap(True).create({"positions": pos, "atomic_numbers": Z, "cell": cell, "pbc": [True] * 3})
