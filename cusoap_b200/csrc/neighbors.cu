@@ -296,8 +296,7 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   const double* H = g.H;
   const double det = H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
                      H[2] * (H[3] * H[7] - H[4] * H[6]);
-  int bad = fabs(det) < 1e-300;
-  const double id = !anyp ? 1.0 : bad ? 0.0 : 1.0 / det;
+  const double id = !anyp ? 1.0 : fabs(det) < 1e-300 ? 0.0 : 1.0 / det;
   // inverse of the row-vector matrix: x = f H  =>  f = x H^-1
   g.Hinv[0] = (H[4] * H[8] - H[5] * H[7]) * id;
   g.Hinv[1] = (H[2] * H[7] - H[1] * H[8]) * id;
@@ -334,7 +333,6 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
     w.fbox[i * 6 + k] = ord_encode(INFINITY);
     w.fbox[i * 6 + 3 + k] = ord_encode(-INFINITY);
   }
-  if (bad && anyp) atomicOr(w.status, 1);
 }
 
 // Smallest (largest) key of a warp: the high words, then the low words of those that have it.
@@ -405,7 +403,12 @@ __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& 
 
 __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork& w, double cutoff, int i) {
   GridDesc g = w.grids[i];
+  const double* H = g.H;
+  const double det = fabs(H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
+                          H[2] * (H[3] * H[7] - H[4] * H[6]));
   if (g.orth < 0) {  // one bin of which nothing is visited (its window would have no end)
+    // (flagged here, behind a barrier from the clear of the flags)
+    if (det < 1e-300) atomicOr(w.status, 1);
     w.bins_per_struct[i] = 1;
     if (s.n_struct == 1) {
       w.bin_off[0] = 0;
@@ -413,9 +416,6 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
     }
     return;
   }
-  const double* H = g.H;
-  const double det = fabs(H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
-                          H[2] * (H[3] * H[7] - H[4] * H[6]));
   double perp[3] = {1.0, 1.0, 1.0}, binw[3];
   if (g.any_per())
     for (int k = 0; k < 3; ++k) {

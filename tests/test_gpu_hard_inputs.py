@@ -61,3 +61,15 @@ def test_cell_not_of_numbers(n, value):
     cell[1, 1] = value
     with pytest.raises(ValueError, match="outside its periodic cell"):
         _soap(True).create({"positions": pos, "atomic_numbers": Z, "cell": cell, "pbc": [True] * 3})
+
+
+@pytest.mark.parametrize("at", [0, 31, 32, 511, 512, 699])
+def test_one_cell_without_a_volume_among_many(at):
+    """The flag of every structure of a batch is seen, whichever thread block finds it."""
+    soap = _soap(True)
+    systems = [{"positions": np.ones((1, 3)), "atomic_numbers": [1], "cell": np.eye(3) * 9.0, "pbc": [True] * 3}
+               for _ in range(700)]
+    systems[at] = dict(systems[at], cell=np.diag([9.0, 0.0, 9.0]))
+    for _ in range(20):
+        with pytest.raises(ValueError, match="singular cell"):
+            soap.create(systems)
