@@ -40,7 +40,9 @@ struct GridDesc {
   short nb[3];
   signed char per[3];
   signed char orth;  // 1: diagonal frame (every non-periodic structure, rectangular cells), 0: another,
-                     // -1: no frame (a periodic cell without a volume, or not of numbers): no pairs
+                     // -1: no frame (a periodic cell without a volume, or so thin that its images
+                     // could not be counted, or not of numbers): no pairs
+  signed char wide;  // an axis has more images than pack3 holds: image shifts in pack_wide
   // FP32 geometry of the window (Angstrom): perpendicular bin widths; for other than diagonal
   // frames the direction of lattice row a, the reciprocal of a bin's length along it, the edges
   // of a bin along b and c, and the largest distance of a bin's point from the bin row's axis
@@ -96,6 +98,21 @@ __device__ __forceinline__ void unpack3(int p, int (&v)[3]) {
   v[0] = (p & 1023) - 512;
   v[1] = ((p >> 10) & 1023) - 512;
   v[2] = ((p >> 20) & 1023) - 512;
+}
+// Cell-window shifts of a frame with more images than 10 bits hold (a cell thinner
+// than about cutoff / 500): fields as wide as the axes need.
+constexpr int kPackedReps = 508;  // largest n_rep of pack3 (the window reaches one cell further)
+__device__ __forceinline__ int shift_bits(int nrep) { return 32 - __clz(2 * (nrep + 2)); }
+__device__ __forceinline__ int pack_wide(const int* nrep, int a, int b, int c) {
+  const int s1 = shift_bits(nrep[0]), s2 = s1 + shift_bits(nrep[1]);
+  return (int)((unsigned)(a + nrep[0] + 2) | (unsigned)(b + nrep[1] + 2) << s1 | (unsigned)(c + nrep[2] + 2) << s2);
+}
+__device__ __forceinline__ void unpack_wide(const int* nrep, int p, int (&v)[3]) {
+  const int s1 = shift_bits(nrep[0]), s2 = s1 + shift_bits(nrep[1]);
+  const unsigned u = (unsigned)p;
+  v[0] = (int)(u & ((1u << s1) - 1u)) - nrep[0] - 2;
+  v[1] = (int)((u >> s1) & ((1u << (s2 - s1)) - 1u)) - nrep[1] - 2;
+  v[2] = (int)(u >> s2) - nrep[2] - 2;
 }
 // atom (27 bits) | species (5 bits) | packed wrap shifts (30 bits), carried in
 // the fourth double of a sorted-atom record so a candidate is one 32-byte load
@@ -328,6 +345,11 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
       const double perp = fabs(det) / (sqrt(cx * cx + cy * cy + cz * cz) + 1e-12);
       if (g.per[k]) g.nrep[k] = (int)ceil(cutoff / (perp + 1e-12));  // SG:389
     }
+  g.wide = max(g.nrep[0], max(g.nrep[1], g.nrep[2])) > kPackedReps;
+  // thinner than a millionth of the cutoff (vectors in a plane, up to rounding): millions of images
+  for (int k = 0; k < 3; ++k)
+    if (g.nrep[k] > 1 << 20) g.orth = -1;
+  if (g.orth >= 0 && shift_bits(g.nrep[0]) + shift_bits(g.nrep[1]) + shift_bits(g.nrep[2]) > 32) g.orth = -1;
   w.grids[i] = g;
   for (int k = 0; k < 3; ++k) {
     w.fbox[i * 6 + k] = ord_encode(INFINITY);
@@ -408,7 +430,7 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
                           H[2] * (H[3] * H[7] - H[4] * H[6]));
   if (g.orth < 0) {  // one bin of which nothing is visited (its window would have no end)
     // (flagged here, behind a barrier from the clear of the flags)
-    if (det < 1e-300) atomicOr(w.status, 1);
+    if (det < INFINITY) atomicOr(w.status, 1);
     w.bins_per_struct[i] = 1;
     if (s.n_struct == 1) {
       w.bin_off[0] = 0;
@@ -711,6 +733,13 @@ struct VisitCentre {
   int cw[3];
   const GridDesc* g;
   bool per;
+  __device__ __forceinline__ int pack(int a, int b, int c) const {
+    return g->wide ? pack_wide(g->nrep, a, b, c) : pack3(a, b, c);
+  }
+  __device__ __forceinline__ void unpack(int p, int (&v)[3]) const {
+    if (g->wide) unpack_wide(g->nrep, p, v);
+    else unpack3(p, v);
+  }
 };
 
 // One sorted-atom record through the read-only path (the lists are built by earlier kernels).
@@ -719,17 +748,15 @@ __device__ __forceinline__ double4 load_record(const double4* p) {
   return make_double4(a.x, a.y, b.x, b.y);
 }
 
-// rvec of the candidate in a slot with cell-window shift T, in FP64.
-__device__ __forceinline__ void exact_rvec(const VisitCentre& C, const double4& p, int Tpacked, double& rx, double& ry,
-                                           double& rz) {
+// rvec of the candidate in a slot with cell-window shift T (of a periodic frame), in FP64.
+__device__ __forceinline__ void exact_rvec(const VisitCentre& C, const double4& p, const int (&T)[3], double& rx,
+                                           double& ry, double& rz) {
   if (!C.per) {
     rx = p.x - C.cp.x;
     ry = p.y - C.cp.y;
     rz = p.z - C.cp.z;
   } else {
     const double* H = C.g->H;
-    int T[3];
-    unpack3(Tpacked, T);
     rx = p.x + (T[0] * H[0] + T[1] * H[3] + T[2] * H[6] - C.cp.x);
     ry = p.y + (T[0] * H[1] + T[1] * H[4] + T[2] * H[7] - C.cp.y);
     rz = p.z + (T[0] * H[2] + T[1] * H[5] + T[2] * H[8] - C.cp.z);
@@ -740,15 +767,16 @@ __device__ __forceinline__ void exact_rvec(const VisitCentre& C, const double4& 
 // create() the r <= 1e-12 edges other than the centre's own (SG:1171-1179).
 __device__ __forceinline__ bool exact_test(const VisitArgs& A, const VisitCentre& C, int slot, int Tpacked) {
   const double4 p = load_record(A.sorted_pos + slot);
+  int T[3] = {0, 0, 0};
+  if (C.per) C.unpack(Tpacked, T);
   double rx, ry, rz;
-  exact_rvec(C, p, Tpacked, rx, ry, rz);
+  exact_rvec(C, p, T, rx, ry, rz);
   const double r2 = rx * rx + ry * ry + rz * rz;
   if (!(r2 <= A.cutoff2)) return false;
   int atom, sp, wrap;
   unpack_info(p.w, atom, sp, wrap);
   if (C.per) {
-    int T[3], aw[3];
-    unpack3(Tpacked, T);
+    int aw[3];
     unpack3(wrap, aw);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
@@ -810,11 +838,14 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
       f[k] = fminf(fmaxf(f[k], -1e6f), 1e6f);
       iw[k] = 1.0f / g.wp[k];
       const float reach = fmaf(R, iw[k], 1e-3f);
-      lo[k] = (int)floorf(fmaxf(f[k] - reach, -1e6f));
-      hi[k] = (int)floorf(fminf(f[k] + reach, 1e6f));
+      lo[k] = (int)floorf(fmaxf(f[k] - reach, -1e9f));
+      hi[k] = (int)floorf(fminf(f[k] + reach, 1e9f));
       if (!PER || !g.per[k]) {
         lo[k] = max(lo[k], -cb[k]);
         hi[k] = min(hi[k], g.nb[k] - 1 - cb[k]);
+      } else {  // (R is 1e-3 A longer than the cutoff: many cells, if they are thin)
+        lo[k] = max(lo[k], -(g.nrep[k] + 1) * g.nb[k] - cb[k]);
+        hi[k] = min(hi[k], (g.nrep[k] + 2) * g.nb[k] - 1 - cb[k]);
       }
     }
   }
@@ -824,9 +855,10 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
     T0 = floordiv(cb[0] + lo[0], g.nb[0]);
     nT = floordiv(cb[0] + hi[0], g.nb[0]) - T0 + 1;
   }
-  // (a cell far thinner than 1e-2 A can have more rows than an int holds)
-  const int64_t nrows64 = (ny > 0 && nz > 0 && lo[0] <= hi[0]) ? (int64_t)ny * nz : 0;
-  const float inv_ny = 1.0f / (float)ny;  // row / ny for rows below 2^20: exact with the half added
+  int nrows = (ny > 0 && nz > 0 && lo[0] <= hi[0]) ? ny * nz : 0;
+  // row / ny is exact with the half added for rows below 2^20 (open axes have at most 1023 bins) and
+  // off by one at most for more of them
+  const float inv_ny = 1.0f / (float)ny;
   const int boff = (int)A.bin_off[ci.y];
   double o[3];
   coord_origin(g, o);
@@ -837,7 +869,9 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
   const unsigned upto = 0xffffffffu >> (31 - lane);
   const bool orth = !PER || g.orth;
   const int groups = PER ? (nT + 1) >> 1 : 1;  // pairs of images of a row
-  const int nrows = (int)min(nrows64, (int64_t)0x7fffff00 / groups), nlanes = nrows * groups;
+  // (thin cells have more rows than an int holds)
+  if (PER && (float)ny * (float)nz * (float)groups > 2e9f) nrows = nrows != 0 ? 2000000000 / groups : 0;
+  const int nlanes = nrows * groups;
   for (int p0 = 0; p0 < nlanes; p0 += 32) {
     int row = p0 + lane, tg = 0;
     if (PER && groups > 1) {
@@ -854,7 +888,12 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
       sh[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     if (row < nrows) {
-      const int iz = nrows <= 1 << 20 ? (int)(((float)row + 0.5f) * inv_ny) : row / ny, dz = lo[2] + iz, dy = lo[1] + row - iz * ny;
+      int iz = (int)(((float)row + 0.5f) * inv_ny), iy = row - iz * ny;
+      if (PER) {
+        if (iy < 0) { --iz; iy += ny; }
+        if (iy >= ny) { ++iz; iy -= ny; }
+      }
+      const int dz = lo[2] + iz, dy = lo[1] + iy;
       float mid, ext2, slack = 1e-3f, iwx;  // x range in bins from the centre's: mid +- (sqrt(ext2) iwx + slack)
       if (orth) {
         const float ay = fmaxf(0.0f, fmaxf((float)dy - f[1], f[1] - (float)(dy + 1)) * g.wp[1]);
@@ -876,8 +915,8 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
       }
       if (ext2 >= 0.0f) {
         const float e = fmaf(sqrt_approx(ext2), iwx, slack);
-        const int x0 = max((int)floorf(fmaxf(mid - e, -1e6f)), lo[0]),
-                  x1 = min((int)floorf(fminf(mid + e, 1e6f)), hi[0]);
+        const int x0 = max((int)floorf(fmaxf(mid - e, -1e9f)), lo[0]),
+                  x1 = min((int)floorf(fminf(mid + e, 1e9f)), hi[0]);
         int byw = cb[1] + dy, bzw = cb[2] + dz, Ty = 0, Tz = 0;
         if (PER) {
           if (g.per[1]) { Ty = floordiv(byw, g.nb[1]); byw -= Ty * g.nb[1]; }
@@ -901,7 +940,7 @@ __device__ __forceinline__ void visit_runs(const VisitArgs& A, VisitMem& M, cons
               sh[q] = make_float4((float)(Tx * H[0] + Ty * H[3] + Tz * H[6] - C.cp.x),
                                   (float)(Tx * H[1] + Ty * H[4] + Tz * H[7] - C.cp.y),
                                   (float)(Tx * H[2] + Ty * H[5] + Tz * H[8] - C.cp.z),
-                                  __int_as_float(pack3(Tx, Ty, Tz)));
+                                  __int_as_float(C.pack(Tx, Ty, Tz)));
             }
           }
         }
@@ -1127,7 +1166,7 @@ __global__ void __launch_bounds__(128, 7) k_fill(VisitArgs A, int64_t n_centres,
     const int64_t P = pair_off[c + 1] - base;
     __syncwarp();
     VisitCentre C;
-    auto record = [&](int slot, int T) {
+    auto record = [&](int slot, const int (&T)[3]) {
       const double4 p = load_record(A.sorted_pos + slot);
       double rx, ry, rz;
       exact_rvec(C, p, T, rx, ry, rz);
@@ -1136,8 +1175,13 @@ __global__ void __launch_bounds__(128, 7) k_fill(VisitArgs A, int64_t n_centres,
     };
     auto staged = [&](int i) {
       const unsigned t = st_meta[i];
-      return record(st_slot[i], C.per ? pack3((int)(t & 15u) - 8, (int)((t >> 4) & 15u) - 8, (int)((t >> 8) & 15u) - 8)
-                                      : 0);
+      const int T[3] = {(int)(t & 15u) - 8, (int)((t >> 4) & 15u) - 8, (int)((t >> 8) & 15u) - 8};
+      return record(st_slot[i], T);
+    };
+    auto unstaged = [&](int slot, int Tpacked) {
+      int T[3] = {0, 0, 0};
+      if (C.per) C.unpack(Tpacked, T);
+      return record(slot, T);
     };
     // slots of one key in a warp's 32 pairs, ranked in lane order behind those counted before
     auto rank_in_key = [&](bool ok, int key) {
@@ -1184,13 +1228,13 @@ __global__ void __launch_bounds__(128, 7) k_fill(VisitArgs A, int64_t n_centres,
       }
     } else {
       visit<1>(A, c, M, C, [&](bool ok, int slot, int T) {
-        if (ok) atomicAdd(&hist[keyof(record(slot, T))], 1);
+        if (ok) atomicAdd(&hist[keyof(unstaged(slot, T))], 1);
       });
       __syncwarp();
       scan_hist();
       visit<1>(A, c, M, C, [&](bool ok, int slot, int T) {
         float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ok) rec = record(slot, T);
+        if (ok) rec = unstaged(slot, T);
         const int pos = rank_in_key(ok, ok ? keyof(rec) : 0);
         if (ok) pairs[base + pos] = rec;
       });

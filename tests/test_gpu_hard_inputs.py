@@ -73,3 +73,26 @@ def test_one_cell_without_a_volume_among_many(at):
     for _ in range(20):
         with pytest.raises(ValueError, match="singular cell"):
             soap.create(systems)
+
+
+@pytest.mark.parametrize("cell,pbc", [(np.diag([0.006, 9.0, 8.0]), [True] * 3),
+                                      (np.diag([9.0, 8.0, 0.003]), [True] * 3),
+                                      (np.array([[9.0, 0.0, 0.0], [5.0, 0.008, 0.0], [0.0, 2.0, 9.0]]), [True] * 3),
+                                      (np.diag([8.0, 0.004, 9.0]), [False, True, False])])
+def test_thin_cells(cell, pbc):
+    """More images along an axis than a 10-bit shift holds."""
+    from test_gpu_neighbors import _check
+    rng = np.random.default_rng(9)
+    _check(_soap(True, n_max=2, l_max=1),
+           [{"positions": rng.uniform(0.0, 1.0, (3, 3)) @ cell, "atomic_numbers": np.array([1, 8, 1]), "cell": cell,
+             "pbc": pbc}])
+
+
+def test_cell_without_a_volume_by_rounding():
+    """Vectors in a plane up to rounding: as many images as no list can hold."""
+    pos, Z = _atoms(20, 3)
+    cell = np.array([[3.0, 0.1, 0.7], [0.3, 2.9, 0.2], [0.0, 0.0, 0.0]])
+    cell[2] = 0.1 * cell[0] + 0.7 * cell[1]
+    assert abs(np.linalg.det(cell)) < 1e-12
+    with pytest.raises(ValueError, match="singular cell"):
+        _soap(True).create({"positions": pos, "atomic_numbers": Z, "cell": cell, "pbc": [True] * 3})
