@@ -392,7 +392,11 @@ class _Pairs:
         ws = ctypes.c_int64(0)
         b = ctypes.byref(soap._basis)
         check(lib.soapb_neighbors_workspace(b, ctypes.byref(batch.cs), ctypes.byref(batch.cc), ctypes.byref(ws)))
-        self.work = torch.empty(max(int(ws.value), 256), dtype=torch.uint8, device=dev)
+        nbytes = (int(ws.value) + 255) & ~255
+        self.work = torch.empty(nbytes + 256, dtype=torch.uint8, device=dev)
+        # work-queue word of the descriptor and adjoint kernels on these pairs: one a call, since
+        # its reset and the kernel are two steps between which another thread may launch
+        self.counter = self.work.data_ptr() + nbytes
         self.pair_off = torch.empty(batch.n_centres + 1, dtype=torch.int64, device=dev)
         # total pairs, largest per-centre count and status flags, written by the count into
         # page-locked host memory: read after one stream synchronisation
@@ -680,7 +684,6 @@ class SOAP:
         self._cutoff = self._r_cut + self._cutoff_padding
         self._poly_grid = _poly_grid(self._r_cut, self._n_max, self.quad_n) if self._rbf == "polynomial" else None
         self._build_basis()
-        self._counter = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._stage_pool: List[torch.Tensor] = []  # page-locked staging buffers of uploads
         self._stats_pool: List[torch.Tensor] = []  # page-locked int64[3] buffers of the neighbour summaries
         self._topology = None  # device copies of the last batch's species, offsets, cells (see _Batch)
@@ -885,7 +888,7 @@ class SOAP:
         coeff = (torch.empty((batch.n_centres, int(self._basis.n_feat_cc)), dtype=torch.float32, device=self.device)
                  if want_coeff else None)
         self._call("descriptor", lib.soapb_descriptor, ctypes.byref(self._basis), batch.n_centres,
-                   _ptr(pairs.pair_off), _ptr(pairs.pairs), mode, _ptr(out), _ptr(coeff), _ptr(self._counter),
+                   _ptr(pairs.pair_off), _ptr(pairs.pairs), mode, _ptr(out), _ptr(coeff), pairs.counter,
                    _stream(self.device))
         return out, coeff
 
@@ -898,7 +901,7 @@ class SOAP:
         self._call("forces", lib.soapb_forces, ctypes.byref(self._basis), batch.n_centres, _ptr(pairs.pair_off),
                    _ptr(pairs.pairs), _ptr(coeff), _ptr(dEdp), self._out_mode() if mode is None else mode,
                    _ptr(batch.centre_attach), int(bool(attach)), _ptr(forces), _ptr(work), work.numel(),
-                   _ptr(self._counter), _stream(self.device))
+                   pairs.counter, _stream(self.device))
         self._last_forces_work = (work, batch.n_centres)
         return forces
 
