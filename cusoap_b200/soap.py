@@ -87,6 +87,14 @@ def _index_centres(centres) -> bool:
     return all(isinstance(c, (int, np.integer)) for c in centres)
 
 
+def _take(pool: list):
+    """A buffer from a pool that other threads take from as well, or None."""
+    try:
+        return pool.pop()
+    except IndexError:
+        return None
+
+
 _TORCH_TYPES = {np.dtype(np.int32): torch.int32, np.dtype(np.int64): torch.int64,
                 np.dtype(np.float64): torch.float64, np.dtype(np.uint8): torch.uint8}
 
@@ -95,8 +103,8 @@ class _DevArrays:
     """Named host arrays copied to the device in one buffer: addresses for the
     library, tensor views made when asked for."""
 
-    def __init__(self, buf: torch.Tensor, where: Dict[str, Tuple[int, np.ndarray]], stage: torch.Tensor):
-        self.buf, self.base, self.stage = buf, buf.data_ptr(), stage
+    def __init__(self, buf: torch.Tensor, where: Dict[str, Tuple[int, np.ndarray]]):
+        self.buf, self.base = buf, buf.data_ptr()
         self.where = {name: (off, a.dtype, a.shape, a.nbytes) for name, (off, a) in where.items()}
 
     def ptr(self, name: str) -> int:
@@ -232,10 +240,13 @@ class _Batch:
                                        and np.array_equal(cached["cells"], cells)
                                        and np.array_equal(cached["pbcs"], pbcs)):
             cached = None
+        self._stage = self._publish = None  # this batch's staging buffer and topology, until staged()
         # centres that are all atom indices (or every atom) are described by host arrays
         by_index = not all_atoms and all(c is None or _index_centres(c) for c in centers_list)
         if cached is not None:
             self._dev = cached["dev"]
+            if cached["stream"] != _stream(dev):  # uploaded on another stream (which has been waited for)
+                self._dev.buf.record_stream(torch.cuda.current_stream(dev))
         else:
             # the small host arrays (and host positions) go to the device in ONE
             # asynchronous copy from a pinned staging buffer
@@ -252,10 +263,10 @@ class _Batch:
                 arrays.append(("centre_atom", np.arange(self.n_atoms, dtype=np.int32)))
             elif by_index:
                 arrays += self._index_arrays(centers_list, counts_a, host)
-            self._dev = soap._upload(arrays)
+            self._dev, self._stage = soap._upload(arrays)
             if all_atoms and not host_pos:
-                soap._topology = {"counts": list(counts_a), "Z": Zall.copy(), "cells": cells.copy(),
-                                  "pbcs": pbcs.copy(), "dev": self._dev}
+                self._publish = {"counts": list(counts_a), "Z": Zall.copy(), "cells": cells.copy(),
+                                 "pbcs": pbcs.copy(), "dev": self._dev, "stream": _stream(dev)}
         self._alias = {"centre_attach": "centre_atom"}
         self.grad_positions = None
         if host_pos:
@@ -343,11 +354,13 @@ class _Batch:
         raise AttributeError(name)
 
     def staged(self, soap: "SOAP") -> None:
-        """The stream of the upload has been synchronised: its staging buffer is free."""
-        dev = self.__dict__.get("_dev")
-        if dev is not None and dev.stage is not None:
-            soap._stage_pool.append(dev.stage)
-            dev.stage = None
+        """The stream of this batch's upload has been synchronised: the staging
+        buffer is free, and other calls, on any stream, may use the arrays."""
+        if self._stage is not None:
+            soap._stage_pool.append(self._stage)
+            self._stage = None
+        if self._publish is not None:
+            soap._topology, self._publish = self._publish, None
 
     def _describe(self, n_struct: int):
         self.cs = Structs(n_struct, self.n_atoms, _ptr(self.atom_off), _ptr(self.positions),
@@ -362,6 +375,7 @@ class _Batch:
         concatenated, counts_a atoms each; centres concatenated, counts per
         structure).  No host-side adapters and no copies."""
         self = cls.__new__(cls)
+        self._stage = self._publish = None
         dev = positions.device
         atom_off = np.concatenate([[0], np.cumsum(counts_a)]).astype(np.int64)
         self.atom_off_list = atom_off.tolist()
@@ -400,9 +414,11 @@ class _Pairs:
         self.pair_off = torch.empty(batch.n_centres + 1, dtype=torch.int64, device=dev)
         # total pairs, largest per-centre count and status flags, written by the count into
         # page-locked host memory: read after one stream synchronisation
-        # (a buffer belongs to one call until it has been read, so threads may share the object)
+        # (a buffer belongs to one call until it has been read)
         pool = soap._stats_pool
-        stats = pool.pop() if pool else torch.empty(3, dtype=torch.int64, pin_memory=True)
+        stats = _take(pool)
+        if stats is None:
+            stats = torch.empty(3, dtype=torch.int64, pin_memory=True)
         soap._call("neighbors_count", lib.soapb_neighbors_count_stats, b, ctypes.byref(batch.cs),
                    ctypes.byref(batch.cc), mode, _ptr(self.work), self.work.numel(), _ptr(self.pair_off), _ptr(stats),
                    st)
@@ -823,19 +839,18 @@ class SOAP:
     def _species_index(self, Z) -> torch.Tensor:
         return torch.as_tensor(self._species_lookup(Z)).to(self.device)
 
-    def _upload(self, arrays) -> _DevArrays:
+    def _upload(self, arrays) -> Tuple[_DevArrays, torch.Tensor]:
         """Copy named host arrays to the device in one asynchronous copy from a
-        page-locked staging buffer.  The buffer goes back to this object's pool
-        once the stream has been synchronised (``_Batch.staged``), so calls of
-        other threads take their own."""
+        page-locked staging buffer: the arrays and the buffer, which the caller
+        puts back into this object's pool once the stream has been synchronised
+        (``_Batch.staged``).  Calls of other threads take their own."""
         where, off = {}, 0
         for name, a in arrays:
             a = np.ascontiguousarray(a)
             where[name] = (off, a)
             off = (off + a.nbytes + 255) & ~255
         total = max(off, 256)
-        pool = self._stage_pool
-        stage = pool.pop() if pool else None
+        stage = _take(self._stage_pool)
         if stage is None or stage.numel() < total:
             stage = torch.empty(max(total, 1 << 16), dtype=torch.uint8, pin_memory=True)
         base = stage.data_ptr()
@@ -843,7 +858,7 @@ class SOAP:
             ctypes.memmove(base + o, a.__array_interface__["data"][0], a.nbytes)
         dbuf = torch.empty(total, dtype=torch.uint8, device=self.device)
         dbuf.copy_(stage[:total], non_blocking=True)
-        return _DevArrays(dbuf, where, stage)
+        return _DevArrays(dbuf, where), stage
 
     def _prepare_centres(self, pos: torch.Tensor, centers):
         """(xyz, self atom, attached atom) per centre.  Index centres are

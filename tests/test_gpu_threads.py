@@ -57,3 +57,48 @@ def test_work_queues(own_stream):
                 assert float((g - want[i][1]).norm() / want[i][1].norm()) < 2e-6
 
     _run(work, 3)
+
+
+class _Emptied(list):
+    """A pool whose last buffer another thread takes between a look at it and the pop."""
+
+    def __bool__(self):
+        return True
+
+    def __len__(self):
+        return 1
+
+    def pop(self, *a):
+        raise IndexError("pop from empty list")
+
+
+def test_pool_emptied_by_another_thread():
+    soap, s = _soap(), W.water_cluster(2, 2, 2, seed=1)
+    want = soap.create(s)
+    soap._stage_pool, soap._stats_pool = _Emptied(), _Emptied()
+    assert torch.equal(soap.create(s), want)
+
+
+def test_topology_of_an_upload_that_waits():
+    """Arrays whose copy still waits on one stream are not used on another, and their staging buffer
+    is not given out again, whoever waits for what."""
+    from cusoap_b200 import _lib
+    from cusoap_b200.soap import _Batch, _Pairs
+    soap, s = _soap(), W.water_cluster(3, 3, 3, seed=1)
+    want = _soap().create(s)
+    sysd = dict(s, positions=torch.as_tensor(s["positions"], device="cuda"))
+    torch.cuda.synchronize()
+    first, other = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(200_000_000)
+        batch = _Batch(soap, [sysd], [None])
+    assert soap._topology is None and not soap._stage_pool
+    with torch.cuda.stream(other):
+        assert torch.equal(soap.create(sysd), want)
+    assert len(soap._stage_pool) == 1 and soap._topology["dev"] is not batch._dev
+    with torch.cuda.stream(first):
+        pairs = _Pairs(soap, batch, _lib.NL_CREATE)
+        assert torch.equal(soap._run_descriptor(batch, pairs, _lib.OUT_PS)[0], want)
+    assert len({p.data_ptr() for p in soap._stage_pool}) == len(soap._stage_pool) == 2
+    with torch.cuda.stream(other):  # the arrays of the first stream's upload, complete by now
+        assert torch.equal(soap.create(sysd), want)
