@@ -960,9 +960,9 @@ class SOAP:
                         raise ValueError("centers list must match number of systems.")
                 if not systems:
                     return []
-                out = self._evaluate_batch(systems, centers_list)
-                parts = list(torch.split(out, [int(c) for c in self._last_counts]))
-                if len(set(self._last_counts)) > 1 and not self.sparse:
+                out, counts = self._evaluate_batch(systems, centers_list)
+                parts = list(torch.split(out, [int(c) for c in counts]))
+                if len(set(counts)) > 1 and not self.sparse:
                     return parts  # uneven shapes do not stack
                 if self.sparse:  # each system's rows in COO, then stacked if possible (SG:1716-1737)
                     parts = [p.to_sparse_coo() for p in parts]
@@ -970,7 +970,7 @@ class SOAP:
                     return torch.stack(parts, dim=0)
                 except Exception:
                     return parts
-            out = self._evaluate_batch([system], [centers])
+            out, _ = self._evaluate_batch([system], [centers])
             return out.to_sparse_coo() if self.sparse else out
 
     def create_flat(self, systems: List[Any], centers=None) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -990,14 +990,14 @@ class SOAP:
             if not systems:
                 return (torch.zeros((0, self.get_number_of_features()), dtype=self.dtype, device=self.device),
                         torch.zeros(1, dtype=torch.int64))
-            out = self._evaluate_batch(systems, centers_list)
+            out, counts = self._evaluate_batch(systems, centers_list)
             offsets = torch.zeros(len(systems) + 1, dtype=torch.int64)
-            offsets[1:] = torch.cumsum(torch.tensor(self._last_counts, dtype=torch.int64), 0)
+            offsets[1:] = torch.cumsum(torch.tensor(counts, dtype=torch.int64), 0)
             return out, offsets
 
-    def _evaluate_batch(self, systems, centers_list) -> torch.Tensor:
+    def _evaluate_batch(self, systems, centers_list) -> Tuple[torch.Tensor, List[int]]:
+        """Descriptors of all centres, and the number of them in each system."""
         batch = _Batch(self, systems, centers_list)
-        self._last_counts = batch.counts
         mode = self._out_mode()
         grad = torch.is_grad_enabled() and any(p.requires_grad for p in batch.pos_tensors)
         if grad:
@@ -1010,7 +1010,7 @@ class SOAP:
         else:
             pairs = _Pairs(self, batch, _lib.NL_CREATE)
             out, _ = self._run_descriptor(batch, pairs, mode)
-        return out.to(self.dtype) if self.dtype != torch.float32 else out
+        return (out.to(self.dtype) if self.dtype != torch.float32 else out), batch.counts
 
     def autotune(self, system, reps: int = 3, cache_path: Optional[str] = None, force: bool = False):
         """Time the candidate launch shapes of the descriptor and adjoint

@@ -102,3 +102,20 @@ def test_topology_of_an_upload_that_waits():
     assert len({p.data_ptr() for p in soap._stage_pool}) == len(soap._stage_pool) == 2
     with torch.cuda.stream(other):  # the arrays of the first stream's upload, complete by now
         assert torch.equal(soap.create(sysd), want)
+
+
+def test_lists_of_systems():
+    """Every call splits its output by its own counts."""
+    soap = _soap()
+    lists = [[W.water_cluster(1, 1, k + i, seed=k) for k in range(1, 4 + i)] for i in range(4)]
+    want = [soap.create(v) for v in lists]
+
+    def work(i):
+        for _ in range(40):
+            got = soap.create(lists[i])
+            assert len(got) == len(want[i]) and all(torch.equal(a, b) for a, b in zip(got, want[i]))
+            flat, off = soap.create_flat(lists[i])
+            assert np.diff(off.numpy()).tolist() == [len(w) for w in want[i]]
+            assert torch.equal(flat, torch.cat(want[i]))
+
+    _run(work, 4)
