@@ -59,7 +59,8 @@ struct JacArgs {
   float* out;
   int* status;
   int* counter;                  // {next task, next zero chunk, tasks, 0}
-  int4* tasks;                   // {centre, entries (negative: the centre's own row), first entry in ent (low, high word)}
+  int2* tasks;                   // {centre, entries (negative: the centre's own row)}, {first entry in ent: low, high
+                                 // word}; 8-byte loads, the alignment that a workspace always needed
   unsigned long long* ent;       // sorted entries, centre c at ent_mult * pair_off[c]
   unsigned long long* ent_tmp;   // merge buffer of a centre with more than cap entries, same offsets
   unsigned int* bitmap;          // (n_centres * n_inc) nonzero-row bits
@@ -306,7 +307,9 @@ __global__ void __launch_bounds__(kEntThreads) k_jac_entries(JacArgs a) {
         e = row_boundary(g1 + (k - own - n0 + 1) * a.eb);
       }
       const unsigned long long first = (unsigned long long)((size_t)a.ent_mult * p0 + b);
-      a.tasks[s_task0 + k] = make_int4((int)c, k < own ? b - e : e - b, (int)(unsigned)first, (int)(unsigned)(first >> 32));
+      int2* t = a.tasks + 2 * (int64_t)(s_task0 + k);
+      t[0] = make_int2((int)c, k < own ? b - e : e - b);
+      t[1] = make_int2((int)(unsigned)first, (int)(unsigned)(first >> 32));
     }
     __syncthreads();
   }
@@ -682,7 +685,9 @@ __global__ void __launch_bounds__(256, 2) k_jacobian(JacArgs a) {
   const int NF = N * (L + 1), SNK = S * N * K;
   auto claim = [&]() {
     const int t = atomicAdd(a.counter, 1);
-    return t < ntasks ? a.tasks[t] : make_int4(-1, 0, 0, 0);
+    if (t >= ntasks) return make_int4(-1, 0, 0, 0);
+    const int2 u = a.tasks[2 * (int64_t)t], v = a.tasks[2 * (int64_t)t + 1];
+    return make_int4(u.x, u.y, v.x, v.y);
   };
   auto keys_of = [&](const int4& t) {
     return a.ent + (((unsigned long long)(unsigned)t.w << 32) | (unsigned)t.z);
@@ -924,7 +929,7 @@ extern "C" int soapb_jacobian(const soapb_basis* b, int64_t n_centres, const int
   a.out = d_out;
   a.status = d_status;
   a.counter = (int*)(w + Lw.counter);
-  a.tasks = (int4*)(w + Lw.tasks);
+  a.tasks = (int2*)(w + Lw.tasks);
   a.ent = (unsigned long long*)(w + Lw.ent);
   a.ent_tmp = (unsigned long long*)(w + Lw.ent_tmp);
   a.bitmap = (unsigned int*)(w + Lw.bitmap);

@@ -96,3 +96,28 @@ def test_cell_without_a_volume_by_rounding():
     assert abs(np.linalg.det(cell)) < 1e-12
     with pytest.raises(ValueError, match="singular cell"):
         _soap(True).create({"positions": pos, "atomic_numbers": Z, "cell": cell, "pbc": [True] * 3})
+
+
+def test_jacobian_workspace_of_eight_byte_alignment():
+    """The library's Jacobian in a workspace that starts 8 bytes behind a 256-byte boundary."""
+    import ctypes
+    from cusoap_b200 import _lib
+    from cusoap_b200.soap import _Batch, _Pairs
+    soap = _soap()
+    pos, Z = _atoms(60, 4)
+    s = {"positions": pos, "atomic_numbers": Z}
+    want, _ = soap.derivatives(s)
+    batch = _Batch(soap, [s], [None])
+    pairs = _Pairs(soap, batch, _lib.NL_ALL)
+    _, coeff = soap._run_descriptor(batch, pairs, _lib.OUT_PS, want_coeff=True)
+    lib, need = _lib.load(), ctypes.c_int64(0)
+    _lib.check(lib.soapb_jacobian_workspace(ctypes.byref(soap._basis), 60, pairs.total, 60, 0, ctypes.byref(need)))
+    work = torch.empty(need.value + 256, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(want)
+    status = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+    _lib.check(lib.soapb_jacobian(ctypes.byref(soap._basis), 60, pairs.pair_off.data_ptr(), pairs.pairs.data_ptr(),
+                                  pairs.total, coeff.data_ptr(), batch.centre_atom.data_ptr(), 60,
+                                  batch.centre_attach.data_ptr(), 0, pairs.max_pairs, _lib.OUT_PS, out.data_ptr(),
+                                  work.data_ptr() + 8, need.value, status.data_ptr(),
+                                  torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(out, want)
