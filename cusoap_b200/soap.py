@@ -534,6 +534,21 @@ class SOAPBatch:
             self._backward_calls()
         torch.cuda.synchronize(dev)
         b.staged(soap)
+        self.finished = torch.cuda.Event()  # behind the plan's last graph, and that one's stream
+        self._last_stream = st
+
+    def _on_stream(self):
+        """The plan's graphs share their buffers, so one replayed on another stream
+        than the last waits for that one on the device; the buffers may then not be
+        given back to their own stream before this one is done with them."""
+        st = _stream(self.soap.device)
+        if st != self._last_stream:
+            cur = torch.cuda.current_stream(self.soap.device)
+            cur.wait_event(self.finished)
+            for t in (self.b._dev.buf, self.b.positions, self.work, self.pair_off, self.pairs, self.desc, self.coeff,
+                      self.dEdp, self.forces, self.fwork, self.counter):
+                t.record_stream(cur)
+            self._last_stream = st
 
     def _list_calls(self):
         soap, b, lib = self.soap, self.b, _lib.load()
@@ -560,17 +575,21 @@ class SOAPBatch:
                                _ptr(self.fwork), self.fwork.numel(), _ptr(self.counter), _stream(soap.device)))
 
     def _replay_forward(self, positions: Optional[torch.Tensor]):
+        self._on_stream()
         if positions is not None:
             self.b.positions.copy_(positions.detach().reshape(-1, 3))
         self.g_list.replay()
         self.listed.record()
         self.g_desc.replay()
+        self.finished.record()
         self.listed.synchronize()
         need = int(self.total.item())
         if need > self.capacity:  # the lists outgrew the pair buffer: re-plan and run again
+            self.finished.synchronize()  # the descriptor of the empty lists is done with the old buffers
             self._build(capacity=int(need * self.headroom) + 1024)
             self.g_list.replay()
             self.g_desc.replay()
+            self.finished.record()
         return self.desc
 
     def create(self, positions: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -586,8 +605,10 @@ class SOAPBatch:
         """-dE/dx (n_atoms, 3) for a given dE/dp (n_atoms, F), at the
         positions of the last ``create``."""
         with _on_device(self.soap.device):
+            self._on_stream()
             self.dEdp.copy_(dEdp)
             self.g_bwd.replay()
+            self.finished.record()
             return self.forces
 
     def split(self, out: torch.Tensor) -> List[torch.Tensor]:

@@ -119,3 +119,56 @@ def test_lists_of_systems():
             assert torch.equal(flat, torch.cat(want[i]))
 
     _run(work, 4)
+
+
+class _Late:
+    """A graph whose replay waits on the device for about 50 ms first."""
+
+    def __init__(self, graph):
+        self.graph = graph
+
+    def replay(self):
+        torch.cuda._sleep(100_000_000)
+        self.graph.replay()
+
+
+@pytest.mark.parametrize("late", ["g_desc", "g_bwd"])
+def test_plan_on_another_stream(late):
+    """A call of a plan on another stream than the last waits for that one's graphs."""
+    soap, s = _soap(), W.water_cluster(4, 4, 4, seed=1)
+    plan = soap.batch([s])
+    pos = torch.as_tensor(s["positions"], device="cuda")
+    moved = pos + 0.05 * torch.sin(torch.arange(pos.numel(), device="cuda").reshape(pos.shape))
+    w = torch.linspace(-1.0, 1.0, soap.get_number_of_features(), device="cuda").expand(len(pos), -1)
+    want = plan.create(moved).clone()
+    first, other = torch.cuda.Stream(), torch.cuda.Stream()
+    setattr(plan, late, _Late(getattr(plan, late)))
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    with torch.cuda.stream(first):
+        plan.create(pos)
+        if late == "g_bwd":
+            plan.forces_from(w)
+        done.record()
+    with torch.cuda.stream(other):
+        got = plan.create(moved)  # returns when its pair lists are there
+        assert done.query()
+        assert torch.equal(got, want)
+
+
+def test_plan_is_made_anew_when_its_graphs_are_done():
+    soap, s = _soap(), W.water_cluster(4, 4, 4, seed=1)
+    plan = soap.batch([s], headroom=1.0)
+    pos = torch.as_tensor(s["positions"], device="cuda")
+    plan.g_desc = _Late(plan.g_desc)
+    build, done = plan._build, torch.cuda.Event()
+
+    def checked(capacity):
+        assert plan.finished.query()
+        done.record()
+        build(capacity)
+
+    plan._build = checked
+    with torch.cuda.stream(torch.cuda.Stream()):
+        got = plan.create(pos * 0.5)
+        assert done.query() and torch.equal(got, soap.create(dict(s, positions=pos * 0.5)))
