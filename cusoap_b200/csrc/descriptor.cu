@@ -246,17 +246,10 @@ __device__ __forceinline__ void descriptor_body(const DescArgs& a) {
     selfb[g] = (active && n < N) ? __ldg(a.selfv + fn_index(n, lme, N)) : 0.0f;
   }
 
-  bool first = true;
   for (;;) {
-    int64_t c;
-    if (a.counter) {
-      int c32 = 0;
-      if (lane == 0) c32 = atomicAdd(a.counter, 1);
-      c = __shfl_sync(0xffffffffu, c32, 0);
-    } else {
-      c = first ? (int64_t)blockIdx.x * (blockDim.x >> 5) + wid : a.n_centres;
-      first = false;
-    }
+    int c32 = 0;
+    if (lane == 0) c32 = atomicAdd(a.counter, 1);
+    const int64_t c = __shfl_sync(0xffffffffu, c32, 0);
     if (c >= a.n_centres) break;
     for (int i = lane; i < cbn; i += 32) cbuf[i] = 0.0f;
     float acc[GN][M];
@@ -914,14 +907,9 @@ static int launch_descriptor(const DescArgs& a, int wpb_tuned, cudaStream_t st) 
   if (occ < 1) occ = 1;
   int64_t blocks = (int64_t)nsm * occ;
   const int64_t need = (a.n_centres + wpb - 1) / wpb;
-  DescArgs b = a;
-  if (blocks >= need) {  // one centre per warp: no work queue to reset
-    blocks = need;
-    b.counter = nullptr;
-  } else if ((rc = check_cuda(cudaMemsetAsync(a.counter, 0, sizeof(int32_t), st), "reset work counter"))) {
-    return rc;
-  }
-  kern<<<(unsigned)blocks, 32 * wpb, smem, st>>>(b);
+  if (blocks > need) blocks = need;
+  if ((rc = check_cuda(cudaMemsetAsync(a.counter, 0, sizeof(int32_t), st), "reset work counter"))) return rc;
+  kern<<<(unsigned)blocks, 32 * wpb, smem, st>>>(a);
   return check_launch("k_descriptor");
 }
 
