@@ -470,41 +470,51 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
       }
       const ulonglong2* x2 = reinterpret_cast<const ulonglong2*>(cbuf + (j * N + n) * KR);
       const ulonglong2* y2 = reinterpret_cast<const ulonglong2*>(cbuf + (jd * N + nd) * KR);
-      // sums of slot pairs with the same two l: one per l pair of the table, then the leftovers
-      constexpr int NLP = YO::NLP, NSUM = NLP + (NLP + 1) / 2;
-      f32x2 sum[NSUM > 0 ? NSUM : 1];
+      // sums of slot pairs with the same two l, one per l pair of the table; the last two products
+      // of the larger l follow, packed with those of the next l pair: every sum runs over m in order
+      constexpr int NLP = YO::NLP;
+      f32x2 sum[NLP > 0 ? NLP : 1], tail = 0ull;
 #pragma unroll
-      for (int k = 0; k < NSUM; ++k) sum[k] = 0ull;
-      float s0 = 0.0f;
+      for (int k = 0; k < NLP; ++k) sum[k] = 0ull;
+      float sl[L + 1];
 #pragma unroll
       for (int q = 0; q < (K + 3) / 4; ++q) {
         const ulonglong2 u = x2[q], v = y2[q];
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           const int i = 2 * q + hh;  // slot pair
+          const f32x2 x = hh ? u.y : u.x, y = hh ? v.y : v.x;
           if (i < YO::NS) {
-            const int la = YO::l_of(kYOrder<L>.lm[2 * i]), lb = YO::l_of(kYOrder<L>.lm[2 * i + 1]);
-            const int k = (lb == la - 1) ? (L - la) / 2 : NLP + (L - la) / 4;
-            sum[k] = fma2(hh ? u.y : u.x, hh ? v.y : v.x, sum[k]);
+            const int ma = kYOrder<L>.lm[2 * i], la = YO::l_of(ma), lb = YO::l_of(kYOrder<L>.lm[2 * i + 1]);
+            const int k = (L - la) / 2;
+            if (lb == la - 1) {
+              sum[k] = fma2(x, y, sum[k]);
+            } else {
+              float s0, s1, t_;
+              if (ma == la * la + 2 * la - 1) {  // the first of the last two
+                unpack2(sum[k], s0, sl[la - 1]);
+                if (lb == la) {
+                  float xa, xb, ya, yb;
+                  unpack2(x, xa, xb);
+                  unpack2(y, ya, yb);
+                  sl[la] = fmaf(xb, yb, fmaf(xa, ya, s0));
+                } else {
+                  unpack2(sum[k + 1 < NLP ? k + 1 : k], s1, t_);
+                  sl[lb - 1] = t_;
+                  tail = fma2(x, y, pack2(s0, s1));
+                }
+              } else {
+                tail = fma2(x, y, tail);
+                unpack2(tail, sl[la], sl[lb]);
+              }
+            }
           } else if (K % 2 == 1 && i == YO::NS) {
             float xa, xb, ya, yb;
-            unpack2(hh ? u.y : u.x, xa, xb);
-            unpack2(hh ? v.y : v.x, ya, yb);
-            s0 = xa * ya;
+            unpack2(x, xa, xb);
+            unpack2(y, ya, yb);
+            sl[0] = xa * ya;
           }
         }
-      }
-      float sl[L + 1];
-      sl[0] = s0;
-#pragma unroll
-      for (int k = 0; k < NLP; ++k) unpack2(sum[k], sl[L - 2 * k], sl[L - 2 * k - 1]);
-#pragma unroll
-      for (int k = NLP; k < NSUM; ++k) {
-        const int ha = L - 4 * (k - NLP), hb = (2 * (k - NLP) + 1 < NLP) ? ha - 2 : ha;
-        float xa, xb;
-        unpack2(sum[k], xa, xb);
-        sl[ha] += xa;
-        sl[hb] += xb;
       }
       float* o = orow + fb0 + p;
 #pragma unroll
