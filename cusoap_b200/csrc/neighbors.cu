@@ -1135,8 +1135,10 @@ __global__ void __launch_bounds__(128, 7) k_fill(VisitArgs A, int64_t n_centres,
     if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(status, 4);
     return;
   }
-  auto keyof = [&](const float4& p) {  // species * nseg + segment of the FP32 record
-    const float r = sqrtf(p.x * p.x + p.y * p.y + p.z * p.z);
+  // species * nseg + segment of the FP32 record.  The roundings are written out: they place a pair
+  // within one of them of a segment's edge, and so the order of the centre's sums.
+  auto keyof = [&](const float4& p) {
+    const float r = sqrtf(fmaf(p.z, p.z, fmaf(p.x, p.x, __fmul_rn(p.y, p.y))));
     return (int)((unsigned)__float_as_int(p.w) >> kAtomBits) * nseg + min((int)(r * inv_h), nseg - 1);
   };
   auto scan_hist = [&]() {  // exclusive scan of hist (each lane a contiguous chunk)

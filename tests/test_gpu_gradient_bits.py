@@ -184,3 +184,33 @@ def test_coefficients(structure, basis):
 @pytest.mark.parametrize("structure", G_STRUCTURES)
 def test_gradient_of_one_centre(structure, basis):
     assert gradients(structure, basis) == GRADIENTS[structure + basis]
+
+
+def _radius(v, order):
+    """FP32 radius of FP32 vectors, squares added in an order, by FMAs (exact products in float64)."""
+    f = lambda x: x.astype(np.float32).astype(np.float64)  # noqa: E731
+    x, y, z = (v[:, order.index(k)].astype(np.float64) for k in "abc")
+    return np.sqrt(f(z * z + f(y * y + f(x * x))).astype(np.float32))
+
+
+def test_pairs_at_segment_edges():
+    """Pairs whose segment depends on the rounding of their radius: that of z z + (x x + y y)."""
+    from cusoap_b200 import _lib
+    from cusoap_b200.soap import _Batch, _Pairs
+    soap = _soap("open", 1, r_cut=6.0, n_max=4, l_max=3, sigma=0.4)
+    h, nseg = soap._basis.seg_width, int(soap._basis.n_seg)
+    rng = np.random.default_rng(2)
+    v = rng.standard_normal((40000, 3))
+    v *= (rng.integers(1, nseg, (40000, 1)) * h) / np.linalg.norm(v, axis=1, keepdims=True)
+    v = v.astype(np.float32)
+    seg = lambda order: np.minimum((_radius(v, order) * np.float32(1.0 / h)).astype(np.int64), nseg - 1)  # noqa: E731
+    edge = (seg("bac") != seg("abc")) | (seg("bac") != seg("cba"))
+    v = v[edge & (np.linalg.norm(v, axis=1) < 0.99 * soap._cutoff)][:300]
+    assert len(v) == 300
+    pos = np.concatenate([np.zeros((1, 3)), v.astype(np.float64)])
+    batch = _Batch(soap, [{"positions": pos, "atomic_numbers": np.ones(301, int)}], [[0]])
+    p = _Pairs(soap, batch, _lib.NL_ALL)
+    got = p.pairs[:p.total].cpu().numpy()
+    assert p.total == 301
+    r = _radius(got[:, :3], "bac")
+    assert (np.diff(np.minimum((r * np.float32(1.0 / h)).astype(np.int64), nseg - 1)) >= 0).all()
