@@ -329,14 +329,16 @@ __device__ __forceinline__ void bulk_s2g(void* g, const void* s, uint32_t bytes)
 // asynchronously and the lane waits for all of them before returning (the
 // tile must outlive them).  Every block's zero warp runs this from the start
 // and its compute warps join once the task queue is empty, so the zero
-// stream ends together with the compute work.  Rows are 12 F bytes, a
-// multiple of 16 (F % 4 == 0).
-__device__ void jac_zero_rows_tma(const JacArgs& a, const void* ztile, int* zq) {
+// stream ends together with the compute work.  Rows are 12 F bytes: a run of
+// rows that does not start or end on 16 bytes (F not a multiple of 4) gets its
+// first and last words by plain stores.  (4-byte stores of such runs by the
+// zero warps alone, of two blocks per SM, made them the longer part: 501 atoms,
+// F = 63: 196 us, 118 us with these copies.)
+__device__ void jac_zero_rows(const JacArgs& a, const void* ztile, int* zq) {
   if ((threadIdx.x & 31) != 0) return;
   const int64_t nrows = a.n_centres * a.n_inc;
-  const int64_t row_bytes = 12 * (int64_t)a.F;
+  const int64_t row_words = 3 * (int64_t)a.F;
   const int64_t nchunks = (nrows + kZeroChunkRows - 1) / kZeroChunkRows;
-  char* out = reinterpret_cast<char*>(a.out);
   for (;;) {
     const int64_t k = (int64_t)(unsigned)atomicAdd(zq, 1);
     if (k >= nchunks) break;
@@ -346,36 +348,20 @@ __device__ void jac_zero_rows_tma(const JacArgs& a, const void* ztile, int* zq) 
       const bool zero = (r < r1) && !((a.bitmap[r >> 5] >> (r & 31)) & 1u);
       if (zero && run < 0) run = r;
       if (!zero && run >= 0) {  // zero rows [run, r)
-        char* p = out + run * row_bytes;
-        int64_t n = (r - run) * row_bytes;
-        while (n > 0) {
-          const uint32_t c = (uint32_t)(n < kZeroTile ? n : kZeroTile);
-          bulk_s2g(p, ztile, c);
-          p += c;
-          n -= c;
+        const int64_t i0 = run * row_words, i1 = r * row_words;
+        const int64_t b0 = min((i0 + 3) & ~(int64_t)3, i1), b1 = max(i1 & ~(int64_t)3, b0);  // multiples of 16 bytes
+        for (int64_t i = i0; i < b0; ++i) __stcs(a.out + i, 0.0f);
+        for (int64_t i = b0; i < b1; i += kZeroTile / 4) {
+          const int64_t bytes = 4 * (b1 - i);
+          bulk_s2g(a.out + i, ztile, (uint32_t)(bytes < kZeroTile ? bytes : kZeroTile));
         }
+        for (int64_t i = b1; i < i1; ++i) __stcs(a.out + i, 0.0f);
         run = -1;
       }
     }
     asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
   }
   asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
-}
-
-// Zero rows with 16-byte stores (rows not a multiple of 16 bytes), same chunks.
-__device__ void jac_zero_rows_st(const JacArgs& a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nrows = a.n_centres * a.n_inc;
-  const int64_t rowf = 3 * (int64_t)a.F;
-  const int64_t nchunks = (nrows + kZeroChunkRows - 1) / kZeroChunkRows;
-  for (int64_t k = blockIdx.x; k < nchunks; k += gridDim.x) {
-    const int64_t r0 = k * kZeroChunkRows, r1 = min(r0 + (int64_t)kZeroChunkRows, nrows);
-    for (int64_t r = r0; r < r1; ++r) {
-      if ((a.bitmap[r >> 5] >> (r & 31)) & 1u) continue;
-      float* p = a.out + r * rowf;
-      for (int64_t i = lane; i < rowf; i += 32) __stcs(p + i, 0.0f);
-    }
-  }
 }
 
 // Named barrier over the compute warps only (id 1; id 0 is __syncthreads).
@@ -671,8 +657,7 @@ __global__ void __launch_bounds__(256, 2) k_jacobian(JacArgs a) {
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // tile visible to the bulk-copy engine
   __syncthreads();
   if (threadIdx.x < 32) {  // zero role
-    if (vec) jac_zero_rows_tma(a, ztile, a.counter + 1);
-    else jac_zero_rows_st(a);
+    jac_zero_rows(a, ztile, a.counter + 1);
     return;
   }
   // compute role: warps 1..7, named barrier 1
@@ -801,7 +786,7 @@ __global__ void __launch_bounds__(256, 2) k_jacobian(JacArgs a) {
     task = s_task[it];
   }
   // task queue empty: this warp joins the zero-row stream
-  if (vec) jac_zero_rows_tma(a, ztile, a.counter + 1);
+  jac_zero_rows(a, ztile, a.counter + 1);
 }
 
 // ---------------------------------------------------------------------------

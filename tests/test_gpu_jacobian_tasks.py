@@ -68,3 +68,26 @@ def test_moving_centres(basis, kind, average):
     # the centre whose atom is left out has no centre row; the others keep theirs
     assert (Jx[0, 0] - Ja[0, 0]).norm() <= TOL * Ja[0, 0].norm()
     assert torch.isfinite(Jx).all()
+
+
+@pytest.mark.parametrize("n_max,l_max,n_species", [(1, 0, 1), (1, 1, 2), (1, 2, 2), (1, 0, 2), (3, 2, 2), (2, 1, 2)])
+def test_zero_rows_of_any_length(monkeypatch, n_max, l_max, n_species):
+    """Runs of zero rows that start and end anywhere within 16 bytes: every element is written."""
+    s = W.water_cluster(1, 1, 9, seed=6)
+    if n_species == 1:
+        s = dict(s, atomic_numbers=np.ones(len(s["atomic_numbers"]), int))
+    basis = dict(species=[1, 8][:n_species], r_cut=2.5, n_max=n_max, l_max=l_max, sigma=0.3)
+    n = len(s["atomic_numbers"])
+    centres, include = [0, 7, n - 1], [i for i in range(n) if i % 7 != 3]
+    from cusoap_b200 import SOAP
+    soap, empty = SOAP(**basis), torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: (lambda t: t.fill_(float("nan")) if t.is_floating_point() else t)(
+        empty(*a, **k)))
+    J = soap.derivatives(s, centers=centres, include=include, return_descriptor=False)
+    monkeypatch.undo()
+    Jo, _ = OracleSOAP(**basis).derivatives(s["positions"], s["atomic_numbers"], centers=centres, include=include)
+    J, far = J.cpu().numpy(), (np.asarray(Jo) == 0.0).all((2, 3))
+    assert far.any(1).all() and not far.all(1).any()
+    assert (J[far] == 0.0).all()
+    for k in range(3):
+        assert rel_l2(J[k], Jo[k]) < TOL
