@@ -631,8 +631,12 @@ __device__ void centre_row(const JacArgs& a, int64_t p0, const unsigned long lon
 // pairs during the contraction, and the centre's coefficient row comes in by
 // asynchronous copies.  1536 atoms, entries (then 67 us) included: 2.08 ms
 // without this, 1.83 ms with it (12 GB take 1.81 ms at the measured copy rate).
-template <int L>
-__global__ void __launch_bounds__(256, 2) k_jacobian(JacArgs a) {
+//
+// Two blocks per SM, whose registers hold the four features of a thread; three
+// (80 registers, small spills) for rows of few features, where the stages'
+// latencies are the time (see JacDispatch).
+template <int L, int B>
+__global__ void __launch_bounds__(256, B) k_jacobian(JacArgs a) {
   using Sh = JacShape<L>;
   constexpr int K = Sh::K, KC = Sh::KC;
   constexpr int kCT = 224;  // compute threads (warps 1..7)
@@ -855,7 +859,13 @@ struct JacDispatch {
     // 2. one launch: in every block warp 0 streams zero rows, warps 1..7 compute
     const size_t smem = base + 4 * (size_t)eb * EF;
     if (smem > 220 * 1024) return set_error(SOAPB_ERR_UNSUPPORTED, "jacobian shared memory %zu B too large", smem);
-    auto kern = k_jacobian<L>;
+    // Three blocks per SM for l_max <= 4 with at most 192 features and a centre for each block.
+    // 900 atoms: F = 8 97 -> 85 us, F = 144 284 -> 263, F = 180 359 -> 327; 1536 atoms, F = 72:
+    // 607 -> 540.  More features or fewer centres are slower with three (900 atoms, F = 272: 407
+    // and 415 us; 192 atoms, F = 144: 46 and 53).
+    auto kern = k_jacobian<L, 2>;
+    if constexpr (L <= 4)
+      if (a.F <= 192 && a.n_centres >= 3 * (int64_t)nsm) kern = k_jacobian<L, 3>;
     rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                     "jacobian smem attribute");
     if (rc) return rc;

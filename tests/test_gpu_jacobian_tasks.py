@@ -91,3 +91,18 @@ def test_zero_rows_of_any_length(monkeypatch, n_max, l_max, n_species):
     assert (J[far] == 0.0).all()
     for k in range(3):
         assert rel_l2(J[k], Jo[k]) < TOL
+
+
+@pytest.mark.parametrize("average", ["off", "cc"])
+@pytest.mark.parametrize("n_max,l_max", [(3, 0), (2, 1), (4, 2), (4, 3), (4, 4), (2, 4)])
+def test_many_centres_of_few_features(n_max, l_max, average):
+    """More centres than three blocks on every SM take: the blocks of centres evaluated alone."""
+    s = W.water_cluster(5, 5, 8, seed=8)
+    soap = _soap(r_cut=2.5, n_max=n_max, l_max=l_max, sigma=0.3, average=average)
+    assert len(s["atomic_numbers"]) == 600
+    for attach in (False, True):
+        J = soap.derivatives(s, attach=attach, return_descriptor=False)
+        pick = list(range(0, 600, 37))
+        few = soap.derivatives(s, centers=pick, attach=attach, return_descriptor=False)
+        assert torch.equal(J[pick] == 0.0, few == 0.0)
+        assert (J[pick].double() - few.double()).norm() <= TOL * few.double().norm()
