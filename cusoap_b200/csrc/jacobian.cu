@@ -548,7 +548,10 @@ __device__ __forceinline__ void quad_values(const JacArgs& a, const float* ed, i
 // 12 FMAs an edge for every feature in batches of eb that follow one another
 // (192 atoms, 130 edges a centre, cc: 193 us against 89 us, entries
 // included).  The edges are sorted by species, so a thread keeps its
-// (n, lm) in registers and adds it to D when the species changes.
+// (n, lm) in registers and adds it to D when the species changes.  An edge's
+// two terms, which often cancel, are added first, then eight edges, then those
+// of a batch: 1.74e-7 from float64 for these 192 atoms.  One FMA after the other
+// is 1.92e-7 away, batches of edges for every feature 1.81e-7; the time is the same.
 template <int L>
 __device__ void centre_row(const JacArgs& a, int64_t p0, const unsigned long long* keys, int n, const float* cs,
                            float* smem, float* orow, const float* sqrt_pref, int tid, int nth) {
@@ -570,14 +573,14 @@ __device__ void centre_row(const JacArgs& a, int64_t p0, const unsigned long lon
       int l = 0;
       while ((l + 1) * (l + 1) <= lm) ++l;
       const int fn = 8 + l * N + nn, iR = 8 + 2 * NF + lm;
-      float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
+      float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f, w0 = 0.0f, w1 = 0.0f, w2 = 0.0f;
       int cur = (int)ed[3];
       auto flush = [&]() {
         float* d = D + cur * NK + it;
-        d[0] -= v0;
-        d[SNK] -= v1;
-        d[2 * SNK] -= v2;
-        v0 = v1 = v2 = 0.0f;
+        d[0] -= w0 + v0;
+        d[SNK] -= w1 + v1;
+        d[2 * SNK] -= w2 + v2;
+        v0 = v1 = v2 = w0 = w1 = w2 = 0.0f;
       };
       for (int i = 0; i < nb; ++i) {
         const float* h = ed + (size_t)i * EF;
@@ -585,10 +588,14 @@ __device__ void centre_row(const JacArgs& a, int64_t p0, const unsigned long lon
           flush();
           cur = (int)h[3];
         }
+        if ((i & 7) == 0) {
+          w0 += v0; w1 += v1; w2 += v2;
+          v0 = v1 = v2 = 0.0f;
+        }
         const float bR = h[fn + NF] * h[iR], b = h[fn];
-        v0 = fmaf(h[0], bR, fmaf(b, h[iR + K], v0));
-        v1 = fmaf(h[1], bR, fmaf(b, h[iR + 2 * K], v1));
-        v2 = fmaf(h[2], bR, fmaf(b, h[iR + 3 * K], v2));
+        v0 += fmaf(h[0], bR, b * h[iR + K]);
+        v1 += fmaf(h[1], bR, b * h[iR + 2 * K]);
+        v2 += fmaf(h[2], bR, b * h[iR + 3 * K]);
       }
       flush();
     }
