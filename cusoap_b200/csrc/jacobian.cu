@@ -552,9 +552,11 @@ __device__ __forceinline__ void quad_values(const JacArgs& a, const float* ed, i
 // two terms, which often cancel, are added first, then eight edges, then those
 // of a batch: 1.74e-7 from float64 for these 192 atoms.  One FMA after the other
 // is 1.92e-7 away, batches of edges for every feature 1.81e-7; the time is the same.
+// pref is the factor sqrt(8 pi^2 / (2 l + 1)) itself: the square of its root that
+// the staged vectors carry is off by up to 1.25e-7, for every feature of an l.
 template <int L>
 __device__ void centre_row(const JacArgs& a, int64_t p0, const unsigned long long* keys, int n, const float* cs,
-                           float* smem, float* orow, const float* sqrt_pref, int tid, int nth) {
+                           float* smem, float* orow, const float* pref, int tid, int nth) {
   using Sh = JacShape<L>;
   constexpr int K = Sh::K, KC = Sh::KC;
   const int N = a.N, SNK = a.S * N * K, NK = N * K, NF = N * (L + 1), EF = Sh::xoff(N), F = a.F;
@@ -614,10 +616,9 @@ __device__ void centre_row(const JacArgs& a, int64_t p0, const unsigned long lon
         v1 += da[SNK + m] * y + x * db[SNK + m];
         v2 += da[2 * SNK + m] * y + x * db[2 * SNK + m];
       }
-      const float pref = sqrt_pref[l] * sqrt_pref[l];
-      __stcs(orow + f, pref * v0);
-      __stcs(orow + F + f, pref * v1);
-      __stcs(orow + 2 * F + f, pref * v2);
+      __stcs(orow + f, pref[l] * v0);
+      __stcs(orow + F + f, pref[l] * v1);
+      __stcs(orow + 2 * F + f, pref[l] * v2);
     }
   } else {
     for (int f = tid; f < F; f += nth) {
@@ -655,7 +656,7 @@ __global__ void __launch_bounds__(256, B) k_jacobian(JacArgs a) {
   float* cs = ztile + kZeroTile / 4;
   float* ed = cs + Sh::cs_floats(N, S);
   const int EF = Sh::entry_floats(N, S, a.mode);
-  __shared__ float s_sqrt_pref[kMaxL + 1];
+  __shared__ float s_sqrt_pref[kMaxL + 1], s_pref[kMaxL + 1];
   __shared__ int s_gstart[33], s_grow[32];  // first entry and output row of each row group of the batch
   __shared__ int s_ng;
   __shared__ int4 s_task[2];
@@ -663,7 +664,10 @@ __global__ void __launch_bounds__(256, B) k_jacobian(JacArgs a) {
   __shared__ int64_t s_p0;
   __shared__ unsigned long long s_key[32];
   __shared__ __align__(16) float4 s_pair[32];
-  if (threadIdx.x <= L) s_sqrt_pref[threadIdx.x] = sqrtf(sqrtf(8.0f * (float)(kPi * kPi) / (2.0f * threadIdx.x + 1.0f)));
+  if (threadIdx.x <= L) {
+    s_pref[threadIdx.x] = sqrtf(8.0f * (float)(kPi * kPi) / (2.0f * threadIdx.x + 1.0f));
+    s_sqrt_pref[threadIdx.x] = sqrtf(s_pref[threadIdx.x]);
+  }
   for (int i = threadIdx.x; i < kZeroTile / 4; i += blockDim.x) ztile[i] = 0.0f;
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // tile visible to the bulk-copy engine
   __syncthreads();
@@ -707,7 +711,7 @@ __global__ void __launch_bounds__(256, B) k_jacobian(JacArgs a) {
     float* obase = a.out + (size_t)c * a.n_inc * 3 * F;
     if (nent < 0) {
       copy_async_wait();  // cs: visible to all after centre_row's first barrier
-      centre_row<L>(a, a.pair_off[c], keys, -nent, cs, ed, obase + (size_t)crow * 3 * F, s_sqrt_pref, tid, kCT);
+      centre_row<L>(a, a.pair_off[c], keys, -nent, cs, ed, obase + (size_t)crow * 3 * F, s_pref, tid, kCT);
       if (tid == 0) s_task[it] = next;
       compute_bar(kCT);
       task = s_task[it];
