@@ -215,9 +215,12 @@ struct SolidHarmonics {
   // Values and Cartesian gradients: store(idx, v, dx, dy, dz).
   // dQ_l^m/dx = -x Q_{l-1}^{m+1}, dQ_l^m/dy = -y Q_{l-1}^{m+1},
   // dQ_l^m/dz = (l+m) Q_{l-1}^m; d(x+iy)^m = m (x+iy)^{m-1} (dx + i dy).
+  // Which product of a sum is rounded is written out: derivatives are also asked
+  // for as float64, and the compiler's choice moved a tenth of them with the code around it.
   template <class Store>
   __device__ __forceinline__ static void with_gradients(float x, float y, float z, Store&& store) {
-    const float r2 = x * x + y * y + z * z;
+    const float r2 = fmaf(z, z, fmaf(x, x, __fmul_rn(y, y)));
+    auto sum = [](float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); };  // a b + c d
     float Q[NQ];
     legendre(z, r2, Q);
     float C = 1.0f, S = 0.0f, Cp = 0.0f, Sp = 0.0f;  // (x+iy)^m and ^(m-1)
@@ -226,8 +229,8 @@ struct SolidHarmonics {
       if (m > 0) {
         Cp = C;
         Sp = S;
-        const float Cn = x * C - y * S;
-        S = x * S + y * C;
+        const float Cn = sum(x, C, -y, S);
+        S = sum(y, C, x, S);
         C = Cn;
       }
 #pragma unroll
@@ -239,13 +242,13 @@ struct SolidHarmonics {
         if (m == 0) {
           store(l * l + l, nrm * q, nrm * (-x * qp), nrm * (-y * qp), nrm * qz);
         } else {
-          const float fm = (float)m;
+          const float fq = q * (float)m, xq = -x * qp, yq = -y * qp;
           // +m: Re (x+iy)^m
-          store(l * l + l + m, nrm * q * C, nrm * (-x * qp * C + q * fm * Cp), nrm * (-y * qp * C - q * fm * Sp),
-                nrm * qz * C);
+          store(l * l + l + m, nrm * q * C, nrm * (m == 1 ? sum(xq, C, fq, Cp) : sum(fq, Cp, xq, C)),
+                nrm * sum(yq, C, -fq, Sp), nrm * qz * C);
           // -m: Im (x+iy)^m
-          store(l * l + l - m, nrm * q * S, nrm * (-x * qp * S + q * fm * Sp), nrm * (-y * qp * S + q * fm * Cp),
-                nrm * qz * S);
+          store(l * l + l - m, nrm * q * S, nrm * sum(xq, S, fq, Sp),
+                nrm * (m == 1 ? sum(yq, S, fq, Cp) : sum(fq, Cp, yq, S)), nrm * qz * S);
         }
       }
     }

@@ -383,7 +383,7 @@ template <int L>
 __device__ __forceinline__ void stage_harmonics(const JacArgs& a, const float4& pr, bool centre_row, float* h) {
   constexpr int K = JacShape<L>::K;
   const int NF = a.N * (L + 1);
-  const float r = sqrtf(pr.x * pr.x + pr.y * pr.y + pr.z * pr.z);
+  const float r = sqrtf(fmaf(pr.z, pr.z, fmaf(pr.x, pr.x, __fmul_rn(pr.y, pr.y))));
   int seg;
   float t;
   seg_coord(r, a.inv_h, a.nseg, seg, t);
@@ -517,9 +517,9 @@ __device__ __forceinline__ void quad_values(const JacArgs& a, const float* ed, i
       for (int k = 0; k < 4; ++k) {
         const int ia = qc.code[k] & 4095, ib = (qc.code[k] >> 12) & 4095;
         const float4 pa = X[ia], qa = X[SNL + ia], pb = X[ib], qb = X[SNL + ib];
-        v[0][k] += pa.z * pb.x + pa.y * pb.w + pb.z * pa.x + pb.y * pa.w;
-        v[1][k] += qa.x * pb.x + pa.y * qb.y + qb.x * pa.x + pb.y * qa.y;
-        v[2][k] += qa.z * pb.x + pa.y * qb.w + qb.z * pa.x + pb.y * qa.w;
+        v[0][k] += fmaf(pb.y, pa.w, fmaf(pb.z, pa.x, fmaf(pa.z, pb.x, __fmul_rn(pa.y, pb.w))));
+        v[1][k] += fmaf(pb.y, qa.y, fmaf(qb.x, pa.x, fmaf(qa.x, pb.x, __fmul_rn(pa.y, qb.y))));
+        v[2][k] += fmaf(pb.y, qa.w, fmaf(qb.z, pa.x, fmaf(qa.z, pb.x, __fmul_rn(pa.y, qb.w))));
       }
     }
   } else {
