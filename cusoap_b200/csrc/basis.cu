@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(512) k_basis_build(BasisDev a) {
     cheb_to_mono(f, a.tabf + ((size_t)fn * force_tab_stride(a.nseg) + seg) * kNCoef);
   }
   __syncthreads();
-  for (int i = tid; N <= 8 && i < a.nseg * NF; i += blockDim.x) {  // i = seg NF + l N + n
+  for (int i = tid; radial_lanes(N, L) && i < a.nseg * NF; i += blockDim.x) {  // i = seg NF + l N + n
     const int seg = i / NF, fn = i % NF, l = fn / N, n = fn % N, NP = stream_lanes(N);
     for (int k = 0; k < kNCoef; ++k) {
       const int c = pair_coef(l, L, k);

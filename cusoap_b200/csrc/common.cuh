@@ -80,12 +80,16 @@ __device__ __forceinline__ void load_coef(const float* __restrict__ tab, int seg
 // a_0(lo), a_1(hi), ...}, then l = 0 alone when l_max is even.  Segments hold
 // them as [16-byte chunk][n][4 floats], n padded to the lanes of a stream: the
 // lanes load a chunk from consecutive addresses, at immediate offsets.
+constexpr int kMaxLNLanes = 6;
 __host__ __device__ inline int stream_lanes(int N) { return N <= 4 ? 4 : 8; }
 inline int64_t off_tab_pairs(const soapb_basis* b) {
   return b->off_tab_b + align_up(4 * (int64_t)b->n_seg * b->n_max * (b->l_max + 1) * kNCoef, 256);
 }
-inline int64_t tab_pairs_bytes(const soapb_basis* b) {  // built for n_max <= 8
-  return b->n_max > 8 ? 0 : align_up(4 * (int64_t)b->n_seg * stream_lanes(b->n_max) * (b->l_max + 1) * kNCoef, 256);
+// Bases of the radial-index-lane kernel, the only reader (its registers set the largest l_max).
+__host__ __device__ inline bool radial_lanes(int N, int L) { return N <= 8 && L <= kMaxLNLanes; }
+inline int64_t tab_pairs_bytes(const soapb_basis* b) {
+  if (!radial_lanes(b->n_max, b->l_max)) return 0;
+  return align_up(4 * (int64_t)b->n_seg * stream_lanes(b->n_max) * (b->l_max + 1) * kNCoef, 256);
 }
 // Position of coefficient k of l among a radial index's coefficients.
 __host__ __device__ inline int pair_coef(int l, int L, int k) {
@@ -109,11 +113,6 @@ __device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   f32x2 d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 

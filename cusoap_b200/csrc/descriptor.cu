@@ -109,7 +109,6 @@ inline bool desc_two_streams(int N, int L) {
 }
 
 constexpr int kMaxBlocks = kMaxS * (kMaxS + 1) / 2;
-constexpr int kMaxLNLanes = 6;  // largest l_max of the radial-index-lane kernel (registers)
 constexpr int kMaxTri = kMaxN * (kMaxN + 1) / 2;
 
 // Per-block tables of the power-spectrum epilogue: the prefactor
@@ -927,7 +926,7 @@ template <int L>
 struct DescDispatch {
   static int run(const DescArgs& a, int gn, int wpb, bool lgroup_only, cudaStream_t st) {
     if constexpr (L <= kMaxLNLanes) {
-      if (!lgroup_only && a.N <= 8 && isfinite(a.self_ratio))
+      if (!lgroup_only && radial_lanes(a.N, L) && isfinite(a.self_ratio))
         return a.N <= 4 ? launch_descriptor_n<L, 4>(a, wpb, st) : launch_descriptor_n<L, 8>(a, wpb, st);
     }
     if constexpr (L <= 4) {
