@@ -57,7 +57,6 @@ struct JacArgs {
   const float* selfv;    // w0 B_nl(0) for r = 0 edges
   const int* ftab;
   float* out;
-  int* status;
   int* counter;                  // {next task, next zero chunk, tasks, 0}
   int2* tasks;                   // {centre, entries (negative: the centre's own row)}, {first entry in ent: low, high
                                  // word}; 8-byte loads, the alignment that a workspace always needed
@@ -933,7 +932,6 @@ extern "C" int soapb_jacobian(const soapb_basis* b, int64_t n_centres, const int
   a.selfv = (const float*)((const char*)b->dev + b->off_self);
   a.ftab = (const int*)((const char*)b->dev + b->off_ftab);
   a.out = d_out;
-  a.status = d_status;
   a.counter = (int*)(w + Lw.counter);
   a.tasks = (int2*)(w + Lw.tasks);
   a.ent = (unsigned long long*)(w + Lw.ent);

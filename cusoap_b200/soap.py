@@ -857,9 +857,6 @@ class SOAP:
         # species numbers outside the table
         return np.searchsorted(np.asarray(self._atomic_numbers_list), Zc).astype(np.int32)
 
-    def _species_index(self, Z) -> torch.Tensor:
-        return torch.as_tensor(self._species_lookup(Z)).to(self.device)
-
     def _upload(self, arrays) -> Tuple[_DevArrays, torch.Tensor]:
         """Copy named host arrays to the device in one asynchronous copy from a
         page-locked staging buffer: the arrays and the buffer, which the caller
