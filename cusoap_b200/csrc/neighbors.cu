@@ -311,19 +311,22 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
   for (int k = 0; k < 3; ++k) anyp |= s.d_pbc[i * 3 + k] ? 1 : 0;
   for (int k = 0; k < 9; ++k) g.H[k] = anyp ? s.d_cells[i * 9 + k] : ((k % 4 == 0) ? 1.0 : 0.0);
   const double* H = g.H;
-  const double det = H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
-                     H[2] * (H[3] * H[7] - H[4] * H[6]);
+  // inverse of the row-vector matrix: x = f H  =>  f = x H^-1.  The roundings are written out: the
+  // bin of an atom on a bin's edge (a lattice site of a skewed cell) depends on the last one.
+  auto minor = [&](int a, int b, int c, int d) { return fma(H[a], H[b], -__dmul_rn(H[c], H[d])); };
+  const double m0 = minor(4, 8, 5, 7), m6 = minor(3, 7, 4, 6);
+  const double m3 = __dsub_rn(__dmul_rn(H[3], H[8]), __dmul_rn(H[5], H[6]));
+  const double det = fma(H[2], m6, fma(H[0], m0, -__dmul_rn(H[1], m3)));
   const double id = !anyp ? 1.0 : fabs(det) < 1e-300 ? 0.0 : 1.0 / det;
-  // inverse of the row-vector matrix: x = f H  =>  f = x H^-1
-  g.Hinv[0] = (H[4] * H[8] - H[5] * H[7]) * id;
-  g.Hinv[1] = (H[2] * H[7] - H[1] * H[8]) * id;
-  g.Hinv[2] = (H[1] * H[5] - H[2] * H[4]) * id;
-  g.Hinv[3] = (H[5] * H[6] - H[3] * H[8]) * id;
-  g.Hinv[4] = (H[0] * H[8] - H[2] * H[6]) * id;
-  g.Hinv[5] = (H[2] * H[3] - H[0] * H[5]) * id;
-  g.Hinv[6] = (H[3] * H[7] - H[4] * H[6]) * id;
-  g.Hinv[7] = (H[1] * H[6] - H[0] * H[7]) * id;
-  g.Hinv[8] = (H[0] * H[4] - H[1] * H[3]) * id;
+  g.Hinv[0] = m0 * id;
+  g.Hinv[1] = minor(2, 7, 1, 8) * id;
+  g.Hinv[2] = minor(1, 5, 2, 4) * id;
+  g.Hinv[3] = minor(5, 6, 3, 8) * id;
+  g.Hinv[4] = minor(0, 8, 2, 6) * id;
+  g.Hinv[5] = minor(2, 3, 0, 5) * id;
+  g.Hinv[6] = m6 * id;
+  g.Hinv[7] = minor(1, 6, 0, 7) * id;
+  g.Hinv[8] = minor(0, 4, 1, 3) * id;
   for (int k = 0; k < 3; ++k) {
     g.per[k] = anyp ? (s.d_pbc[i * 3 + k] ? 1 : 0) : 0;
     g.fmin[k] = 0.0;
