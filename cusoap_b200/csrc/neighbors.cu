@@ -43,6 +43,7 @@ struct GridDesc {
                      // -1: no frame (a periodic cell without a volume, or so thin that its images
                      // could not be counted, or not of numbers): no pairs
   signed char wide;  // an axis has more images than pack3 holds: image shifts in pack_wide
+  signed char fine;  // diagonal frame with quarter-cutoff bins: an image's shift is one product an axis
   // FP32 geometry of the window (Angstrom): perpendicular bin widths; for other than diagonal
   // frames the direction of lattice row a, the reciprocal of a bin's length along it, the edges
   // of a bin along b and c, and the largest distance of a bin's point from the bin row's axis
@@ -139,9 +140,17 @@ __device__ __forceinline__ int struct_of_atom(const int64_t* atom_off, int n_str
   return lo;
 }
 
+// Arithmetic that decides a bin or a pair has its roundings written out: it is done in several
+// kernels (bins and records, count and fill), which have to agree to the last bit where an atom
+// lies on the edge of a bin or a pair at the cutoff.
 __device__ __forceinline__ void to_frac(const GridDesc& g, double x, double y, double z, double (&f)[3]) {
 #pragma unroll
-  for (int j = 0; j < 3; ++j) f[j] = x * g.Hinv[j] + y * g.Hinv[3 + j] + z * g.Hinv[6 + j];
+  for (int j = 0; j < 3; ++j) f[j] = fma(z, g.Hinv[6 + j], fma(x, g.Hinv[j], __dmul_rn(y, g.Hinv[3 + j])));
+}
+
+// Component k of t[0] a + t[1] b + t[2] c.
+__device__ __forceinline__ double lattice_sum(const double* H, const int (&t)[3], int k) {
+  return fma((double)t[2], H[6 + k], fma((double)t[0], H[k], __dmul_rn((double)t[1], H[3 + k])));
 }
 
 // Bin, wrap shift and wrapped position of a point of structure g.
@@ -165,9 +174,9 @@ __device__ __forceinline__ bool locate(const GridDesc& g, double x, double y, do
       b[i] = min(max(bi, 0), g.nb[i] - 1);
     }
   }
-  wp[0] = x - (w[0] * g.H[0] + w[1] * g.H[3] + w[2] * g.H[6]);
-  wp[1] = y - (w[0] * g.H[1] + w[1] * g.H[4] + w[2] * g.H[7]);
-  wp[2] = z - (w[0] * g.H[2] + w[1] * g.H[5] + w[2] * g.H[8]);
+  wp[0] = __dsub_rn(x, lattice_sum(g.H, w, 0));
+  wp[1] = __dsub_rn(y, lattice_sum(g.H, w, 1));
+  wp[2] = __dsub_rn(z, lattice_sum(g.H, w, 2));
   return ok;
 }
 
@@ -334,7 +343,7 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
     g.nb[k] = 1;
     g.nrep[k] = 0;
   }
-  g.wrapped = 0;
+  g.wrapped = g.fine = 0;
   g.orth = 1;
   for (int k = 0; k < 9; ++k)
     if (k % 4 == 0 ? !(H[k] > 0.0) : H[k] != 0.0) g.orth = 0;
@@ -429,8 +438,11 @@ __device__ __forceinline__ void frac_bbox(const soapb_structs& s, const NLWork& 
 __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork& w, double cutoff, int i) {
   GridDesc g = w.grids[i];
   const double* H = g.H;
-  const double det = fabs(H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
-                          H[2] * (H[3] * H[7] - H[4] * H[6]));
+  // (roundings written out: a width of a whole number of bins, up to the last bit, sets that number)
+  auto minor = [](double a, double b, double c, double d) { return fma(a, b, -__dmul_rn(c, d)); };
+  const double det = fabs(fma(H[2], minor(H[3], H[7], H[4], H[6]),
+                              fma(H[0], minor(H[4], H[8], H[5], H[7]),
+                                  -__dmul_rn(H[1], minor(H[3], H[8], H[5], H[6])))));
   if (g.orth < 0) {  // one bin of which nothing is visited (its window would have no end)
     // (flagged here, behind a barrier from the clear of the flags)
     if (det < INFINITY) atomicOr(w.status, 1);
@@ -446,8 +458,9 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
     for (int k = 0; k < 3; ++k) {
       const double* u = H + 3 * ((k + 1) % 3);
       const double* v = H + 3 * ((k + 2) % 3);
-      const double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2], cz = u[0] * v[1] - u[1] * v[0];
-      perp[k] = det / (sqrt(cx * cx + cy * cy + cz * cz) + 1e-300);
+      const double cx = minor(u[1], v[2], u[2], v[1]), cy = minor(u[2], v[0], u[0], v[2]),
+                   cz = minor(u[0], v[1], u[1], v[0]);
+      perp[k] = det / (sqrt(fma(cz, cz, fma(cx, cx, __dmul_rn(cy, cy)))) + 1e-300);
     }
   const int64_t A = s.d_atom_off[i + 1] - s.d_atom_off[i];
   // Bins of perpendicular width >= cutoff / 4 in diagonal frames, unless a
@@ -456,7 +469,8 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
   // The line is where it always was: the bins set the order of the pairs.
   // Quarter bins everywhere would gain little (501 atoms, triclinic: count 18
   // instead of 19 us, fill 22 instead of 23).
-  const double bin_min = (g.orth && !(g.per[0] && perp[0] < 0.75 * cutoff) ? 0.25 : 0.5) * cutoff;
+  const bool fine = g.orth && !(g.per[0] && perp[0] < 0.75 * cutoff);
+  const double bin_min = (fine ? 0.25 : 0.5) * cutoff;
   double far[3];  // largest |fractional coordinate| of a wrapped atom, from the origin of the FP32 copies
   for (int k = 0; k < 3; ++k) {
     if (g.per[k]) {
@@ -486,6 +500,7 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
     g.nb[k] = max(1, g.nb[k] / 2);
     binw[k] = span / g.nb[k];
   }
+  g.fine = fine && !(g.per[0] && g.nb[0] < 3);
   for (int k = 0; k < 3; ++k) {
     g.binw[k] = binw[k];
     // a single bin of an open axis may be as thin as its atoms; the window takes it at least 1e-3 A wide
@@ -754,15 +769,19 @@ __device__ __forceinline__ double4 load_record(const double4* p) {
 // rvec of the candidate in a slot with cell-window shift T (of a periodic frame), in FP64.
 __device__ __forceinline__ void exact_rvec(const VisitCentre& C, const double4& p, const int (&T)[3], double& rx,
                                            double& ry, double& rz) {
+  const double* H = C.g->H;
   if (!C.per) {
     rx = p.x - C.cp.x;
     ry = p.y - C.cp.y;
     rz = p.z - C.cp.z;
+  } else if (C.g->fine) {  // a diagonal frame: one product an axis
+    rx = __dadd_rn(p.x, fma((double)T[0], H[0], -C.cp.x));
+    ry = __dadd_rn(p.y, fma((double)T[1], H[4], -C.cp.y));
+    rz = __dadd_rn(p.z, fma((double)T[2], H[8], -C.cp.z));
   } else {
-    const double* H = C.g->H;
-    rx = p.x + (T[0] * H[0] + T[1] * H[3] + T[2] * H[6] - C.cp.x);
-    ry = p.y + (T[0] * H[1] + T[1] * H[4] + T[2] * H[7] - C.cp.y);
-    rz = p.z + (T[0] * H[2] + T[1] * H[5] + T[2] * H[8] - C.cp.z);
+    rx = __dadd_rn(p.x, __dsub_rn(lattice_sum(H, T, 0), C.cp.x));
+    ry = __dadd_rn(p.y, __dsub_rn(lattice_sum(H, T, 1), C.cp.y));
+    rz = __dadd_rn(p.z, __dsub_rn(lattice_sum(H, T, 2), C.cp.z));
   }
 }
 
@@ -774,7 +793,7 @@ __device__ __forceinline__ bool exact_test(const VisitArgs& A, const VisitCentre
   if (C.per) C.unpack(Tpacked, T);
   double rx, ry, rz;
   exact_rvec(C, p, T, rx, ry, rz);
-  const double r2 = rx * rx + ry * ry + rz * rz;
+  const double r2 = fma(rz, rz, fma(rx, rx, __dmul_rn(ry, ry)));
   if (!(r2 <= A.cutoff2)) return false;
   int atom, sp, wrap;
   unpack_info(p.w, atom, sp, wrap);

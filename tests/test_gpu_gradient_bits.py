@@ -32,7 +32,7 @@ PAIRS = {
     ("triclinic", 6.0, 21, 2, 3.0): "d63d80bd3b0a5369731af4720dc7d66a",
     ("triclinic", 6.0, 21, 2, 6.0): "3f97027b3989590dda11b215f74e0683",
     ("triclinic", 16.0, 330, 4, 3.0): "069d0b2037a3d9ae8882b54caae2d508",
-    ("triclinic", 16.0, 330, 4, 6.0): "1aa0101ec645095e4bd6445435b44c69",
+    ("triclinic", 16.0, 330, 4, 6.0): "1aa0101ec645095e90c372a3f72a376a",
     ("slab", 12.0, 150, 3, 3.0): "8b1417e9a2456a36e8aa58ac604bf0d0",
     ("slab", 12.0, 150, 3, 6.0): "0a40912671618706edacae3b1509cf77",
 }
@@ -67,11 +67,11 @@ COEFFICIENTS = {
     ("triclinic", 6.0, 21, 2, 8, 4): "5cc9b80bdd9cc9a5", ("triclinic", 6.0, 21, 2, 7, 5): "e06e9b75f3e890aa",
     ("triclinic", 6.0, 21, 2, 8, 6): "ea8472c426c5e7db", ("triclinic", 6.0, 21, 2, 2, 6): "7cb25e7230ae1b33",
     ("triclinic", 6.0, 21, 2, 10, 4): "7e62261c0ff65a17", ("triclinic", 6.0, 21, 2, 8, 8): "7b6fde5b6ebb26a8",
-    ("triclinic", 16.0, 330, 4, 4, 0): "112c9f688b09f2d6", ("triclinic", 16.0, 330, 4, 8, 1): "c53dbcc326d7ba3d",
-    ("triclinic", 16.0, 330, 4, 3, 2): "aa4d9b199cf62227", ("triclinic", 16.0, 330, 4, 4, 3): "427cb64aa4aeba6b",
-    ("triclinic", 16.0, 330, 4, 8, 4): "4002ef0b987aba05", ("triclinic", 16.0, 330, 4, 7, 5): "c71fefa41122083e",
-    ("triclinic", 16.0, 330, 4, 8, 6): "426dddfd5bff9ba0", ("triclinic", 16.0, 330, 4, 2, 6): "e1d3d3185ba031df",
-    ("triclinic", 16.0, 330, 4, 10, 4): "505e71980aec1ae9", ("triclinic", 16.0, 330, 4, 8, 8): "dec873998e04cad4",
+    ("triclinic", 16.0, 330, 4, 4, 0): "f60af04bb369840d", ("triclinic", 16.0, 330, 4, 8, 1): "e9c0c314480df32e",
+    ("triclinic", 16.0, 330, 4, 3, 2): "cf817cc653457566", ("triclinic", 16.0, 330, 4, 4, 3): "87be270f1af210bf",
+    ("triclinic", 16.0, 330, 4, 8, 4): "12e5af0b07320696", ("triclinic", 16.0, 330, 4, 7, 5): "cd74a5cd2ec73a5a",
+    ("triclinic", 16.0, 330, 4, 8, 6): "fbad6e62d3391de6", ("triclinic", 16.0, 330, 4, 2, 6): "d9c0f21b7794dfba",
+    ("triclinic", 16.0, 330, 4, 10, 4): "7b68df470ebd620d", ("triclinic", 16.0, 330, 4, 8, 8): "0a458a2f4c4c7c9d",
     ("slab", 12.0, 150, 3, 4, 0): "f5de31adc52f1cce", ("slab", 12.0, 150, 3, 8, 1): "0836b7d570e65b4f",
     ("slab", 12.0, 150, 3, 3, 2): "4ddd82ec6229f191", ("slab", 12.0, 150, 3, 4, 3): "99c6563be0587636",
     ("slab", 12.0, 150, 3, 8, 4): "f4f068b62a70d534", ("slab", 12.0, 150, 3, 7, 5): "d9b3e2a01711e082",
@@ -111,6 +111,11 @@ def _digest(t):
     return hashlib.sha256((v + np.zeros((), v.dtype)).tobytes()).hexdigest()[:16]  # (+ 0: one zero)
 
 
+def _at(frac, cell):
+    """frac @ cell without a library's choice of FMAs."""
+    return frac[:, :1] * cell[0] + frac[:, 1:2] * cell[1] + frac[:, 2:] * cell[2]
+
+
 def _structure(kind, side, n, n_species):
     """n atoms; a quarter of them on a lattice of the box's bins, where a rounding decides the bin."""
     rng = np.random.default_rng([n, len(kind), int(10 * side)])
@@ -118,7 +123,7 @@ def _structure(kind, side, n, n_species):
     frac[::4] = np.round(frac[::4] * 8) / 8
     cell = {"open": np.eye(3), "cubic": np.eye(3), "slab": np.diag([1.0, 0.9, 1.2]), "thin": np.diag([0.3, 1.4, 2.0]),
             "triclinic": np.array([[1.0, 0.0, 0.0], [0.2, 0.97, 0.0], [0.1, -0.15, 0.95]])}[kind] * side
-    s = {"positions": frac @ cell, "atomic_numbers": rng.choice(np.array([1, 6, 7, 8][:n_species]), n)}
+    s = {"positions": _at(frac, cell), "atomic_numbers": rng.choice(np.array([1, 6, 7, 8][:n_species]), n)}
     if kind != "open":
         s.update(cell=cell, pbc=[True, True, kind != "slab"])
     return s
@@ -214,3 +219,33 @@ def test_pairs_at_segment_edges():
     assert p.total == 301
     r = _radius(got[:, :3], "bac")
     assert (np.diff(np.minimum((r * np.float32(1.0 / h)).astype(np.int64), nseg - 1)) >= 0).all()
+
+
+# by shape of the cell: 12 cells each
+SITES = {"rotated": "f096e2f68e70664b", "skewed": "8817e01d8cbd18b8", "both": "e08721337261f0da"}
+
+
+def sites(shape):
+    """Pair lists of atoms on lattice sites, where a rounding decides the bin and the image."""
+    from cusoap_b200 import _lib
+    from cusoap_b200.soap import _Batch, _Pairs
+    soap = _soap("cubic", 1, r_cut=4.0, n_max=2, l_max=1, sigma=0.3)
+    out = []
+    for i in range(12):
+        rng = np.random.default_rng([i, len(shape)])
+        cell = np.diag(rng.uniform(3.0, 14.0, 3))
+        if shape != "rotated":
+            cell[1] += rng.uniform(-0.5, 0.5) * cell[0]
+            cell[2] += rng.uniform(-0.5, 0.5) * cell[0] + rng.uniform(-0.5, 0.5) * np.array([0.0, cell[1, 1], 0.0])
+        if shape != "skewed":  # (to 20 bits behind the point, whatever the library's last bits)
+            cell = np.round(_at(cell, np.linalg.qr(rng.standard_normal((3, 3)))[0]) * 2.0 ** 20) / 2.0 ** 20
+        pos = _at(rng.integers(0, 24, (40, 3)) / 24.0 + rng.integers(-1, 2, (40, 3)), cell)
+        p = _Pairs(soap, _Batch(soap, [{"positions": pos, "atomic_numbers": np.ones(40, int), "cell": cell,
+                                        "pbc": [True, True, i % 4 > 0]}], [None]), _lib.NL_ALL)
+        out += [_digest(p.pair_off), _digest(p.pairs[:p.total].view(torch.int32))]
+    return hashlib.sha256("".join(out).encode()).hexdigest()[:16]
+
+
+@pytest.mark.parametrize("shape", ["rotated", "skewed", "both"])
+def test_lattice_sites(shape):
+    assert sites(shape) == SITES[shape]

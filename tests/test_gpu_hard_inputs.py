@@ -121,3 +121,49 @@ def test_jacobian_workspace_of_eight_byte_alignment():
                                   work.data_ptr() + 8, need.value, status.data_ptr(),
                                   torch.cuda.current_stream().cuda_stream))
     assert torch.equal(out, want)
+
+
+def _edge_cells():
+    """Cells a whole number of quarter cutoffs wide between their faces, rectangular, skewed and
+    rotated: lattice vectors at exactly the cutoff, atoms on the edges of bins."""
+    out = []
+    for i in range(60):
+        rng = np.random.default_rng(i)
+        quarters = rng.integers(1, 12, 3).astype(float)
+        skew = np.eye(3)
+        if i % 3:
+            skew[1, 0], skew[2, 0], skew[2, 1] = rng.uniform(-0.5, 0.5, 3)
+        turn = np.linalg.qr(rng.standard_normal((3, 3)))[0] if i % 3 == 2 else np.eye(3)
+        n = 1 + i % 9
+        out.append((quarters, skew, turn, rng.integers(0, 12, (n, 3)) / 12.0, rng.choice(np.array([1, 8]), n)))
+    return out
+
+
+def test_pairs_at_the_cutoff(monkeypatch):
+    """The fill finds the pairs that the count found, also where a rounding decides; all pairs nearer
+    than the cutoff and none beyond it, up to that rounding."""
+    from cusoap_b200 import _lib
+    from cusoap_b200.soap import _Batch, _Pairs
+    soap = _soap(True, n_max=1, l_max=0)
+    rc, empty = soap._cutoff, torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: (
+        lambda t: t.fill_(float("nan")) if t.is_floating_point() and t.is_cuda else t)(empty(*a, **k)))
+    lists = []
+    for quarters, skew, turn, frac, Z in _edge_cells():
+        cell = np.diag(quarters * rc / 4) @ skew @ turn
+        batch = _Batch(soap, [{"positions": frac @ cell, "atomic_numbers": Z, "cell": cell, "pbc": [True] * 3}], [None])
+        p = _Pairs(soap, batch, _lib.NL_ALL)
+        lists.append((cell, frac @ cell, p.pair_off.tolist(), p.pairs[:p.total].cpu().numpy()))
+    monkeypatch.undo()
+    for cell, pos, off, pairs in lists:
+        assert np.isfinite(pairs[:, :3]).all()
+        perp = 1.0 / np.linalg.norm(np.linalg.inv(cell), axis=0)
+        reps = [np.arange(-k, k + 1) for k in np.ceil(rc / perp).astype(int) + 1]
+        shifts = np.stack(np.meshgrid(*reps, indexing="ij"), -1).reshape(-1, 3) @ cell
+        for c in range(len(pos)):
+            r = np.linalg.norm((pos[None] - pos[c]) + shifts[:, None], axis=2).reshape(-1)
+            got = np.sort(np.linalg.norm(pairs[off[c]:off[c + 1], :3].astype(np.float64), axis=1))
+            near, far = np.sort(r[r < rc * (1 - 1e-12)]), np.sum(r <= rc * (1 + 1e-12))
+            assert len(near) <= len(got) <= far
+            assert np.abs(got[:len(near)] - near).max(initial=0.0) < 1e-5
+            assert np.abs(got[len(near):] - rc).max(initial=0.0) < 1e-5
