@@ -43,7 +43,6 @@ struct GridDesc {
                      // -1: no frame (a periodic cell without a volume, or so thin that its images
                      // could not be counted, or not of numbers): no pairs
   signed char wide;  // an axis has more images than pack3 holds: image shifts in pack_wide
-  signed char fine;  // diagonal frame with quarter-cutoff bins: an image's shift is one product an axis
   // FP32 geometry of the window (Angstrom): perpendicular bin widths; for other than diagonal
   // frames the direction of lattice row a, the reciprocal of a bin's length along it, the edges
   // of a bin along b and c, and the largest distance of a bin's point from the bin row's axis
@@ -343,7 +342,7 @@ __device__ __forceinline__ void grid_init(const soapb_structs& s, const NLWork& 
     g.nb[k] = 1;
     g.nrep[k] = 0;
   }
-  g.wrapped = g.fine = 0;
+  g.wrapped = 0;
   g.orth = 1;
   for (int k = 0; k < 9; ++k)
     if (k % 4 == 0 ? !(H[k] > 0.0) : H[k] != 0.0) g.orth = 0;
@@ -469,8 +468,7 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
   // The line is where it always was: the bins set the order of the pairs.
   // Quarter bins everywhere would gain little (501 atoms, triclinic: count 18
   // instead of 19 us, fill 22 instead of 23).
-  const bool fine = g.orth && !(g.per[0] && perp[0] < 0.75 * cutoff);
-  const double bin_min = (fine ? 0.25 : 0.5) * cutoff;
+  const double bin_min = (g.orth && !(g.per[0] && perp[0] < 0.75 * cutoff) ? 0.25 : 0.5) * cutoff;
   double far[3];  // largest |fractional coordinate| of a wrapped atom, from the origin of the FP32 copies
   for (int k = 0; k < 3; ++k) {
     if (g.per[k]) {
@@ -500,7 +498,6 @@ __device__ __forceinline__ void grid_setup(const soapb_structs& s, const NLWork&
     g.nb[k] = max(1, g.nb[k] / 2);
     binw[k] = span / g.nb[k];
   }
-  g.fine = fine && !(g.per[0] && g.nb[0] < 3);
   for (int k = 0; k < 3; ++k) {
     g.binw[k] = binw[k];
     // a single bin of an open axis may be as thin as its atoms; the window takes it at least 1e-3 A wide
@@ -774,10 +771,6 @@ __device__ __forceinline__ void exact_rvec(const VisitCentre& C, const double4& 
     rx = p.x - C.cp.x;
     ry = p.y - C.cp.y;
     rz = p.z - C.cp.z;
-  } else if (C.g->fine) {  // a diagonal frame: one product an axis
-    rx = __dadd_rn(p.x, fma((double)T[0], H[0], -C.cp.x));
-    ry = __dadd_rn(p.y, fma((double)T[1], H[4], -C.cp.y));
-    rz = __dadd_rn(p.z, fma((double)T[2], H[8], -C.cp.z));
   } else {
     rx = __dadd_rn(p.x, __dsub_rn(lattice_sum(H, T, 0), C.cp.x));
     ry = __dadd_rn(p.y, __dsub_rn(lattice_sum(H, T, 1), C.cp.y));
