@@ -693,7 +693,8 @@ __device__ __forceinline__ void flush_row(float* row, const LaneSums<L>& acc) {
   }
 }
 
-template <int L, int NP>
+// U: pairs of a batch without a species change that the loop is unrolled over.
+template <int L, int NP, int U>
 __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
   using Sh = NShape<L, NP>;
   constexpr int K = Sh::K, K4 = Sh::K4, KC = Sh::KC, H = Sh::H;
@@ -803,7 +804,7 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
       if (sp_chg == 0) {
         // no species change in any stream: t, a coefficient reload where the segment changes,
         // Horner and the K FMAs per pair
-#pragma unroll
+#pragma unroll (U)
         for (int j = 0; j < NP; ++j) {
           const int q = h * NP + j;
           // one warp-uniform branch for the streams' reloads, kept a branch by the barrier: the ten
@@ -857,12 +858,12 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
 
 // l_max <= 4: 4 blocks of 4 warps per SM at 128 registers; l_max 5: 3 blocks; l_max 6: 2 blocks,
 // so its 49 accumulators and 7 x 8 coefficients per lane stay in registers (at 3 blocks they spill)
-template <int L, int NP>
+template <int L, int NP, int U>
 __global__ void __launch_bounds__(128, (L <= 4) ? 4 : (L == 5 ? 3 : 2)) k_descriptor_n(DescArgs a) {
-  descriptor_n_body<L, NP>(a);
+  descriptor_n_body<L, NP, U>(a);
 }
 
-template <int L, int NP>
+template <int L, int NP, int U = NP>
 static int launch_descriptor_n(const DescArgs& a, int wpb_tuned, cudaStream_t st) {
   const int per_warp = 4 * NShape<L, NP>::warp_floats(a.S, a.N);
   if (per_warp % 16 != 0) return set_error(SOAPB_ERR_ARG, "descriptor: warp slice of %d B not 16-byte aligned", per_warp);
@@ -871,7 +872,7 @@ static int launch_descriptor_n(const DescArgs& a, int wpb_tuned, cudaStream_t st
   if ((wpb_tuned == 1 || wpb_tuned == 2 || wpb_tuned == 4) && wpb_tuned <= wpb) wpb = wpb_tuned;
   if (wpb < 1) return set_error(SOAPB_ERR_UNSUPPORTED, "descriptor shared memory %d B per warp too large", per_warp);
   const int smem = wpb * per_warp;
-  auto kern = k_descriptor_n<L, NP>;
+  auto kern = k_descriptor_n<L, NP, U>;
   int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                       "descriptor smem attribute");
   if (rc) return rc;
@@ -926,8 +927,20 @@ template <int L>
 struct DescDispatch {
   static int run(const DescArgs& a, int gn, int wpb, bool lgroup_only, cudaStream_t st) {
     if constexpr (L <= kMaxLNLanes) {
-      if (!lgroup_only && radial_lanes(a.N, L) && isfinite(a.self_ratio))
-        return a.N <= 4 ? launch_descriptor_n<L, 4>(a, wpb, st) : launch_descriptor_n<L, 8>(a, wpb, st);
+      if (!lgroup_only && radial_lanes(a.N, L) && isfinite(a.self_ratio)) {
+        // At l_max 6 a pair's 49 FMAs and 7 Horner passes are long enough that the unrolled loop, and
+        // the one for batches with a species change, exceed what the instruction caches hold: rolled
+        // with 4 lanes (512 cells, 4 species: 2718 -> 2196 us; 20000 atoms of one species: 391 -> 399),
+        // and with 8 from 3 species on (2634 -> 2495 us; 2001 atoms of 2 species: 75 -> 79).  At
+        // l_max 4 unrolled: 14.05 ms for 1M atoms, 14.7 unrolled by 2.
+        if constexpr (L == 6) {
+          if (a.N <= 4) return launch_descriptor_n<L, 4, 1>(a, wpb, st);
+          if (a.S >= 3) return launch_descriptor_n<L, 8, 1>(a, wpb, st);
+          return launch_descriptor_n<L, 8>(a, wpb, st);
+        } else {
+          return a.N <= 4 ? launch_descriptor_n<L, 4>(a, wpb, st) : launch_descriptor_n<L, 8>(a, wpb, st);
+        }
+      }
     }
     if constexpr (L <= 4) {
       if (desc_two_streams(a.N, L)) {  // functions per lane fixed by (N, L): ceil(N / floor(16 / (L+1)))
