@@ -857,9 +857,12 @@ __device__ __forceinline__ void descriptor_n_body(const DescArgs& a) {
 }
 
 // l_max <= 4: 4 blocks of 4 warps per SM at 128 registers; l_max 5: 3 blocks; l_max 6: 2 blocks,
-// so its 49 accumulators and 7 x 8 coefficients per lane stay in registers (at 3 blocks they spill)
+// so its 49 accumulators and 7 x 8 coefficients per lane stay in registers (at 3 blocks they spill).
+// With few accumulators the unrolled loop's loads would take the registers of further blocks: 8 at
+// l_max 0 and 6 at l_max 2 (96 cells of 4 species, n_max 8: 107 -> 88 and 180 -> 155 us).
+constexpr int lane_blocks(int L) { return L == 0 ? 8 : L == 2 ? 6 : L <= 4 ? 4 : L == 5 ? 3 : 2; }
 template <int L, int NP, int U>
-__global__ void __launch_bounds__(128, (L <= 4) ? 4 : (L == 5 ? 3 : 2)) k_descriptor_n(DescArgs a) {
+__global__ void __launch_bounds__(128, lane_blocks(L)) k_descriptor_n(DescArgs a) {
   descriptor_n_body<L, NP, U>(a);
 }
 
@@ -932,14 +935,12 @@ struct DescDispatch {
         // the one for batches with a species change, exceed what the instruction caches hold: rolled
         // with 4 lanes (512 cells, 4 species: 2718 -> 2196 us; 20000 atoms of one species: 391 -> 399),
         // and with 8 from 3 species on (2634 -> 2495 us; 2001 atoms of 2 species: 75 -> 79).  At
-        // l_max 4 unrolled: 14.05 ms for 1M atoms, 14.7 unrolled by 2.
-        if constexpr (L == 6) {
-          if (a.N <= 4) return launch_descriptor_n<L, 4, 1>(a, wpb, st);
+        // l_max 4 with 8 lanes unrolled: 14.05 ms for 1M atoms, 14.7 unrolled by 2; with 4 lanes, whose
+        // streams are shorter, rolled from l_max 4 on (96 cells of 4 species: 227 -> 212 us, l_max 5 296 -> 269).
+        if (a.N <= 4) return launch_descriptor_n<L, 4, (L >= 4 ? 1 : 4)>(a, wpb, st);
+        if constexpr (L == 6)
           if (a.S >= 3) return launch_descriptor_n<L, 8, 1>(a, wpb, st);
-          return launch_descriptor_n<L, 8>(a, wpb, st);
-        } else {
-          return a.N <= 4 ? launch_descriptor_n<L, 4>(a, wpb, st) : launch_descriptor_n<L, 8>(a, wpb, st);
-        }
+        return launch_descriptor_n<L, 8>(a, wpb, st);
       }
     }
     if constexpr (L <= 4) {
