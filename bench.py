@@ -421,7 +421,7 @@ def batched_vs_plain(soap_cls, torch):
             "batched_atoms_per_s": res["batched"], "plain_atoms_per_s": res["plain"],
             "speedup": res["batched"] / res["plain"],
             "graph_atoms_per_s": res["graph"], "graph_speedup": res["graph"] / res["plain"],
-            "graph_note": "SOAP.batch plan: forward and adjoint replayed as two captured CUDA graphs",
+            "graph_note": "SOAP.batch plan: neighbour list, descriptor and adjoint replayed as captured CUDA graphs",
             "autotuned": {k: tuned[k] for k in ("desc_wpb", "desc_gn", "force_wpb")}}
 
 

@@ -543,12 +543,12 @@ __device__ __forceinline__ void desc_epilogue_n(const DescArgs& a, int64_t c, co
 // order over the neighbours, and the harmonics are staged with their norms: the
 // coefficients are those of scalar FMAs bit by bit, as float64 position gradients
 // need (norms applied to the sums instead: 13.95 against 14.05 ms for 1M atoms, and
-// a larger error).  The pair loop is unrolled over the batch and branches around
-// the coefficient reloads.  1M atoms (l_max 4): 14.65 -> 14.05 ms; 48 cells
-// (l_max 6): 268 -> 262 us; 3000 atoms (l_max 3): 73 -> 70 us.  The gain is less than the
+// a larger error).  The pair loop branches around the coefficient reloads and is
+// unrolled over the batch or not (DescDispatch).  1M atoms (l_max 4): 14.65 -> 14.05 ms;
+// 48 cells (l_max 6): 266 -> 255 us; 3000 atoms (l_max 3): 73 -> 67 us.  The gain is less than the
 // instructions saved because packed and scalar FMAs with three distinct
 // operands share the register ports (2.3 - 2.7 and 1.6 - 1.9 cycles each,
-// measured) and 4 warps per scheduler leave 47 % of the issue slots to the
+// measured) and 4 warps per scheduler leave 45 % of the issue slots to the
 // latency of the reloads and row reads.  Measured slower: the polynomials as
 // trees over t^2, t^4 (14.36 ms), two pairs per step (16.0 ms), 3 blocks per SM
 // (14.8 ms; l_max 6, where they spill: 288 against 268 us for the 48 cells), the

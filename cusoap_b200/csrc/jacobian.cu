@@ -38,7 +38,7 @@
 // A task is one staged batch, not one centre: staging a batch is a chain of
 // barriers and shared-memory latencies, so with centres as tasks a centre's
 // batches ran one after the other in one block while most blocks had no centre
-// (50 centres of a 3000-atom cluster, F = 420: 452 us a launch, 152 us as it is
+// (50 centres of a 3000-atom cluster, F = 420: 452 us a launch, 148 us as it is
 // now, 115 us of it to write the output; 1536 atoms, 12 GB: 2.35 and 1.76 ms).
 // Zero and nonzero rows are disjoint, so every element is written once and the
 // two roles never synchronise.

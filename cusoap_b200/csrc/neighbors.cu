@@ -649,7 +649,8 @@ __global__ void k_gather_atoms(soapb_structs s, NLWork w) {
 // kernels cost their launches (16 launches and 3 memsets, 2-5 us each, for
 // 24 to 3000 atoms).  One cluster of up to 8 CTAs runs them all, with a cluster
 // barrier between stages (one CTA: a block barrier); intermediate arrays stay
-// in the workspace, in L2.  24 atoms: 12 us, 3000: 19 us, 48 cells of 50 atoms: 49 us.
+// in the workspace, in L2.  24 atoms: 15 us, 3000: 21 us, 48 cells
+// of 200 atoms: 53 us.
 constexpr int kCellsThreads = 512;
 constexpr int kCellsMaxCtas = 8;
 
@@ -822,9 +823,9 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 // The enumeration is bound by instruction issue and the latency of the loads: 5
 // warp instructions per pair in the count, against 8 with FP64 row geometry
 // (six divisions and a square root a centre, one a row) and tests (1M atoms:
-// count 3.31 -> 2.2 ms; 48 periodic cells 85 -> 40 us).  Other than diagonal
+// count 3.31 -> 2.32 ms; 48 periodic cells 85 -> 43 us).  Other than diagonal
 // frames scanned the full window of half-cutoff bins before
-// (501 atoms, triclinic: count 38 -> 19 us, fill 45 -> 23 us).
+// (501 atoms, triclinic: count and scan 46 -> 21 us, fill 45 -> 22 us).
 // Writing the candidate slots of all runs into a list first, instead of finding
 // each lane's run, took as many instructions as it saved.
 template <bool PER, int UNROLL, class Fn>
@@ -1065,8 +1066,9 @@ __device__ __forceinline__ int64_t nth_centre(int i, int64_t n_centres) {
 }
 
 // Pairs of every centre, one warp per centre, 8 blocks of 4 warps per SM (64
-// registers): the count is latency-bound with little work per candidate, so
-// more resident warps pay.  The largest count goes to
+// registers, 130 B of spills): the count is latency-bound with little work per
+// candidate, so more resident warps pay (1M atoms with the set-up: 2.48 ms, 6
+// blocks 2.66).  The largest count goes to
 // status[2].  With pair_off, the last block to finish scans the counts into it
 // and, with stats, writes {total, largest, flags} -- the caller gets offsets and
 // summary from this launch (kLastBlockScan centres: the scan by 128 threads
@@ -1129,9 +1131,11 @@ __global__ void __launch_bounds__(128, 8) k_count(VisitArgs A, int64_t n_centres
 // The latency of the record loads and of the ranking bounds this kernel, so it
 // keeps little per pair: 20 bytes (the FP32 record, key and rank, a tile's
 // records loaded while the next is tested) leave fewer warps and less L1 and
-// measured slower (1M atoms: 7.0 ms).  1M atoms: 7.25 -> 5.9 ms; 3000 atoms at
-// 700 pairs a centre: 63 -> 42 us (768 staged pairs, no second enumeration); 48
-// cells: 126 -> 76 us.  7 blocks per SM: 6 take 6.1 ms, 8 spill.
+// measured slower (1M atoms: 7.0 ms).  1M atoms: 7.25 -> 6.01 ms; 3000 atoms at
+// 700 pairs a centre: 63 -> 43 us (768 staged pairs, no second enumeration); 48
+// cells: 124 -> 74 us.  7 blocks per SM, at 72 registers with 200 B of spills
+// around the enumerations: 6 take 6.5 ms; 8 the same, but 3000 atoms 51 us with
+// the launch instead of 48.
 __host__ __device__ inline int fill_warp_bytes(int nkeys, int stage) {
   return (int)sizeof(VisitMem) + 8 * stage + ((4 * nkeys + 15) & ~15);
 }
